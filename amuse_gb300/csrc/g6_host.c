@@ -1723,14 +1723,13 @@ static struct {
   int g_exact, g_niter, g_wpc, g_cps;
   double g_eta;
   long long g_maxsteps;
-  void *g_key;
   /* smallN's unperturbed binaries (g6x_batch_unperturbed) */
   int unp, unp_full;
   double unp_dt_crit, unp_r2_crit, unp_gamma;
   int *d_nbin;
-  int g_unp;
-} BT = {0, 0, NULL, NULL, NULL, NULL, NULL, NULL, NULL, NULL, NULL, NULL, NULL, 4, 2,
-        NULL, 0, 0, 0, 0, 0.0, 0, NULL, 0, 0, 0.0, 0.0, 0.0, NULL, 0};
+  int g_unp, g_full;
+  double g_dt_crit, g_r2_crit, g_gamma;
+} BT = {.wpc = 4, .cps = 2};
 
 static void batch_free(void) {
   cudaFree(BT.d_order); cudaFree(BT.d_off); cudaFree(BT.d_queue); cudaFree(BT.d_status);
@@ -1749,8 +1748,18 @@ static void batch_free(void) {
   BT.unp_gamma = g;
 }
 
+/* The captured graph holds the buffers' addresses: it goes whenever one of
+   them is reallocated (a new address may equal the old one, so comparing
+   addresses is not enough, and a batch can outgrow the per-system buffers
+   alone). */
+static void batch_drop_graph(void) {
+  if (BT.gexec) cudaGraphExecDestroy(BT.gexec);
+  BT.gexec = NULL;
+}
+
 static int batch_ensure(int nsys, int nbody) {
   if (nsys > BT.cap_sys) {
+    batch_drop_graph();
     cudaFree(BT.d_order); cudaFree(BT.d_off); cudaFree(BT.d_tend); cudaFree(BT.d_tout);
     cudaFree(BT.d_steps); cudaFree(BT.d_wall); cudaFree(BT.d_status); cudaFree(BT.d_nbin);
     BT.cap_sys = 0;
@@ -1769,6 +1778,7 @@ static int batch_ensure(int nsys, int nbody) {
     BT.cap_sys = nsys;
   }
   if (nbody > BT.cap_body) {
+    batch_drop_graph();
     cudaFree(BT.d_mass); cudaFree(BT.d_pos); cudaFree(BT.d_vel);
     BT.cap_body = 0;
     size_t b = (size_t)nbody;
@@ -1802,11 +1812,10 @@ static int batch_graph_launch(int nsys, double eta, int n_iter, long long max_st
   CK(cudaMemcpyAsync(BT.d_queue + 1, &nsys, sizeof(int), cudaMemcpyHostToDevice, G.st));
   if (!BT.gexec || BT.g_exact != exact || BT.g_niter != n_iter ||
       BT.g_eta != eta || BT.g_maxsteps != max_steps || BT.g_wpc != BT.wpc ||
-      BT.g_cps != BT.cps || BT.g_key != (void *)BT.d_pos || BT.g_unp != unp) {
-    if (BT.gexec) {
-      cudaGraphExecDestroy(BT.gexec);
-      BT.gexec = NULL;
-    }
+      BT.g_cps != BT.cps || BT.g_unp != unp ||
+      (unp && (BT.g_full != BT.unp_full || BT.g_dt_crit != BT.unp_dt_crit ||
+               BT.g_r2_crit != BT.unp_r2_crit || BT.g_gamma != BT.unp_gamma))) {
+    batch_drop_graph();
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(G.st, cudaStreamCaptureModeThreadLocal));
     int rc = unp ? g6k_batch_launch_unp(BT.d_order, BT.d_off, BT.d_tend, BT.d_mass,
@@ -1836,8 +1845,11 @@ static int batch_graph_launch(int nsys, double eta, int n_iter, long long max_st
     BT.g_maxsteps = max_steps;
     BT.g_wpc = BT.wpc;
     BT.g_cps = BT.cps;
-    BT.g_key = (void *)BT.d_pos;
     BT.g_unp = unp;
+    BT.g_full = BT.unp_full;
+    BT.g_dt_crit = BT.unp_dt_crit;
+    BT.g_r2_crit = BT.unp_r2_crit;
+    BT.g_gamma = BT.unp_gamma;
   }
   CK(cudaGraphLaunch(BT.gexec, G.st));
   return 0;

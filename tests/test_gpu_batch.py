@@ -199,3 +199,21 @@ def test_unperturbed_batching_workload_completes(g6):
           f"{r['steps'].max()}")
     assert np.all(r["status"] == 0) and np.all(r["t_final"] >= t_end)
     assert np.all(np.isfinite(de)) and np.median(de) < 1e-3
+
+
+@pytest.mark.parametrize("first,then", [((4, 60), (40, 3)), ((40, 3), (6, 60)), ((5, 3), (90, 40))])
+def test_batch_growing_in_systems_or_bodies(lib_built, first, then):
+    """A second batch that outgrows the per-system buffers alone (more but
+    smaller systems), the per-body buffers alone, or both: the launch must
+    see the reallocated buffers."""
+    g6 = ag.G6X(0)
+    g6.close()  # start from empty batch buffers
+    g6 = ag.G6X(0)
+    for nsys, n in (first, then):
+        ns, m, x, v, tcr = _systems(nsys, n, n, seed=nsys)
+        r = g6.batch_run(ns, 0.05 * tcr, m, x, v, eta=0.14, exact=True, max_steps=100000)
+        for s in range(0, nsys, 7):
+            a, b = s * n, (s + 1) * n
+            px, pv, tf, st = oracle.smalln(m[a:b], x[a:b], v[a:b], 0.14, 0.05 * tcr)
+            assert r["status"][s] == 0 and r["steps"][s] == st and r["t_final"][s] == tf
+            assert np.array_equal(r["pos"][a:b], px) and np.array_equal(r["vel"][a:b], pv)
