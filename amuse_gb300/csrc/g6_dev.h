@@ -113,6 +113,12 @@ int g6k_sm_count(void);
 int g6k_scatter(const g6_jstate *js, const g6_jupd *d_upd, int n, cudaStream_t st);
 int g6k_predict(const g6_jstate *js, int nj, double ti, int prec, cudaStream_t st);
 int g6k_force(const g6_force_args *a, g6_shape *shape, cudaStream_t st);
+/* The FP64 force (kern_force64.cu), which g6k_force calls for G6_PREC_FP64:
+ * ticket is an array of groups_max counters, zero between launches.       */
+int g6k_force64(const g6_force_args *a, unsigned *ticket, int groups_max, g6_shape *shape,
+                cudaStream_t st);
+size_t g6k_force64_scratch(int ni, int nj, int nn, int force_jl, int force_nsplit,
+                           int groups_max);
 
 /* FP64 Hermite corrector + Aarseth step on the listed slots (in place):
  * idata.cc:399-514.  acc/jerk are the new values at tnext, [ni][3]. */
@@ -184,6 +190,19 @@ int g6k_store_forces(const g6_jstate *js, int ni, const int *ilist,
 #endif
 
 #ifdef __CUDACC__
+/* a / B correctly rounded, for a small whole constant B and rb = 1/B rounded:
+   q = a rb is within an ulp, the FMA residual a - B q is exact, and q plus
+   the residual times rb rounds to the quotient (Markstein 1990, IBM J. Res.
+   Dev. 34, theorem 3: rb is the rounded reciprocal).  3 FP64 instructions
+   where the general division takes about 10 at 16 cycles each.  Outside the
+   range where nothing over- or underflows (zeros among them): __ddiv_rn.
+   Checked against a / B on 3e8 mantissas (random, low and high ends).  */
+__device__ __forceinline__ double g6_div_const(double a, double B, double rb) {
+  const unsigned e = (unsigned)__double2hiint(a) & 0x7fffffffu;
+  if (e - 0x04000000u > 0x78000000u) return __ddiv_rn(a, B); /* |a| below 2^-959 or above 2^961 */
+  const double q = __dmul_rn(a, rb);
+  return __fma_rn(__fma_rn(-B, q, a), rb, q);
+}
 /* ph4's prediction of one position component, x + dt*(v + 0.5*dt*(a +
    dt*j/3)) with its rounding order and no contraction (predict_all,
    src/amuse_ph4/src/jdata.cc:736-744; the host i-prediction idata.cc:346-365
@@ -193,7 +212,7 @@ __device__ __forceinline__ double g6_predict_x(double x, double v, double a, dou
   if (dt == 0) return x;
   const double hdt = __dmul_rn(0.5, dt);
   return __dadd_rn(
-      x, __dmul_rn(dt, __dadd_rn(v, __dmul_rn(hdt, __dadd_rn(a, __ddiv_rn(__dmul_rn(dt, j), 3.0))))));
+      x, __dmul_rn(dt, __dadd_rn(v, __dmul_rn(hdt, __dadd_rn(a, g6_div_const(__dmul_rn(dt, j), 3.0, 1.0 / 3.0))))));
 }
 /* ph4's predicted velocity component, v + dt*(a + 0.5*dt*j) (jdata.cc:741-743). */
 __device__ __forceinline__ double g6_predict_v(double v, double a, double j, double dt) {

@@ -1,5 +1,6 @@
 // kern_force.cu -- the i-block Hermite force kernel (acc, jerk, pot, nearest
-// neighbour) for sm_103a, in two arithmetic policies:
+// neighbour) for sm_103a in split precision (the plain FP64 kernel is
+// kern_force64.cu):
 //
 //   split: positions as double-single (hi+lo float pairs), relative
 //          position formed by (xj_hi - xi_hi) + (xj_lo - xi_lo), all pair
@@ -9,8 +10,6 @@
 //          consecutive j), so each packed f32x2 instruction (add/sub/mul/fma
 //          .rn.f32x2) evaluates one i against two j: half the issue slots of
 //          scalar code for the same FP32 work.
-//   fp64:  the same pair formula in plain FP64 (the "plain FP64 GPU"
-//          kernel; also the GPU-side oracle at N=2^20).
 //
 // The pair formula is ph4's (src/amuse_ph4/src/idata.cc:188-226):
 //   dx = xj - xi, dv = vj - vi, r2 = |dx|^2 + eps2 (+2^-52 as ph4),
@@ -22,8 +21,8 @@
 // here the host resolves id -> j slot once per call and the kernel skips
 // that slot.
 //
-// Structure (one CTA = 128 threads = 4 warps; 2 i-particles per thread in
-// split precision, 3 CTAs per SM; 4 in FP64):
+// Structure (one CTA = 128 threads = 4 warps; 2 i-particles per thread, 3
+// CTAs per SM):
 //   * j-tiles of 256 records are streamed HBM/L2 -> shared memory with
 //     cp.async.bulk (TMA, non-tensor) completing on an mbarrier; warps
 //     consume the ring independently (no CTA barrier in the loop).
@@ -32,7 +31,7 @@
 //     active blocks still fill all 152 SMs.
 //   * Lanes of one i merge with warp shuffles (plus shared memory across
 //     warps for JL > 32); CTAs of one i merge in a second pass kernel, in
-//     fixed order, with float-float (split) or FP64 adds: deterministic.
+//     fixed order, with float-float adds: deterministic.
 //   * Nearest neighbour (optional, a template flag): the hot loop keeps only
 //     a running min of r2 (one FMNMX per pair) and the tile where it last
 //     improved; after the loop that tile is re-read from L2 and re-scanned
@@ -46,16 +45,6 @@
 
 #include "f32x2.cuh"
 #include "g6_dev.h"
-
-// 32-byte aligned FP64 quadruple (CUDA 13 deprecates the unaligned double4).
-struct __align__(32) G6D4 {
-  double x, y, z, w;
-};
-__host__ __device__ __forceinline__ G6D4 g6d4(double x, double y, double z, double w) {
-  G6D4 r;
-  r.x = x; r.y = y; r.z = z; r.w = w;
-  return r;
-}
 
 namespace {
 
@@ -78,9 +67,6 @@ namespace {
 #ifndef G6_MINB
 #define G6_MINB 3
 #endif
-#ifndef G6_IPT_F64
-#define G6_IPT_F64 4
-#endif
 #ifndef G6_XMERGE_MAX
 #define G6_XMERGE_MAX 2  // split merge in the force kernel up to this many i per group
 #endif
@@ -92,10 +78,7 @@ namespace {
 #endif
 constexpr int NT = G6_NT;    // threads per CTA
 constexpr int TJ = G6_TILE;  // j records per tile
-// i-particles per thread: the split kernel's packed f32x2 pair terms need
-// twice the registers per i, so it holds fewer i than the FP64 kernel.
-constexpr int IPT_SPLIT = G6_IPT;
-constexpr int IPT_F64 = G6_IPT_F64;
+constexpr int IPT_SPLIT = G6_IPT;  // i-particles per thread
 constexpr int UNROLL = G6_UNROLL;  // j-loop unroll factor (the best measured:
                                     // 8 plain, 4 with the nearest neighbour)
 constexpr int JLMAX = TJ < NT ? TJ : NT;  // j-lanes per i at most
@@ -110,11 +93,7 @@ enum { ERR_TMA_TIMEOUT = 1, ERR_SHAPE = 2 };
 struct __align__(16) RecS {
   float2 xh, yh, zh, m, xl, yl, zl, ml, vx, vy, vz, pad1;  // ml: the mass's low part
 };
-struct __align__(32) RecD {
-  G6D4 p, v;
-};
 static_assert(sizeof(RecS) == 96, "split record pair");
-static_assert(sizeof(RecD) == 64, "fp64 record");
 
 // ---------------------------------------------------------------- PTX ---
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -475,165 +454,6 @@ struct SplitP {
   __device__ static void finish(const Out &o, int i, const KParams &kp);
 };
 
-struct F64P {
-  using Rec = RecD;
-  using R = double;
-  static constexpr int JPR = 1;     // j per record
-  static constexpr int IPT = IPT_F64;
-  static constexpr int NSTAGE = 2;  // TMA ring depth (2 x 16 KB)
-  static constexpr int MINB = 1;
-  struct I {
-    double x, y, z, vx, vy, vz;
-  };
-  struct Part {
-    double a[3], j[3], p;
-  };
-  struct Tot {
-    double a[3], j[3], p;
-  };
-  struct Out {  // 72 B
-    double a[3], j[3], p;
-    double nnr2;
-    int nn, pad;
-  };
-  __device__ static I load_i_explicit(const double *p, const double *v) {
-    I s;
-    s.x = p[0]; s.y = p[1]; s.z = p[2];
-    s.vx = v[0]; s.vy = v[1]; s.vz = v[2];
-    return s;
-  }
-  __device__ static I load_i_slot(const void *recs, int slot) {
-    const Rec &r = reinterpret_cast<const Rec *>(recs)[slot];
-    I s;
-    s.x = r.p.x; s.y = r.p.y; s.z = r.p.z;
-    s.vx = r.v.x; s.vy = r.v.y; s.vz = r.v.z;
-    return s;
-  }
-  __device__ static double eps(double eps2) { return eps2 + 1.0 / 4503599627370496.0; }
-  __device__ static void zero(Part &q) {
-#pragma unroll
-    for (int k = 0; k < 3; k++) q.a[k] = q.j[k] = 0.0;
-    q.p = 0.0;
-  }
-  __device__ static void zero(Tot &t) {
-#pragma unroll
-    for (int k = 0; k < 3; k++) t.a[k] = t.j[k] = 0.0;
-    t.p = 0.0;
-  }
-  __device__ static void fold(Tot &t, const Part &q) {
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      t.a[k] += q.a[k];
-      t.j[k] += q.j[k];
-    }
-    t.p += q.p;
-  }
-  __device__ static __forceinline__ double r2e(const I &s, const Rec &r, double eps2,
-                                               double &dx, double &dy, double &dz) {
-    dx = r.p.x - s.x;
-    dy = r.p.y - s.y;
-    dz = r.p.z - s.z;
-    double r2 = __fma_rn(dx, dx, eps2);
-    r2 = __fma_rn(dy, dy, r2);
-    return __fma_rn(dz, dz, r2);
-  }
-  // 1/sqrt(x) in FP64: FP32 MUFU seed, then two Newton-Raphson steps
-  // y <- y (3 - x y^2) / 2 (quadratic convergence: 2^-22 -> 2^-44 -> 2^-88).
-  __device__ static __forceinline__ double rsqrt64(double x) {
-    double y = (double)rsqrtf((float)x);
-    const double hx = 0.5 * x;
-    y = y * __fma_rn(-hx * y, y, 1.5);
-    y = y * __fma_rn(-hx * y, y, 1.5);
-    return y;
-  }
-  // ph4's nearest-neighbour key: the unsoftened r^2 summed in component
-  // order without contraction (idata.cc:200-205,214-218), so the argmin
-  // (first slot on equal keys) is ph4's nn bit for bit.
-  __device__ static __forceinline__ double nnkey(double dx, double dy, double dz) {
-    return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-  }
-  template <bool CHECK, bool NN, bool HJ = false>
-  __device__ static __forceinline__ void pair(const I &s, const Rec &r, double eps2, Part &q,
-                                              double &nnmin, int selfrel) {
-    const bool is_self = CHECK && selfrel == 0;
-    double dx, dy, dz;
-    const double r2 = r2e(s, r, eps2, dx, dy, dz);
-    double rinv = rsqrt64(r2);
-    if (CHECK) rinv = is_self ? 0.0 : rinv;
-    if (NN) {
-      const double key = nnkey(dx, dy, dz);
-      nnmin = fmin(nnmin, is_self ? __longlong_as_double(0x7ff0000000000000ll) : key);
-    }
-    const double dvx = r.v.x - s.vx, dvy = r.v.y - s.vy, dvz = r.v.z - s.vz;
-    const double rv = dx * dvx + dy * dvy + dz * dvz;
-    const double rinv2 = rinv * rinv;
-    const double mri = r.p.w * rinv;
-    const double mr3i = mri * rinv2;
-    double a3;
-    if (HJ) {
-      const double r2u = dx * dx + dy * dy + dz * dz;
-      a3 = (CHECK && is_self) ? 0.0 : -3.0 * (rv / r2u);
-    } else {
-      a3 = -3.0 * (rv * rinv2);
-    }
-    q.a[0] = fma(mr3i, dx, q.a[0]);
-    q.a[1] = fma(mr3i, dy, q.a[1]);
-    q.a[2] = fma(mr3i, dz, q.a[2]);
-    q.j[0] = fma(mr3i, fma(a3, dx, dvx), q.j[0]);
-    q.j[1] = fma(mr3i, fma(a3, dy, dvy), q.j[1]);
-    q.j[2] = fma(mr3i, fma(a3, dz, dvz), q.j[2]);
-    q.p += mri;
-  }
-  __device__ static __forceinline__ void rescan(const I &s, const Rec &r, double eps2,
-                                                double best, int slot0, int self, int &idx,
-                                                double &m2) {
-    (void)m2;  // the FP64 key is ph4's own: no gap to prove
-    double dx, dy, dz;
-    (void)r2e(s, r, eps2, dx, dy, dz);
-    if (idx < 0 && slot0 != self && nnkey(dx, dy, dz) == best) idx = slot0;
-  }
-  static constexpr bool JFOLD = false;
-  template <bool NN>
-  __host__ __device__ static constexpr bool tot_shared() {
-    return false;
-  }
-  __device__ static void fold_jerk(Tot &, Part &) {}
-  __device__ static void to_out(const Tot &t, double nnr2, double nnr2b, int nn, Out &o) {
-    (void)nnr2b;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      o.a[k] = t.a[k];
-      o.j[k] = t.j[k];
-    }
-    o.p = t.p;
-    o.nnr2 = nnr2;
-    o.nn = nn;
-    o.pad = 0;
-  }
-  __device__ static void merge(Out &a, const Out &b) {
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      a.a[k] += b.a[k];
-      a.j[k] += b.j[k];
-    }
-    a.p += b.p;
-    if (b.nnr2 < a.nnr2 || (b.nnr2 == a.nnr2 && b.nn < a.nn)) {
-      a.nnr2 = b.nnr2;
-      a.nn = b.nn;
-    }
-  }
-  __device__ static void write_final(const Out &o, int i, double *acc, double *jerk,
-                                     double *pot) {
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      acc[3 * i + k] = o.a[k];
-      jerk[3 * i + k] = o.j[k];
-    }
-    pot[i] = -o.p;
-  }
-  __device__ static void finish(const Out &o, int i, const KParams &kp);
-};
-
 // A partial record written by another CTA of this launch: read around L1.
 template <class O>
 __device__ __forceinline__ O load_out_cg(const O *p) {
@@ -871,13 +691,6 @@ __device__ __noinline__ void SplitP::finish(const Out &o, int i, const KParams &
     kp.nn[i] = -1;
   }
   if (mode) ref_enqueue(kp.refine, i, mode, thr, thr_mt);
-}
-
-__device__ __noinline__ void F64P::finish(const Out &o, int i, const KParams &kp) {
-  write_final(o, i, kp.acc, kp.jerk, kp.pot);
-  const int nn = (o.nn >= 0 && o.nn < kp.nj) ? o.nn : -1;
-  if (kp.nn) kp.nn[i] = kp.want_nn ? nn : -1;
-  if (kp.nn_r2) kp.nn_r2[i] = nn >= 0 ? (float)o.nnr2 : __int_as_float(0x7f800000);
 }
 
 // Number of j per thread between compensated folds.
@@ -1570,19 +1383,19 @@ int sm_count() {
 // JL = 1) stay at JL = 1.  The last few shapes are cached (block steps
 // repeat the same ni).
 struct ShapeKey {
-  int ni, nj, prec, nn, fjl, fns;
+  int ni, nj, nn, fjl, fns;
   int jl, nsplit, jsplit;
 };
 ShapeKey g_shape_cache[256];
 
-void choose_shape(int ni, int nj, int prec, int nn, int force_jl, int force_nsplit, int *jl_out,
+void choose_shape(int ni, int nj, int nn, int force_jl, int force_nsplit, int *jl_out,
                   int *nsplit_out, int *jsplit_out) {
   nn = nn ? 1 : 0;
   const unsigned h =
-      ((unsigned)ni * 2654435761u ^ (unsigned)nj * 40503u ^ (unsigned)prec ^ (unsigned)nn * 97u) &
+      ((unsigned)ni * 2654435761u ^ (unsigned)nj * 40503u ^ (unsigned)nn * 97u) &
       255u;
   ShapeKey &c = g_shape_cache[h];
-  if (c.ni == ni && c.nj == nj && c.prec == prec && c.nn == nn && c.fjl == force_jl &&
+  if (c.ni == ni && c.nj == nj && c.nn == nn && c.fjl == force_jl &&
       c.fns == force_nsplit && c.jl > 0) {
     *jl_out = c.jl;
     *nsplit_out = c.nsplit;
@@ -1590,12 +1403,10 @@ void choose_shape(int ni, int nj, int prec, int nn, int force_jl, int force_nspl
     return;
   }
   const int ntiles = nj > 0 ? (nj + TJ - 1) / TJ : 1;
-  const int minb = prec == G6_PREC_FP64 ? F64P::MINB : SplitP::MINB;
-  const int slots = minb * sm_count();
+  const int slots = SplitP::MINB * sm_count();
   const double A = 150.0, F = 3000.0;
-  // per j and i: ~20 issue slots split (packed j pairs), ~37 x 32 FP64
-  const int IPT = prec == G6_PREC_FP64 ? IPT_F64 : IPT_SPLIT;
-  const double B = (prec == G6_PREC_FP64 ? 32.0 * 37.0 : 20.0) * IPT;
+  const int IPT = IPT_SPLIT;
+  const double B = 20.0 * IPT;  // per j and i: ~20 issue slots (packed j pairs)
   int jl0 = 1;
   while (jl0 < JLMAX && (NT / (jl0 * 2)) * IPT >= ni && ni > 0) jl0 *= 2;
   int jl_lo = jl0, jl_hi = JLMAX;
@@ -1672,7 +1483,6 @@ void choose_shape(int ni, int nj, int prec, int nn, int force_jl, int force_nspl
   *jsplit_out = tp * TJ;
   c.ni = ni;
   c.nj = nj;
-  c.prec = prec;
   c.nn = nn;
   c.fjl = force_jl;
   c.fns = force_nsplit;
@@ -1756,11 +1566,11 @@ extern "C" int g6k_refine_read(const void *refine, int out[4], cudaStream_t st) 
 
 extern "C" size_t g6k_scratch_bytes(int ni, int nj, int prec, int nn, int force_jl,
                                     int force_nsplit) {
+  if (prec == G6_PREC_FP64) return g6k_force64_scratch(ni, nj, nn, force_jl, force_nsplit, XTMAX);
   int jl, nsplit, jsplit;
-  choose_shape(ni, nj, prec, nn, force_jl, force_nsplit, &jl, &nsplit, &jsplit);
+  choose_shape(ni, nj, nn, force_jl, force_nsplit, &jl, &nsplit, &jsplit);
   if (nsplit <= 1) return 0;
-  const size_t rec = prec == G6_PREC_FP64 ? sizeof(F64P::Out) : sizeof(SplitP::Out);
-  return (size_t)nsplit * (size_t)ni * rec;
+  return (size_t)nsplit * (size_t)ni * sizeof(SplitP::Out);
 }
 
 extern "C" int g6k_force(const g6_force_args *a, g6_shape *shape, cudaStream_t st) {
@@ -1768,9 +1578,13 @@ extern "C" int g6k_force(const g6_force_args *a, g6_shape *shape, cudaStream_t s
   if (a->nj <= 0 || !a->acc || !a->jerk || !a->pot || !a->js || !a->err) return -1;
   if (!a->ilist && (!a->ipos || !a->ivel)) return -1;
   if (a->hjerk && (a->want_nn || (a->force_jl != 0 && a->force_jl != 1))) return -2;
+  if (a->force_jl < 0 || a->force_jl > JLMAX || (a->force_jl & (a->force_jl - 1))) return -2;
+  if (a->prec == G6_PREC_FP64)
+    return g6k_force64(a, a->refine ? reinterpret_cast<RefBuf *>(a->refine)->xtick : nullptr,
+                       a->refine ? XTMAX : 0, shape, st);
   int jl, nsplit, jsplit;
-  choose_shape(a->ni, a->nj, a->prec, a->want_nn, a->hjerk ? 1 : a->force_jl, a->force_nsplit,
-               &jl, &nsplit, &jsplit);
+  choose_shape(a->ni, a->nj, a->want_nn, a->hjerk ? 1 : a->force_jl, a->force_nsplit, &jl,
+               &nsplit, &jsplit);
   if (jl < 1 || jl > JLMAX || (jl & (jl - 1))) return -2;
   KParams kp;
   kp.ni = a->ni;
@@ -1797,15 +1611,14 @@ extern "C" int g6k_force(const g6_force_args *a, g6_shape *shape, cudaStream_t s
   // The refinement pass serves the split kernel's g6 results; the hermite
   // jerk form and callers passing kappa < 0 (the fixed-step path) keep plain
   // split arithmetic.
-  kp.refine =
-      (a->prec == G6_PREC_SPLIT && !a->hjerk && a->kappa >= 0.0) ? a->refine : nullptr;
+  kp.refine = !a->hjerk && a->kappa >= 0.0 ? a->refine : nullptr;
   kp.kappa2 = a->kappa > 0.0 ? a->kappa * a->kappa : 0.0;
   kp.stall = a->stall_test;
   kp.wait_ns = a->stall_test ? STALL_TEST_NS : WAIT_NS;
   const size_t need =
       nsplit > 1 ? g6k_scratch_bytes(a->ni, a->nj, a->prec, a->want_nn, jl, nsplit) : 0;
   if (need > a->scratch_bytes) return -4;
-  const int islots = (NT / jl) * (a->prec == G6_PREC_FP64 ? IPT_F64 : IPT_SPLIT);
+  const int islots = (NT / jl) * IPT_SPLIT;
   const int gx = (a->ni + islots - 1) / islots;
   if (shape) {
     shape->jl = jl;
@@ -1824,10 +1637,6 @@ extern "C" int g6k_force(const g6_force_args *a, g6_shape *shape, cudaStream_t s
   kp.xtick = (a->refine && nsplit > 1 && gx <= XTMAX && islots <= G6_XMERGE_MAX)
                  ? reinterpret_cast<RefBuf *>(a->refine)->xtick
                  : nullptr;
-  if (a->prec == G6_PREC_FP64) {
-    kp.jrec = a->js->jp_f64;
-    return launch<F64P>(kp, jl, gx, st, a->ev_mid);
-  }
   kp.jrec = a->js->jp_split;
   return launch<SplitP>(kp, jl, gx, st, a->ev_mid);
 }

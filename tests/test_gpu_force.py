@@ -491,3 +491,39 @@ def test_results_do_not_depend_on_the_launch_shape(g6):
         g6.set_shape(0, 0)
     for o in outs[1:]:
         assert np.array_equal(o["nn"], outs[0]["nn"])
+
+
+@pytest.mark.parametrize("n,ni", [(1, 1), (2, 2), (31, 3), (33, 33), (255, 17), (257, 257),
+                                  (1000, 31), (1025, 65), (5000, 1), (5000, 129), (20001, 40)])
+def test_fp64_force_edges(g6, n, ni):
+    """The FP64 kernel at the edges of its i-lane widths and j chunks, with
+    and without the neighbour, listed slots and explicit points, against the
+    oracle: each result within 1e-14 of the sum of its terms' magnitudes
+    (about 100 roundings of 2^-53), the neighbour equal."""
+    rng = np.random.RandomState(n + ni)
+    m = rng.uniform(0.5, 1.5, n) / n
+    x, v = rng.normal(size=(n, 3)), rng.normal(size=(n, 3))
+    ids = np.arange(n, dtype=np.int32)
+    g6.set_precision(ag.FP64)
+    try:
+        g6.load_particles(m, x, v)
+        sel = np.sort(rng.permutation(n)[:ni]).astype(np.int32)
+        ref = oracle.force(m, x, v, 1e-4, x[sel], v[sel])
+        d = np.linalg.norm(x[None] - x[sel][:, None], axis=2) ** 2 + 1e-4
+        w = np.linalg.norm(v[None] - v[sel][:, None], axis=2)
+        d[np.arange(ni), sel] = np.inf
+        sa, sp = (m / d).sum(1), (m / np.sqrt(d)).sum(1)
+        sj = (4 * m * w / d ** 1.5).sum(1)
+        for shape in ((0, 0), (1, 1), (4, 3), (32, 5)):
+            g6.set_shape(*shape)
+            o = g6.force(0.0, 1e-4, n, x[sel], v[sel], self_slot=sel)
+            assert np.all(np.abs(o["acc"] - ref["acc"]).max(1) <= 1e-14 * sa + 1e-300)
+            assert np.all(np.abs(o["jerk"] - ref["jerk"]).max(1) <= 1e-14 * sj + 1e-300)
+            assert np.all(np.abs(o["pot"] - ref["pot"]) <= 1e-14 * sp + 1e-300)
+            if n > 1:
+                assert np.array_equal(o["nn"], ref["nn"])
+            else:
+                assert np.all(o["nn"] == -1)
+    finally:
+        g6.set_shape(0, 0)
+        g6.set_precision(ag.SPLIT)
