@@ -147,6 +147,11 @@ __global__ void __launch_bounds__(PT) list_predict_kernel(g6_jstate js, int nj, 
   predict_one<PREC>(js, s, nj, tn);
 }
 
+// Threads per CTA: ~36 FP64 instructions per slot at 16 cycles each per warp
+// and SM, so while there are fewer than eight warps for every SM they go out
+// one per CTA (1024 slots in CTAs of 256 kept 8 warps on each of 4 SMs).
+int predict_threads(int nj_pad) { return nj_pad <= 8 * 32 * g6k_sm_count() ? 32 : PT; }
+
 }  // namespace
 
 extern "C" int g6k_scatter(const g6_jstate *js, const g6_jupd *d_upd, int n, cudaStream_t st) {
@@ -159,11 +164,12 @@ extern "C" int g6k_predict(const g6_jstate *js, int nj, double ti, int prec, cud
   if (nj <= 0) return 0;
   const int nj_pad = (nj + G6_TILE - 1) / G6_TILE * G6_TILE;
   if (nj_pad > js->cap) return -1;
-  const int grid = (nj_pad + PT - 1) / PT;
+  const int threads = predict_threads(nj_pad);
+  const int grid = (nj_pad + threads - 1) / threads;
   if (prec == G6_PREC_FP64)
-    predict_kernel<G6_PREC_FP64><<<grid, PT, 0, st>>>(*js, nj, nj_pad, ti);
+    predict_kernel<G6_PREC_FP64><<<grid, threads, 0, st>>>(*js, nj, nj_pad, ti);
   else
-    predict_kernel<G6_PREC_SPLIT><<<grid, PT, 0, st>>>(*js, nj, nj_pad, ti);
+    predict_kernel<G6_PREC_SPLIT><<<grid, threads, 0, st>>>(*js, nj, nj_pad, ti);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -173,12 +179,13 @@ extern "C" int g6k_list_predict(const g6_jstate *js, int nj, int prec,
   if (nj <= 0) return 0;
   const int nj_pad = (nj + G6_TILE - 1) / G6_TILE * G6_TILE;
   if (nj_pad > js->cap) return -1;
-  const int grid = (nj_pad + PT - 1) / PT;
+  const int threads = predict_threads(nj_pad);
+  const int grid = (nj_pad + threads - 1) / threads;
   const cudaError_t e =
       prec == G6_PREC_FP64
-          ? launch_pdl(list_predict_kernel<G6_PREC_FP64>, dim3(grid), dim3(PT), 0, st, *js, nj,
+          ? launch_pdl(list_predict_kernel<G6_PREC_FP64>, dim3(grid), dim3(threads), 0, st, *js, nj,
                        nj_pad, dmin, dmin_next, d_ilist, d_ni, d_tnext)
-          : launch_pdl(list_predict_kernel<G6_PREC_SPLIT>, dim3(grid), dim3(PT), 0, st, *js, nj,
+          : launch_pdl(list_predict_kernel<G6_PREC_SPLIT>, dim3(grid), dim3(threads), 0, st, *js, nj,
                        nj_pad, dmin, dmin_next, d_ilist, d_ni, d_tnext);
   return e == cudaSuccess ? 0 : -3;
 }

@@ -30,6 +30,7 @@ __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a,
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a, b); }
+__device__ __forceinline__ double div3(double a) { return g6_div_const(a, 3.0, 1.0 / 3.0); }
 
 // fmod(t, p) == 0 for p a positive normal power of two, without the
 // iterative double-precision fmod: t = m * 2^e (m an integer) is a multiple
@@ -90,15 +91,18 @@ __global__ void correct_kernel(g6_jstate js, int ni, const int *__restrict__ ili
     } else {
       // x + dt*(v + 0.5*dt*(a + dt*j/3)),  v + dt*(a + 0.5*dt*j)
       const double hdt = dmul(0.5, dt);
-      xp = dadd(x, dmul(dt, dadd(v, dmul(hdt, dadd(oa, ddiv(dmul(dt, oj), 3.0))))));
+      xp = dadd(x, dmul(dt, dadd(v, dmul(hdt, dadd(oa, div3(dmul(dt, oj)))))));
       vp = dadd(v, dmul(dt, dadd(oa, dmul(hdt, oj))));
     }
     const double ia = acc[3 * ii + kc], ij = jerk[3 * ii + kc];
     const double da = dsub(oa, ia);
     const double alpha = dsub(dmul(-3.0, da), dmul(dt, dadd(dmul(2.0, oj), ij)));
     const double beta = dadd(dmul(2.0, da), dmul(dt, dadd(oj, ij)));
-    xp = dadd(xp, dmul(dadd(ddiv(alpha, 12.0), ddiv(beta, 20.0)), dt2));
-    vp = dadd(vp, dmul(dadd(ddiv(alpha, 3.0), ddiv(beta, 4.0)), dt));
+    // (a quarter of a double is exact or rounds as the division does)
+    xp = dadd(xp, dmul(dadd(g6_div_const(alpha, 12.0, 1.0 / 12.0),
+                            g6_div_const(beta, 20.0, 1.0 / 20.0)),
+                       dt2));
+    vp = dadd(vp, dmul(dadd(div3(alpha), dmul(beta, 0.25)), dt));
     pa2 = dmul(ia, ia);
     const double dj = dmul(dt, ij);
     pj2 = dmul(dj, dj);
@@ -132,9 +136,9 @@ __global__ void correct_kernel(g6_jstate js, int ni, const int *__restrict__ ili
   int expo;
   double oldstep2 = ddiv(olds, dmul(2.0, frexp(olds, &expo)));
   for (int guard = 0; guard < 1100 && !multiple_of_pow2(tnext, oldstep2); guard++)
-    oldstep2 = ddiv(oldstep2, 2.0);
+    oldstep2 = dmul(oldstep2, 0.5);  // as the division by 2, to the last bit
   if (newstep < oldstep2) {
-    newstep = ddiv(oldstep2, 2.0);
+    newstep = dmul(oldstep2, 0.5);
   } else {
     const double t2 = dmul(2.0, oldstep2);
     if (newstep >= t2 && multiple_of_pow2(tnext, t2))
@@ -450,8 +454,9 @@ extern "C" int g6k_correct(const g6_jstate *js, int ni, const int *ilist, double
                            double eta, const double *acc, const double *jerk, const double *pot,
                            const int *nn, cudaStream_t st) {
   if (ni <= 0) return 0;
-  // 4 lanes per particle, 32 particles per 128-thread block
-  return launch_pdl(correct_kernel, dim3((ni + 31) / 32), dim3(128), 0, st, *js, ni, ilist, tnext,
+  // 4 lanes per particle, one warp (8 particles) per CTA: an SM issues FP64
+  // at 2 lanes a cycle, so a block's few warps go to as many SMs
+  return launch_pdl(correct_kernel, dim3((ni + 7) / 8), dim3(32), 0, st, *js, ni, ilist, tnext,
                     eta, acc, jerk, pot, nn) == cudaSuccess
              ? 0
              : -3;
