@@ -228,7 +228,7 @@ struct SplitP {
   struct Tot {  // compensated totals (s: plain sum, an estimate), largest chunk of s
     float ah[3], al[3], jh[3], jl[3], ph, pl, s, mt, pad;  // 17 words: odd stride
   };
-  struct Out {  // partial record exchanged between CTAs, 80 B
+  struct __align__(16) Out {  // partial record exchanged between CTAs, 80 B
     float2 a[3], j[3], p;
     float nnr2;   // smallest nearest-neighbour key (r^2 + eps^2, FP32)
     float nnr2b;  // second smallest key over the other j
@@ -423,6 +423,15 @@ struct SplitP {
     o.s1 = t.s;
     o.mt = t.mt;
     o.nn = nn;
+    o.pad = 0;
+  }
+  __device__ static void to_out_zero(Out &o) {  // merge's neutral element
+#pragma unroll
+    for (int k = 0; k < 3; k++) o.a[k] = o.j[k] = make_float2(0.f, 0.f);
+    o.p = make_float2(0.f, 0.f);
+    o.nnr2 = o.nnr2b = __int_as_float(0x7f800000);
+    o.s1 = o.mt = 0.f;
+    o.nn = 0x7fffffff;
     o.pad = 0;
   }
   __device__ static void merge(Out &a, const Out &b) {
@@ -624,17 +633,23 @@ __device__ __forceinline__ double ph4_r2(const double xi[3], const double xj[3])
   const double d0 = dsub(xj[0], xi[0]), d1 = dsub(xj[1], xi[1]), d2 = dsub(xj[2], xi[2]);
   return __dadd_rn(__dadd_rn(__dmul_rn(d0, d0), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
 }
-// Tk(D) of the header, rounded up to FP32.
-__device__ __forceinline__ float nn_bound(double D, double e, const double xi[3]) {
-  const double sD = sqrt(D);
-  const double X = fmax(fabs(xi[0]), fmax(fabs(xi[1]), fabs(xi[2]))) + sD * (1.0 + 1.0 / 1048576.0);
-  const double E = X * (1.0 + 1.0 / 1048576.0) * (1.0 / 1073741824.0);
-  const double T = (1.0 + 1.0 / 65536.0) * (D + e) + 4.0 * E * sD + 4.0 * E * E;
-  return __double2float_ru(T);
+// An FP32 upper bound of Tk(D): every factor is rounded up or padded by more
+// than the roundings of the FP32 evaluation (a larger bound only queues a
+// few more particles, whose neighbour the redo finds either way).
+__device__ __forceinline__ float nn_bound(double D, float e, const double xi[3]) {
+  const float d = __double2float_ru(D);
+  const float sD = __fsqrt_ru(d);
+  const float X = __fadd_ru(fmaxf(fabsf(__double2float_rn(xi[0])),
+                                  fmaxf(fabsf(__double2float_rn(xi[1])),
+                                        fabsf(__double2float_rn(xi[2])))),
+                            sD);
+  const float E = __fmul_ru(X, (1.0f + 1.0f / 524288.0f) * (1.0f / 1073741824.0f));
+  const float t = __fmul_ru(1.0f + 1.0f / 65536.0f, __fadd_ru(d, e));
+  return __fmaf_ru(4.0f, __fmul_ru(E, __fadd_ru(sD, E)), t);
 }
-// The FP32 softening of the split key (SplitP::eps), as a double.
-__device__ __forceinline__ double split_eps(double eps2) {
-  return (double)((float)eps2 + (float)(1.0 / 4503599627370496.0));
+// The FP32 softening of the split key (SplitP::eps).
+__device__ __forceinline__ float split_eps(double eps2) {
+  return (float)eps2 + (float)(1.0 / 4503599627370496.0);
 }
 
 __device__ __forceinline__ void ref_enqueue(void *buf, int i, int mode, float thr,
@@ -655,7 +670,15 @@ __device__ __noinline__ void SplitP::finish(const Out &o, int i, const KParams &
   write_final(o, i, kp.acc, kp.jerk, kp.pot);
   int mode = 0;
   float thr = 0.f, thr_mt = 0.f;
-  if (kp.refine && kp.kappa2 > 0.0) {
+  // Most sums are far from both limits: an FP32 test with a margin of 1e-3
+  // settles those, the FP64 one (16 cycles of the SM per instruction)
+  // decides the rest.
+  const float a2f = __fmaf_rn(o.a[0].x, o.a[0].x,
+                              __fmaf_rn(o.a[1].x, o.a[1].x, __fmul_rn(o.a[2].x, o.a[2].x)));
+  const float lim = 0.999f * (float)kp.kappa2 * a2f;
+  const bool clear = a2f > 1e-30f && lim < 1e37f && __fmul_rn(o.s1, o.s1) < lim &&
+                     __fmul_rn(o.mt, o.mt) < 0.999f * (float)(MU0 * MU0) * a2f;
+  if (kp.refine && kp.kappa2 > 0.0 && !clear) {
     double a2 = 0.0;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -693,6 +716,131 @@ __device__ __noinline__ void SplitP::finish(const Out &o, int i, const KParams &
   if (mode) ref_enqueue(kp.refine, i, mode, thr, thr_mt);
 }
 
+// ---------------------------------------------------------- lane table ---
+//
+// The sums of one i over its NL lanes (j-lanes of a CTA, or splits) by way
+// of shared memory.  A shuffle tree makes every lane carry all 20 words of
+// the record through every level (1250 instructions per warp at JL = 128,
+// five times the pair work of one tile).  Here each lane stores its words,
+// NT / NI threads per i then take one float-float quantity per eighth of
+// them: PARTS threads add NL / PARTS lanes each (independent TwoSums, the
+// dependent chain is one addition per lane) and merge by shuffle; the last
+// eighth does the condition sum, the largest chunk and the neighbour keys.
+// Row pitch NI * NL + 8 words: the eight rows a warp reads start in
+// different banks.  The results go to column 0 of the i's first lane.
+// For NL >= TAB_JL, where NT / NI >= 8.
+constexpr int TAB_JL = 16;
+constexpr int TAB_ROWS = 19;  // 7 x (hi, lo), key, second key, s, mt, slot
+template <int NL, int NI>
+__host__ __device__ constexpr int lane_table_pitch() {
+  return NI * NL + 8;
+}
+template <int NL, int NI>
+__host__ __device__ constexpr int lane_table_words() {
+  return TAB_ROWS * lane_table_pitch<NL, NI>();
+}
+template <int NL, int NI>
+__device__ __forceinline__ void lane_table_put(float *tab, int i, int l, const SplitP::Out &o) {
+  constexpr int P = lane_table_pitch<NL, NI>();
+  float *t = tab + i * NL + l;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    t[(2 * k) * P] = o.a[k].x;
+    t[(2 * k + 1) * P] = o.a[k].y;
+    t[(6 + 2 * k) * P] = o.j[k].x;
+    t[(7 + 2 * k) * P] = o.j[k].y;
+  }
+  t[12 * P] = o.p.x;
+  t[13 * P] = o.p.y;
+  t[14 * P] = o.nnr2;
+  t[15 * P] = o.nnr2b;
+  t[16 * P] = o.s1;
+  t[17 * P] = o.mt;
+  t[18 * P] = __int_as_float(o.nn);
+}
+template <int NL, int NI>
+__device__ __forceinline__ SplitP::Out lane_table_get(const float *tab, int i) {
+  constexpr int P = lane_table_pitch<NL, NI>();
+  const float *t = tab + i * NL;
+  SplitP::Out o;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    o.a[k] = make_float2(t[(2 * k) * P], t[(2 * k + 1) * P]);
+    o.j[k] = make_float2(t[(6 + 2 * k) * P], t[(7 + 2 * k) * P]);
+  }
+  o.p = make_float2(t[12 * P], t[13 * P]);
+  o.nnr2 = t[14 * P];
+  o.nnr2b = t[15 * P];
+  o.s1 = t[16 * P];
+  o.mt = t[17 * P];
+  o.nn = __float_as_int(t[18 * P]);
+  o.pad = 0;
+  return o;
+}
+template <int NL, int NI>
+__device__ __forceinline__ void lane_table_sum(float *tab) {
+  constexpr int P = lane_table_pitch<NL, NI>();
+  constexpr int TPI = NT / NI;       // threads per i
+  constexpr int PARTS = TPI / 8;     // threads per quantity
+  static_assert(TPI >= 8 && NL % PARTS == 0 && PARTS <= 32, "table");
+  const int i = threadIdx.x / TPI, r = threadIdx.x % TPI;
+  const int c = r / PARTS, part = r % PARTS;
+  float *t = tab + i * NL;
+  SplitP::Out o;
+  SplitP::to_out_zero(o);
+  float h = 0.f, l = 0.f;
+  if (c < 7) {
+    const float *th = t + 2 * c * P + part, *tl = th + P;
+#pragma unroll 4
+    for (int q = 0; q < NL / PARTS; q++) {
+      ff_acc(h, l, th[q * PARTS]);
+      l = __fadd_rn(l, tl[q * PARTS]);
+    }
+  } else {
+    for (int q = 0; q < NL / PARTS; q++) {
+      const float *u = t + 14 * P + part + q * PARTS;
+      const float k1 = u[0], k2 = u[P];
+      const int s = __float_as_int(u[4 * P]);
+      o.nnr2b = fminf(fmaxf(o.nnr2, k1), fminf(o.nnr2b, k2));
+      if (k1 < o.nnr2 || (k1 == o.nnr2 && s < o.nn)) {
+        o.nnr2 = k1;
+        o.nn = s;
+      }
+      o.s1 += u[2 * P];
+      o.mt = fmaxf(o.mt, u[3 * P]);
+    }
+  }
+#pragma unroll
+  for (int m = 1; m < PARTS; m <<= 1) {
+    ff_add(h, l, __shfl_down_sync(0xffffffffu, h, m), __shfl_down_sync(0xffffffffu, l, m));
+    const float k1 = __shfl_down_sync(0xffffffffu, o.nnr2, m);
+    const float k2 = __shfl_down_sync(0xffffffffu, o.nnr2b, m);
+    const float s1 = __shfl_down_sync(0xffffffffu, o.s1, m);
+    const float mt = __shfl_down_sync(0xffffffffu, o.mt, m);
+    const int s = __shfl_down_sync(0xffffffffu, o.nn, m);
+    o.nnr2b = fminf(fmaxf(o.nnr2, k1), fminf(o.nnr2b, k2));
+    if (k1 < o.nnr2 || (k1 == o.nnr2 && s < o.nn)) {
+      o.nnr2 = k1;
+      o.nn = s;
+    }
+    o.s1 += s1;
+    o.mt = fmaxf(o.mt, mt);
+  }
+  __syncthreads();  // every lane's words are read before column 0 is written
+  if (part == 0) {
+    if (c < 7) {
+      t[2 * c * P] = h;
+      t[(2 * c + 1) * P] = l;
+    } else {
+      t[14 * P] = o.nnr2;
+      t[15 * P] = o.nnr2b;
+      t[16 * P] = o.s1;
+      t[17 * P] = o.mt;
+      t[18 * P] = __int_as_float(o.nn);
+    }
+  }
+}
+
 // Number of j per thread between compensated folds.
 constexpr int FOLD_J = 64;
 
@@ -724,25 +872,6 @@ __global__ void __launch_bounds__(NT, P::MINB) force_kernel(KParams kp) {
   const int lane = tid & 31;
   pdl_wait();  // the predictor's records and the block list are complete
 
-  // ---- i-particles of this thread ----
-  typename P::I I[IPT];
-  int self[IPT];
-  bool valid[IPT];
-#pragma unroll
-  for (int k = 0; k < IPT; k++) {
-    const int i = blockIdx.x * ISLOTS + k * NIL + il;
-    valid[k] = i < kp.ni;
-    const int ii = valid[k] ? i : 0;
-    if (kp.ilist) {
-      const int slot = kp.ilist[ii];
-      I[k] = P::load_i_slot(kp.jrec, slot);
-      self[k] = valid[k] ? (kp.iself ? kp.iself[ii] : slot) : -1;
-    } else {
-      I[k] = P::load_i_explicit(kp.ipos + 3 * ii, kp.ivel + 3 * ii);
-      self[k] = valid[k] && kp.iself ? kp.iself[ii] : -1;
-    }
-  }
-
   // ---- j-range of this CTA ----
   const int js = blockIdx.y * kp.jsplit;
   int je = js + kp.jsplit;
@@ -768,6 +897,25 @@ __global__ void __launch_bounds__(NT, P::MINB) force_kernel(KParams kp) {
     for (int s = 0; s < NSTAGE && s < ntiles; s++) {
       mbar_expect_tx(&full[s], RPT * sizeof(Rec));
       tma_load_1d(&tiles[s][0], gj + s * RPT, RPT * sizeof(Rec), &full[s]);
+    }
+  }
+
+  // ---- i-particles of this thread ----
+  typename P::I I[IPT];
+  int self[IPT];
+  bool valid[IPT];
+#pragma unroll
+  for (int k = 0; k < IPT; k++) {
+    const int i = blockIdx.x * ISLOTS + k * NIL + il;
+    valid[k] = i < kp.ni;
+    const int ii = valid[k] ? i : 0;
+    if (kp.ilist) {
+      const int slot = kp.ilist[ii];
+      I[k] = P::load_i_slot(kp.jrec, slot);
+      self[k] = valid[k] ? (kp.iself ? kp.iself[ii] : slot) : -1;
+    } else {
+      I[k] = P::load_i_explicit(kp.ipos + 3 * ii, kp.ivel + 3 * ii);
+      self[k] = valid[k] && kp.iself ? kp.iself[ii] : -1;
     }
   }
 
@@ -932,9 +1080,29 @@ __global__ void __launch_bounds__(NT, P::MINB) force_kernel(KParams kp) {
     P::fold(T(k), q[k]);
     P::to_out(T(k), nnbest[k], nnm2[k], nnidx[k], o[k]);
   }
-  if (JL > 1) {
+  if constexpr (JL >= TAB_JL) {
+    // many lanes per i: through a shared-memory table (see lane_table)
+    float *tab = reinterpret_cast<float *>(&tiles[0][0]);
+    static_assert(lane_table_words<JL, ISLOTS>() * 4 <= sizeof(Rec) * RPT * NSTAGE, "table");
+    __syncthreads();  // the tiles are read
 #pragma unroll
-    for (int m = 1; m < (JL < 32 ? JL : 32); m <<= 1) {
+    for (int k = 0; k < IPT; k++) lane_table_put<JL, ISLOTS>(tab, k * NIL + il, jl, o[k]);
+    __syncthreads();
+    lane_table_sum<JL, ISLOTS>(tab);
+    __syncthreads();
+    if (tid < ISLOTS) {
+      const int i = blockIdx.x * ISLOTS + tid;
+      const typename P::Out m = lane_table_get<JL, ISLOTS>(tab, tid);
+      if (i < kp.ni) {
+        if (kp.nsplit == 1)
+          P::finish(m, i, kp);
+        else
+          reinterpret_cast<typename P::Out *>(kp.part)[(size_t)blockIdx.y * kp.ni_pad + i] = m;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int m = 1; m < JL; m <<= 1) {
 #pragma unroll
       for (int k = 0; k < IPT; k++) {
         typename P::Out other = shfl_xor_out(o[k], m);
@@ -947,121 +1115,89 @@ __global__ void __launch_bounds__(NT, P::MINB) force_kernel(KParams kp) {
         }
       }
     }
-  }
-  (void)lane;
-  if (JL > 32) {
-    // Cross-warp: warps w0..w0+JL/32-1 own one i-lane group.
-    __syncthreads();
-    typename P::Out *buf = reinterpret_cast<typename P::Out *>(&tiles[0][0]);
-    static_assert(sizeof(typename P::Out) * IPT * (NT / 32) <= sizeof(Rec) * RPT * NSTAGE, "smem");
-    const int warp = tid >> 5;
-    if (lane == 0) {
-#pragma unroll
-      for (int k = 0; k < IPT; k++) buf[warp * IPT + k] = o[k];
-    }
-    __syncthreads();
     if (jl == 0) {
-      constexpr int WPG = JL / 32;
 #pragma unroll
       for (int k = 0; k < IPT; k++) {
-        typename P::Out acc = buf[warp * IPT + k];
-        for (int w = 1; w < WPG; w++) P::merge(acc, buf[(warp + w) * IPT + k]);
-        o[k] = acc;
+        if (!valid[k]) continue;
+        const int i = blockIdx.x * ISLOTS + k * NIL + il;
+        if (kp.nsplit == 1)
+          P::finish(o[k], i, kp);
+        else
+          reinterpret_cast<typename P::Out *>(kp.part)[(size_t)blockIdx.y * kp.ni_pad + i] = o[k];
       }
     }
   }
-  if (jl == 0) {
-#pragma unroll
-    for (int k = 0; k < IPT; k++) {
-      if (!valid[k]) continue;
-      const int i = blockIdx.x * ISLOTS + k * NIL + il;
-      if (kp.nsplit == 1) {
-        P::finish(o[k], i, kp);
-      } else {
-        reinterpret_cast<typename P::Out *>(kp.part)[(size_t)blockIdx.y * kp.ni_pad + i] = o[k];
-      }
-    }
-  }
+  if constexpr (ISLOTS > G6_XMERGE_MAX) return;
   if (kp.nsplit == 1 || !kp.xtick) return;
 
-  // ---- split merge in the last CTA of the i-group (no second launch): the
-  // CTA whose ticket completes the group merges the nsplit partial records
-  // of each of the group's i, a warp per i, lane l taking splits l, l+32, ...
-  // in order and the lanes merging in a fixed shuffle-down tree (as
-  // reduce_warp_kernel).  The ticket is reset for the next launch. ----
-  __shared__ int last_s;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) last_s = atomicAdd(&kp.xtick[blockIdx.x], 1u) == (unsigned)(kp.nsplit - 1);
-  __syncthreads();
-  if (!last_s) return;
-  __threadfence();
-  using Out = typename P::Out;
-  const Out *part = reinterpret_cast<const Out *>(kp.part);
-  const int warp = tid >> 5;
-  const int i0 = blockIdx.x * ISLOTS;
-  for (int qq = warp; qq < ISLOTS; qq += NWARP) {
-    const int i = i0 + qq;
-    if (i >= kp.ni) break;
-    Out m = load_out_cg(part + (size_t)(lane < kp.nsplit ? lane : 0) * kp.ni_pad + i);
-    for (int sp = lane + 32; sp < kp.nsplit; sp += 32)
-      P::merge(m, load_out_cg(part + (size_t)sp * kp.ni_pad + i));
-    const int have = kp.nsplit < 32 ? kp.nsplit : 32;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      Out b;
-      const int *src = reinterpret_cast<const int *>(&m);
-      int *dst = reinterpret_cast<int *>(&b);
-#pragma unroll
-      for (int w = 0; w < (int)(sizeof(Out) / 4); w++)
-        dst[w] = __shfl_down_sync(0xffffffffu, src[w], off);
-      if (lane < off && lane + off < have) P::merge(m, b);
+  // ---- split merge in the last CTA of the i-group (no second launch): NT /
+  // ISLOTS threads per i, thread l taking splits l, l + ML, ... in order,
+  // then the table sums them as it sums the lanes.  The ticket is reset for
+  // the next launch. ----
+  if constexpr (ISLOTS <= G6_XMERGE_MAX) {
+    constexpr int ML = NT / ISLOTS;
+    __shared__ int last_s;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last_s = atomicAdd(&kp.xtick[blockIdx.x], 1u) == (unsigned)(kp.nsplit - 1);
+    __syncthreads();
+    if (!last_s) return;
+    __threadfence();
+    using Out = typename P::Out;
+    float *tab = reinterpret_cast<float *>(&tiles[0][0]);
+    const int q = tid / ML, l = tid % ML;
+    const int i = blockIdx.x * ISLOTS + q;
+    const Out *part = reinterpret_cast<const Out *>(kp.part) + (i < kp.ni ? i : 0);
+    Out m;
+    P::to_out_zero(m);
+    if (l < kp.nsplit) {
+      m = load_out_cg(part + (size_t)l * kp.ni_pad);
+      for (int sp = l + ML; sp < kp.nsplit; sp += ML)
+        P::merge(m, load_out_cg(part + (size_t)sp * kp.ni_pad));
     }
-    if (lane == 0) P::finish(m, i, kp);
+    lane_table_put<ML, ISLOTS>(tab, q, l, m);
+    __syncthreads();
+    lane_table_sum<ML, ISLOTS>(tab);
+    __syncthreads();
+    if (tid < ISLOTS && blockIdx.x * ISLOTS + tid < kp.ni)
+      P::finish(lane_table_get<ML, ISLOTS>(tab, tid), blockIdx.x * ISLOTS + tid, kp);
+    if (tid == 0) kp.xtick[blockIdx.x] = 0u;
   }
-  if (tid == 0) kp.xtick[blockIdx.x] = 0u;
 }
 
-// Second pass: merge the nsplit partial records of each i in split order
-// (one thread per i; for large blocks).
-template <class P>
-__global__ void reduce_kernel(KParams kp) {
+// Second pass: merge the nsplit partial records of each i.  A CTA takes IPB
+// i; thread (l, i) merges splits l, l + 128/IPB, ... in order, the 128/IPB
+// threads of an i merge in a fixed tree through shared memory, and the first
+// IPB threads finish their i together (finish's FP64 instructions cost 16
+// cycles of the SM each, whether one lane or 32 have an i: with a warp per i
+// they were most of this pass).  Deterministic for a given (ni, nsplit).
+// IPB = 8 while that gives every SM at most one CTA (splits in parallel), 32
+// above (dense finish); measured with the whole force call, see launch().
+template <class P, int IPB>
+__global__ void __launch_bounds__(128) reduce_kernel(KParams kp) {
+  constexpr int SL = 128 / IPB;
+  using Out = typename P::Out;
+  __shared__ Out sh[SL / 2][IPB];
   pdl_wait();
   pdl_trigger();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kp.ni) return;
-  const typename P::Out *part = reinterpret_cast<const typename P::Out *>(kp.part);
-  typename P::Out o = part[i];
-  for (int s = 1; s < kp.nsplit; s++) P::merge(o, part[(size_t)s * kp.ni_pad + i]);
-  P::finish(o, i, kp);
-}
-
-// The same merge with one warp per i, for small blocks, where the splits are
-// many and the i few (a thread walking 128 splits alone took ~90 us): lane l
-// merges splits l, l+32, ... in order, then the lanes merge in a fixed
-// shuffle-down tree.  Deterministic for a given (ni, nsplit).
-template <class P>
-__global__ void reduce_warp_kernel(KParams kp) {
-  pdl_wait();
-  pdl_trigger();
-  const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (i >= kp.ni) return;  // whole warps exit together
-  const typename P::Out *part = reinterpret_cast<const typename P::Out *>(kp.part);
-  typename P::Out o = part[(size_t)(lane < kp.nsplit ? lane : 0) * kp.ni_pad + i];
-  for (int s = lane + 32; s < kp.nsplit; s += 32) P::merge(o, part[(size_t)s * kp.ni_pad + i]);
-  const int have = kp.nsplit < 32 ? kp.nsplit : 32;  // lanes holding a partial
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    typename P::Out b;
-    const int *src = reinterpret_cast<const int *>(&o);
-    int *dst = reinterpret_cast<int *>(&b);
-#pragma unroll
-    for (int w = 0; w < (int)(sizeof(b) / 4); w++)
-      dst[w] = __shfl_down_sync(0xffffffffu, src[w], off);
-    if (lane < off && lane + off < have) P::merge(o, b);
+  const int il = threadIdx.x % IPB, l = threadIdx.x / IPB;
+  const int i = blockIdx.x * IPB + il;
+  const Out *part = reinterpret_cast<const Out *>(kp.part) + (i < kp.ni ? i : 0);
+  Out o;
+  P::to_out_zero(o);
+  if (l < kp.nsplit) {
+    o = part[(size_t)l * kp.ni_pad];
+#pragma unroll 2
+    for (int s = l + SL; s < kp.nsplit; s += SL) P::merge(o, part[(size_t)s * kp.ni_pad]);
   }
-  if (lane == 0) P::finish(o, i, kp);
+#pragma unroll
+  for (int h = SL / 2; h > 0; h >>= 1) {
+    if (l >= h && l < 2 * h) sh[l - h][il] = o;
+    __syncthreads();
+    if (l < h) P::merge(o, sh[l][il]);
+    __syncthreads();
+  }
+  if (l == 0 && i < kp.ni) P::finish(o, i, kp);
 }
 
 // FP64 redo of the queued i-particles (see "nearest neighbour proof" and
@@ -1072,20 +1208,47 @@ __global__ void reduce_warp_kernel(KParams kp) {
 // depends only on the number of queued entries, so results are
 // deterministic.  The last CTA to finish resets the queue.
 //
-// 1/sqrt(x): FP32 MUFU seed (relative error < 2^-22) and one Newton step,
-// relative error < 2^-42, far below the 1e-6 the pass is for.
+// What bounds it: the FP64 unit (2 lanes per SM and cycle: 16 cycles per warp
+// instruction, however many lanes have work).  So the REF_MT terms that are
+// due in FP64 are not evaluated where they are met, one or two lanes at a
+// time, but listed per warp in shared memory and evaluated 32 at a time;
+// cross-lane sums are float-float where the terms were FP32, and the FP64
+// ones exchange halves of the four quantities instead of all of them
+// (6 additions for 20).  Measured on a Salpeter cluster, N = 16384, blocks of
+// 139 to 2000 particles: 79-97 us before, see launch() for the figures now.
+//
+// 1/sqrt(x) as in kern_force64.cu: FP64 MUFU seed and one third-order step.
 __device__ __forceinline__ double refine_rsqrt(double x) {
-  double y = (double)rsqrt_approx((float)x);
-  return y * __fma_rn(-0.5 * x * y, y, 1.5);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = __fma_rn(-(x * y), y, 1.0);
+  return __fma_rn(h * y, __fma_rn(0.375, h, 0.5), y);
+}
+
+// FP64 term of j on the i at xi, added to sa and sp.
+__device__ __forceinline__ void f64_term(const void *rec, int j, const double xi[3], double eps2,
+                                         double sa[3], double &sp) {
+  double dx[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    dx[k] = ((double)g6_split_get(rec, j, k) + (double)g6_split_get(rec, j, 4 + k)) - xi[k];
+  const double m = (double)g6_split_get(rec, j, 3) + (double)g6_split_get(rec, j, 7);
+  const double r2 = __fma_rn(dx[2], dx[2], __fma_rn(dx[1], dx[1], __fma_rn(dx[0], dx[0], eps2)));
+  const double rinv = refine_rsqrt(r2);
+  const double mri = m * rinv;
+  const double mr3i = mri * (rinv * rinv);
+#pragma unroll
+  for (int k = 0; k < 3; k++) sa[k] = __fma_rn(mr3i, dx[k], sa[k]);
+  sp += mri;
 }
 
 // One j of a REF_MT entry: the force kernel's FP32 term (same operations,
 // so the same value up to the final product's rounding) into compensated
-// FP32 sums, or, above thr = TAU |a|, the FP64 term into the FP64 sums.
-__device__ __forceinline__ void mt_term(float xh, float yh, float zh, float m, float ml, float xl,
+// FP32 sums; true (and nothing added) above thr = TAU |a|, where the term is
+// due in FP64.
+__device__ __forceinline__ bool mt_term(float xh, float yh, float zh, float m, float ml, float xl,
                                         float yl, float zl, const float ih[3], const float il[3],
-                                        const double xi[3], float e32, double eps2, float thr,
-                                        double sa[3], double &sp, float ah[3], float al[3],
+                                        float e32, float thr, bool skip, float ah[3], float al[3],
                                         float &ph, float &pl) {
   const float jh[3] = {xh, yh, zh}, jl[3] = {xl, yl, zl};
   float d[3];
@@ -1094,30 +1257,44 @@ __device__ __forceinline__ void mt_term(float xh, float yh, float zh, float m, f
   const float r2f = __fmaf_rn(d[2], d[2], __fmaf_rn(d[1], d[1], __fmaf_rn(d[0], d[0], e32)));
   const float rinv = rsqrt_approx(r2f);
   const float mri = __fmul_rn(m, rinv);
-  if (__fmul_rn(mri, rinv) > thr) {
-    double dx[3];
+  if (skip) return false;
+  if (__fmul_rn(mri, rinv) > thr) return true;
+  // the FP32 term with the mass's high part, compensated; its low part
+  // (2^-24 of the term) goes straight into the low words
+  const float r3 = __fmul_rn(rinv, __fmul_rn(rinv, rinv));
+  const float mr3i = __fmul_rn(mri, __fmul_rn(rinv, rinv));
+  const float lr3 = __fmul_rn(ml, r3);
 #pragma unroll
-    for (int k = 0; k < 3; k++) dx[k] = ((double)jh[k] + (double)jl[k]) - xi[k];
-    const double r2 = __fma_rn(dx[2], dx[2], __fma_rn(dx[1], dx[1], __fma_rn(dx[0], dx[0], eps2)));
-    const double ri = refine_rsqrt(r2);
-    const double mr = ((double)m + (double)ml) * ri;
-    const double mr3 = mr * (ri * ri);
+  for (int k = 0; k < 3; k++) {
+    ff_acc(ah[k], al[k], __fmul_rn(mr3i, d[k]));
+    al[k] = __fmaf_rn(lr3, d[k], al[k]);
+  }
+  ff_acc(ph, pl, mri);
+  pl = __fmaf_rn(ml, rinv, pl);
+  return false;
+}
+
+// Warp sums of four FP64 quantities: halves of them change lanes first, so
+// every lane of group lane >> 3 ends with the sum of v[lane >> 3].
+__device__ __forceinline__ double warp_sum4(const double v[4], int lane) {
+  const bool hi = lane & 16, h2 = lane & 8;
+  double a = hi ? v[2] : v[0], b = hi ? v[3] : v[1];
+  a += __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
+  b += __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 16);
+  double c = h2 ? b : a;
+  c += __shfl_xor_sync(0xffffffffu, h2 ? a : b, 8);
 #pragma unroll
-    for (int k = 0; k < 3; k++) sa[k] = __fma_rn(mr3, dx[k], sa[k]);
-    sp += mr;
-  } else {
-    // the FP32 term with the mass's high part, compensated; its low part
-    // (2^-24 of the term) goes straight into the low words
-    const float r3 = __fmul_rn(rinv, __fmul_rn(rinv, rinv));
-    const float mr3i = __fmul_rn(mri, __fmul_rn(rinv, rinv));
-    const float lr3 = __fmul_rn(ml, r3);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      ff_acc(ah[k], al[k], __fmul_rn(mr3i, d[k]));
-      al[k] = __fmaf_rn(lr3, d[k], al[k]);
-    }
-    ff_acc(ph, pl, mri);
-    pl = __fmaf_rn(ml, rinv, pl);
+  for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  return c;
+}
+
+// The nearer of two neighbour candidates, the smaller slot on equal r^2
+// (slot < 0: none).  r^2 >= +0, so the bits order like the values.
+__device__ __forceinline__ void ref_nn_take(double &r2, int &slot, double or2, int os) {
+  const long long a = __double_as_longlong(r2), b = __double_as_longlong(or2);
+  if (os >= 0 && (slot < 0 || b < a || (b == a && os < slot))) {
+    r2 = or2;
+    slot = os;
   }
 }
 
@@ -1126,9 +1303,10 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
   pdl_trigger();
   RefBuf *b = reinterpret_cast<RefBuf *>(kp.refine);
   __shared__ unsigned s_cnt;
-  __shared__ double s_sum[RNT / 32][5];
+  __shared__ double s_sum[RNT / 32][4], s_r2[RNT / 32];
   __shared__ int s_slot[RNT / 32];
   __shared__ int s_last;
+  __shared__ int s_due[RNT / 32][96];  // per warp: j whose REF_MT term is due in FP64
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) s_cnt = *reinterpret_cast<volatile unsigned *>(&b->h.count);
   __syncthreads();
@@ -1155,7 +1333,7 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
   }
   const int units = ne * nch;
   const double eps2 = kp.eps2 + 1.0 / 4503599627370496.0;  // ph4's + 2^-52
-  const float e32 = (float)split_eps(kp.eps2);
+  const float e32 = split_eps(kp.eps2);
   const double inf = __longlong_as_double(0x7ff0000000000000ll);
   const void *rec = kp.jrec;
   for (int u = blockIdx.x; u < units; u += gridDim.x) {
@@ -1192,47 +1370,78 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
     for (int k = 0; k < 3; k++) xi[k] = (double)ih[k] + (double)il[k];
     if (mode & REF_NN) ipos64(kp, i, xi64);
     double sa[3] = {0.0, 0.0, 0.0}, sp = 0.0;
-    float ah[3] = {0.f, 0.f, 0.f}, al[3] = {0.f, 0.f, 0.f}, ph = 0.f, pl = 0.f;  // REF_MT
     double br2 = inf;
     int bslot = -1;
-    if (mode == REF_MT) {
-      // the common case alone: whole record pairs in four 16-byte loads,
-      // two pairs in flight per thread
+    double sum4 = 0.0;  // this lane group's quantity (warp_sum4's order)
+    if (mode & REF_MT) {
+      // whole record pairs in four 16-byte loads, two pairs in flight per
+      // thread; all lanes of a warp take the same number of steps
+      float ah[3] = {0.f, 0.f, 0.f}, al[3] = {0.f, 0.f, 0.f}, ph = 0.f, pl = 0.f;
       const float4 *q4 = reinterpret_cast<const float4 *>(rec);
+      int *due = s_due[warp];
+      int nd = 0;  // listed and not yet evaluated (the same in every lane)
+      bool any = false;
+      const unsigned below = (1u << lane) - 1u;
+      const int steps = (p1 - p0 - 32 * warp + RNT - 1) / RNT;
 #pragma unroll 2
-      for (int rp = p0 + tid; rp < p1; rp += RNT) {
-        const float4 A = __ldg(q4 + 6 * rp), B = __ldg(q4 + 6 * rp + 1);
-        const float4 C = __ldg(q4 + 6 * rp + 2), D = __ldg(q4 + 6 * rp + 3);
-        if (2 * rp != self && 2 * rp < kp.nj)
-          mt_term(A.x, A.z, B.x, B.z, D.z, C.x, C.z, D.x, ih, il, xi, e32, eps2, thr_mt, sa, sp,
-                  ah, al, ph, pl);
-        if (2 * rp + 1 != self && 2 * rp + 1 < kp.nj)
-          mt_term(A.y, A.w, B.y, B.w, D.w, C.y, C.w, D.y, ih, il, xi, e32, eps2, thr_mt, sa, sp,
-                  ah, al, ph, pl);
+      for (int st = 0; st < steps; st++) {
+        const int rp = p0 + 32 * warp + lane + st * RNT;
+        const int rq = rp < p1 ? rp : p1 - 1;
+        const float4 A = __ldg(q4 + 6 * rq), B = __ldg(q4 + 6 * rq + 1);
+        const float4 C = __ldg(q4 + 6 * rq + 2), D = __ldg(q4 + 6 * rq + 3);
+        const int j = 2 * rp;
+        const bool d0 = mt_term(A.x, A.z, B.x, B.z, D.z, C.x, C.z, D.x, ih, il, e32, thr_mt,
+                                rp >= p1 || j == self || j >= kp.nj, ah, al, ph, pl);
+        const bool d1 = mt_term(A.y, A.w, B.y, B.w, D.w, C.y, C.w, D.y, ih, il, e32, thr_mt,
+                                rp >= p1 || j + 1 == self || j + 1 >= kp.nj, ah, al, ph, pl);
+        const unsigned m0 = __ballot_sync(0xffffffffu, d0), m1 = __ballot_sync(0xffffffffu, d1);
+        if (m0 | m1) {
+          if (d0) due[nd + __popc(m0 & below)] = j;
+          nd += __popc(m0);
+          if (d1) due[nd + __popc(m1 & below)] = j + 1;
+          nd += __popc(m1);
+          __syncwarp();
+          while (nd >= 32) {
+            nd -= 32;
+            f64_term(rec, due[nd + lane], xi, eps2, sa, sp);
+            any = true;
+          }
+          __syncwarp();
+        }
       }
-    }
-    for (int j = j0 + tid; mode != REF_MT && j < j1; j += RNT) {
-      if (j == self) continue;
-      if (mode & REF_MT)
-        mt_term(g6_split_get(rec, j, 0), g6_split_get(rec, j, 1), g6_split_get(rec, j, 2),
-                g6_split_get(rec, j, 3), g6_split_get(rec, j, 7), g6_split_get(rec, j, 4),
-                g6_split_get(rec, j, 5), g6_split_get(rec, j, 6), ih, il, xi, e32, eps2, thr_mt,
-                sa, sp, ah, al, ph, pl);
-      if (mode & REF_ACC) {  // acceleration and potential; the jerk stays
-        double dx[3];
+      if (nd > 0) {
+        if (lane < nd) f64_term(rec, due[lane], xi, eps2, sa, sp);
+        any = true;
+        __syncwarp();
+      }
+      // FP32 sums: float-float over the warp
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
 #pragma unroll
         for (int k = 0; k < 3; k++)
-          dx[k] = ((double)g6_split_get(rec, j, k) + (double)g6_split_get(rec, j, 4 + k)) - xi[k];
-        const double m = (double)g6_split_get(rec, j, 3) + (double)g6_split_get(rec, j, 7);
-        const double r2 = __fma_rn(dx[2], dx[2], __fma_rn(dx[1], dx[1], __fma_rn(dx[0], dx[0], eps2)));
-        const double rinv = refine_rsqrt(r2);
-        const double mri = m * rinv;
-        const double mr3i = mri * (rinv * rinv);
-#pragma unroll
-        for (int k = 0; k < 3; k++) sa[k] = __fma_rn(mr3i, dx[k], sa[k]);
-        sp += mri;
+          ff_add(ah[k], al[k], __shfl_xor_sync(0xffffffffu, ah[k], off),
+                 __shfl_xor_sync(0xffffffffu, al[k], off));
+        ff_add(ph, pl, __shfl_xor_sync(0xffffffffu, ph, off),
+               __shfl_xor_sync(0xffffffffu, pl, off));
       }
-      if (mode & REF_NN) {
+      const int c = lane >> 3;
+      const float fh = c == 0 ? ah[0] : c == 1 ? ah[1] : c == 2 ? ah[2] : ph;
+      const float fl = c == 0 ? al[0] : c == 1 ? al[1] : c == 2 ? al[2] : pl;
+      sum4 = (double)fh + (double)fl;
+      if (any) {
+        const double v[4] = {sa[0], sa[1], sa[2], sp};
+        sum4 += warp_sum4(v, lane);
+      }
+    }
+    if (mode & REF_ACC) {  // acceleration and potential; the jerk stays
+      for (int j = j0 + tid; j < j1; j += RNT)
+        if (j != self) f64_term(rec, j, xi, eps2, sa, sp);
+      const double v[4] = {sa[0], sa[1], sa[2], sp};
+      sum4 = warp_sum4(v, lane);
+    }
+    if (mode & REF_NN) {
+      for (int j = j0 + tid; j < j1; j += RNT) {
+        if (j == self) continue;
         float d[3];
 #pragma unroll
         for (int k = 0; k < 3; k++)
@@ -1242,57 +1451,43 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
         if (key <= thr) {
           double xj[3];
           jpos64(kp.js, kp.ti, j, xj);
-          const double r2 = ph4_r2(xi64, xj);
-          if (r2 < br2 || (r2 == br2 && j < bslot)) {
-            br2 = r2;
-            bslot = j;
-          }
+          ref_nn_take(br2, bslot, ph4_r2(xi64, xj), j);
         }
       }
-    }
-    if (mode & REF_MT) {
 #pragma unroll
-      for (int k = 0; k < 3; k++) sa[k] += (double)ah[k] + (double)al[k];
-      sp += (double)ph + (double)pl;
-    }
-    // fixed-order reduction: shuffle-down tree, then warps in order
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-      for (int k = 0; k < 3; k++) sa[k] += __shfl_down_sync(0xffffffffu, sa[k], off);
-      sp += __shfl_down_sync(0xffffffffu, sp, off);
-      const double or2 = __shfl_down_sync(0xffffffffu, br2, off);
-      const int os = __shfl_down_sync(0xffffffffu, bslot, off);
-      if (or2 < br2 || (or2 == br2 && os >= 0 && (bslot < 0 || os < bslot))) {
-        br2 = or2;
-        bslot = os;
+      for (int off = 16; off > 0; off >>= 1) {
+        const double or2 = __shfl_down_sync(0xffffffffu, br2, off);
+        const int os = __shfl_down_sync(0xffffffffu, bslot, off);
+        ref_nn_take(br2, bslot, or2, os);
       }
     }
+    if ((lane & 7) == 0) s_sum[warp][lane >> 3] = sum4;
     if (lane == 0) {
-      for (int k = 0; k < 3; k++) s_sum[warp][k] = sa[k];
-      s_sum[warp][3] = sp;
-      s_sum[warp][4] = br2;
+      s_r2[warp] = br2;
       s_slot[warp] = bslot;
     }
     __syncthreads();
-    if (tid == 0) {
-      RefPart q;
-      for (int k = 0; k < 3; k++) q.a[k] = 0.0;
-      q.p = 0.0;
-      q.r2 = inf;
-      q.slot = -1;
-      q.pad = 0;
-      for (int w = 0; w < RNT / 32; w++) {
-        for (int k = 0; k < 3; k++) q.a[k] += s_sum[w][k];
-        q.p += s_sum[w][3];
-        if (s_slot[w] >= 0 && (s_sum[w][4] < q.r2 || (s_sum[w][4] == q.r2 && s_slot[w] < q.slot))) {
-          q.r2 = s_sum[w][4];
-          q.slot = s_slot[w];
-        }
-      }
-      b->part[e * nch + c] = q;
+    // the warps in order: one lane per quantity
+    RefPart *out = &b->part[e * nch + c];
+    if (tid < 4) {
+      double q = s_sum[0][tid];
+      for (int w = 1; w < RNT / 32; w++) q += s_sum[w][tid];
+      if (tid < 3)
+        out->a[tid] = q;
+      else
+        out->p = q;
+    } else if (tid == 4) {
+      double r2 = inf;
+      int sl = -1;
+      for (int w = 0; w < RNT / 32; w++) ref_nn_take(r2, sl, s_r2[w], s_slot[w]);
+      out->r2 = r2;
+      out->slot = sl;
+      out->pad = 0;
+    }
+    if (warp == 0) {
       __threadfence();
-      s_last = atomicAdd(&b->ticket[e], 1u) == (unsigned)(nch - 1);
+      __syncwarp();
+      if (lane == 0) s_last = atomicAdd(&b->ticket[e], 1u) == (unsigned)(nch - 1);
     }
     __syncthreads();
     // The CTA that completed the entry merges its chunks: warp 0, lane l
@@ -1301,35 +1496,29 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
     if (s_last && warp == 0) {
       __threadfence();
       const volatile RefPart *vp = b->part + (size_t)e * nch;
-      double fa[3] = {0.0, 0.0, 0.0}, fp = 0.0, fr2 = inf;
+      double f[4] = {0.0, 0.0, 0.0, 0.0}, fr2 = inf;
       int fs = -1;
       for (int cc = lane; cc < nch; cc += 32) {
-        for (int k = 0; k < 3; k++) fa[k] += vp[cc].a[k];
-        fp += vp[cc].p;
-        const int sl = vp[cc].slot;
-        const double r2 = vp[cc].r2;
-        if (sl >= 0 && (r2 < fr2 || (r2 == fr2 && sl < fs))) {
-          fr2 = r2;
-          fs = sl;
-        }
+        for (int k = 0; k < 3; k++) f[k] += vp[cc].a[k];
+        f[3] += vp[cc].p;
+        if (mode & REF_NN) ref_nn_take(fr2, fs, vp[cc].r2, vp[cc].slot);
       }
+      const double q = warp_sum4(f, lane);
+      if ((mode & (REF_ACC | REF_MT)) && (lane & 7) == 0) {
+        if (lane < 24)
+          kp.acc[3 * i + (lane >> 3)] = q;
+        else
+          kp.pot[i] = -q;
+      }
+      if (mode & REF_NN) {
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-        for (int k = 0; k < 3; k++) fa[k] += __shfl_down_sync(0xffffffffu, fa[k], off);
-        fp += __shfl_down_sync(0xffffffffu, fp, off);
-        const double or2 = __shfl_down_sync(0xffffffffu, fr2, off);
-        const int os = __shfl_down_sync(0xffffffffu, fs, off);
-        if (os >= 0 && (or2 < fr2 || (or2 == fr2 && (fs < 0 || os < fs)))) {
-          fr2 = or2;
-          fs = os;
+        for (int off = 16; off > 0; off >>= 1) {
+          const double or2 = __shfl_down_sync(0xffffffffu, fr2, off);
+          const int os = __shfl_down_sync(0xffffffffu, fs, off);
+          ref_nn_take(fr2, fs, or2, os);
         }
       }
       if (lane == 0) {
-        if (mode & (REF_ACC | REF_MT)) {
-          for (int k = 0; k < 3; k++) kp.acc[3 * i + k] = fa[k];
-          kp.pot[i] = -fp;
-        }
         if ((mode & REF_NN) && fs >= 0) {
           if (kp.nn) kp.nn[i] = fs;
           if (kp.nn_r2) kp.nn_r2[i] = (float)fr2;
@@ -1523,10 +1712,10 @@ int launch(const KParams &kp, int jl, int gx, cudaStream_t st, cudaEvent_t ev_mi
       return -2;
   }
   if (kp.nsplit > 1 && !kp.xtick) {
-    if (kp.ni < 4096)
-      launch_pdl(reduce_warp_kernel<P>, dim3((kp.ni + 3) / 4), dim3(128), 0, st, kp);
+    if (kp.ni <= 8 * sm_count())
+      launch_pdl(reduce_kernel<P, 8>, dim3((kp.ni + 7) / 8), dim3(128), 0, st, kp);
     else
-      launch_pdl(reduce_kernel<P>, dim3((kp.ni + 127) / 128), dim3(128), 0, st, kp);
+      launch_pdl(reduce_kernel<P, 32>, dim3((kp.ni + 31) / 32), dim3(128), 0, st, kp);
   }
   if (ev_mid) cudaEventRecord(ev_mid, st);
   // refine_kernel: units of (entry, j-chunk), at most RCHMAX chunks per

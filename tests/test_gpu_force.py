@@ -527,3 +527,30 @@ def test_fp64_force_edges(g6, n, ni):
     finally:
         g6.set_shape(0, 0)
         g6.set_precision(ag.SPLIT)
+
+
+@pytest.mark.parametrize("jl,ns", [(128, 1), (128, 2), (128, 63), (128, 65), (128, 130), (64, 3),
+                                   (32, 33), (16, 1), (16, 130), (8, 9), (1, 5)])
+@pytest.mark.parametrize("ni", [1, 2, 17, 257])
+def test_lane_and_split_merges(g6, jl, ns, ni):
+    """Every way the partial sums of an i meet (shuffles, the lane table, the
+    last CTA of a group, the second pass with 8 or 32 i per CTA), ragged
+    splits among them: within the split contract of the oracle, the neighbour
+    equal, the potential within 1e-6."""
+    n = 130 * 256 - 77
+    rng = np.random.RandomState(ni)
+    m = rng.uniform(0.5, 1.5, n) / n
+    x, v = rng.normal(size=(n, 3)), rng.normal(size=(n, 3))
+    sel = np.sort(rng.permutation(n)[:ni]).astype(np.int32)
+    ref = oracle.force(m, x, v, 1e-4, x[sel], v[sel])
+    g6.load_particles(m, x, v)
+    try:
+        g6.set_shape(jl, ns)
+        o = g6.force(0.0, 1e-4, n, x[sel], v[sel], self_slot=sel)
+    finally:
+        g6.set_shape(0, 0)
+    ea = np.linalg.norm(o["acc"] - ref["acc"], axis=1) / np.linalg.norm(ref["acc"], axis=1)
+    ej = np.linalg.norm(o["jerk"] - ref["jerk"], axis=1) / np.linalg.norm(ref["jerk"], axis=1)
+    assert ea.max() <= 1e-6 and ej.max() <= 1e-4
+    assert np.all(np.abs(o["pot"] - ref["pot"]) <= 1e-6 * np.abs(ref["pot"]))
+    assert np.array_equal(o["nn"], ref["nn"])
