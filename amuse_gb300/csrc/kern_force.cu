@@ -542,7 +542,7 @@ struct KParams {
 // largest partial sum over 32 j of one thread) above MU0 |a| are queued for
 // the cheaper REF_MT pass: the sum redone with the kernel's FP32 pair terms
 // but compensated (TwoSum) accumulation, every term above TAU |a| replaced
-// by its FP64 value.  That removes the dominant terms' own errors and the
+// by its float-float value.  That removes the dominant terms' own errors and the
 // FP32 partial sums' roundings relative to them, which are what does not
 // average out there; the remaining terms are each below TAU |a|, so their
 // random errors add up to ~1e-7 sqrt(TAU kappa) |a|.  Common in clusters
@@ -568,14 +568,14 @@ enum { REF_ACC = 1, REF_NN = 2, REF_MT = 4 };
 // with a term of 1.4 |a| reached 1.23e-6 (a star pulling against a cluster,
 // 6000 bodies); at 1.0 the worst left unrefined is one term's error.
 constexpr double MU0 = 1.0;
-// Terms above TAU |a| are evaluated in FP64 in the REF_MT pass.  A warp
-// takes the FP64 branch whenever one of its lanes does, at 1/64 of the FP32
-// rate, so TAU is kept where few terms reach it: at 0.02 the remaining
-// terms' random errors stay below ~1e-7 sqrt(0.02 kappa) |a| (C2 at 65536
-// Salpeter: the same largest error as at 0.005, and the block loop 2 %
-// faster).
+// Terms above TAU |a| are evaluated in float-float in the REF_MT pass: at
+// 0.02 the remaining terms' random errors stay below ~1e-7 sqrt(0.02 kappa)
+// |a| (C2 at 65536 Salpeter: the same largest error as at 0.005).
+#ifndef G6_REF_CTAS
+#define G6_REF_CTAS 4  // refine_kernel: CTAs per SM (62 registers, 256 threads)
+#endif
 #ifndef G6_REF_UNITS
-#define G6_REF_UNITS 4  // refine_kernel: (entry, j-chunk) units per CTA to aim for
+#define G6_REF_UNITS 2  // refine_kernel: (entry, j-chunk) units per CTA to aim for
 #endif
 #ifndef G6_TAU
 #define G6_TAU 0.02f
@@ -1172,7 +1172,8 @@ __global__ void __launch_bounds__(NT, P::MINB) force_kernel(KParams kp) {
 // cycles of the SM each, whether one lane or 32 have an i: with a warp per i
 // they were most of this pass).  Deterministic for a given (ni, nsplit).
 // IPB = 8 while that gives every SM at most one CTA (splits in parallel), 32
-// above (dense finish); measured with the whole force call, see launch().
+// above (dense finish).  8.5 -> 7.9 us at 651 i x 11 splits, 18 -> 11 us at
+// 4004 x 13, 16 -> 14 us at 722 x 37 with neighbours (a warp per i before).
 template <class P, int IPB>
 __global__ void __launch_bounds__(128) reduce_kernel(KParams kp) {
   constexpr int SL = 128 / IPB;
@@ -1208,14 +1209,14 @@ __global__ void __launch_bounds__(128) reduce_kernel(KParams kp) {
 // depends only on the number of queued entries, so results are
 // deterministic.  The last CTA to finish resets the queue.
 //
-// What bounds it: the FP64 unit (2 lanes per SM and cycle: 16 cycles per warp
-// instruction, however many lanes have work).  So the REF_MT terms that are
-// due in FP64 are not evaluated where they are met, one or two lanes at a
-// time, but listed per warp in shared memory and evaluated 32 at a time;
-// cross-lane sums are float-float where the terms were FP32, and the FP64
-// ones exchange halves of the four quantities instead of all of them
-// (6 additions for 20).  Measured on a Salpeter cluster, N = 16384, blocks of
-// 139 to 2000 particles: 79-97 us before, see launch() for the figures now.
+// What bounds it: FP64 issues at 2 lanes per SM and cycle (16 cycles per warp
+// instruction, however many lanes have work), so REF_MT entries, nearly all
+// of them, use none inside a unit: the terms that need more than FP32 are
+// evaluated in float-float (about 150 FP32 instructions, relative error
+// ~1e-12, where FP64 took 30 at 16 cycles) and, because few lanes meet one at
+// a time, listed per warp in shared memory and evaluated 32 at a time; lane
+// sums merge in float-float.  REF_ACC entries exchange halves of their four
+// FP64 quantities across lanes (6 additions for 20).
 //
 // 1/sqrt(x) as in kern_force64.cu: FP64 MUFU seed and one third-order step.
 __device__ __forceinline__ double refine_rsqrt(double x) {
@@ -1245,7 +1246,7 @@ __device__ __forceinline__ void f64_term(const void *rec, int j, const double xi
 // One j of a REF_MT entry: the force kernel's FP32 term (same operations,
 // so the same value up to the final product's rounding) into compensated
 // FP32 sums; true (and nothing added) above thr = TAU |a|, where the term is
-// due in FP64.
+// due in float-float.
 __device__ __forceinline__ bool mt_term(float xh, float yh, float zh, float m, float ml, float xl,
                                         float yl, float zl, const float ih[3], const float il[3],
                                         float e32, float thr, bool skip, float ah[3], float al[3],
@@ -1272,6 +1273,56 @@ __device__ __forceinline__ bool mt_term(float xh, float yh, float zh, float m, f
   ff_acc(ph, pl, mri);
   pl = __fmaf_rn(ml, rinv, pl);
   return false;
+}
+
+__device__ __forceinline__ float2 ff_mul(float2 a, float2 b) {
+  const float p = __fmul_rn(a.x, b.x);
+  float e = __fmaf_rn(a.x, b.x, -p);
+  e = __fmaf_rn(a.x, b.y, e);
+  e = __fmaf_rn(a.y, b.x, e);
+  const float h = __fadd_rn(p, e);
+  return make_float2(h, __fsub_rn(e, __fsub_rn(h, p)));
+}
+
+// The term of j in float-float, added to the compensated sums.
+__device__ __forceinline__ void ff_term(const void *rec, int j, const float ih[3],
+                                        const float il[3], float2 eps2, float ah[3], float al[3],
+                                        float &ph, float &pl) {
+  float2 d[3], r2 = eps2;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    // (xh_j - xh_i) exactly as s + e (TwoSum), then the low words
+    const float a = g6_split_get(rec, j, k), b = -ih[k];
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    const float t = __fadd_rn(e, __fsub_rn(g6_split_get(rec, j, 4 + k), il[k]));
+    d[k].x = __fadd_rn(s, t);
+    const float tt = __fsub_rn(d[k].x, s);
+    d[k].y = __fadd_rn(__fsub_rn(s, __fsub_rn(d[k].x, tt)), __fsub_rn(t, tt));
+    const float q = __fmul_rn(d[k].x, d[k].x);
+    const float ql = __fmaf_rn(2.0f * d[k].x, d[k].y, __fmaf_rn(d[k].x, d[k].x, -q));
+    ff_add(r2.x, r2.y, q, ql);
+  }
+  // 1/sqrt: y + y h (1/2 + 3/8 h), h = 1 - r2 y^2 from exact products (1 - u
+  // is exact, u being near 1)
+  const float y = rsqrt_approx(r2.x);
+  const float t = __fmul_rn(y, y), te = __fmaf_rn(y, y, -t);
+  const float u = __fmul_rn(t, r2.x), ue = __fmaf_rn(t, r2.x, -u);
+  const float h = __fsub_rn(__fsub_rn(1.0f, u), __fmaf_rn(t, r2.y, __fmaf_rn(te, r2.x, ue)));
+  float2 ri;
+  const float c = __fmul_rn(y, __fmaf_rn(__fmul_rn(0.375f, h), h, __fmul_rn(0.5f, h)));
+  ri.x = __fadd_rn(y, c);
+  ri.y = __fsub_rn(c, __fsub_rn(ri.x, y));
+  const float2 mr = ff_mul(make_float2(g6_split_get(rec, j, 3), g6_split_get(rec, j, 7)), ri);
+  const float2 mr3 = ff_mul(mr, ff_mul(ri, ri));
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const float2 f = ff_mul(mr3, d[k]);
+    ff_acc(ah[k], al[k], f.x);
+    al[k] = __fadd_rn(al[k], f.y);
+  }
+  ff_acc(ph, pl, mr.x);
+  pl = __fadd_rn(pl, mr.y);
 }
 
 // Warp sums of four FP64 quantities: halves of them change lanes first, so
@@ -1306,7 +1357,7 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
   __shared__ double s_sum[RNT / 32][4], s_r2[RNT / 32];
   __shared__ int s_slot[RNT / 32];
   __shared__ int s_last;
-  __shared__ int s_due[RNT / 32][96];  // per warp: j whose REF_MT term is due in FP64
+  __shared__ int s_due[RNT / 32][96];  // per warp: j whose REF_MT term is due in float-float
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) s_cnt = *reinterpret_cast<volatile unsigned *>(&b->h.count);
   __syncthreads();
@@ -1319,11 +1370,11 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
   if (cnt > (unsigned)RCAP && blockIdx.x == 0 && tid == 0) atomicMax(&b->h.overflow, cnt);
   int nch = 1;
   if (ne > 0) {
-    // About one unit per CTA while the entries are few (each unit then
-    // covers more j and the CTA reduces once); four per CTA once they are
-    // many, for balance (measured on config 2's blocks: 8 entries 34 -> 24
-    // us, 25 entries 68 -> 40 us at one per CTA; 366 entries 282 us at four,
-    // 652 us at one)
+    // One unit per CTA while the entries are few (the CTA reduces once), two
+    // once they are many, for balance.  Salpeter cluster, N = 16384, 4 CTAs
+    // per SM: 165 entries 72 us at one, 62 at two, 61 at four; 59 entries 26,
+    // 28, 30; at 2 CTAs per SM and four units 78 and 39.  (With the FP64
+    // terms and reductions this pass had before: 87 and 54 us.)
     const int upc = ne * 4 > (int)gridDim.x ? G6_REF_UNITS : 1;
     nch = (upc * (int)gridDim.x + ne - 1) / ne;
     nch = min(nch, RCHMAX);
@@ -1369,7 +1420,6 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
 #pragma unroll
     for (int k = 0; k < 3; k++) xi[k] = (double)ih[k] + (double)il[k];
     if (mode & REF_NN) ipos64(kp, i, xi64);
-    double sa[3] = {0.0, 0.0, 0.0}, sp = 0.0;
     double br2 = inf;
     int bslot = -1;
     double sum4 = 0.0;  // this lane group's quantity (warp_sum4's order)
@@ -1380,7 +1430,7 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
       const float4 *q4 = reinterpret_cast<const float4 *>(rec);
       int *due = s_due[warp];
       int nd = 0;  // listed and not yet evaluated (the same in every lane)
-      bool any = false;
+      const float2 eps2f = make_float2((float)eps2, (float)(eps2 - (double)(float)eps2));
       const unsigned below = (1u << lane) - 1u;
       const int steps = (p1 - p0 - 32 * warp + RNT - 1) / RNT;
 #pragma unroll 2
@@ -1403,15 +1453,13 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
           __syncwarp();
           while (nd >= 32) {
             nd -= 32;
-            f64_term(rec, due[nd + lane], xi, eps2, sa, sp);
-            any = true;
+            ff_term(rec, due[nd + lane], ih, il, eps2f, ah, al, ph, pl);
           }
           __syncwarp();
         }
       }
       if (nd > 0) {
-        if (lane < nd) f64_term(rec, due[lane], xi, eps2, sa, sp);
-        any = true;
+        if (lane < nd) ff_term(rec, due[lane], ih, il, eps2f, ah, al, ph, pl);
         __syncwarp();
       }
       // FP32 sums: float-float over the warp
@@ -1428,12 +1476,9 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
       const float fh = c == 0 ? ah[0] : c == 1 ? ah[1] : c == 2 ? ah[2] : ph;
       const float fl = c == 0 ? al[0] : c == 1 ? al[1] : c == 2 ? al[2] : pl;
       sum4 = (double)fh + (double)fl;
-      if (any) {
-        const double v[4] = {sa[0], sa[1], sa[2], sp};
-        sum4 += warp_sum4(v, lane);
-      }
     }
     if (mode & REF_ACC) {  // acceleration and potential; the jerk stays
+      double sa[3] = {0.0, 0.0, 0.0}, sp = 0.0;
       for (int j = j0 + tid; j < j1; j += RNT)
         if (j != self) f64_term(rec, j, xi, eps2, sa, sp);
       const double v[4] = {sa[0], sa[1], sa[2], sp};
@@ -1722,7 +1767,7 @@ int launch(const KParams &kp, int jl, int gx, cudaStream_t st, cudaEvent_t ev_mi
   // entry and ni entries, so small blocks get a small grid
   if (kp.refine) {
     const long long cap = (long long)kp.ni * RCHMAX;
-    const int grid = cap < 2LL * sm_count() ? (int)cap : 2 * sm_count();
+    const int grid = cap < (long long)G6_REF_CTAS * sm_count() ? (int)cap : G6_REF_CTAS * sm_count();
     launch_pdl(refine_kernel, dim3(grid), dim3(RNT), 0, st, kp);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
