@@ -72,3 +72,40 @@ def test_knn_edges(g6):
             g6.knn(5, k=k)
     with pytest.raises(ag.G6Error):
         g6.knn(5, k=2, slots=[7])
+
+
+def _cell_system(name, n, rng):
+    if name == "plummer":
+        return ic.plummer(n, rng=rng)[1]
+    if name == "lattice":  # ties everywhere, far from the origin
+        k = int(np.ceil(n ** (1 / 3)))
+        g = np.arange(k) * 0.0625
+        return (np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3) + 1000.0)[:n]
+    if name == "outlier":  # one particle sets the filter's slack for all
+        x = rng.normal(size=(n, 3))
+        x[n // 3] = [3e4, -1e4, 2e4]
+        return x
+    if name == "plane":  # no extent along one axis
+        x = rng.uniform(-1, 1, size=(n, 3))
+        x[:, 2] = 0.25
+        return x
+    x = rng.normal(size=(n, 3)) * 1e-3  # two clumps far apart, many coincident
+    x[: n // 2] += 50.0
+    x[: n // 8] = x[0]
+    return x
+
+
+@pytest.mark.parametrize("name", ["plummer", "lattice", "outlier", "plane", "clumps"])
+@pytest.mark.parametrize("n,ni,k", [(9261, 9261, 12), (4099, 4097, 8), (16421, 4127, 32), (70001, 9001, 1)])
+def test_knn_cells(g6, name, n, ni, k):
+    """The cell path (many pairs, dense lists): the exact lists, whatever the
+    cells hold; ragged tiles, listed slots in any order, some twice."""
+    rng = np.random.RandomState(n)
+    x = _cell_system(name, n, rng)
+    g6.load_particles(np.full(n, 1.0 / n), x, np.zeros_like(x))
+    slots = np.arange(n) if ni == n else rng.randint(0, n, ni)
+    ids, d2 = g6.knn(n, k=k, slots=slots)
+    few = rng.permutation(ni)[:600]
+    ref_j, ref_d = oracle.knn(x, k, slots[few])
+    _check(ids[few], d2[few], ref_j, ref_d)
+    assert np.all(np.diff(d2, axis=1) >= 0)
