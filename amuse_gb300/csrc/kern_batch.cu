@@ -5,9 +5,9 @@
 // a host-chosen order, largest systems first), integrates it to its end
 // time, writes it back and takes the next one, so uneven systems balance
 // themselves.  The integrator is smallN's (src/amuse_ph4/src/smallN.cc):
-// without the unperturbed-binary tree in batch_kernel (its EXACT mode is
-// bit-identical to smallN with dt_crit = 0), with it in batch_unp_kernel
-// (below) -- a shared-step, time-symmetrised
+// batch_exact_kernel without the unperturbed-binary tree (bit-identical to
+// smallN with dt_crit = 0), batch_tree_kernel (the fast and split modes) with
+// it or without -- a shared-step, time-symmetrised
 // 4th-order Hermite scheme --
 //   predict_loworder (hdyn.h:192-201) from the stored old acc/jerk,
 //   n_iter + 1 force evaluations per step, each followed by
@@ -15,15 +15,14 @@
 //   iterated step new_dt (smallN.cc:617-660),
 //   step from the Kepler criterion eta * sqrt(min over pairs of
 //   min(0.5 r^3 / (m_i + m_j), r^2 / v^2)) (smallN.cc:85-116, :318-363).
-// State is FP64.  Lane l owns bodies l and l + 32 (n <= 64).
+// State is FP64.  n <= 64.
 //
-// EXACT = true evaluates every expression with the same IEEE operations, in
+// The exact mode evaluates every expression with the same IEEE operations, in
 // the same order, as smallN on the CPU (each pair in its (i < j) orientation,
 // contributions accumulated in smallN's pair order, no fused multiply-adds,
-// IEEE divides and square roots), so results are bit-identical to smallN.
-// MODE_FAST uses one reciprocal square root per pair and FMAs (about 7x
-// fewer FP64 instructions; results differ from smallN at the last-bit
-// level, which chaotic systems amplify).
+// correctly rounded divides and square roots).
+// MODE_FAST uses one reciprocal square root per pair and FMAs (results differ
+// from smallN at the last-bit level, which chaotic systems amplify).
 // MODE_SPLIT keeps the state, the predictor and the corrector in FP64 but
 // evaluates the pair terms in FP32 from double-single positions (the
 // relative position is exact to FP32 precision of |r|, as in the g6 force
@@ -32,11 +31,14 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "f32x2.cuh"
+#include "g6_dev.h"
+
 namespace {
 
 constexpr int MAXN = 64;
 constexpr int WARPS_MAX = 8;
-enum { MODE_FAST = 0, MODE_EXACT = 1, MODE_SPLIT = 2 };
+enum { MODE_FAST = 0, MODE_EXACT = 1, MODE_SPLIT = 2 };  // the ABI's G6_BATCH_*
 
 
 __device__ __forceinline__ double ADD(double a, double b) { return __dadd_rn(a, b); }
@@ -49,152 +51,71 @@ struct Body {
   double pos[3], vel[3], pp[3], pv[3], acc[3], jerk[3], oacc[3], ojerk[3];
 };
 
-struct WarpSmem {
-  union {
-    struct {
-      double pp[MAXN][3];
-      double pv[MAXN][3];
-    } d;
-    struct {  // MODE_SPLIT: double-single positions, FP32 velocities
-      float ph[MAXN][3];
-      float pl[MAXN][3];
-      float vf[MAXN][3];
-    } f;
-  };
-  double m[MAXN];
-  float mf[MAXN];
+struct alignas(16) double4_16 {
+  double x, y, z, w;
 };
 
-// 1/sqrt(x): FP32 MUFU seed, two Newton-Raphson steps.
-__device__ __forceinline__ double rsqrt64(double x) {
-  double y = (double)rsqrtf((float)x);
-  const double hx = 0.5 * x;
-  y = y * fma(-hx * y, y, 1.5);
-  y = y * fma(-hx * y, y, 1.5);
-  return y;
+struct WarpSmem {
+  double pp[MAXN][3];
+  double pv[MAXN][3];
+  double m[MAXN];
+};
+
+// a / b correctly rounded from y, the correctly rounded 1 / b: q = a y is
+// within an ulp, its FMA residual is exact, and one correction rounds right
+// (Markstein 1990, theorem 3; checked against a / b on 4e8 operands, the ends
+// of the mantissa range among them).  3 FP64 instructions for each further
+// quotient by the same b instead of about 10.  Where a product could leave
+// the normal range (a = 0 too), the division itself.
+__device__ __forceinline__ bool mid_range(double x) {  // 2^-300 <= |x| < 2^300
+  const unsigned e = (unsigned)__double2hiint(x) & 0x7ff00000u;
+  return e - (723u << 20) < (600u << 20);
+}
+__device__ __forceinline__ double div_by(double a, double b, double y, bool bmid) {
+  if (!(bmid && mid_range(a))) return __ddiv_rn(a, b);
+  const double q = __dmul_rn(a, y);
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 
 // Contribution of the pair (a, b), a < b in smallN's orientation, to body
 // `me` (me == a or me == b), plus the pair's Kepler time-step^2.
-template <bool EXACT>
 __device__ __forceinline__ double pair_term(const WarpSmem &S, int a, int b, bool me_is_a,
                                             double inv_me, double acc[3], double jerk[3]) {
   const double ma = S.m[a], mb = S.m[b];
   double dx[3], dv[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    dx[k] = SUB(S.d.pp[b][k], S.d.pp[a][k]);
-    dv[k] = SUB(S.d.pv[b][k], S.d.pv[a][k]);
+    dx[k] = SUB(S.pp[b][k], S.pp[a][k]);
+    dv[k] = SUB(S.pv[b][k], S.pv[a][k]);
   }
-  if (EXACT) {
-    const double d2 = ADD(ADD(MUL(dx[0], dx[0]), MUL(dx[1], dx[1])), MUL(dx[2], dx[2]));
-    const double d = __dsqrt_rn(d2);
-    const double d3 = MUL(d2, d);
-    const double xv = ADD(ADD(MUL(dx[0], dv[0]), MUL(dx[1], dv[1])), MUL(dx[2], dv[2]));
-    const double d5 = MUL(d3, d2);
-    const double s = me_is_a ? inv_me : -inv_me;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      const double iforce = DIV(MUL(mb, dx[k]), d3);
-      const double ijerk = MUL(mb, SUB(DIV(dv[k], d3), DIV(MUL(MUL(3.0, dx[k]), xv), d5)));
-      const double force = MUL(ma, iforce);
-      const double jk = MUL(ma, ijerk);
-      acc[k] = ADD(acc[k], MUL(s, force));
-      jerk[k] = ADD(jerk[k], MUL(s, jk));
-    }
-    const double mass = ADD(mb, ma);
-    const double vel2 = ADD(ADD(MUL(dv[0], dv[0]), MUL(dv[1], dv[1])), MUL(dv[2], dv[2]));
-    const double dtff2 = DIV(MUL(0.5, d3), mass);
-    const double dtv2 = DIV(d2, fabs(vel2));
-    return fmin(dtff2, dtv2);
-  } else {
-    const double d2 = dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2];
-    const double rinv = rsqrt64(d2);
-    const double rinv2 = rinv * rinv;
-    const double rinv3 = rinv * rinv2;
-    const double xv = dx[0] * dv[0] + dx[1] * dv[1] + dx[2] * dv[2];
-    const double mo = me_is_a ? mb : -ma;  // force/m_me on me
-    const double f = mo * rinv3;
-    const double a3 = -3.0 * xv * rinv2;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      acc[k] = fma(f, dx[k], acc[k]);
-      jerk[k] = fma(f, fma(a3, dx[k], dv[k]), jerk[k]);
-    }
-    (void)inv_me;
-    const double vel2 = dv[0] * dv[0] + dv[1] * dv[1] + dv[2] * dv[2];
-    const double d3 = d2 * d2 * rinv;
-    const double dtff2 = 0.5 * d3 / (ma + mb);
-    const double dtv2 = d2 / vel2;
-    return fmin(dtff2, dtv2);
-  }
-}
-
-__device__ __forceinline__ float rsqrt_approx(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// MODE_SPLIT pair term: contribution of j to body i, and the pair's Kepler
-// step^2.  FP32 unless the pair is closer than 1e-9 (d^2 < 1e-18): there
-// m / d^3 times a relative velocity ~ sqrt(M / d) can leave the FP32 range,
-// so such (rare) pairs are evaluated in FP64 into separate accumulators.
-// The pair j == i (self) is evaluated too, with its contribution masked to
-// zero and its step to +inf, so the j loop has no divergent skip.  The step
-// quotients use the approximate division (split mode is not bit-exact with
-// anything, and the step only has to follow the criterion closely).
-__device__ __forceinline__ float pair_split(const WarpSmem &S, int i, int j, float acc[3],
-                                            float jerk[3], double accd[3], double jerkd[3]) {
-  const bool self = j == i;
-  float dx[3], dv[3];
+  const double d2 = ADD(ADD(MUL(dx[0], dx[0]), MUL(dx[1], dx[1])), MUL(dx[2], dx[2]));
+  const double d = __dsqrt_rn(d2);
+  const double d3 = MUL(d2, d);
+  const double xv = ADD(ADD(MUL(dx[0], dv[0]), MUL(dx[1], dv[1])), MUL(dx[2], dv[2]));
+  const double d5 = MUL(d3, d2);
+  const double y3 = __drcp_rn(d3), y5 = __drcp_rn(d5);
+  const bool r3 = mid_range(d3), r5 = mid_range(d5);
+  const double s = me_is_a ? inv_me : -inv_me;
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    dx[k] = __fadd_rn(__fsub_rn(S.f.ph[j][k], S.f.ph[i][k]), __fsub_rn(S.f.pl[j][k], S.f.pl[i][k]));
-    dv[k] = S.f.vf[j][k] - S.f.vf[i][k];
+    const double iforce = div_by(MUL(mb, dx[k]), d3, y3, r3);
+    const double ijerk = MUL(mb, SUB(div_by(dv[k], d3, y3, r3),
+                                     div_by(MUL(MUL(3.0, dx[k]), xv), d5, y5, r5)));
+    const double force = MUL(ma, iforce);
+    const double jk = MUL(ma, ijerk);
+    acc[k] = ADD(acc[k], MUL(s, force));
+    jerk[k] = ADD(jerk[k], MUL(s, jk));
   }
-  const float d2 = fmaf(dx[2], dx[2], fmaf(dx[1], dx[1], dx[0] * dx[0]));
-  const float v2 = fmaf(dv[2], dv[2], fmaf(dv[1], dv[1], dv[0] * dv[0]));
-  const float mt = S.mf[i] + S.mf[j];
-  if (self || d2 >= 1e-18f) {
-    const float rinv = self ? 0.f : rsqrt_approx(d2);
-    const float rinv2 = rinv * rinv;
-    const float f = S.mf[j] * rinv * rinv2;
-    const float xv = fmaf(dx[2], dv[2], fmaf(dx[1], dv[1], dx[0] * dv[0]));
-    const float a3 = -3.0f * xv * rinv2;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      acc[k] = fmaf(f, dx[k], acc[k]);
-      jerk[k] = fmaf(f, fmaf(a3, dx[k], dv[k]), jerk[k]);
-    }
-    const float ts = fminf(__fdividef(0.5f * d2 * (d2 * rinv), mt), __fdividef(d2, v2));
-    return self ? __int_as_float(0x7f800000) : ts;
-  }
-  double X[3], W[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    X[k] = (double)dx[k];
-    W[k] = (double)dv[k];
-  }
-  const double dd2 = X[0] * X[0] + X[1] * X[1] + X[2] * X[2];
-  const double d = sqrt(dd2);
-  const double rinv2 = 1.0 / dd2;
-  const double f = (double)S.mf[j] * rinv2 / d;
-  const double a3 = -3.0 * (X[0] * W[0] + X[1] * W[1] + X[2] * W[2]) * rinv2;
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    accd[k] += f * X[k];
-    jerkd[k] += f * (a3 * X[k] + W[k]);
-  }
-  const double vv = W[0] * W[0] + W[1] * W[1] + W[2] * W[2];
-  return (float)fmin(0.5 * dd2 * d / (double)mt, dd2 / vv);
+  const double mass = ADD(mb, ma);
+  const double vel2 = ADD(ADD(MUL(dv[0], dv[0]), MUL(dv[1], dv[1])), MUL(dv[2], dv[2]));
+  const double dtff2 = DIV(MUL(0.5, d3), mass);
+  const double dtv2 = DIV(d2, fabs(vel2));
+  return fmin(dtff2, dtv2);
 }
 
 // acc/jerk of the lane's bodies from the predicted state in S; returns the
 // system's min Kepler step^2 (warp-uniform).
-template <int MODE>
 __device__ double forces(const WarpSmem &S, int n, int lane, Body B[2]) {
-  constexpr bool EXACT = MODE == MODE_EXACT;
   double ts2 = __longlong_as_double(0x7ff0000000000000ll);
 #pragma unroll
   for (int q = 0; q < 2; q++) {
@@ -202,38 +123,18 @@ __device__ double forces(const WarpSmem &S, int n, int lane, Body B[2]) {
 #pragma unroll
     for (int k = 0; k < 3; k++) B[q].acc[k] = B[q].jerk[k] = 0.0;
     if (i >= n) continue;
-    if (MODE == MODE_SPLIT) {
-      float a[3] = {0.f, 0.f, 0.f}, jk[3] = {0.f, 0.f, 0.f};
-      double ad[3] = {0.0, 0.0, 0.0}, jd[3] = {0.0, 0.0, 0.0};
-      float m2 = __int_as_float(0x7f800000);
-      for (int j = 0; j < n; j++) m2 = fminf(m2, pair_split(S, i, j, a, jk, ad, jd));
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        B[q].acc[k] = (double)a[k] + ad[k];
-        B[q].jerk[k] = (double)jk[k] + jd[k];
-      }
-      ts2 = fmin(ts2, (double)m2);
-    } else if (EXACT) {
-      // smallN's pair order: (j, i) for j < i first, then (i, j) for j > i,
-      // each pair in its (i < j) orientation.
-      for (int j = 0; j < i; j++)
-        ts2 = fmin(ts2, pair_term<true>(S, j, i, false, B[q].inv_m, B[q].acc, B[q].jerk));
-      for (int j = i + 1; j < n; j++)
-        ts2 = fmin(ts2, pair_term<true>(S, i, j, true, B[q].inv_m, B[q].acc, B[q].jerk));
-    } else {
-      // orientation-free (same instruction stream in every lane)
-      for (int j = 0; j < n; j++) {
-        if (j == i) continue;
-        ts2 = fmin(ts2, pair_term<false>(S, i, j, true, B[q].inv_m, B[q].acc, B[q].jerk));
-      }
-    }
+    // smallN's pair order: (j, i) for j < i first, then (i, j) for j > i,
+    // each pair in its (i < j) orientation.
+    for (int j = 0; j < i; j++)
+      ts2 = fmin(ts2, pair_term(S, j, i, false, B[q].inv_m, B[q].acc, B[q].jerk));
+    for (int j = i + 1; j < n; j++)
+      ts2 = fmin(ts2, pair_term(S, i, j, true, B[q].inv_m, B[q].acc, B[q].jerk));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) ts2 = fmin(ts2, __shfl_xor_sync(0xffffffffu, ts2, o));
   return ts2;
 }
 
-template <int MODE>
 __device__ __forceinline__ void publish(WarpSmem &S, int n, int lane, const Body B[2]) {
   __syncwarp();
 #pragma unroll
@@ -242,38 +143,37 @@ __device__ __forceinline__ void publish(WarpSmem &S, int n, int lane, const Body
     if (i < n) {
 #pragma unroll
       for (int k = 0; k < 3; k++) {
-        if (MODE == MODE_SPLIT) {
-          const float h = __double2float_rn(B[q].pp[k]);
-          S.f.ph[i][k] = h;
-          S.f.pl[i][k] = __double2float_rn(B[q].pp[k] - (double)h);
-          S.f.vf[i][k] = __double2float_rn(B[q].pv[k]);
-        } else {
-          S.d.pp[i][k] = B[q].pp[k];
-          S.d.pv[i][k] = B[q].pv[k];
-        }
+        S.pp[i][k] = B[q].pp[k];
+        S.pv[i][k] = B[q].pv[k];
       }
     }
   }
   __syncwarp();
 }
 
-template <int MODE>
-__global__ void batch_kernel(const int *__restrict__ order, const int *__restrict__ off,
-                             const double *__restrict__ t_end_s, const double *__restrict__ mass,
-                             double *pos, double *vel, double eta, int n_iter,
-                             long long max_steps, int *queue, double *t_out, long long *steps_out,
-                             unsigned long long *wall_ns, int *status) {
-  constexpr bool EXACT = MODE == MODE_EXACT;
+// The queue: a warp's first system is its rank with the CTAs counted first,
+// so that the first (largest) systems, or the only ones, go to different SMs
+// (FP64 issues at 2 lanes per SM: four warps of one CTA at work beside idle
+// SMs ran at a quarter of their speed); the others come from the counter.
+__device__ __forceinline__ int first_system(int w) { return w * gridDim.x + blockIdx.x; }
+__device__ __forceinline__ int next_system(int *queue, int lane) {
+  int q = 0;
+  if (lane == 0) q = atomicAdd(queue, 1);
+  return (int)(gridDim.x * (blockDim.x >> 5)) + __shfl_sync(0xffffffffu, q, 0);
+}
+
+__global__ void batch_exact_kernel(const int *__restrict__ order, const int *__restrict__ off,
+                                   const double *__restrict__ t_end_s,
+                                   const double *__restrict__ mass, double *pos, double *vel,
+                                   double eta, int n_iter, long long max_steps, int *queue,
+                                   double *t_out, long long *steps_out,
+                                   unsigned long long *wall_ns, int *status) {
   __shared__ WarpSmem smem[WARPS_MAX];
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
   WarpSmem &S = smem[w];
   const int nsys = queue[1];  // written by the host before the launch
-  while (true) {
-    int q = 0;
-    if (lane == 0) q = atomicAdd(queue, 1);
-    q = __shfl_sync(0xffffffffu, q, 0);
-    if (q >= nsys) break;
+  for (int q = first_system(w); q < nsys; q = next_system(queue, lane)) {
     const int s = order[q];
     unsigned long long t0;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
@@ -288,13 +188,14 @@ __global__ void batch_kernel(const int *__restrict__ order, const int *__restric
       }
       continue;
     }
+    const int nq = n > 32 ? 2 : 1;  // bodies per lane
     Body B[2];
 #pragma unroll
     for (int qq = 0; qq < 2; qq++) {
       const int i = lane + 32 * qq;
       const int ii = i < n ? i : 0;
       B[qq].m = mass[base + ii];
-      B[qq].inv_m = EXACT ? DIV(1.0, B[qq].m) : 1.0 / B[qq].m;
+      B[qq].inv_m = DIV(1.0, B[qq].m);
 #pragma unroll
       for (int k = 0; k < 3; k++) {
         B[qq].pos[k] = pos[3 * (base + ii) + k];
@@ -303,15 +204,11 @@ __global__ void batch_kernel(const int *__restrict__ order, const int *__restric
         B[qq].pv[k] = B[qq].vel[k];
         B[qq].oacc[k] = B[qq].ojerk[k] = 0.0;  // hdyn() zeroes them
       }
-      if (i < n) {
-        S.m[i] = B[qq].m;
-        S.mf[i] = __double2float_rn(B[qq].m);
-      }
+      if (i < n) S.m[i] = B[qq].m;
     }
-    publish<MODE>(S, n, lane, B);
+    publish(S, n, lane, B);
     double t = 0.0, t_pred = -1.0;
-    double dt = EXACT ? MUL(eta, __dsqrt_rn(forces<MODE>(S, n, lane, B)))
-                      : eta * sqrt(forces<MODE>(S, n, lane, B));
+    double dt = MUL(eta, __dsqrt_rn(forces(S, n, lane, B)));
     long long nsteps = 0;
     int st = 0;
     while (t < t_end) {
@@ -319,23 +216,19 @@ __global__ void batch_kernel(const int *__restrict__ order, const int *__restric
         st = 1;  // step budget exhausted
         break;
       }
-      const double tn = EXACT ? ADD(t, dt) : t + dt;
+      const double tn = ADD(t, dt);
       if (tn != t_pred) {  // predict_loworder_all
-        const double h = EXACT ? SUB(tn, t) : tn - t;
-        const double h3 = EXACT ? DIV(h, 3.0) : h / 3.0;
-        const double h2 = EXACT ? DIV(h, 2.0) : h * 0.5;
+        const double h = SUB(tn, t);
+        const double h3 = DIV(h, 3.0);
+        const double h2 = MUL(h, 0.5);  // halving rounds as the division by 2
 #pragma unroll
         for (int qq = 0; qq < 2; qq++) {
+          if (qq >= nq) break;
 #pragma unroll
           for (int k = 0; k < 3; k++) {
             const double oj = B[qq].ojerk[k], oa = B[qq].oacc[k];
-            if (EXACT) {
-              B[qq].pp[k] = ADD(MUL(ADD(MUL(ADD(MUL(oj, h3), oa), h2), B[qq].vel[k]), h), B[qq].pos[k]);
-              B[qq].pv[k] = ADD(MUL(ADD(MUL(oj, h2), oa), h), B[qq].vel[k]);
-            } else {
-              B[qq].pp[k] = fma(fma(fma(oj, h3, oa), h2, B[qq].vel[k]), h, B[qq].pos[k]);
-              B[qq].pv[k] = fma(fma(oj, h2, oa), h, B[qq].vel[k]);
-            }
+            B[qq].pp[k] = ADD(MUL(ADD(MUL(ADD(MUL(oj, h3), oa), h2), B[qq].vel[k]), h), B[qq].pos[k]);
+            B[qq].pv[k] = ADD(MUL(ADD(MUL(oj, h2), oa), h), B[qq].vel[k]);
           }
         }
         t_pred = tn;
@@ -350,78 +243,51 @@ __global__ void batch_kernel(const int *__restrict__ order, const int *__restric
       double new_dt = dt, end_dt = dt;
       for (int it = 0; it <= n_iter; it++) {
         const double prev = new_dt;
-        publish<MODE>(S, n, lane, B);
-        const double ts2 = forces<MODE>(S, n, lane, B);
-        end_dt = EXACT ? MUL(eta, __dsqrt_rn(ts2)) : eta * sqrt(ts2);
+        publish(S, n, lane, B);
+        const double ts2 = forces(S, n, lane, B);
+        end_dt = MUL(eta, __dsqrt_rn(ts2));
         if (it < n_iter) {
-          if (EXACT) {
-            new_dt = MUL(0.5, ADD(dt, end_dt));
-            new_dt = ADD(dt, MUL(MUL(0.5, SUB(end_dt, dt)), DIV(new_dt, prev)));
-          } else {
-            new_dt = 0.5 * (dt + end_dt);
-            new_dt = dt + 0.5 * (end_dt - dt) * (new_dt / prev);
-          }
+          new_dt = MUL(0.5, ADD(dt, end_dt));
+          new_dt = ADD(dt, MUL(MUL(0.5, SUB(end_dt, dt)), DIV(new_dt, prev)));
         }
         const bool cj = new_dt != prev;
         double tau = 0, tau2 = 0, tau3 = 0, theta = 0, inv_theta = 0;
         if (cj) {
-          if (EXACT) {
-            const double dt_off = SUB(new_dt, MUL(0.5, prev));
-            theta = MUL(0.5, prev);
-            tau = DIV(dt_off, theta);
-            inv_theta = DIV(1.0, theta);
-            tau2 = MUL(tau, tau);
-            tau3 = MUL(tau2, tau);
-          } else {
-            theta = 0.5 * prev;
-            tau = (new_dt - theta) / theta;
-            inv_theta = 1.0 / theta;
-            tau2 = tau * tau;
-            tau3 = tau2 * tau;
-          }
+          const double dt_off = SUB(new_dt, MUL(0.5, prev));
+          theta = MUL(0.5, prev);
+          tau = DIV(dt_off, theta);
+          inv_theta = DIV(1.0, theta);
+          tau2 = MUL(tau, tau);
+          tau3 = MUL(tau2, tau);
         }
-        const double nd2 = EXACT ? MUL(new_dt, new_dt) : new_dt * new_dt;
+        const double nd2 = MUL(new_dt, new_dt);
 #pragma unroll
         for (int qq = 0; qq < 2; qq++) {
+          if (qq >= nq) break;  // an FP64 instruction costs the same without bodies
           Body &b = B[qq];
 #pragma unroll
           for (int k = 0; k < 3; k++) {
             if (cj) {  // correct_acc_and_jerk(new_dt, prev)
               const double pa = b.acc[k], pj = b.jerk[k], oa = b.oacc[k], oj = b.ojerk[k];
-              if (EXACT) {
-                const double c1 = ADD(SUB(2.0, MUL(3.0, tau)), tau3);
-                const double c2 = SUB(ADD(2.0, MUL(3.0, tau)), tau3);
-                const double c3 = ADD(SUB(SUB(1.0, tau), tau2), tau3);
-                const double c4 = ADD(ADD(SUB(-1.0, tau), tau2), tau3);
-                b.acc[k] = MUL(0.25, ADD(ADD(ADD(MUL(oa, c1), MUL(pa, c2)), MUL(MUL(oj, theta), c3)),
-                                         MUL(MUL(pj, theta), c4)));
-                const double e1 = ADD(-1.0, tau2), e2 = SUB(1.0, tau2);
-                const double e3 = ADD(SUB(-1.0, MUL(2.0, tau)), MUL(3.0, tau2));
-                const double e4 = ADD(ADD(-1.0, MUL(2.0, tau)), MUL(3.0, tau2));
-                b.jerk[k] = MUL(0.25, ADD(ADD(ADD(MUL(MUL(MUL(oa, inv_theta), 3.0), e1),
-                                                  MUL(MUL(MUL(pa, inv_theta), 3.0), e2)),
-                                              MUL(oj, e3)),
-                                          MUL(pj, e4)));
-              } else {
-                b.acc[k] = 0.25 * (oa * (2 - 3 * tau + tau3) + pa * (2 + 3 * tau - tau3) +
-                                   oj * theta * (1 - tau - tau2 + tau3) +
-                                   pj * theta * (-1 - tau + tau2 + tau3));
-                b.jerk[k] = 0.25 * (oa * inv_theta * 3 * (-1 + tau2) + pa * inv_theta * 3 * (1 - tau2) +
-                                    oj * (-1 - 2 * tau + 3 * tau2) + pj * (-1 + 2 * tau + 3 * tau2));
-              }
+              const double c1 = ADD(SUB(2.0, MUL(3.0, tau)), tau3);
+              const double c2 = SUB(ADD(2.0, MUL(3.0, tau)), tau3);
+              const double c3 = ADD(SUB(SUB(1.0, tau), tau2), tau3);
+              const double c4 = ADD(ADD(SUB(-1.0, tau), tau2), tau3);
+              b.acc[k] = MUL(0.25, ADD(ADD(ADD(MUL(oa, c1), MUL(pa, c2)), MUL(MUL(oj, theta), c3)),
+                                       MUL(MUL(pj, theta), c4)));
+              const double e1 = ADD(-1.0, tau2), e2 = SUB(1.0, tau2);
+              const double e3 = ADD(SUB(-1.0, MUL(2.0, tau)), MUL(3.0, tau2));
+              const double e4 = ADD(ADD(-1.0, MUL(2.0, tau)), MUL(3.0, tau2));
+              b.jerk[k] = MUL(0.25, ADD(ADD(ADD(MUL(MUL(MUL(oa, inv_theta), 3.0), e1),
+                                                MUL(MUL(MUL(pa, inv_theta), 3.0), e2)),
+                                            MUL(oj, e3)),
+                                        MUL(pj, e4)));
             }
             // correct_pos_and_vel(new_dt)
-            if (EXACT) {
-              b.pv[k] = SUB(ADD(b.vel[k], DIV(MUL(new_dt, ADD(b.acc[k], b.oacc[k])), 2.0)),
-                            DIV(MUL(nd2, SUB(b.jerk[k], b.ojerk[k])), 12.0));
-              b.pp[k] = SUB(ADD(b.pos[k], DIV(MUL(new_dt, ADD(b.pv[k], b.vel[k])), 2.0)),
-                            DIV(MUL(nd2, SUB(b.acc[k], b.oacc[k])), 12.0));
-            } else {
-              b.pv[k] = b.vel[k] + new_dt * (b.acc[k] + b.oacc[k]) * 0.5 -
-                        nd2 * (b.jerk[k] - b.ojerk[k]) * (1.0 / 12.0);
-              b.pp[k] = b.pos[k] + new_dt * (b.pv[k] + b.vel[k]) * 0.5 -
-                        nd2 * (b.acc[k] - b.oacc[k]) * (1.0 / 12.0);
-            }
+            b.pv[k] = SUB(ADD(b.vel[k], MUL(MUL(new_dt, ADD(b.acc[k], b.oacc[k])), 0.5)),
+                          g6_div_const(MUL(nd2, SUB(b.jerk[k], b.ojerk[k])), 12.0, 1.0 / 12.0));
+            b.pp[k] = SUB(ADD(b.pos[k], MUL(MUL(new_dt, ADD(b.pv[k], b.vel[k])), 0.5)),
+                          g6_div_const(MUL(nd2, SUB(b.acc[k], b.oacc[k])), 12.0, 1.0 / 12.0));
           }
         }
       }
@@ -433,7 +299,7 @@ __global__ void batch_kernel(const int *__restrict__ order, const int *__restric
           B[qq].vel[k] = B[qq].pv[k];
         }
       dt = end_dt;
-      t = EXACT ? ADD(t, new_dt) : t + new_dt;
+      t = ADD(t, new_dt);
       nsteps++;
     }
 #pragma unroll
@@ -480,8 +346,27 @@ __global__ void batch_kernel(const int *__restrict__ order, const int *__restric
 // orc_smalln_unpert.  FAST (FP64 pair terms) and SPLIT (FP32 pair terms)
 // modes; all tree decisions are taken redundantly by every lane of the
 // warp from shared data, so they are warp-uniform.
-constexpr int NB = 8;             // binaries per system at most
-constexpr int WARPS_MAX_UNP = 4;  // shared memory per warp is larger here
+//
+// What bounds it: FP64 issues at 2 lanes per SM and cycle, half a lane per
+// scheduler, so an FP64 instruction holds a warp's scheduler for 64 cycles
+// however few lanes need it.  So the per-body work is laid out by component:
+// lane l holds components l, l + 32, ... of the system's 3n (a 3-body system
+// has 9 lanes at work in one pass, where a lane per body took three passes of
+// three lanes, and two more for bodies 33 .. 64 that were not there); the
+// corrector's eight coefficients are evaluated by eight lanes at once;
+// divisions and square roots of step quantities are a MUFU seed and one
+// third-order step; and comparisons of non-negative values are integer
+// compares.  A lone warp is bound by instruction latency (5.7 cycles per
+// instruction of 32,000 a step at n = 52), so the split mode's pair loop reads
+// a body in three or four 16-byte loads and evaluates two pairs per packed
+// f32x2 instruction.
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+constexpr int NB = 8;  // binaries per system at most
 
 struct BinRec {
   int li, lj, full, pad;
@@ -494,32 +379,60 @@ struct BinRec {
 struct UnpParams {
   double dt_crit, r2_crit, gamma2, gamma_inv3;
   int allow_full;
+  int on;  // 0: no binaries are made
 };
 
-struct UnpSmem {
-  union {  // leaves for the force loop; node positions/velocities for the tree logic
-    struct {
-      double pp[MAXN][3];
-      double pv[MAXN][3];
-    } d;
-    struct {
-      float ph[MAXN][3];
-      float pl[MAXN][3];
-      float vf[MAXN][3];
-    } f;
-  } A;
+struct alignas(16) UnpSmem {
+  // leaves for the force loop; in split mode d holds the nodes for the tree
+  struct {
+    double4_16 pp[MAXN];  // x, y, z, leaf mass
+    double4_16 pv[MAXN];  // velocity, mass of the leaf's node
+  } d;
+  struct {
+    float4 hi[MAXN];  // x, y, z (high words), leaf mass
+    float4 lo[MAXN];  // x, y, z (low words), -
+    float4 vf[MAXN];  // velocity, mass of the leaf's node
+    float4 cv[MAXN];  // velocity of the leaf's node
+  } f;
+  double4_16 cv[MAXN];  // fast mode: velocity of the leaf's node
   double la[MAXN][3], lj[MAXN][3];  // leaf forces, then node accelerations
-  double m[MAXN];                    // leaf masses
-  float mf[MAXN];
   double nm[MAXN];                   // node masses (at node slots)
-  float nmf[MAXN];                   // the same in FP32 (split mode's step criterion)
-  double cv[MAXN][3];                // node predicted velocities (at node slots)
-  float cvf[MAXN][3];
+  double kr[NB][6];                  // binaries' relative position and velocity
   int nd[MAXN];                      // node (leader slot) of every leaf slot
+  int bi[MAXN];                      // binary of a node slot, -1: a single leaf
   BinRec bin[NB];
   int nb;
 };
 
+__device__ __forceinline__ bool mid_positive(double x) {  // 2^-300 <= x < 2^300
+  return (unsigned)__double2hiint(x) - (723u << 20) < (600u << 20);
+}
+// 1/x: FP64 MUFU seed (relative error below 2^-19) and one third-order step,
+// x (1 + h + h^2) with h = 1 - x y; the division outside the seed's range.
+__device__ __forceinline__ double rcp64(double x) {
+  if (!mid_range(x)) return 1.0 / x;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = __fma_rn(-x, y, 1.0);
+  return __fma_rn(y, __fma_rn(h, h, h), y);
+}
+// 1/sqrt(x) the same way (y + y h (1/2 + 3/8 h), h = 1 - x y^2); for x
+// normal, in the pair loop (where the FP32 seed of before needed x in the FP32
+// range), and for any x.
+__device__ __forceinline__ double rsqrt64_normal(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = __fma_rn(-(x * y), y, 1.0);
+  return __fma_rn(h * y, __fma_rn(0.375, h, 0.5), y);
+}
+__device__ __forceinline__ double rsqrt64(double x) {
+  return mid_positive(x) ? rsqrt64_normal(x) : 1.0 / sqrt(x);
+}
+__device__ __forceinline__ double sqrt64(double x) {
+  if (!mid_positive(x)) return sqrt(x);
+  const double y = rsqrt64(x), q = x * y;
+  return __fma_rn(__fma_rn(-q, q, x), 0.5 * y, q);
+}
 // Stumpff functions C(z) = (1 - cos sqrt z) / z, S(z) = (sqrt z - sin sqrt z)
 // / z^(3/2) (cosh, sinh for z < 0), both from one sincos (one exp) of
 // sqrt(|z|) / 2: 1 - cos s = 2 sin^2(s/2) (no cancellation), sin s = 2
@@ -528,16 +441,18 @@ struct UnpSmem {
 // Newton step rather than two.
 __device__ __forceinline__ void kst_cs(double z, double &C, double &S) {
   if (z > 0.1) {
-    const double s = sqrt(z);
+    const double s = sqrt64(z);
     double sh, ch;
     sincos(0.5 * s, &sh, &ch);
-    C = 2.0 * sh * sh / z;
-    S = (s - 2.0 * sh * ch) / (s * z);
+    const double i = rcp64(s * z);  // 1 / z^(3/2)
+    C = 2.0 * sh * sh * (s * i);
+    S = (s - 2.0 * sh * ch) * i;
   } else if (z < -0.1) {
-    const double s = sqrt(-z), e = exp(0.5 * s), ei = 1.0 / e;
+    const double s = sqrt64(-z), e = exp(0.5 * s), ei = rcp64(e);
     const double sh = 0.5 * (e - ei), ch = 0.5 * (e + ei);
-    C = 2.0 * sh * sh / -z;
-    S = (2.0 * sh * ch - s) / (s * -z);
+    const double i = rcp64(s * -z);
+    C = 2.0 * sh * sh * (s * i);
+    S = (2.0 * sh * ch - s) * i;
   } else {
     C = 1.0 / 2 +
         z * (-1.0 / 24 +
@@ -564,14 +479,16 @@ __device__ __forceinline__ void kst_cs(double z, double &C, double &S) {
 // orbit), xw + sqrt(mu) (dt - dtw) / rw (dx/dt = sqrt(mu) / r); x grows with
 // dt, so xw then also bounds the root from one side.  The C and S of the
 // step whose correction is below 1e-15 x give the f and g functions.
-__device__ void kep_prop(double mu, const double r0[3], const double v0[3], double dt,
+__device__ __noinline__ void kep_prop(double mu, const double r0[3], const double v0[3], double dt,
                          double r[3], double v[3], double *xw = nullptr, double *dtw = nullptr,
                          double *rw = nullptr) {
-  const double rn = sqrt(r0[0] * r0[0] + r0[1] * r0[1] + r0[2] * r0[2]);
+  const double r2 = r0[0] * r0[0] + r0[1] * r0[1] + r0[2] * r0[2];
+  const double irn = rsqrt64(r2), rn = sqrt64(r2);
   const double v2 = v0[0] * v0[0] + v0[1] * v0[1] + v0[2] * v0[2];
   const double rv = r0[0] * v0[0] + r0[1] * v0[1] + r0[2] * v0[2];
-  const double alpha = 2.0 / rn - v2 / mu, smu = sqrt(mu);
-  const double c1 = rv / smu, c2 = 1.0 - alpha * rn;
+  const double ismu = rsqrt64(mu), smu = sqrt64(mu);
+  const double alpha = 2.0 * irn - v2 * (ismu * ismu);
+  const double c1 = rv * ismu, c2 = 1.0 - alpha * rn;
   if (dt == 0.0) {
     for (int k = 0; k < 3; k++) r[k] = r0[k], v[k] = v0[k];
     return;
@@ -583,14 +500,14 @@ __device__ void kep_prop(double mu, const double r0[3], const double v0[3], doub
   };
   const bool warm = xw && *dtw > 0.0 && dt > 0.0;
   const double inf = __longlong_as_double(0x7ff0000000000000ll);
-  double x0 = alpha > 0.0 ? smu * dt * alpha : smu * dt / rn;  // sign of dt
+  double x0 = alpha > 0.0 ? smu * dt * alpha : smu * dt * irn;  // sign of dt
   double lo, hi;
   if (warm) {
     // The root lies above xw when dt >= dtw (F(xw) <= 0), else in (0, xw).
     // No evaluation before the first Newton step: with hi = +inf, steps from
     // below (F < 0, dF > 0) only move up, until one lands above the root and
     // bounds it.
-    x0 = *xw + smu * (dt - *dtw) / *rw;
+    x0 = *xw + smu * (dt - *dtw) * rcp64(*rw);
     lo = dt >= *dtw ? *xw : 0.0;
     hi = dt >= *dtw ? inf : *xw;
     if (!(x0 > lo && x0 < hi)) x0 = hi < inf ? 0.5 * (lo + hi) : lo + fabs(lo) + 1e-300;
@@ -613,22 +530,24 @@ __device__ void kep_prop(double mu, const double r0[3], const double v0[3], doub
       lo = x;
     else
       hi = x;
-    double xn = x - F / dF;
+    const double newton = F * rcp64(dF);
+    double xn = x - newton;
     if (hi < inf && (!(xn > lo && xn < hi) || fabs(2.0 * F) > fabs(step_old * dF))) {
       step_old = step;
       step = 0.5 * (hi - lo);
       xn = lo + step;
     } else {
       step_old = step;
-      step = F / dF;
+      step = newton;
     }
     if (xn == x) break;
     x = xn;
   }
-  const double f = 1.0 - x * x * C / rn, g = dt - x * x * x * S / smu;
+  const double f = 1.0 - x * x * C * irn, g = dt - x * x * x * S * ismu;
   for (int k = 0; k < 3; k++) r[k] = f * r0[k] + g * v0[k];
-  const double rr = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
-  const double fd = smu / (rr * rn) * (alpha * x * x * x * S - x), gd = 1.0 - x * x * C / rr;
+  const double rr2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+  const double irr = rsqrt64(rr2), rr = sqrt64(rr2);
+  const double fd = smu * (irr * irn) * (alpha * x * x * x * S - x), gd = 1.0 - x * x * C * irr;
   for (int k = 0; k < 3; k++) v[k] = fd * r0[k] + gd * v0[k];
   if (xw && dt > 0.0) {
     *xw = x;
@@ -640,7 +559,7 @@ __device__ void kep_prop(double mu, const double r0[3], const double v0[3], doub
 // Time to the next pericentre (0: not approaching it) and the period (inf
 // unless bound): mean anomaly from the eccentric (hyperbolic) anomaly;
 // Barker's equation near e = 1.
-__device__ int kep_peri(double mu, const double r[3], const double v[3], double *dt_peri,
+__device__ __noinline__ int kep_peri(double mu, const double r[3], const double v[3], double *dt_peri,
                         double *period) {
   const double rn = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
   const double v2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
@@ -675,9 +594,10 @@ __device__ int kep_peri(double mu, const double r[3], const double v[3], double 
   return 1;
 }
 
-__device__ __forceinline__ double dist3(const double a[3], const double b[3]) {
-  const double d0 = a[0] - b[0], d1 = a[1] - b[1], d2 = a[2] - b[2];
-  return sqrt(d0 * d0 + d1 * d1 + d2 * d2);
+// 1 / |a - b|
+__device__ __forceinline__ double idist(const double a[3], const double4_16 &b) {
+  const double d0 = a[0] - b.x, d1 = a[1] - b.y, d2 = a[2] - b.z;
+  return rsqrt64(d0 * d0 + d1 * d1 + d2 * d2);
 }
 
 // The relative state of a binary at time t (frozen when fully unperturbed).
@@ -712,10 +632,10 @@ __device__ __forceinline__ double warp_min(double x) {
 }
 
 // Tidal potential of the other top-level nodes on leaves (xi, xj) around
-// the centre of mass xc (smallN_unpert.cc:17-40); node positions in S.A.d.
+// the centre of mass xc (smallN_unpert.cc:17-40); node positions in S.d.
 // The whole warp calls it (uniform arguments); each lane sums its two node
 // slots (the tree's loops over nodes run at 1/32 of the FP64 work per lane).
-__device__ double tidal_pot(const UnpSmem &S, int n, int lane, int li, int lj, double mi,
+__device__ __noinline__ double tidal_pot(const UnpSmem &S, int n, int lane, int li, int lj, double mi,
                             double mj, const double xi[3], const double xj[3],
                             const double xc[3]) {
   double phi = 0.0;
@@ -723,257 +643,471 @@ __device__ double tidal_pot(const UnpSmem &S, int n, int lane, int li, int lj, d
   for (int q = 0; q < 2; q++) {
     const int k = lane + 32 * q;
     if (k >= n || S.nd[k] != k || k == li || k == lj) continue;
-    phi += S.nm[k] * (-mi / dist3(xi, S.A.d.pp[k]) - mj / dist3(xj, S.A.d.pp[k]) +
-                      (mi + mj) / dist3(xc, S.A.d.pp[k]));
+    phi += S.nm[k] * (-mi * idist(xi, S.d.pp[k]) - mj * idist(xj, S.d.pp[k]) +
+                      (mi + mj) * idist(xc, S.d.pp[k]));
   }
   return warp_sum(phi);
 }
 
-template <int MODE>
-__device__ __forceinline__ void unp_store_leaf(UnpSmem &S, int s, const double x[3],
-                                               const double v[3]) {
+// What every lane keeps of the components c = lane + 32 r of the 3n: body
+// c / 3, coordinate c % 3.  NS slots, a template parameter of all that
+// follows: slots a system does not have would be predicated off, and an FP64
+// instruction costs its time all the same (a 3-body step issued 813 of them
+// with six slots).
+template <int NS>
+struct Comp {
+  double pos[NS], vel[NS], pp[NS], pv[NS], acc[NS], jerk[NS], oacc[NS], ojerk[NS];
+};
+
+#define FOR_COMP(r, c, n)                          \
+  _Pragma("unroll") for (int r = 0; r < NS; r++) \
+    if (const int c = lane + 32 * r; c < 3 * (n))
+
+__device__ __forceinline__ double &elem(double4_16 &v, int k) { return (&v.x)[k]; }
+__device__ __forceinline__ float &elem(float4 &v, int k) { return (&v.x)[k]; }
+
+// One component of a leaf's predicted state, and (TREE) of its node's
+// velocity.
+template <int MODE, bool TREE>
+__device__ __forceinline__ void store_leaf(UnpSmem &S, int s, int k, double x, double v,
+                                           double cv) {
   if (MODE == MODE_SPLIT) {
-    for (int k = 0; k < 3; k++) {
-      const float h = __double2float_rn(x[k]);
-      S.A.f.ph[s][k] = h;
-      S.A.f.pl[s][k] = __double2float_rn(x[k] - (double)h);
-      S.A.f.vf[s][k] = __double2float_rn(v[k]);
-    }
+    const float h = __double2float_rn(x);
+    elem(S.f.hi[s], k) = h;
+    elem(S.f.lo[s], k) = __double2float_rn(x - (double)h);
+    elem(S.f.vf[s], k) = __double2float_rn(v);
+    if (TREE) elem(S.f.cv[s], k) = __double2float_rn(cv);
   } else {
-    for (int k = 0; k < 3; k++) S.A.d.pp[s][k] = x[k], S.A.d.pv[s][k] = v[k];
+    elem(S.d.pp[s], k) = x;
+    elem(S.d.pv[s], k) = v;
+    if (TREE) elem(S.cv[s], k) = cv;
   }
 }
 
-// Resolved forces on the top-level nodes from the predicted states in B:
-// returns the system's min step^2 (warp-uniform) and the node pair setting it.
+// The masses beside the leaves (their own and their node's), and the binary
+// of every node slot: after the tree changed.
 template <int MODE>
-__device__ double unp_forces(UnpSmem &S, int n, int lane, Body B[2], double t, int *imin,
-                             int *jmin) {
+__device__ void tree_masses(UnpSmem &S, int n, int lane) {
   __syncwarp();
-  // publish: node slots of this lane (singles: their leaf; leaders: both leaves)
+  for (int s = lane; s < n; s += 32) {
+    int b = -1;
+    for (int q = 0; q < S.nb; q++)
+      if (S.bin[q].li == s) b = q;
+    S.bi[s] = b;
+    const double nm = S.nm[S.nd[s]];
+    if (MODE == MODE_SPLIT)
+      S.f.vf[s].w = __double2float_rn(nm);
+    else
+      S.d.pv[s].w = nm;
+  }
+  __syncwarp();
+}
+
+// MODE_SPLIT pair loop for the lane's leaves i = lane (and lane + 32): sums
+// over all leaves of other nodes, the smallest step^2 and its node pair, two
+// pairs per packed instruction: both leaves of the lane with one j (NQ = 2),
+// or one leaf with two j, whose terms are then added one after the other, so
+// the sums run over j in order either way.  Pairs within one node (the leaf
+// itself among them) are evaluated with rinv = 0, so the loop does not
+// diverge.  The pair that sets the step is the one with the largest max(2 M /
+// r^3, v^2 / r^2); its step^2 is then taken from the quotients (approximate
+// division).  FP32 unless a pair is closer than 1e-9 (d^2 < 1e-18): there m /
+// d^3 times a relative velocity ~ sqrt(M / d) can leave the FP32 range, so
+// such (rare) pairs are left out of the loop and evaluated in FP64 after it.
+// TREE false: no binaries, every leaf is its node.
+struct Leaf {
+  float4 h, l, v, c;  // position words (mass), velocity (node mass), node velocity
+  int node;
+};
+template <bool TREE>
+__device__ __forceinline__ Leaf get_leaf(const UnpSmem &S, int j) {
+  Leaf b;
+  b.h = S.f.hi[j];
+  b.l = S.f.lo[j];
+  b.v = S.f.vf[j];
+  b.c = TREE ? S.f.cv[j] : b.v;
+  b.node = TREE ? S.nd[j] : j;
+  return b;
+}
+struct Pair2 {  // two leaves, one per half
+  f2x hx, hy, hz, lx, ly, lz, vx, vy, vz, cx, cy, cz, m, nm;
+};
+__device__ __forceinline__ Pair2 pack_leaves(const Leaf &a, const Leaf &b) {
+  Pair2 p;
+  p.hx = f2_pack(a.h.x, b.h.x), p.hy = f2_pack(a.h.y, b.h.y), p.hz = f2_pack(a.h.z, b.h.z);
+  p.lx = f2_pack(a.l.x, b.l.x), p.ly = f2_pack(a.l.y, b.l.y), p.lz = f2_pack(a.l.z, b.l.z);
+  p.vx = f2_pack(a.v.x, b.v.x), p.vy = f2_pack(a.v.y, b.v.y), p.vz = f2_pack(a.v.z, b.v.z);
+  p.cx = f2_pack(a.c.x, b.c.x), p.cy = f2_pack(a.c.y, b.c.y), p.cz = f2_pack(a.c.z, b.c.z);
+  p.m = f2_pack(a.h.w, b.h.w), p.nm = f2_pack(a.v.w, b.v.w);
+  return p;
+}
+// The terms of the pairs (i, j) of both halves: f dx is the acceleration, f u
+// the jerk, w the step's measure; near is set where a pair is too close.
+template <bool TREE>
+__device__ __forceinline__ void pair_terms(const Pair2 &i, const Pair2 &j, bool same0, bool same1,
+                                           f2x &f, f2x dx[3], f2x u[3], float &w0, float &w1,
+                                           bool &near0, bool &near1) {
+  dx[0] = f2_add(f2_sub(j.hx, i.hx), f2_sub(j.lx, i.lx));
+  dx[1] = f2_add(f2_sub(j.hy, i.hy), f2_sub(j.ly, i.ly));
+  dx[2] = f2_add(f2_sub(j.hz, i.hz), f2_sub(j.lz, i.lz));
+  const f2x dv[3] = {f2_sub(j.vx, i.vx), f2_sub(j.vy, i.vy), f2_sub(j.vz, i.vz)};
+  const f2x d2 = f2_fma(dx[2], dx[2], f2_fma(dx[1], dx[1], f2_mul(dx[0], dx[0])));
+  f2x v2;
+  if (TREE) {
+    const f2x c0 = f2_sub(j.cx, i.cx), c1 = f2_sub(j.cy, i.cy), c2 = f2_sub(j.cz, i.cz);
+    v2 = f2_fma(c2, c2, f2_fma(c1, c1, f2_mul(c0, c0)));
+  } else {
+    v2 = f2_fma(dv[2], dv[2], f2_fma(dv[1], dv[1], f2_mul(dv[0], dv[0])));
+  }
+  float a, b;
+  f2_unpack(d2, a, b);
+  const bool n0 = !(a >= 1e-18f), n1 = !(b >= 1e-18f);
+  near0 |= n0 && !same0;
+  near1 |= n1 && !same1;
+  const f2x rinv = f2_pack(same0 || n0 ? 0.f : rsqrt_approx(a), same1 || n1 ? 0.f : rsqrt_approx(b));
+  const f2x rinv2 = f2_mul(rinv, rinv);
+  f = f2_mul(f2_mul(j.m, rinv), rinv2);
+  const f2x xv = f2_fma(dx[2], dv[2], f2_fma(dx[1], dv[1], f2_mul(dx[0], dv[0])));
+  const f2x a3 = f2_mul(f2_mul(f2_dup(-3.0f), xv), rinv2);
 #pragma unroll
-  for (int q = 0; q < 2; q++) {
-    const int s = lane + 32 * q;
-    if (s >= n || S.nd[s] != s) continue;
-    for (int k = 0; k < 3; k++) {
-      S.cv[s][k] = B[q].pv[k];
-      S.cvf[s][k] = __double2float_rn(B[q].pv[k]);
-    }
-    S.nm[s] = B[q].m;
-    S.nmf[s] = __double2float_rn(B[q].m);
-    int qb = -1;
-    for (int b = 0; b < S.nb; b++)
-      if (S.bin[b].li == s) qb = b;
-    if (qb < 0) {
-      unp_store_leaf<MODE>(S, s, B[q].pp, B[q].pv);
-    } else {
-      BinRec &bb = S.bin[qb];  // this lane's binary (its leader slot is the lane's)
-      double r[3], v[3], xi[3], vi[3], xj[3], vj[3];
-      bin_rel_warm(bb, t, r, v);
-      const double M = bb.mi + bb.mj, fi = bb.mj / M, fj = bb.mi / M;
+  for (int k = 0; k < 3; k++) u[k] = f2_fma(a3, dx[k], dv[k]);
+  const f2x M = f2_add(i.nm, j.nm);
+  const f2x wm = f2_mul(f2_mul(f2_add(M, M), rinv), rinv2), wv = f2_mul(v2, rinv2);
+  w0 = fmaxf(f2_lo(wm), f2_lo(wv));
+  w1 = fmaxf(f2_hi(wm), f2_hi(wv));
+}
+
+template <bool TREE, int NQ>
+__device__ __forceinline__ void pairs_split(UnpSmem &S, int n, int lane, double la[2][3],
+                                            double lj[2][3], float tsq[2], int pq[2]) {
+  float a[NQ][3], jk[NQ][3], wb[NQ];
+  int jb[NQ], ni[NQ];
+  bool near[2] = {false, false};
+#pragma unroll
+  for (int q = 0; q < NQ; q++) {
+    wb[q] = 0.f;
+    jb[q] = -1;
+    ni[q] = TREE ? S.nd[min(lane + 32 * q, n - 1)] : lane + 32 * q;
+  }
+  f2x f, dx[3], u[3];
+  float w0, w1;
+  if (NQ == 2) {
+    const Pair2 I = pack_leaves(get_leaf<TREE>(S, lane), get_leaf<TREE>(S, min(lane + 32, n - 1)));
+    f2x A[3] = {0ull, 0ull, 0ull}, J[3] = {0ull, 0ull, 0ull};
+#pragma unroll 1
+    for (int j = 0; j < n; j++) {
+      const Leaf b = get_leaf<TREE>(S, j);
+      pair_terms<TREE>(I, pack_leaves(b, b), b.node == ni[0], b.node == ni[NQ - 1], f, dx, u, w0,
+                       w1, near[0], near[1]);
+#pragma unroll
       for (int k = 0; k < 3; k++) {
-        xi[k] = B[q].pp[k] - fi * r[k];
-        vi[k] = B[q].pv[k] - fi * v[k];
-        xj[k] = B[q].pp[k] + fj * r[k];
-        vj[k] = B[q].pv[k] + fj * v[k];
+        A[k] = f2_fma(f, dx[k], A[k]);
+        J[k] = f2_fma(f, u[k], J[k]);
       }
-      unp_store_leaf<MODE>(S, bb.li, xi, vi);
-      unp_store_leaf<MODE>(S, bb.lj, xj, vj);
+      if (w0 > wb[0]) wb[0] = w0, jb[0] = j;
+      if (w1 > wb[NQ - 1]) wb[NQ - 1] = w1, jb[NQ - 1] = j;
     }
-  }
-  __syncwarp();
-  double ts2 = __longlong_as_double(0x7ff0000000000000ll);
-  int pmin = 0x7fffffff;  // node pair id a * MAXN + b (a < b) of ts2
-  double la[2][3], lj[2][3];
 #pragma unroll
-  for (int q = 0; q < 2; q++) {
+    for (int k = 0; k < 3; k++) {
+      f2_unpack(A[k], a[0][k], a[NQ - 1][k]);
+      f2_unpack(J[k], jk[0][k], jk[NQ - 1][k]);
+    }
+  } else {
+    const Leaf me = get_leaf<TREE>(S, min(lane, n - 1));
+    const Pair2 I = pack_leaves(me, me);
+#pragma unroll
+    for (int k = 0; k < 3; k++) a[0][k] = jk[0][k] = 0.f;
+#pragma unroll 1
+    for (int j = 0; j < n; j += 2) {
+      const bool two = j + 1 < n;
+      const Leaf b = get_leaf<TREE>(S, j), c = get_leaf<TREE>(S, two ? j + 1 : j);
+      pair_terms<TREE>(I, pack_leaves(b, c), b.node == ni[0], !two || c.node == ni[0], f, dx, u,
+                       w0, w1, near[0], near[1]);
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        a[0][k] = fmaf(f2_hi(f), f2_hi(dx[k]), fmaf(f2_lo(f), f2_lo(dx[k]), a[0][k]));
+        jk[0][k] = fmaf(f2_hi(f), f2_hi(u[k]), fmaf(f2_lo(f), f2_lo(u[k]), jk[0][k]));
+      }
+      if (w0 > wb[0]) wb[0] = w0, jb[0] = j;
+      if (w1 > wb[0]) wb[0] = w1, jb[0] = j + 1;
+    }
+    near[0] |= near[1];
+  }
+#pragma unroll
+  for (int q = 0; q < NQ; q++) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) la[q][k] = (double)a[q][k], lj[q][k] = (double)jk[q][k];
     const int i = lane + 32 * q;
-    for (int k = 0; k < 3; k++) la[q][k] = lj[q][k] = 0.0;
+    tsq[q] = __int_as_float(0x7f800000);
+    pq[q] = 0x7fffffff;
     if (i >= n) continue;
-    const int ni = S.nd[i];
-    if (MODE == MODE_SPLIT) {
-      // FP32 throughout the loop (FP64 runs at 1/64 of the FP32 rate): the
-      // pairs within one node (the leaf itself, its binary companion) are
-      // evaluated with their terms masked to zero and their step to +inf,
-      // so the loop does not diverge; the smallest step and its node pair
-      // are kept in FP32 and merged into the FP64 minimum afterwards.
-      float a[3] = {0.f, 0.f, 0.f}, jk[3] = {0.f, 0.f, 0.f};
-      float tsq = __int_as_float(0x7f800000);
-      int pq = 0x7fffffff;
+    const Leaf me = get_leaf<TREE>(S, i);
+    if (jb[q] >= 0) {
+      const Leaf b = get_leaf<TREE>(S, jb[q]);
+      const float d0 = __fadd_rn(__fsub_rn(b.h.x, me.h.x), __fsub_rn(b.l.x, me.l.x));
+      const float d1 = __fadd_rn(__fsub_rn(b.h.y, me.h.y), __fsub_rn(b.l.y, me.l.y));
+      const float d2 = __fadd_rn(__fsub_rn(b.h.z, me.h.z), __fsub_rn(b.l.z, me.l.z));
+      const float c0 = b.c.x - me.c.x, c1 = b.c.y - me.c.y, c2 = b.c.z - me.c.z;
+      const float dd = fmaf(d2, d2, fmaf(d1, d1, d0 * d0));
+      const float v2 = fmaf(c2, c2, fmaf(c1, c1, c0 * c0));
+      tsq[q] = fminf(__fdividef(0.5f * dd * (dd * rsqrt_approx(dd)), me.v.w + b.v.w),
+                     __fdividef(dd, v2));
+      pq[q] = ni[q] < b.node ? ni[q] * MAXN + b.node : b.node * MAXN + ni[q];
+    }
+    if (near[q]) {  // pairs too close for FP32: FP64
       for (int j = 0; j < n; j++) {
-        const int nj = S.nd[j];
-        const bool same = nj == ni;
-        float dx[3], dv[3], dc[3];
+        const Leaf b = get_leaf<TREE>(S, j);
+        if (b.node == ni[q]) continue;
+        const float e0 = __fadd_rn(__fsub_rn(b.h.x, me.h.x), __fsub_rn(b.l.x, me.l.x));
+        const float e1 = __fadd_rn(__fsub_rn(b.h.y, me.h.y), __fsub_rn(b.l.y, me.l.y));
+        const float e2 = __fadd_rn(__fsub_rn(b.h.z, me.h.z), __fsub_rn(b.l.z, me.l.z));
+        if (fmaf(e2, e2, fmaf(e1, e1, e0 * e0)) >= 1e-18f) continue;
+        const float c0 = b.c.x - me.c.x, c1 = b.c.y - me.c.y, c2 = b.c.z - me.c.z;
+        const double v2 = (double)fmaf(c2, c2, fmaf(c1, c1, c0 * c0));
+        const double X[3] = {(double)e0, (double)e1, (double)e2};
+        const double U[3] = {(double)(b.v.x - me.v.x), (double)(b.v.y - me.v.y),
+                             (double)(b.v.z - me.v.z)};
+        const double dd2 = X[0] * X[0] + X[1] * X[1] + X[2] * X[2];
+        const double d = sqrt(dd2), ri2 = 1.0 / dd2, fd = S.d.pp[j].w * ri2 / d;
+        const double a3 = -3.0 * (X[0] * U[0] + X[1] * U[1] + X[2] * U[2]) * ri2;
         for (int k = 0; k < 3; k++) {
-          dx[k] = __fadd_rn(__fsub_rn(S.A.f.ph[j][k], S.A.f.ph[i][k]),
-                            __fsub_rn(S.A.f.pl[j][k], S.A.f.pl[i][k]));
-          dv[k] = S.A.f.vf[j][k] - S.A.f.vf[i][k];
-          dc[k] = S.cvf[nj][k] - S.cvf[ni][k];
+          la[q][k] += fd * X[k];
+          lj[q][k] += fd * (a3 * X[k] + U[k]);
         }
-        const float d2 = fmaf(dx[2], dx[2], fmaf(dx[1], dx[1], dx[0] * dx[0]));
-        const float v2 = fmaf(dc[2], dc[2], fmaf(dc[1], dc[1], dc[0] * dc[0]));
-        const float mt = S.nmf[ni] + S.nmf[nj];
-        float ts;
-        if (same || d2 >= 1e-18f) {
-          const float rinv = same ? 0.f : rsqrt_approx(d2);
-          const float rinv2 = rinv * rinv;
-          const float f = S.mf[j] * rinv * rinv2;
-          const float xv = fmaf(dx[2], dv[2], fmaf(dx[1], dv[1], dx[0] * dv[0]));
-          const float a3 = -3.0f * xv * rinv2;
-          for (int k = 0; k < 3; k++) {
-            a[k] = fmaf(f, dx[k], a[k]);
-            jk[k] = fmaf(f, fmaf(a3, dx[k], dv[k]), jk[k]);
-          }
-          ts = same ? __int_as_float(0x7f800000)
-                    : fminf(__fdividef(0.5f * d2 * (d2 * rinv), mt), __fdividef(d2, v2));
-        } else {  // too close for FP32: FP64
-          double X[3], W[3];
-          for (int k = 0; k < 3; k++) X[k] = (double)dx[k], W[k] = (double)dv[k];
-          const double dd2 = X[0] * X[0] + X[1] * X[1] + X[2] * X[2];
-          const double d = sqrt(dd2), ri2 = 1.0 / dd2, fd = S.m[j] * ri2 / d;
-          const double a3 = -3.0 * (X[0] * W[0] + X[1] * W[1] + X[2] * W[2]) * ri2;
-          for (int k = 0; k < 3; k++) {
-            la[q][k] += fd * X[k];
-            lj[q][k] += fd * (a3 * X[k] + W[k]);
-          }
-          ts = (float)fmin(0.5 * dd2 * d / (double)mt, dd2 / (double)v2);
-        }
-        const int pid = ni < nj ? ni * MAXN + nj : nj * MAXN + ni;
-        if (ts < tsq || (ts == tsq && pid < pq)) {
-          tsq = ts;
-          pq = pid;
-        }
+        const float ts =
+            (float)fmin(0.5 * dd2 * d / (double)(me.v.w + b.v.w), dd2 / v2);
+        const int pid = ni[q] < b.node ? ni[q] * MAXN + b.node : b.node * MAXN + ni[q];
+        if (ts < tsq[q] || (ts == tsq[q] && pid < pq[q])) tsq[q] = ts, pq[q] = pid;
       }
-      if ((double)tsq < ts2 || ((double)tsq == ts2 && pq < pmin)) {
-        ts2 = (double)tsq;
-        pmin = pq;
+    }
+  }
+}
+
+// MODE_FAST pair loop: FP64, with the largest 1 / step^2 = max(2 M / r^3,
+// v^2 / r^2) in the place of the smallest step^2 (no divisions).  The pairs of
+// one node are masked (rinv = 0).  Bound by FP64 issue: about 40 instructions
+// per pair at 64 cycles (52 bodies: 150 us per evaluation, 240 before).
+template <bool TREE, int NQ>
+__device__ __forceinline__ void pairs_fast(UnpSmem &S, int n, int lane, double la[2][3],
+                                           double lj[2][3], double &wmax, int &pmin) {
+  double4_16 X[NQ], V[NQ], C[NQ];
+  int ni[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; q++) {
+    const int i = min(lane + 32 * q, n - 1);
+    X[q] = S.d.pp[i];
+    V[q] = S.d.pv[i];
+    if (TREE) C[q] = S.cv[i];
+    ni[q] = TREE ? S.nd[i] : i;
+#pragma unroll
+    for (int k = 0; k < 3; k++) la[q][k] = lj[q][k] = 0.0;
+  }
+  constexpr int UNR = NQ == 2 ? 1 : 2;
+#pragma unroll UNR
+  for (int j = 0; j < n; j++) {
+    const int nj = TREE ? S.nd[j] : j;
+    const double4_16 Y = S.d.pp[j], U = S.d.pv[j];
+    double4_16 D;
+    if (TREE) D = S.cv[j];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+      const bool same = nj == ni[q];
+      const double dx = Y.x - X[q].x, dy = Y.y - X[q].y, dz = Y.z - X[q].z;
+      const double du = U.x - V[q].x, dv = U.y - V[q].y, dw = U.z - V[q].z;
+      const double d2 = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
+      const double rinv = same ? 0.0 : rsqrt64_normal(d2);
+      const double rinv2 = rinv * rinv, rinv3 = rinv * rinv2;
+      const double f = Y.w * rinv3;
+      const double a3 = -3.0 * __fma_rn(dz, dw, __fma_rn(dy, dv, dx * du)) * rinv2;
+      la[q][0] = __fma_rn(f, dx, la[q][0]);
+      la[q][1] = __fma_rn(f, dy, la[q][1]);
+      la[q][2] = __fma_rn(f, dz, la[q][2]);
+      lj[q][0] = __fma_rn(f, __fma_rn(a3, dx, du), lj[q][0]);
+      lj[q][1] = __fma_rn(f, __fma_rn(a3, dy, dv), lj[q][1]);
+      lj[q][2] = __fma_rn(f, __fma_rn(a3, dz, dw), lj[q][2]);
+      double c0 = du, c1 = dv, c2 = dw;
+      if (TREE) c0 = D.x - C[q].x, c1 = D.y - C[q].y, c2 = D.z - C[q].z;
+      const double v2 = __fma_rn(c2, c2, __fma_rn(c1, c1, c0 * c0));
+      const double w1 = (V[q].w + U.w) * (rinv3 + rinv3), w2 = v2 * rinv2;
+      // both are >= 0 (0 when masked): integer compares
+      const long long b1 = __double_as_longlong(w1), b2 = __double_as_longlong(w2);
+      const long long bw = b1 > b2 ? b1 : b2, b0 = __double_as_longlong(wmax);
+      const int pid = ni[q] < nj ? ni[q] * MAXN + nj : nj * MAXN + ni[q];
+      if (!same && (bw > b0 || (bw == b0 && pid < pmin))) {
+        wmax = __longlong_as_double(bw);
+        pmin = pid;
       }
-      for (int k = 0; k < 3; k++) la[q][k] += (double)a[k], lj[q][k] += (double)jk[k];
-    } else {
-      for (int j = 0; j < n; j++) {
-        const int nj = S.nd[j];
-        if (nj == ni) continue;
-        double dx[3], dv[3], dc[3];
-        for (int k = 0; k < 3; k++) {
-          dx[k] = S.A.d.pp[j][k] - S.A.d.pp[i][k];
-          dv[k] = S.A.d.pv[j][k] - S.A.d.pv[i][k];
-          dc[k] = S.cv[nj][k] - S.cv[ni][k];
-        }
-        const double d2 = dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2];
-        const double rinv = rsqrt64(d2);
-        const double rinv2 = rinv * rinv;
-        const double f = S.m[j] * rinv * rinv2;
-        const double a3 = -3.0 * (dx[0] * dv[0] + dx[1] * dv[1] + dx[2] * dv[2]) * rinv2;
-        for (int k = 0; k < 3; k++) {
-          la[q][k] = fma(f, dx[k], la[q][k]);
-          lj[q][k] = fma(f, fma(a3, dx[k], dv[k]), lj[q][k]);
-        }
-        const double v2 = dc[0] * dc[0] + dc[1] * dc[1] + dc[2] * dc[2];
-        const double d3 = d2 * d2 * rinv;
-        const double ts = fmin(0.5 * d3 / (S.nm[ni] + S.nm[nj]), d2 / v2);
-        const int pid = ni < nj ? ni * MAXN + nj : nj * MAXN + ni;
-        if (ts < ts2 || (ts == ts2 && pid < pmin)) {
-          ts2 = ts;
-          pmin = pid;
-        }
+    }
+  }
+}
+
+// Resolved forces on the top-level nodes from the predicted components:
+// returns the natural step (warp-uniform, eta sqrt(min step^2)) and the node
+// pair setting it.
+template <int MODE, int NS>
+__device__ __forceinline__ double tree_forces(UnpSmem &S, int n, int lane, Comp<NS> &B, double t, double eta,
+                              int *imin, int *jmin) {
+  const unsigned FULL = 0xffffffffu;
+  constexpr int NQ = NS > 3 ? 2 : 1;  // leaves per lane
+  const int nb = S.nb;
+  __syncwarp();
+  if (nb > 0) {
+    if (lane < nb) {  // a lane per binary: its components' relative state at t
+      double r[3], v[3];
+      bin_rel_warm(S.bin[lane], t, r, v);
+      for (int k = 0; k < 3; k++) S.kr[lane][k] = r[k], S.kr[lane][3 + k] = v[k];
+    }
+    __syncwarp();
+  }
+  FOR_COMP(r, c, n) {
+    const int s = c / 3, k = c - 3 * s;
+    if (nb == 0) {
+      store_leaf<MODE, false>(S, s, k, B.pp[r], B.pv[r], B.pv[r]);
+    } else if (S.nd[s] == s) {
+      const int b = S.bi[s];
+      if (b < 0) {
+        store_leaf<MODE, true>(S, s, k, B.pp[r], B.pv[r], B.pv[r]);
+      } else {
+        const BinRec &bb = S.bin[b];
+        const double iM = rcp64(bb.mi + bb.mj), fi = bb.mj * iM, fj = bb.mi * iM;
+        const double x = S.kr[b][k], v = S.kr[b][3 + k];
+        store_leaf<MODE, true>(S, bb.li, k, B.pp[r] - fi * x, B.pv[r] - fi * v, B.pv[r]);
+        store_leaf<MODE, true>(S, bb.lj, k, B.pp[r] + fj * x, B.pv[r] + fj * v, B.pv[r]);
       }
     }
   }
   __syncwarp();
+  double dt;
+  int pmin = 0x7fffffff;
+  double la[2][3], lj[2][3];
+  if (MODE == MODE_SPLIT) {
+    float ts[2];
+    int pq[2];
+    ts[1] = __int_as_float(0x7f800000);
+    pq[1] = 0x7fffffff;
+    if (nb == 0)
+      pairs_split<false, NQ>(S, n, lane, la, lj, ts, pq);
+    else
+      pairs_split<true, NQ>(S, n, lane, la, lj, ts, pq);
+    if (ts[1] < ts[0] || (ts[1] == ts[0] && pq[1] < pq[0])) ts[0] = ts[1], pq[0] = pq[1];
+    const unsigned u = __float_as_uint(ts[0]);  // >= +0, or +inf: ordered as its bits
+    const unsigned m = __reduce_min_sync(FULL, u);
+    pmin = (int)__reduce_min_sync(FULL, u == m ? (unsigned)pq[0] : 0x7fffffffu);
+    dt = eta * sqrt64((double)(__uint_as_float(m)));
+  } else {
+    double w = 0.0;
+    if (nb == 0)
+      pairs_fast<false, NQ>(S, n, lane, la, lj, w, pmin);
+    else
+      pairs_fast<true, NQ>(S, n, lane, la, lj, w, pmin);
+    long long b = __double_as_longlong(w);
 #pragma unroll
-  for (int q = 0; q < 2; q++) {
+    for (int o = 16; o > 0; o >>= 1) {
+      const long long ob = __shfl_xor_sync(FULL, b, o);
+      const int op = __shfl_xor_sync(FULL, pmin, o);
+      if (ob > b || (ob == b && op < pmin)) {
+        b = ob;
+        pmin = op;
+      }
+    }
+    dt = eta * rsqrt64(__longlong_as_double(b));
+  }
+  *imin = pmin == 0x7fffffff ? -1 : pmin / MAXN;
+  *jmin = pmin == 0x7fffffff ? -1 : pmin % MAXN;
+#pragma unroll
+  for (int q = 0; q < NQ; q++) {
     const int i = lane + 32 * q;
     if (i < n)
       for (int k = 0; k < 3; k++) S.la[i][k] = la[q][k], S.lj[i][k] = lj[q][k];
   }
   __syncwarp();
   // node forces: mass-weighted leaf forces
-#pragma unroll
-  for (int q = 0; q < 2; q++) {
-    const int s = lane + 32 * q;
-    for (int k = 0; k < 3; k++) B[q].acc[k] = B[q].jerk[k] = 0.0;
-    if (s >= n || S.nd[s] != s) continue;
-    int qb = -1;
-    for (int b = 0; b < S.nb; b++)
-      if (S.bin[b].li == s) qb = b;
-    if (qb < 0) {
-      for (int k = 0; k < 3; k++) B[q].acc[k] = S.la[s][k], B[q].jerk[k] = S.lj[s][k];
+  FOR_COMP(r, c, n) {
+    const int s = c / 3, k = c - 3 * s;
+    const int b = nb > 0 ? S.bi[s] : -1;
+    if (b < 0) {
+      const bool node = nb == 0 || S.nd[s] == s;
+      B.acc[r] = node ? S.la[s][k] : 0.0;
+      B.jerk[r] = node ? S.lj[s][k] : 0.0;
     } else {
-      const BinRec &bb = S.bin[qb];
-      const double M = bb.mi + bb.mj;
-      for (int k = 0; k < 3; k++) {
-        B[q].acc[k] = (bb.mi * S.la[bb.li][k] + bb.mj * S.la[bb.lj][k]) / M;
-        B[q].jerk[k] = (bb.mi * S.lj[bb.li][k] + bb.mj * S.lj[bb.lj][k]) / M;
-      }
+      const BinRec &bb = S.bin[b];
+      const double iM = rcp64(bb.mi + bb.mj);
+      B.acc[r] = (bb.mi * S.la[bb.li][k] + bb.mj * S.la[bb.lj][k]) * iM;
+      B.jerk[r] = (bb.mi * S.lj[bb.li][k] + bb.mj * S.lj[bb.lj][k]) * iM;
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double ot = __shfl_xor_sync(0xffffffffu, ts2, o);
-    const int op = __shfl_xor_sync(0xffffffffu, pmin, o);
-    if (ot < ts2 || (ot == ts2 && op < pmin)) {
-      ts2 = ot;
-      pmin = op;
-    }
-  }
-  *imin = pmin == 0x7fffffff ? -1 : pmin / MAXN;
-  *jmin = pmin == 0x7fffffff ? -1 : pmin % MAXN;
-  return ts2;
+  return dt;
 }
 
 // Node states (after a step) into shared memory for the tree logic: positions
-// and velocities in A.d, accelerations in la, masses in nm.
-__device__ __forceinline__ void unp_publish_nodes(UnpSmem &S, int n, int lane, const Body B[2]) {
+// and velocities in d, accelerations in la.
+template <int NS>
+__device__ __forceinline__ void publish_nodes(UnpSmem &S, int n, int lane, const Comp<NS> &B) {
   __syncwarp();
-#pragma unroll
-  for (int q = 0; q < 2; q++) {
-    const int s = lane + 32 * q;
-    if (s >= n || S.nd[s] != s) continue;
-    for (int k = 0; k < 3; k++) {
-      S.A.d.pp[s][k] = B[q].pos[k];
-      S.A.d.pv[s][k] = B[q].vel[k];
-      S.la[s][k] = B[q].acc[k];
+  FOR_COMP(r, c, n) {
+    const int s = c / 3, k = c - 3 * s;
+    if (S.nd[s] == s) {
+      elem(S.d.pp[s], k) = B.pos[r];
+      elem(S.d.pv[s], k) = B.vel[r];
+      S.la[s][k] = B.acc[r];
     }
-    S.nm[s] = B[q].m;
   }
   __syncwarp();
 }
 
-__device__ __forceinline__ void body_set(Body &b, double m, const double x[3], const double v[3]) {
-  b.m = m;
-  b.inv_m = 1.0 / m;
-  for (int k = 0; k < 3; k++) {
-    b.pos[k] = b.pp[k] = x[k];
-    b.vel[k] = b.pv[k] = v[k];
-    b.oacc[k] = b.ojerk[k] = 0.0;  // a node the tree has just made
+// The components of node slot i after the tree made it anew.
+template <int NS>
+__device__ __forceinline__ void node_set(Comp<NS> &B, int n, int lane, int i, const double x[3],
+                                         const double v[3]) {
+  FOR_COMP(r, c, n) {
+    const int s = c / 3, k = c - 3 * s;
+    if (s == i) {
+      B.pos[r] = B.pp[r] = k == 0 ? x[0] : k == 1 ? x[1] : x[2];
+      B.vel[r] = B.pv[r] = k == 0 ? v[0] : k == 1 ? v[1] : v[2];
+      B.oacc[r] = B.ojerk[r] = 0.0;
+    }
   }
+}
+
+__device__ __forceinline__ void get3(const double4_16 &v, double x[3]) {
+  x[0] = v.x, x[1] = v.y, x[2] = v.z;
+}
+__device__ __forceinline__ void put3(double4_16 &v, const double x[3]) {
+  v.x = x[0], v.y = x[1], v.z = x[2];
 }
 
 // The tree changes after a step (smallN.cc:1022-1060): binary creation from
 // the pair that set the step, then the end of every segment due now.  Every
 // lane evaluates the same decisions from shared data; lane 0 writes the
-// shared records, the owners of the slots update their bodies.  Returns 0
+// shared records, the owners of the components update theirs.  Returns 0
 // (no change), 1 (changed), 3 (changed, a binary made).
-__device__ int unp_tree(UnpSmem &S, int n, int lane, Body B[2], double t, double dt_nat, int bim,
-                        int bjm, const UnpParams &P) {
-  unp_publish_nodes(S, n, lane, B);
+template <int MODE, int NS>
+__device__ __forceinline__ int tree_step(UnpSmem &S, int n, int lane, Comp<NS> &B, double t, double dt_nat, int bim,
+                         int bjm, const UnpParams &P) {
+  const bool create = bim >= 0 && S.nb < NB && dt_nat <= P.dt_crit;
+  bool due = false;
+  for (int b = 0; b < S.nb; b++) due |= !(S.bin[b].tpred > t);
+  if (!create && !due) return 0;
+  publish_nodes(S, n, lane, B);
   int changed = 0;
   // --- creation (is_unperturbed_and_approaching, create_binary)
-  if (bim >= 0 && S.nb < NB && dt_nat <= P.dt_crit) {
+  if (create) {
     bool leaves = true;
     for (int b = 0; b < S.nb; b++)
       if (S.bin[b].li == bim || S.bin[b].li == bjm) leaves = false;
     const int i = bim, j = bjm;
-    const double *xi = S.A.d.pp[i], *xj = S.A.d.pp[j], *vi = S.A.d.pv[i], *vj = S.A.d.pv[j];
+    double xi[3], xj[3], vi[3], vj[3];
+    get3(S.d.pp[i], xi), get3(S.d.pp[j], xj), get3(S.d.pv[i], vi), get3(S.d.pv[j], vj);
     double r[3], v[3];
     for (int k = 0; k < 3; k++) r[k] = xj[k] - xi[k], v[k] = vj[k] - vi[k];
     const double d2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
     const double rv = r[0] * v[0] + r[1] * v[1] + r[2] * v[2];
     if (leaves && d2 <= P.r2_crit && rv <= 0.0) {
-      const double mi = S.nm[i], mj = S.nm[j], M = mi + mj;
+      const double mi = S.nm[i], mj = S.nm[j], M = mi + mj, iM = rcp64(M);
       double cm[3], cmv[3];
       for (int k = 0; k < 3; k++) {
-        cm[k] = (mi * xi[k] + mj * xj[k]) / M;
-        cmv[k] = (mi * vi[k] + mj * vj[k]) / M;
+        cm[k] = (mi * xi[k] + mj * xj[k]) * iM;
+        cmv[k] = (mi * vi[k] + mj * vj[k]) * iM;
       }
       // the strongest perturber (largest m^2 / d^2 from the CM; the first
       // node on ties): each lane its two node slots, then a warp argmax
@@ -983,10 +1117,11 @@ __device__ int unp_tree(UnpSmem &S, int n, int lane, Body B[2], double t, double
       for (int q = 0; q < 2; q++) {
         const int k2 = lane + 32 * q;
         if (k2 >= n || S.nd[k2] != k2 || k2 == i || k2 == j) continue;
-        double e2 = 0.0;
-        for (int k = 0; k < 3; k++) e2 += (S.A.d.pp[k2][k] - cm[k]) * (S.A.d.pp[k2][k] - cm[k]);
-        const double p2 = S.nm[k2] * S.nm[k2] / e2;
-        if (p2 > maxp) maxp = p2, nnd2 = e2, mk = S.nm[k2], kk = k2;
+        const double4_16 y = S.d.pp[k2];
+        const double e0 = y.x - cm[0], e1 = y.y - cm[1], e2 = y.z - cm[2];
+        const double ee = e0 * e0 + e1 * e1 + e2 * e2;
+        const double p2 = S.nm[k2] * S.nm[k2] * rcp64(ee);
+        if (p2 > maxp) maxp = p2, nnd2 = ee, mk = S.nm[k2], kk = k2;
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -994,18 +1129,17 @@ __device__ int unp_tree(UnpSmem &S, int n, int lane, Body B[2], double t, double
         const double od = __shfl_xor_sync(0xffffffffu, nnd2, o);
         const double om = __shfl_xor_sync(0xffffffffu, mk, o);
         const int ok = __shfl_xor_sync(0xffffffffu, kk, o);
-        if (op > maxp || (op == maxp && ok < kk)) maxp = op, nnd2 = od, mk = om, kk = ok;
+        const long long bo = __double_as_longlong(op), bm = __double_as_longlong(maxp);
+        if (bo > bm || (bo == bm && ok < kk)) maxp = op, nnd2 = od, mk = om, kk = ok;
       }
       bool unp = true;
       if (maxp > 0.0) {
-        const double q = d2 / nnd2;
-        unp = 4.0 * (mk / M) * (mk / M) * q * q * q < P.gamma2;
+        const double q = d2 * rcp64(nnd2);
+        unp = 4.0 * (mk * iM) * (mk * iM) * q * q * q < P.gamma2;
       }
       double dtp, per;
       if (unp && kep_peri(M, r, v, &dtp, &per)) {
-        double pxi[3], pxj[3];
-        for (int k = 0; k < 3; k++) pxi[k] = xi[k], pxj[k] = xj[k];
-        const double tid = tidal_pot(S, n, lane, i, j, mi, mj, pxi, pxj, cm);
+        const double tid = tidal_pot(S, n, lane, i, j, mi, mj, xi, xj, cm);
         __syncwarp();
         if (lane == 0) {
           BinRec &b = S.bin[S.nb];
@@ -1021,12 +1155,11 @@ __device__ int unp_tree(UnpSmem &S, int n, int lane, Body B[2], double t, double
           b.tidal = tid;
           S.nd[j] = i;
           S.nm[i] = M;
-          for (int k = 0; k < 3; k++) S.A.d.pp[i][k] = cm[k], S.A.d.pv[i][k] = cmv[k];
+          put3(S.d.pp[i], cm);
+          put3(S.d.pv[i], cmv);
           S.nb++;
         }
-#pragma unroll
-        for (int q = 0; q < 2; q++)
-          if (lane + 32 * q == i) body_set(B[q], M, cm, cmv);
+        node_set(B, n, lane, i, cm, cmv);
         __syncwarp();
         changed = 3;
       }
@@ -1037,18 +1170,19 @@ __device__ int unp_tree(UnpSmem &S, int n, int lane, Body B[2], double t, double
     const BinRec bb = S.bin[qb];
     if (bb.tpred > t) continue;
     const int i = bb.li, j = bb.lj;
-    const double M = bb.mi + bb.mj;
+    const double M = bb.mi + bb.mj, iM = rcp64(M);
     double r[3], v[3], xi[3], xj[3], xc[3], vc[3];
     BinRec bw = bb;  // warm-started solve on a copy (every lane, same values)
     bin_rel_warm(bw, t, r, v);
-    for (int k = 0; k < 3; k++) xc[k] = S.A.d.pp[i][k], vc[k] = S.A.d.pv[i][k];
+    get3(S.d.pp[i], xc);
+    get3(S.d.pv[i], vc);
     for (int k = 0; k < 3; k++) {
-      xi[k] = xc[k] - bb.mj / M * r[k];
-      xj[k] = xc[k] + bb.mi / M * r[k];
+      xi[k] = xc[k] - bb.mj * iM * r[k];
+      xj[k] = xc[k] + bb.mi * iM * r[k];
     }
     const double tid = tidal_pot(S, n, lane, i, j, bb.mi, bb.mj, xi, xj, xc);
     if (!bb.full) {
-      const double mu = bb.mi * bb.mj / M, v2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+      const double mu = bb.mi * bb.mj * iM, v2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
       const double fac = 1.0 - 2.0 * (tid - bb.tidal) / (mu * v2);
       if (fac > 0.0) {
         const double sf = sqrt(fac);
@@ -1069,10 +1203,12 @@ __device__ int unp_tree(UnpSmem &S, int n, int lane, Body B[2], double t, double
         const int k2 = lane + 32 * q;
         if (k2 >= n || S.nd[k2] != k2 || k2 == i) continue;
         const double rp = P.gamma_inv3 * a * cbrt(2.0 * S.nm[k2] / M);
-        double dp[3], dvl[3], da[3];
+        double yp[3], yv[3], dp[3], dvl[3], da[3];
+        get3(S.d.pp[k2], yp);
+        get3(S.d.pv[k2], yv);
         for (int k = 0; k < 3; k++) {
-          dp[k] = S.A.d.pp[k2][k] - xc[k];
-          dvl[k] = S.A.d.pv[k2][k] - vc[k];
+          dp[k] = yp[k] - xc[k];
+          dvl[k] = yv[k] - vc[k];
           da[k] = S.la[k2][k] - S.la[i][k];
         }
         const double dr = sqrt(dp[0] * dp[0] + dp[1] * dp[1] + dp[2] * dp[2]);
@@ -1106,24 +1242,19 @@ __device__ int unp_tree(UnpSmem &S, int n, int lane, Body B[2], double t, double
     // dissolve: the components become top-level nodes again
     double yi[3], yj[3], wi[3], wj[3];
     for (int k = 0; k < 3; k++) {
-      yi[k] = xc[k] - bb.mj / M * r[k];
-      yj[k] = xc[k] + bb.mi / M * r[k];
-      wi[k] = vc[k] - bb.mj / M * v[k];
-      wj[k] = vc[k] + bb.mi / M * v[k];
+      yi[k] = xc[k] - bb.mj * iM * r[k];
+      yj[k] = xc[k] + bb.mi * iM * r[k];
+      wi[k] = vc[k] - bb.mj * iM * v[k];
+      wj[k] = vc[k] + bb.mi * iM * v[k];
     }
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      if (lane + 32 * q == i) body_set(B[q], bb.mi, yi, wi);
-      if (lane + 32 * q == j) body_set(B[q], bb.mj, yj, wj);
-    }
+    node_set(B, n, lane, i, yi, wi);
+    node_set(B, n, lane, j, yj, wj);
     __syncwarp();
     if (lane == 0) {
-      for (int k = 0; k < 3; k++) {
-        S.A.d.pp[i][k] = yi[k];
-        S.A.d.pv[i][k] = wi[k];
-        S.A.d.pp[j][k] = yj[k];
-        S.A.d.pv[j][k] = wj[k];
-      }
+      put3(S.d.pp[i], yi);
+      put3(S.d.pv[i], wi);
+      put3(S.d.pp[j], yj);
+      put3(S.d.pv[j], wj);
       S.nd[j] = j;
       S.nm[i] = bb.mi;
       S.nm[j] = bb.mj;
@@ -1134,188 +1265,245 @@ __device__ int unp_tree(UnpSmem &S, int n, int lane, Body B[2], double t, double
     qb--;
     changed |= 1;
   }
+  if (changed) tree_masses<MODE>(S, n, lane);
   return changed;
 }
 
+struct TreeRun {  // one system's integration
+  int n, n_iter;
+  double t_end, eta;
+  long long max_steps;
+  double *pos, *vel;  // its first body
+  const double *mass;
+  // results
+  double t;
+  long long steps;
+  int status, made;
+};
+
+template <int MODE, int NS>
+__device__ __noinline__ void integrate(UnpSmem &S, int lane, TreeRun &run, const UnpParams &P) {
+  const int n = run.n, n_iter = run.n_iter;
+  const double t_end = run.t_end, eta = run.eta;
+  const long long max_steps = run.max_steps;
+  double *pos = run.pos, *vel = run.vel;
+  const double *mass = run.mass;
+  // lane & 7: one of the corrector's coefficients, a cubic in tau, a quarter
+  // included: acc = c0 oa + c1 pa + theta (c2 oj + c3 pj),
+  // jerk = (c4 oa + c5 pa) / theta + c6 oj + c7 pj (smallN.cc:487-510)
+  double q0, q1, q2, q3;
+  {
+    const int l = lane & 7;
+    q0 = l < 2 ? 0.5 : l == 2 ? 0.25 : l == 4 ? -0.75 : l == 5 ? 0.75 : -0.25;
+    q1 = l == 0 ? -0.75 : l == 1 ? 0.75 : l == 2 || l == 3 ? -0.25 : l == 6 ? -0.5 : l == 7 ? 0.5 : 0.0;
+    q2 = l < 2 ? 0.0 : l == 2 ? -0.25 : l == 3 ? 0.25 : l == 5 ? -0.75 : 0.75;
+    q3 = l == 0 || l == 2 || l == 3 ? 0.25 : l == 1 ? -0.25 : 0.0;
+  }
+  Comp<NS> B;
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < NS; r++) {
+    const int c = lane + 32 * r;
+    B.pos[r] = B.pp[r] = c < 3 * n ? pos[c] : 0.0;
+    B.vel[r] = B.pv[r] = c < 3 * n ? vel[c] : 0.0;
+    B.acc[r] = B.jerk[r] = B.oacc[r] = B.ojerk[r] = 0.0;
+  }
+  for (int i = lane; i < n; i += 32) {
+    const double m = mass[i];
+    S.nd[i] = i;
+    S.nm[i] = m;
+    S.d.pp[i].w = m;
+    if (MODE == MODE_SPLIT) S.f.hi[i].w = __double2float_rn(m);
+  }
+  if (lane == 0) S.nb = 0;
+  tree_masses<MODE>(S, n, lane);
+  int bim, bjm, made = 0;
+  double t = 0.0;
+  double dt = tree_forces<MODE, NS>(S, n, lane, B, t, eta, &bim, &bjm);
+  long long nsteps = 0;
+  int st = 0;
+  while (t < t_end) {
+    if (nsteps >= max_steps) {
+      st = 1;  // step budget exhausted
+      break;
+    }
+    double lim = __longlong_as_double(0x7ff0000000000000ll);
+    for (int b = 0; b < S.nb; b++) lim = fmin(lim, S.bin[b].tpred - t);
+    int nit = n_iter;
+    if (dt >= lim) {
+      dt = lim;
+      nit = 0;
+    }
+    // predict_loworder (hdyn.h:192-201: with the stored old force)
+    {
+      const double h = dt, h3 = h * (1.0 / 3.0), h2 = h * 0.5;
+      FOR_COMP(r, c, n) {
+        const double oj = B.ojerk[r], oa = B.oacc[r];
+        B.pp[r] = fma(fma(fma(oj, h3, oa), h2, B.vel[r]), h, B.pos[r]);
+        B.pv[r] = fma(fma(oj, h2, oa), h, B.vel[r]);
+        B.oacc[r] = B.acc[r];
+        B.ojerk[r] = B.jerk[r];
+      }
+    }
+    double new_dt = dt, end_dt = dt;
+    for (int it = 0; it <= nit; it++) {
+      const double prev = new_dt;
+      end_dt = tree_forces<MODE, NS>(S, n, lane, B, t + new_dt, eta, &bim, &bjm);
+      double iprev = 0.0;
+      if (it < nit) {
+        iprev = rcp64(prev);
+        new_dt = 0.5 * (dt + end_dt);
+        new_dt = dt + 0.5 * (end_dt - dt) * (new_dt * iprev);
+        if (new_dt >= lim) {
+          new_dt = lim;
+          nit = 0;
+        }
+      }
+      if (new_dt != prev) {  // correct_acc_and_jerk(new_dt, prev)
+        const double theta = 0.5 * prev, itheta = 2.0 * iprev;
+        const double tau = (new_dt - theta) * itheta;
+        double cc = fma(fma(fma(q3, tau, q2), tau, q1), tau, q0);
+        const int l = lane & 7;
+        cc *= (l & 6) == 2 ? theta : (l & 6) == 4 ? itheta : 1.0;
+        double k[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) k[q] = __shfl_sync(0xffffffffu, cc, q);
+        FOR_COMP(r, c, n) {
+          const double pa = B.acc[r], pj = B.jerk[r], oa = B.oacc[r], oj = B.ojerk[r];
+          B.acc[r] = fma(k[3], pj, fma(k[2], oj, fma(k[1], pa, k[0] * oa)));
+          B.jerk[r] = fma(k[7], pj, fma(k[6], oj, fma(k[5], pa, k[4] * oa)));
+        }
+      }
+      // correct_pos_and_vel(new_dt)
+      const double hh = 0.5 * new_dt, h12 = new_dt * new_dt * (1.0 / 12.0);
+      FOR_COMP(r, c, n) {
+        B.pv[r] = fma(-h12, B.jerk[r] - B.ojerk[r], fma(hh, B.acc[r] + B.oacc[r], B.vel[r]));
+        B.pp[r] = fma(-h12, B.acc[r] - B.oacc[r], fma(hh, B.pv[r] + B.vel[r], B.pos[r]));
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < NS; r++) B.pos[r] = B.pp[r], B.vel[r] = B.pv[r];
+    dt = end_dt;
+    t = t + new_dt;
+    nsteps++;
+    if (P.on) {
+      const int tc = tree_step<MODE, NS>(S, n, lane, B, t, dt, bim, bjm, P);
+      if (tc) {
+        if (tc & 2) made++;
+        dt = tree_forces<MODE, NS>(S, n, lane, B, t, eta, &bim, &bjm);
+      }
+    }
+  }
+  // resolve the binaries left at the end into their components
+  __syncwarp();
+  if (lane < S.nb) {
+    double r[3], v[3];
+    bin_rel(S.bin[lane], t, r, v);
+    for (int k = 0; k < 3; k++) S.kr[lane][k] = r[k], S.kr[lane][3 + k] = v[k];
+  }
+  __syncwarp();
+  FOR_COMP(r, c, n) {
+    const int i = c / 3, k = c - 3 * i;
+    const int b = S.bi[i];
+    if (S.nd[i] == i && b < 0) {
+      pos[c] = B.pos[r];
+      vel[c] = B.vel[r];
+    } else if (S.nd[i] == i) {
+      const BinRec &bb = S.bin[b];
+      const double iM = rcp64(bb.mi + bb.mj), x = S.kr[b][k], v = S.kr[b][3 + k];
+      pos[3 * bb.li + k] = B.pos[r] - bb.mj * iM * x;
+      vel[3 * bb.li + k] = B.vel[r] - bb.mj * iM * v;
+      pos[3 * bb.lj + k] = B.pos[r] + bb.mi * iM * x;
+      vel[3 * bb.lj + k] = B.vel[r] + bb.mi * iM * v;
+    }
+  }
+  run.t = t;
+  run.steps = nsteps;
+  run.status = st;
+  run.made = made;
+}
+#undef FOR_COMP
+
 template <int MODE>
-__global__ void batch_unp_kernel(const int *__restrict__ order, const int *__restrict__ off,
-                                 const double *__restrict__ t_end_s, const double *__restrict__ mass,
-                                 double *pos, double *vel, double eta, int n_iter,
-                                 long long max_steps, int *queue, double *t_out,
-                                 long long *steps_out, unsigned long long *wall_ns, int *status,
-                                 int *nbin_out, UnpParams P) {
-  __shared__ UnpSmem smem[WARPS_MAX_UNP];
+__global__ void batch_tree_kernel(const int *__restrict__ order, const int *__restrict__ off,
+                                  const double *__restrict__ t_end_s,
+                                  const double *__restrict__ mass, double *pos, double *vel,
+                                  double eta, int n_iter, long long max_steps, int *queue,
+                                  double *t_out, long long *steps_out,
+                                  unsigned long long *wall_ns, int *status, int *nbin_out,
+                                  UnpParams P) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
-  UnpSmem &S = smem[w];
+  UnpSmem &S = reinterpret_cast<UnpSmem *>(smem_raw)[w];
   const int nsys = queue[1];  // written by the host before the launch
-  while (true) {
-    int qq0 = 0;
-    if (lane == 0) qq0 = atomicAdd(queue, 1);
-    qq0 = __shfl_sync(0xffffffffu, qq0, 0);
-    if (qq0 >= nsys) break;
-    const int s = order[qq0];
+  for (int q = first_system(w); q < nsys; q = next_system(queue, lane)) {
+    const int s = order[q];
     unsigned long long t0;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
     const int base = off[s];
     const int n = off[s + 1] - base;
-    const double t_end = t_end_s[s];
     if (n < 2 || n > MAXN) {
       if (lane == 0) {
-        status[s] = 2;
+        status[s] = 2;  // unsupported size (host also checks)
         steps_out[s] = 0;
         t_out[s] = 0.0;
-        nbin_out[s] = 0;
+        if (nbin_out) nbin_out[s] = 0;
       }
       continue;
     }
-    Body B[2];
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      const int i = lane + 32 * q;
-      const int ii = i < n ? i : 0;
-      double x[3], v[3];
-      for (int k = 0; k < 3; k++) x[k] = pos[3 * (base + ii) + k], v[k] = vel[3 * (base + ii) + k];
-      body_set(B[q], mass[base + ii], x, v);
-      if (i < n) {
-        S.m[i] = B[q].m;
-        S.mf[i] = __double2float_rn(B[q].m);
-        S.nd[i] = i;
-      }
-    }
-    if (lane == 0) S.nb = 0;
-    __syncwarp();
-    int bim, bjm, made = 0;
-    double t = 0.0;
-    double dt = eta * sqrt(unp_forces<MODE>(S, n, lane, B, t, &bim, &bjm));
-    long long nsteps = 0;
-    int st = 0;
-    while (t < t_end) {
-      if (nsteps >= max_steps) {
-        st = 1;
-        break;
-      }
-      double lim = __longlong_as_double(0x7ff0000000000000ll);
-      for (int b = 0; b < S.nb; b++) lim = fmin(lim, S.bin[b].tpred - t);
-      int nit = n_iter;
-      if (dt >= lim) {
-        dt = lim;
-        nit = 0;
-      }
-      // predict_loworder (hdyn.h:192-201: with the stored old force)
-      const double h = dt, h3 = h / 3.0, h2 = h * 0.5;
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        if (lane + 32 * q >= n || S.nd[lane + 32 * q] != lane + 32 * q) continue;
-        for (int k = 0; k < 3; k++) {
-          const double oj = B[q].ojerk[k], oa = B[q].oacc[k];
-          B[q].pp[k] = fma(fma(fma(oj, h3, oa), h2, B[q].vel[k]), h, B[q].pos[k]);
-          B[q].pv[k] = fma(fma(oj, h2, oa), h, B[q].vel[k]);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 2; q++)
-        for (int k = 0; k < 3; k++) B[q].oacc[k] = B[q].acc[k], B[q].ojerk[k] = B[q].jerk[k];
-      double new_dt = dt, end_dt = dt;
-      for (int it = 0; it <= nit; it++) {
-        const double prev = new_dt;
-        const double ts2 = unp_forces<MODE>(S, n, lane, B, t + new_dt, &bim, &bjm);
-        end_dt = eta * sqrt(ts2);
-        if (it < nit) {
-          new_dt = 0.5 * (dt + end_dt);
-          new_dt = dt + 0.5 * (end_dt - dt) * (new_dt / prev);
-          if (new_dt >= lim) {
-            new_dt = lim;
-            nit = 0;
-          }
-        }
-        const bool cj = new_dt != prev;
-        double tau = 0, tau2 = 0, tau3 = 0, theta = 0, inv_theta = 0;
-        if (cj) {
-          theta = 0.5 * prev;
-          tau = (new_dt - theta) / theta;
-          inv_theta = 1.0 / theta;
-          tau2 = tau * tau;
-          tau3 = tau2 * tau;
-        }
-        const double nd2 = new_dt * new_dt;
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-          Body &b = B[q];
-          for (int k = 0; k < 3; k++) {
-            if (cj) {
-              const double pa = b.acc[k], pj = b.jerk[k], oa = b.oacc[k], oj = b.ojerk[k];
-              b.acc[k] = 0.25 * (oa * (2 - 3 * tau + tau3) + pa * (2 + 3 * tau - tau3) +
-                                 oj * theta * (1 - tau - tau2 + tau3) +
-                                 pj * theta * (-1 - tau + tau2 + tau3));
-              b.jerk[k] = 0.25 * (oa * inv_theta * 3 * (-1 + tau2) + pa * inv_theta * 3 * (1 - tau2) +
-                                  oj * (-1 - 2 * tau + 3 * tau2) + pj * (-1 + 2 * tau + 3 * tau2));
-            }
-            b.pv[k] = b.vel[k] + new_dt * (b.acc[k] + b.oacc[k]) * 0.5 -
-                      nd2 * (b.jerk[k] - b.ojerk[k]) * (1.0 / 12.0);
-            b.pp[k] = b.pos[k] + new_dt * (b.pv[k] + b.vel[k]) * 0.5 -
-                      nd2 * (b.acc[k] - b.oacc[k]) * (1.0 / 12.0);
-          }
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 2; q++)
-        for (int k = 0; k < 3; k++) B[q].pos[k] = B[q].pp[k], B[q].vel[k] = B[q].pv[k];
-      dt = end_dt;
-      t = t + new_dt;
-      nsteps++;
-      const int tc = unp_tree(S, n, lane, B, t, dt, bim, bjm, P);
-      if (tc) {
-        if (tc & 2) made++;
-        dt = eta * sqrt(unp_forces<MODE>(S, n, lane, B, t, &bim, &bjm));
-      }
-    }
-    // resolve the binaries left at the end into their components
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      const int i = lane + 32 * q;
-      if (i >= n || S.nd[i] != i) continue;
-      int qb = -1;
-      for (int b = 0; b < S.nb; b++)
-        if (S.bin[b].li == i) qb = b;
-      if (qb < 0) {
-        for (int k = 0; k < 3; k++) {
-          pos[3 * (base + i) + k] = B[q].pos[k];
-          vel[3 * (base + i) + k] = B[q].vel[k];
-        }
-      } else {
-        const BinRec &bb = S.bin[qb];
-        double r[3], v[3];
-        bin_rel(bb, t, r, v);
-        const double M = bb.mi + bb.mj;
-        for (int k = 0; k < 3; k++) {
-          pos[3 * (base + bb.li) + k] = B[q].pos[k] - bb.mj / M * r[k];
-          vel[3 * (base + bb.li) + k] = B[q].vel[k] - bb.mj / M * v[k];
-          pos[3 * (base + bb.lj) + k] = B[q].pos[k] + bb.mi / M * r[k];
-          vel[3 * (base + bb.lj) + k] = B[q].vel[k] + bb.mi / M * v[k];
-        }
-      }
+    TreeRun run;
+    run.n = n;
+    run.n_iter = n_iter;
+    run.t_end = t_end_s[s];
+    run.eta = eta;
+    run.max_steps = max_steps;
+    run.pos = pos + 3 * (size_t)base;
+    run.vel = vel + 3 * (size_t)base;
+    run.mass = mass + base;
+    switch ((3 * n + 31) / 32) {
+      case 1: integrate<MODE, 1>(S, lane, run, P); break;  // 2 to 10 bodies
+      case 2: integrate<MODE, 2>(S, lane, run, P); break;  // to 21
+      case 3: integrate<MODE, 3>(S, lane, run, P); break;  // to 32
+      default: integrate<MODE, 6>(S, lane, run, P); break;
     }
     if (lane == 0) {
       unsigned long long t1;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-      t_out[s] = t;
-      steps_out[s] = nsteps;
+      t_out[s] = run.t;
+      steps_out[s] = run.steps;
       wall_ns[s] = t1 - t0;
-      status[s] = st;
-      nbin_out[s] = made;
+      status[s] = run.status;
+      if (nbin_out) nbin_out[s] = run.made;
     }
     __syncwarp();
   }
 }
+
 
 __global__ void queue_reset(int *queue) { queue[0] = 0; }
 
 }  // namespace
 
 extern "C" int g6k_batch_max_n(void) { return MAXN; }
+
+// The fast and split modes: dynamic shared memory for warps_per_cta warps.
+static int launch_tree(int mode, const int *order, const int *off, const double *t_end,
+                       const double *mass, double *pos, double *vel, double eta, int n_iter,
+                       long long max_steps, int warps_per_cta, int ctas, int *queue,
+                       double *t_out, long long *steps_out, unsigned long long *wall_ns,
+                       int *status, int *nbin_out, const UnpParams &P, cudaStream_t st) {
+  const size_t sm = sizeof(UnpSmem) * (size_t)warps_per_cta;
+  const int most = (int)(sizeof(UnpSmem) * WARPS_MAX);
+  auto kern = mode == MODE_SPLIT ? batch_tree_kernel<MODE_SPLIT> : batch_tree_kernel<MODE_FAST>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) !=
+      cudaSuccess)
+    return -3;
+  kern<<<ctas, 32 * warps_per_cta, sm, st>>>(order, off, t_end, mass, pos, vel, eta, n_iter,
+                                             max_steps, queue, t_out, steps_out, wall_ns, status,
+                                             nbin_out, P);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
 
 // One persistent launch: grid = ctas_per_sm * SMs, warps_per_cta warps each.
 // Resets the queue counter first (same stream), so the pair can be captured
@@ -1330,24 +1518,22 @@ extern "C" int g6k_batch_launch(const int *order, const int *off, const double *
   if (warps_per_cta < 1 || warps_per_cta > WARPS_MAX || ctas < 1) return -2;
   if (exact < MODE_FAST || exact > MODE_SPLIT) return -2;
   queue_reset<<<1, 1, 0, st>>>(queue);
-#define G6_BATCH(M)                                                                           \
-  batch_kernel<M><<<ctas, 32 * warps_per_cta, 0, st>>>(order, off, t_end, mass, pos, vel,       \
-                                                       eta, n_iter, max_steps, queue, t_out,    \
-                                                       steps_out, wall_ns, status)
-  if (exact == MODE_EXACT)
-    G6_BATCH(MODE_EXACT);
-  else if (exact == MODE_SPLIT)
-    G6_BATCH(MODE_SPLIT);
-  else
-    G6_BATCH(MODE_FAST);
-#undef G6_BATCH
+  if (exact != MODE_EXACT) {
+    UnpParams P = {};
+    return launch_tree(exact, order, off, t_end, mass, pos, vel, eta, n_iter, max_steps,
+                       warps_per_cta, ctas, queue, t_out, steps_out, wall_ns, status, nullptr, P,
+                       st);
+  }
+  batch_exact_kernel<<<ctas, 32 * warps_per_cta, 0, st>>>(order, off, t_end, mass, pos, vel, eta,
+                                                          n_iter, max_steps, queue, t_out,
+                                                          steps_out, wall_ns, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-// The same with smallN's unperturbed binaries (FAST or SPLIT pair terms):
-// dt_crit, r2_crit, gamma and allow_full as smallN's set_dt_crit,
-// set_r2_crit, set_gamma, set_allow_full_unperturbed; nbin_out[s] counts the
-// binaries made in system s.
+// The fast or split mode with smallN's unperturbed binaries: dt_crit,
+// r2_crit, gamma and allow_full as smallN's set_dt_crit, set_r2_crit,
+// set_gamma, set_allow_full_unperturbed; nbin_out[s] counts the binaries made
+// in system s.
 extern "C" int g6k_batch_launch_unp(const int *order, const int *off,
                                     const double *t_end, const double *mass, double *pos,
                                     double *vel, double eta, int n_iter, long long max_steps,
@@ -1356,7 +1542,7 @@ extern "C" int g6k_batch_launch_unp(const int *order, const int *off,
                                     double *t_out, long long *steps_out,
                                     unsigned long long *wall_ns, int *status, int *nbin_out,
                                     cudaStream_t st) {
-  if (warps_per_cta < 1 || warps_per_cta > WARPS_MAX_UNP || ctas < 1) return -2;
+  if (warps_per_cta < 1 || warps_per_cta > 4 || ctas < 1) return -2;
   if (mode != MODE_FAST && mode != MODE_SPLIT) return -2;
   UnpParams P;
   P.dt_crit = dt_crit;
@@ -1364,14 +1550,9 @@ extern "C" int g6k_batch_launch_unp(const int *order, const int *off,
   P.gamma2 = gamma * gamma;
   P.gamma_inv3 = pow(fmax(P.gamma2, 1e-120), -1.0 / 6.0);
   P.allow_full = allow_full;
+  P.on = 1;
   queue_reset<<<1, 1, 0, st>>>(queue);
-  if (mode == MODE_SPLIT)
-    batch_unp_kernel<MODE_SPLIT><<<ctas, 32 * warps_per_cta, 0, st>>>(
-        order, off, t_end, mass, pos, vel, eta, n_iter, max_steps, queue, t_out, steps_out,
-        wall_ns, status, nbin_out, P);
-  else
-    batch_unp_kernel<MODE_FAST><<<ctas, 32 * warps_per_cta, 0, st>>>(
-        order, off, t_end, mass, pos, vel, eta, n_iter, max_steps, queue, t_out, steps_out,
-        wall_ns, status, nbin_out, P);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch_tree(mode, order, off, t_end, mass, pos, vel, eta, n_iter, max_steps,
+                     warps_per_cta, ctas, queue, t_out, steps_out, wall_ns, status, nbin_out, P,
+                     st);
 }

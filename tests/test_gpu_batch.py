@@ -217,3 +217,35 @@ def test_batch_growing_in_systems_or_bodies(lib_built, first, then):
             px, pv, tf, st = oracle.smalln(m[a:b], x[a:b], v[a:b], 0.14, 0.05 * tcr)
             assert r["status"][s] == 0 and r["steps"][s] == st and r["t_final"][s] == tf
             assert np.array_equal(r["pos"][a:b], px) and np.array_equal(r["vel"][a:b], pv)
+
+
+@pytest.mark.parametrize("mode,tol", [("fast", 1e-9), ("split", 1e-6)])
+@pytest.mark.parametrize("unp", [False, True])
+def test_component_layout_edges(g6, mode, tol, unp):
+    """Sizes at the edges of the component slots (3n = 32 k) and of the two
+    leaves per lane, a few steps, against smallN: FP64 roundings amplified by
+    at most 1e6, FP32 pair terms moving bodies by 1e-7 of a t^2 / 2 ~ 2e-3 of
+    the size, amplified by 1e3 at the closest pair."""
+    sizes = [2, 3, 10, 11, 21, 22, 32, 33, 42, 43, 53, 54, 63, 64]
+    rng = np.random.RandomState(12)
+    sysm = [ic.plummer(n, do_scale=True, rng=rng) for n in sizes]
+    ns = np.array(sizes, np.int32)
+    m = np.concatenate([s[0] for s in sysm])
+    x = np.concatenate([s[1] for s in sysm]) * 1e-3
+    v = np.concatenate([s[2] for s in sysm]) / np.sqrt(1e-3)
+    t_end = 0.02 * 2 * np.sqrt(2) * 1e-3 ** 1.5
+    # dt_crit = 0 makes no binaries: the tree's code with smallN's trajectory
+    g6.batch_unperturbed(unp, dt_crit=0.0)
+    try:
+        r = g6.batch_run(ns, t_end, m, x, v, mode=mode, max_steps=100000)
+    finally:
+        g6.batch_unperturbed(False)
+    off = np.concatenate([[0], np.cumsum(ns)])
+    for s, n in enumerate(sizes):
+        a, b = off[s], off[s + 1]
+        px, pv, tf, st = oracle.smalln(m[a:b], x[a:b], v[a:b], 0.14, t_end)
+        assert r["status"][s] == 0
+        if mode == "fast":
+            assert r["steps"][s] == st, n
+        assert np.abs(r["pos"][a:b] - px).max() <= tol * 1e-3, n
+        assert np.abs(r["vel"][a:b] - pv).max() <= tol * 1e3 * np.abs(pv).max(), n
