@@ -7,7 +7,7 @@
  *   - the j-store grows on demand (no nj_max = 131072 cap, sapporo.cpp:30);
  *   - j updates are staged in pinned memory, deduplicated per slot with an
  *     O(1) slot index (the reference uses a std::map, sapporo.cpp:83-110) and
- *     applied with one copy + one scatter kernel per force call;
+ *     applied with one scatter kernel per force call;
  *   - inputs and outputs move with one asynchronous copy each way;
  *   - errors return negative codes instead of exit(-1).
  * There is no CPU force path: every force is computed by the CUDA kernels.
@@ -119,7 +119,8 @@ typedef struct {
   double pred_t;
   /* i / out buffers: pinned host block + device block, capacity cap_i */
   int cap_i;
-  void *h_in, *d_in;   /* [ipos 3n][ivel 3n][h2 n] doubles, [iself n] ints */
+  int io_n; /* the n of the call the blocks are laid out for: each moves in one copy */
+  void *h_in, *d_in;   /* [ipos 3n][ivel 3n] doubles, [iself n (even)] ints, [h2 n] doubles */
   void *h_out, *d_out; /* [err 2 ints][acc 3n][jerk 3n][pot n] doubles, [nn n] ints, [nnr2 n] floats */
   int *d_err;
   void *d_scratch;
@@ -286,7 +287,7 @@ static int ensure_io(int ni) {
   if (ni <= G.cap_i) return 0;
   int cap = G.cap_i ? G.cap_i : 1024;
   while (cap < ni) cap *= 2;
-  size_t in_b = (size_t)cap * (7 * sizeof(double) + sizeof(int));
+  size_t in_b = (size_t)cap * (7 * sizeof(double) + sizeof(int)) + sizeof(double);
   size_t out_b = 16 + (size_t)cap * (7 * sizeof(double) + sizeof(int) + sizeof(float));
   if (G.h_in) cudaFreeHost(G.h_in);
   if (G.h_out) cudaFreeHost(G.h_out);
@@ -311,17 +312,17 @@ static int ensure_io(int ni) {
   return 0;
 }
 
-/* Views into the i/o blocks for capacity cap_i. */
+/* Views into the i/o blocks for the current call's io_n particles. */
 #define IN_POS(b) ((double *)(b))
-#define IN_VEL(b) ((double *)(b) + 3 * (size_t)G.cap_i)
-#define IN_H2(b) ((double *)(b) + 6 * (size_t)G.cap_i)
-#define IN_SELF(b) ((int *)((double *)(b) + 7 * (size_t)G.cap_i))
+#define IN_VEL(b) ((double *)(b) + 3 * (size_t)G.io_n)
+#define IN_SELF(b) ((int *)((double *)(b) + 6 * (size_t)G.io_n))
+#define IN_H2(b) ((double *)(b) + 6 * (size_t)G.io_n + ((size_t)G.io_n + 1) / 2)
 #define OUT_ERR(b) ((int *)(b))
 #define OUT_ACC(b) ((double *)((char *)(b) + 16))
-#define OUT_JERK(b) (OUT_ACC(b) + 3 * (size_t)G.cap_i)
-#define OUT_POT(b) (OUT_ACC(b) + 6 * (size_t)G.cap_i)
-#define OUT_NN(b) ((int *)(OUT_ACC(b) + 7 * (size_t)G.cap_i))
-#define OUT_NNR2(b) ((float *)(OUT_NN(b) + (size_t)G.cap_i))
+#define OUT_JERK(b) (OUT_ACC(b) + 3 * (size_t)G.io_n)
+#define OUT_POT(b) (OUT_ACC(b) + 6 * (size_t)G.io_n)
+#define OUT_NN(b) ((int *)(OUT_ACC(b) + 7 * (size_t)G.io_n))
+#define OUT_NNR2(b) ((float *)(OUT_NN(b) + (size_t)G.io_n))
 
 static int ensure_scratch(size_t bytes) {
   if (bytes <= G.scratch_bytes) return 0;
@@ -345,10 +346,15 @@ static int check_open(void) {
   return 0;
 }
 
-/* Apply staged j updates: one H2D copy + one scatter kernel. */
+/* Apply staged j updates.  Up to UPD_DIRECT records (a block's) the scatter
+   kernel reads them where they are, in pinned host memory: it needs each once,
+   and a copy before it costs more than the reads (ph4's block of 8: one copy
+   and its gap, about 4 us).  More go by one copy. */
+#define UPD_DIRECT 1024
 static int flush_updates(void) {
   if (G.n_upd == 0) return 0;
-  if (G.n_upd > G.cap_dupd) {
+  const int direct = G.n_upd <= UPD_DIRECT;
+  if (!direct && G.n_upd > G.cap_dupd) {
     cudaFree(G.d_upd);
     G.d_upd = NULL;
     G.cap_dupd = 0;
@@ -359,15 +365,18 @@ static int flush_updates(void) {
     }
     G.cap_dupd = c;
   }
-  CK(cudaMemcpyAsync(G.d_upd, G.h_upd, sizeof(g6_jupd) * (size_t)G.n_upd,
-                     cudaMemcpyHostToDevice, G.st));
-  CK(cudaEventRecord(G.ev_upd, G.st));
-  G.upd_inflight = 1;
-  int rc = g6k_scatter(&G.js, G.d_upd, G.n_upd, G.st);
+  if (!direct) {
+    CK(cudaMemcpyAsync(G.d_upd, G.h_upd, sizeof(g6_jupd) * (size_t)G.n_upd,
+                       cudaMemcpyHostToDevice, G.st));
+    CK(cudaEventRecord(G.ev_upd, G.st)); /* h_upd may be written again after this */
+  }
+  int rc = g6k_scatter(&G.js, direct ? G.h_upd : G.d_upd, G.n_upd, G.st);
   if (rc) {
     seterr("scatter launch failed");
     return G6_ERR_CUDA;
   }
+  if (direct) CK(cudaEventRecord(G.ev_upd, G.st));
+  G.upd_inflight = 1;
   for (int u = 0; u < G.n_upd; u++) G.stage_pos[G.h_upd[u].addr] = -1;
   G.n_upd = 0;
   G.pred_valid = 0;
@@ -651,10 +660,7 @@ static int stage_force_host(int nj, int ni, const int *index, const double *xi,
   if (ni > 0) {
     rc = ensure_io(ni);
     if (rc) return rc;
-    rc = flush_updates();
-    if (rc) return rc;
-    rc = predict_if_needed(nj);
-    if (rc) return rc;
+    G.io_n = ni;
     memcpy(IN_POS(G.h_in), xi, sizeof(double) * 3 * (size_t)ni);
     memcpy(IN_VEL(G.h_in), vi, sizeof(double) * 3 * (size_t)ni);
     if (h2)
@@ -670,13 +676,16 @@ static int stage_force_host(int nj, int ni, const int *index, const double *xi,
         hs[i] = (s >= 0 && s < nj) ? s : -1;
       }
     }
-    /* One copy of the live prefix of each input section. */
-    CK(cudaMemcpyAsync(IN_POS(G.d_in), IN_POS(G.h_in), sizeof(double) * 3 * (size_t)ni,
+    /* One copy of positions, velocities and self slots (a copy each cost
+       about 3 us apiece); first, so that the kernels below follow each other
+       without a copy between them. */
+    CK(cudaMemcpyAsync(G.d_in, G.h_in,
+                       sizeof(double) * 6 * (size_t)ni + sizeof(int) * (size_t)ni,
                        cudaMemcpyHostToDevice, G.st));
-    CK(cudaMemcpyAsync(IN_VEL(G.d_in), IN_VEL(G.h_in), sizeof(double) * 3 * (size_t)ni,
-                       cudaMemcpyHostToDevice, G.st));
-    CK(cudaMemcpyAsync(IN_SELF(G.d_in), hs, sizeof(int) * (size_t)ni, cudaMemcpyHostToDevice,
-                       G.st));
+    rc = flush_updates();
+    if (rc) return rc;
+    rc = predict_if_needed(nj);
+    if (rc) return rc;
     if (index && ni <= G.pending_cap) memcpy(G.pending_ids, index, sizeof(int) * (size_t)ni);
   }
   G.pending_nj = nj;
@@ -718,20 +727,11 @@ static int launch_force_host(int want_nn) {
     G.pending = 0;
     return rc;
   }
-  /* Error word + live prefix of each output section. */
-  CK(cudaMemcpyAsync(G.h_out, G.d_out, 16, cudaMemcpyDeviceToHost, G.st));
-  CK(cudaMemcpyAsync(OUT_ACC(G.h_out), OUT_ACC(G.d_out), sizeof(double) * 3 * (size_t)ni,
+  /* Error word and results in one copy (the neighbours at its end). */
+  CK(cudaMemcpyAsync(G.h_out, G.d_out,
+                     16 + sizeof(double) * 7 * (size_t)ni +
+                         (want_nn ? (sizeof(int) + sizeof(float)) * (size_t)ni : 0),
                      cudaMemcpyDeviceToHost, G.st));
-  CK(cudaMemcpyAsync(OUT_JERK(G.h_out), OUT_JERK(G.d_out), sizeof(double) * 3 * (size_t)ni,
-                     cudaMemcpyDeviceToHost, G.st));
-  CK(cudaMemcpyAsync(OUT_POT(G.h_out), OUT_POT(G.d_out), sizeof(double) * (size_t)ni,
-                     cudaMemcpyDeviceToHost, G.st));
-  if (want_nn) {
-    CK(cudaMemcpyAsync(OUT_NN(G.h_out), OUT_NN(G.d_out), sizeof(int) * (size_t)ni,
-                       cudaMemcpyDeviceToHost, G.st));
-    CK(cudaMemcpyAsync(OUT_NNR2(G.h_out), OUT_NNR2(G.d_out), sizeof(float) * (size_t)ni,
-                       cudaMemcpyDeviceToHost, G.st));
-  }
   CK(cudaEventRecord(G.ev_done, G.st));
   return 0;
 }
@@ -847,7 +847,8 @@ int g6_read_neighbour_list_(int *cluster_id) {
     seterr("g6_read_neighbour_list before g6calc_lasthalf");
     return G6_ERR_STATE;
   }
-  const int ni = G.pending_ni;
+  /* (a firsthalf since then may have laid the block out for fewer) */
+  const int ni = G.pending_ni < G.io_n ? G.pending_ni : G.io_n;
   if (ni <= 0) return 0;
   const size_t per = (size_t)(G6_NGB_MAX + 1);
   if (ni > ngb_cap) {

@@ -1732,14 +1732,14 @@ int launch(const KParams &kp, int jl, int gx, cudaStream_t st, cudaEvent_t ev_mi
   // instantiation; small blocks are latency-bound and keep the nn code.
   if (kp.hjerk) {
     if (jl != 1 || kp.want_nn) return -2;
-    force_kernel<P, 1, false, true><<<grid, block, 0, st>>>(kp);
+    launch_pdl(force_kernel<P, 1, false, true>, grid, block, 0, st, kp);
   } else switch (jl) {
 #define G6_CASE(J)                                            \
   case J:                                                     \
     if (kp.want_nn)                                           \
-      force_kernel<P, J, true><<<grid, block, 0, st>>>(kp);  \
+      launch_pdl(force_kernel<P, J, true>, grid, block, 0, st, kp);  \
     else                                                      \
-      force_kernel<P, J, false><<<grid, block, 0, st>>>(kp); \
+      launch_pdl(force_kernel<P, J, false>, grid, block, 0, st, kp); \
     break;
     G6_CASE(1)
     G6_CASE(2)

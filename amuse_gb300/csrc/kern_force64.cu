@@ -365,11 +365,11 @@ extern "C" int g6k_force64(const g6_force_args *a, unsigned *ticket, int groups_
   }
   const dim3 grid(gx, s.nsplit), block(32);
   if (a->hjerk)
-    force64_kernel<false, true><<<grid, block, 0, st>>>(k, s.il_log2);
+    launch_pdl(force64_kernel<false, true>, grid, block, 0, st, k, s.il_log2);
   else if (a->want_nn)
-    force64_kernel<true, false><<<grid, block, 0, st>>>(k, s.il_log2);
+    launch_pdl(force64_kernel<true, false>, grid, block, 0, st, k, s.il_log2);
   else
-    force64_kernel<false, false><<<grid, block, 0, st>>>(k, s.il_log2);
+    launch_pdl(force64_kernel<false, false>, grid, block, 0, st, k, s.il_log2);
   if (a->ev_mid) cudaEventRecord(a->ev_mid, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

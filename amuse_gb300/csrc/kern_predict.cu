@@ -37,6 +37,7 @@ constexpr int PT = 256;
 constexpr double FAR = 1.0e18;
 
 __global__ void scatter_kernel(g6_jstate js, const g6_jupd *__restrict__ upd, int n) {
+  pdl_trigger();  // the predictor waits for this kernel's end
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n) return;
   const g6_jupd r = upd[u];
@@ -118,6 +119,8 @@ __device__ __forceinline__ void predict_one(const g6_jstate &js, int s, int nj, 
 
 template <int PREC>
 __global__ void __launch_bounds__(PT) predict_kernel(g6_jstate js, int nj, int nj_pad, double ti) {
+  pdl_wait();
+  pdl_trigger();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nj_pad) return;
   predict_one<PREC>(js, s, nj, ti);
@@ -156,7 +159,9 @@ int predict_threads(int nj_pad) { return nj_pad <= 8 * 32 * g6k_sm_count() ? 32 
 
 extern "C" int g6k_scatter(const g6_jstate *js, const g6_jupd *d_upd, int n, cudaStream_t st) {
   if (n <= 0) return 0;
-  scatter_kernel<<<(n + PT - 1) / PT, PT, 0, st>>>(*js, d_upd, n);
+  // one record per thread, a warp per CTA: the records' latency (host memory,
+  // for a block's) is what this takes, not their number
+  scatter_kernel<<<(n + 31) / 32, 32, 0, st>>>(*js, d_upd, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -166,11 +171,13 @@ extern "C" int g6k_predict(const g6_jstate *js, int nj, double ti, int prec, cud
   if (nj_pad > js->cap) return -1;
   const int threads = predict_threads(nj_pad);
   const int grid = (nj_pad + threads - 1) / threads;
-  if (prec == G6_PREC_FP64)
-    predict_kernel<G6_PREC_FP64><<<grid, threads, 0, st>>>(*js, nj, nj_pad, ti);
-  else
-    predict_kernel<G6_PREC_SPLIT><<<grid, threads, 0, st>>>(*js, nj, nj_pad, ti);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  const cudaError_t e =
+      prec == G6_PREC_FP64
+          ? launch_pdl(predict_kernel<G6_PREC_FP64>, dim3(grid), dim3(threads), 0, st, *js, nj,
+                       nj_pad, ti)
+          : launch_pdl(predict_kernel<G6_PREC_SPLIT>, dim3(grid), dim3(threads), 0, st, *js, nj,
+                       nj_pad, ti);
+  return e == cudaSuccess ? 0 : -3;
 }
 
 extern "C" int g6k_list_predict(const g6_jstate *js, int nj, int prec,
