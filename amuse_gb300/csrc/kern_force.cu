@@ -873,11 +873,20 @@ __global__ void __launch_bounds__(NT, P::MINB) force_kernel(KParams kp) {
   pdl_wait();  // the predictor's records and the block list are complete
 
   // ---- j-range of this CTA ----
-  const int js = blockIdx.y * kp.jsplit;
-  int je = js + kp.jsplit;
-  const int nj_pad = (kp.nj + TJ - 1) / TJ * TJ;
-  if (je > nj_pad) je = nj_pad;
-  const int ntiles = je > js ? (je - js) / TJ : 0;
+  // Where every tile is folded by itself (JL <= 4) the splits differ by one
+  // tile at most; with more j-lanes a fold covers several tiles, counted from
+  // the split's first, and the splits keep equal lengths.
+  const int all = (kp.nj + TJ - 1) / TJ;
+  int t0, t1;
+  if (FOLD_TILES == 1) {
+    t0 = (int)((long long)all * blockIdx.y / kp.nsplit);
+    t1 = (int)((long long)all * (blockIdx.y + 1) / kp.nsplit);
+  } else {
+    t0 = min(all, (int)blockIdx.y * (kp.jsplit / TJ));
+    t1 = min(all, t0 + kp.jsplit / TJ);
+  }
+  const int js = t0 * TJ;
+  const int ntiles = t1 - t0;
   const Rec *gj = reinterpret_cast<const Rec *>(kp.jrec) + js / JPR;
 
   constexpr int NWARP = NT / 32;
@@ -1622,6 +1631,43 @@ struct ShapeKey {
 };
 ShapeKey g_shape_cache[256];
 
+// The number of splits where their lengths may differ by a tile (JL <= 4):
+// what counts is the tiles of the busiest SM.  In units of one tile's time on
+// an SM of its own, a CTA costs its tiles and OV; with up to three CTAs per SM
+// all run at once, fewer leave FP32 cycles unused (EFF); beyond that slots
+// refill as CTAs end; the partial records cost their traffic.  Another count
+// than ns0 (choose_shape's, equal lengths) is taken where it should gain 1 %.
+// Measured with the second pass: 8192 x 8192 121 -> 103 us (11 -> 32 splits:
+// 2.3 CTAs of three tiles per SM, some SMs with three, became 6.7 of one),
+// 16384 x 16384 with neighbours 449 -> 429 us, 11719 x 2^20 13.22 -> 12.97 ms
+// (11.8 CTAs per SM -> 23.0).
+int balanced_splits(int ni, int ntiles, int jl, int ns0, int force_nsplit) {
+  if (force_nsplit > 0) return force_nsplit < ntiles ? force_nsplit : ntiles;
+  const int sms = sm_count(), islots = (NT / jl) * IPT_SPLIT;
+  const long long gx = (ni + islots - 1) / islots;
+  const double OV = 0.28 * jl, EFF[3] = {0.6, 0.9, 0.96};
+  auto cost = [&](int ns) {
+    const long long c = (gx * ns + sms - 1) / sms;  // CTAs of the busiest SM
+    const double tiles = (double)ntiles / ns, merge = 3e-6 * jl * ni * (double)ns;
+    if (c <= 3) return (double)c * ((ntiles + ns - 1) / ns + OV) / EFF[c - 1] + merge;
+    return (double)c * (tiles + OV) + merge;
+  };
+  // within the fixed scratch array where the count before was
+  const size_t room = (size_t)16 << 20, rec = (size_t)ni * sizeof(SplitP::Out);
+  int best = ns0;
+  double bc = cost(ns0) * 0.99;
+  const int most = ntiles < 128 ? ntiles : 128;
+  for (int ns = 1; ns <= most; ns++) {
+    if (ns > ns0 && (size_t)ns0 * rec <= room && (size_t)ns * rec > room) break;
+    const double c = cost(ns);
+    if (c < bc) {
+      bc = c;
+      best = ns;
+    }
+  }
+  return best;
+}
+
 void choose_shape(int ni, int nj, int nn, int force_jl, int force_nsplit, int *jl_out,
                   int *nsplit_out, int *jsplit_out) {
   nn = nn ? 1 : 0;
@@ -1715,6 +1761,7 @@ void choose_shape(int ni, int nj, int nn, int force_jl, int force_nsplit, int *j
   *jl_out = bjl;
   *nsplit_out = (ntiles + tp - 1) / tp;
   *jsplit_out = tp * TJ;
+  if (bjl <= 4) *nsplit_out = balanced_splits(ni, ntiles, bjl, *nsplit_out, force_nsplit);
   c.ni = ni;
   c.nj = nj;
   c.nn = nn;
