@@ -2030,15 +2030,13 @@ int g6x_batch_tune(int nsys, const int *n_per_sys, const double *t_end, const do
  * torch.autograd.Function).  All calls are blocking. */
 int g6k_fixed_records(const g6_jstate *js, int n, const double *x, const double *v,
                       const double *m, int prec, cudaStream_t st);
-int g6k_fixed_predict(int n, double h, const double *x, const double *v, const double *a,
-                      const double *j, double *xp, double *vp, cudaStream_t st);
-int g6k_fixed_correct(int n, double h, double *x, double *v, double *a, double *j,
-                      const double *a1, const double *j1, cudaStream_t st);
-int g6k_fixed_adj_pre(int n, double h, double *lx, double *lv, double *la, double *lj,
-                      double *la1, double *lj1, cudaStream_t st);
-int g6k_fixed_adj_post(int n, double h, double *lx, double *lv, double *la, double *lj,
-                       const double *gxp, const double *gvp, double *lm, const double *gm,
-                       cudaStream_t st);
+int g6k_fixed_advance(const g6_jstate *js, int n, double h, int correct, int predict, double *x,
+                      double *v, double *a, double *j, const double *a1, const double *j1,
+                      const double *m, double *xp, double *vp, int prec, cudaStream_t st);
+int g6k_fixed_adjoint(int n, double h, double eps2, int nsteps, int prec, int hjerk,
+                      const double *xp_all, const double *vp_all, const double *m, double *lx,
+                      double *lv, double *la, double *lj, double *lm, double *la1, double *lj1,
+                      double *gxp, double *gvp, double *gm, void *scratch, cudaStream_t st);
 size_t g6k_vjp_scratch_bytes(int n);
 int g6k_force_vjp(int n, double eps2, int prec, int hjerk, const double *x, const double *v,
                   const double *m, const double *la1, const double *lj1, double *gx, double *gv,
@@ -2092,15 +2090,16 @@ static int fixed_buffers(int n) {
 /* The fixed-step calls enqueue on the library stream; the public entry
    points below synchronise once at their end and then check the force
    kernel's error word. */
-static int fixed_force_async(int n, double eps2, const double *d_x, const double *d_v,
-                             const double *d_m, double *d_a, double *d_j) {
+static int fixed_ready(int n) {
   int rc = grow_j((n + G6_TILE - 1) / G6_TILE * G6_TILE);
   if (rc) return rc;
   rc = ensure_run_buffers(n);
   if (rc) return rc;
-  rc = identity_list(n);
-  if (rc) return rc;
-  if (g6k_fixed_records(&G.js, n, d_x, d_v, d_m, G.prec, G.st)) return G6_ERR_CUDA;
+  return identity_list(n);
+}
+
+/* The force on all bodies from the records, which are ready. */
+static int fixed_force_records(int n, double eps2, double *d_a, double *d_j) {
   G.pred_valid = 0; /* the records no longer hold a prediction of the j-state */
   g6_force_args a;
   memset(&a, 0, sizeof(a));
@@ -2117,27 +2116,43 @@ static int fixed_force_async(int n, double eps2, const double *d_x, const double
   return run_force(&a);
 }
 
-static int fixed_step_async(int n, double h, double eps2, double *d_x, double *d_v, double *d_a,
-                            double *d_j, const double *d_m, double *d_xp, double *d_vp) {
-  if (g6k_fixed_predict(n, h, d_x, d_v, d_a, d_j, d_xp, d_vp, G.st)) return G6_ERR_CUDA;
-  int rc = fixed_force_async(n, eps2, d_xp, d_vp, d_m, fx_a1, fx_j1);
+static int fixed_force_async(int n, double eps2, const double *d_x, const double *d_v,
+                             const double *d_m, double *d_a, double *d_j) {
+  int rc = fixed_ready(n);
   if (rc) return rc;
-  if (g6k_fixed_correct(n, h, d_x, d_v, d_a, d_j, fx_a1, fx_j1, G.st)) return G6_ERR_CUDA;
+  if (g6k_fixed_records(&G.js, n, d_x, d_v, d_m, G.prec, G.st)) return G6_ERR_CUDA;
+  return fixed_force_records(n, eps2, d_a, d_j);
+}
+
+/* nsteps steps in place; step s's predicted state goes to d_xp + s * stride. */
+static int fixed_steps_async(int n, double h, double eps2, int nsteps, double *d_x, double *d_v,
+                             double *d_a, double *d_j, const double *d_m, double *d_xp,
+                             double *d_vp, size_t stride) {
+  if (nsteps <= 0) return 0;
+  int rc = fixed_ready(n);
+  if (rc) return rc;
+  G.pred_valid = 0;
+  for (int s = 0; s <= nsteps; s++) {
+    const size_t o = stride * (size_t)s;
+    if (g6k_fixed_advance(&G.js, n, h, s > 0, s < nsteps, d_x, d_v, d_a, d_j, fx_a1, fx_j1, d_m,
+                          s < nsteps ? d_xp + o : NULL, s < nsteps ? d_vp + o : NULL, G.prec,
+                          G.st))
+      return G6_ERR_CUDA;
+    if (s == nsteps) break;
+    rc = fixed_force_records(n, eps2, fx_a1, fx_j1);
+    if (rc) return rc;
+  }
   return 0;
 }
 
-static int fixed_step_adjoint_async(int n, double h, double eps2, const double *d_xp,
-                                    const double *d_vp, const double *d_m, double *d_lx,
-                                    double *d_lv, double *d_la, double *d_lj, double *d_lm,
-                                    double *d_work) {
-  double *gxp = d_work, *gvp = d_work + 3 * (size_t)n, *gm = d_work + 6 * (size_t)n;
-  if (g6k_fixed_adj_pre(n, h, d_lx, d_lv, d_la, d_lj, fx_a1, fx_j1, G.st)) return G6_ERR_CUDA;
-  if (g6k_force_vjp(n, eps2, G.prec, fx_form == G6_JERK_HERMITE, d_xp, d_vp, d_m, fx_a1, fx_j1,
-                    gxp, gvp, gm, fx_part, G.st))
-    return G6_ERR_CUDA;
-  if (g6k_fixed_adj_post(n, h, d_lx, d_lv, d_la, d_lj, gxp, gvp, d_lm, gm, G.st))
-    return G6_ERR_CUDA;
-  return 0;
+static int fixed_adjoints_async(int n, double h, double eps2, int nsteps, const double *d_xp,
+                                const double *d_vp, const double *d_m, double *d_lx, double *d_lv,
+                                double *d_la, double *d_lj, double *d_lm, double *d_work) {
+  return g6k_fixed_adjoint(n, h, eps2, nsteps, G.prec, fx_form == G6_JERK_HERMITE, d_xp, d_vp, d_m,
+                           d_lx, d_lv, d_la, d_lj, d_lm, fx_a1, fx_j1, d_work,
+                           d_work + 3 * (size_t)n, d_work + 6 * (size_t)n, fx_part, G.st)
+             ? G6_ERR_CUDA
+             : 0;
 }
 
 static int fixed_finish(void) {
@@ -2164,7 +2179,7 @@ int g6x_fixed_step(int n, double h, double eps2, double *d_x, double *d_v, doubl
   if (n <= 0 || !d_xp || !d_vp) return G6_ERR_ARG;
   rc = fixed_buffers(n);
   if (rc) return rc;
-  rc = fixed_step_async(n, h, eps2, d_x, d_v, d_a, d_j, d_m, d_xp, d_vp);
+  rc = fixed_steps_async(n, h, eps2, 1, d_x, d_v, d_a, d_j, d_m, d_xp, d_vp, 0);
   return rc ? rc : fixed_finish();
 }
 
@@ -2179,13 +2194,10 @@ int g6x_fixed_run(int n, double h, double eps2, int nsteps, double *d_x, double 
   if (n <= 0 || nsteps < 0 || (!d_xp_all) != (!d_vp_all)) return G6_ERR_ARG;
   rc = fixed_buffers(n);
   if (rc) return rc;
-  for (int s = 0; s < nsteps; s++) {
-    const size_t o = d_xp_all ? 3 * (size_t)n * (size_t)s : 0;
-    rc = fixed_step_async(n, h, eps2, d_x, d_v, d_a, d_j, d_m, d_xp_all ? d_xp_all + o : fx_xp,
-                          d_vp_all ? d_vp_all + o : fx_vp);
-    if (rc) return rc;
-  }
-  return fixed_finish();
+  rc = fixed_steps_async(n, h, eps2, nsteps, d_x, d_v, d_a, d_j, d_m,
+                         d_xp_all ? d_xp_all : fx_xp, d_vp_all ? d_vp_all : fx_vp,
+                         d_xp_all ? 3 * (size_t)n : 0);
+  return rc ? rc : fixed_finish();
 }
 
 /* Vector-Jacobian product of the force at (x, v): given cotangents la/lj of
@@ -2214,8 +2226,7 @@ int g6x_fixed_step_adjoint(int n, double h, double eps2, const double *d_xp, con
   if (n <= 0 || !d_work) return G6_ERR_ARG;
   rc = fixed_buffers(n);
   if (rc) return rc;
-  rc = fixed_step_adjoint_async(n, h, eps2, d_xp, d_vp, d_m, d_lx, d_lv, d_la, d_lj, d_lm,
-                                d_work);
+  rc = fixed_adjoints_async(n, h, eps2, 1, d_xp, d_vp, d_m, d_lx, d_lv, d_la, d_lj, d_lm, d_work);
   return rc ? rc : fixed_finish();
 }
 
@@ -2230,11 +2241,7 @@ int g6x_fixed_adjoint_run(int n, double h, double eps2, int nsteps, const double
   if (n <= 0 || nsteps < 0 || !d_work || !d_xp_all || !d_vp_all) return G6_ERR_ARG;
   rc = fixed_buffers(n);
   if (rc) return rc;
-  for (int s = nsteps - 1; s >= 0; s--) {
-    const size_t o = 3 * (size_t)n * (size_t)s;
-    rc = fixed_step_adjoint_async(n, h, eps2, d_xp_all + o, d_vp_all + o, d_m, d_lx, d_lv, d_la,
-                                  d_lj, d_lm, d_work);
-    if (rc) return rc;
-  }
-  return fixed_finish();
+  rc = fixed_adjoints_async(n, h, eps2, nsteps, d_xp_all, d_vp_all, d_m, d_lx, d_lv, d_la, d_lj,
+                            d_lm, d_work);
+  return rc ? rc : fixed_finish();
 }

@@ -34,6 +34,7 @@
 // (q = s recovers the softened form).
 // The VJP runs in split precision (double-single r, FP32 pair math, per-tile
 // FP32 partials folded into FP64 totals) or in FP64.
+#include "pdl.cuh"
 #include <cuda_runtime.h>
 
 #include "f32x2.cuh"
@@ -45,28 +46,18 @@ struct __align__(32) G6D4 {
 
 namespace {
 
-constexpr int PT = 256;
-constexpr int VT = 128;  // VJP threads per CTA
+constexpr int VT = 32;  // FP64 VJP threads per CTA
 constexpr int VTILE = 128;
 
-__global__ void records_kernel(int n, int n_pad, const double *__restrict__ x,
-                               const double *__restrict__ v, const double *__restrict__ m,
-                               int prec, void *jp_split, void *jp_f64) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n_pad) return;
-  double xp[3], vp[3], mm;
-  if (s < n) {
-    for (int k = 0; k < 3; k++) {
-      xp[k] = x[3 * s + k];
-      vp[k] = v[3 * s + k];
-    }
-    mm = m[s];
-  } else {
-    for (int k = 0; k < 3; k++) {
-      xp[k] = 1.0e18;
-      vp[k] = 0.0;
-    }
-    mm = 0.0;
+// One force record from a body's state (s >= n: padding, massless and far).
+__device__ __forceinline__ void store_record(int s, int n, const double x[3], const double v[3],
+                                             double m, int prec, void *jp_split, void *jp_f64) {
+  double xp[3], vp[3];
+  const double mm = s < n ? m : 0.0;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    xp[k] = s < n ? x[k] : 1.0e18;
+    vp[k] = s < n ? v[k] : 0.0;
   }
   if (prec == G6_PREC_FP64) {
     G6D4 *r = reinterpret_cast<G6D4 *>(jp_f64) + 2 * (size_t)s;
@@ -85,59 +76,64 @@ __global__ void records_kernel(int n, int n_pad, const double *__restrict__ x,
   }
 }
 
-__global__ void predict_kernel(int n, double h, const double *__restrict__ x,
-                               const double *__restrict__ v, const double *__restrict__ a,
-                               const double *__restrict__ j, double *xp, double *vp) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 3 * n) return;
-  // hermite predict_step: pos += vel*dt + acc*dt*dt/2 + jerk*dt*dt*dt/6
-  xp[e] = x[e] + (v[e] * h + a[e] * h * h / 2 + j[e] * h * h * h / 6);
-  vp[e] = v[e] + (a[e] * h + j[e] * h * h / 2);
+__global__ void records_kernel(int n, int n_pad, const double *__restrict__ x,
+                               const double *__restrict__ v, const double *__restrict__ m,
+                               int prec, void *jp_split, void *jp_f64) {
+  pdl_wait();
+  pdl_trigger();
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= n_pad) return;
+  double xs[3] = {0, 0, 0}, vs[3] = {0, 0, 0};
+  if (s < n)
+    for (int k = 0; k < 3; k++) xs[k] = x[3 * s + k], vs[k] = v[3 * s + k];
+  store_record(s, n, xs, vs, s < n ? m[s] : 0.0, prec, jp_split, jp_f64);
 }
 
-__global__ void correct_kernel(int n, double h, double *x, double *v, double *a, double *j,
-                               const double *__restrict__ a1, const double *__restrict__ j1) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 3 * n) return;
-  const double v0 = v[e], a0 = a[e], jj0 = j[e], an = a1[e], jn = j1[e];
-  // hermite correct_step
-  const double vn = v0 + (a0 + an) * h / 2 + (jj0 - jn) * h * h / 12;
-  x[e] = x[e] + (v0 + vn) * h / 2 + (a0 - an) * h * h / 12;
-  v[e] = vn;
-  a[e] = an;
-  j[e] = jn;
-}
-
-// Adjoint, first half: step-output adjoints in (lx, lv, la, lj) become the
-// corrector's input-adjoint contributions (in place); la1/lj1 receive the
-// adjoints of the force outputs (the VJP's cotangents).
-__global__ void adj_pre_kernel(int n, double h, double *lx, double *lv, double *la, double *lj,
-                               double *la1, double *lj1) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 3 * n) return;
-  const double Lx = lx[e], Lv = lv[e], La = la[e], Lj = lj[e];
-  const double Lvt = Lv + Lx * h / 2;
-  la1[e] = La - Lx * h * h / 12 + Lvt * h / 2;
-  lj1[e] = Lj - Lvt * h * h / 12;
-  lx[e] = Lx;
-  lv[e] = Lx * h / 2 + Lvt;
-  la[e] = Lx * h * h / 12 + Lvt * h / 2;
-  lj[e] = Lvt * h * h / 12;
-}
-
-// Adjoint, second half: add the predictor's pull-back of (gxp, gvp).
-// lm (if not NULL) accumulates the mass cotangent gm.
-__global__ void adj_post_kernel(int n, double h, double *lx, double *lv, double *la, double *lj,
-                                const double *__restrict__ gxp, const double *__restrict__ gvp,
-                                double *lm, const double *__restrict__ gm) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 3 * n) return;
-  if (lm && e < n) lm[e] += gm[e];
-  const double gx = gxp[e], gv = gvp[e];
-  lx[e] += gx;
-  lv[e] += gx * h + gv;
-  la[e] += gx * h * h / 2 + gv * h;
-  lj[e] += gx * h * h * h / 6 + gv * h * h / 2;
+// What lies between two force evaluations of a fixed-step run, a body per
+// thread: the corrector of the step that ends (CORRECT) and the prediction
+// and force records of the one that begins (PREDICT).  Three launches before,
+// 4 us each at n = 8192; one warp per CTA, since the ~60 FP64 instructions of a
+// warp take 64 cycles of its scheduler each.
+template <bool CORRECT, bool PREDICT>
+__global__ void __launch_bounds__(32) advance_kernel(int n, int n_pad, double h, double *x,
+                                                     double *v, double *a, double *j,
+                                                     const double *__restrict__ a1,
+                                                     const double *__restrict__ j1,
+                                                     const double *__restrict__ m, double *xp,
+                                                     double *vp, int prec, void *jp_split,
+                                                     void *jp_f64) {
+  pdl_wait();
+  pdl_trigger();
+  const int s = blockIdx.x * 32 + threadIdx.x;
+  if (s >= n_pad) return;
+  double xs[3] = {0, 0, 0}, vs[3] = {0, 0, 0};
+  if (s < n) {
+    const double hh = 0.5 * h, h2 = h * h / 2, h12 = h * h / 12, h6 = h * h * h / 6;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const int e = 3 * s + k;
+      double X = x[e], V = v[e], A = a[e], J = j[e];
+      if (CORRECT) {  // hermite correct_step
+        const double an = a1[e], jn = j1[e];
+        const double vn = V + (A + an) * hh + (J - jn) * h12;
+        X = X + (V + vn) * hh + (A - an) * h12;
+        V = vn;
+        A = an;
+        J = jn;
+        x[e] = X;
+        v[e] = V;
+        a[e] = A;
+        j[e] = J;
+      }
+      if (PREDICT) {  // predict_step: pos += vel*dt + acc*dt*dt/2 + jerk*dt*dt*dt/6
+        xs[k] = X + (V * h + A * h2 + J * h6);
+        vs[k] = V + (A * h + J * h2);
+        xp[e] = xs[k];
+        vp[e] = vs[k];
+      }
+    }
+  }
+  if (PREDICT) store_record(s, n, xs, vs, s < n ? m[s] : 0.0, prec, jp_split, jp_f64);
 }
 
 // ---- force VJP, FP64 ----
@@ -145,8 +141,33 @@ struct VRecD {
   double x[3], v[3], m, la[3], lj[3];
 };
 
-// One body k per thread, j in shared-memory tiles of VTILE, the j range
-// split over gridDim.y CTA rows; m < 0 marks padding.
+// FP64 MUFU seeds and one third-order step (kern_force64.cu); the divisions
+// outside the seeds' range.
+__device__ __forceinline__ bool mid_range(double x) {
+  return (unsigned)__double2hiint(x) - (723u << 20) < (600u << 20);  // 2^-300 <= x < 2^300
+}
+__device__ __forceinline__ double rsqrt64(double x) {
+  if (!mid_range(x)) return 1.0 / sqrt(x);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = __fma_rn(-(x * y), y, 1.0);
+  return __fma_rn(h * y, __fma_rn(0.375, h, 0.5), y);
+}
+__device__ __forceinline__ double rcp64(double x) {
+  if (!mid_range(x)) return 1.0 / x;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = __fma_rn(-x, y, 1.0);
+  return __fma_rn(y, __fma_rn(h, h, h), y);
+}
+
+// One body k per thread, one warp per CTA (an FP64 instruction takes 64 cycles
+// of the warp's scheduler: warps spread over the SMs), j in shared-memory
+// tiles of VTD, the j range split over gridDim.y CTA rows.  Of n = 128 .. 1024
+// bodies, four-warp CTAs with IEEE divisions and a square root per pair took 7
+// to 15 times as long (8 steps with their adjoint, n = 1024: 39.9 -> 4.9 ms
+// with the FP64 force's part).
+constexpr int VTD = 32;
 template <bool HJ>
 __global__ void __launch_bounds__(VT) vjp_f64_kernel(int n, double eps2,
                                                      const double *__restrict__ x,
@@ -155,7 +176,9 @@ __global__ void __launch_bounds__(VT) vjp_f64_kernel(int n, double eps2,
                                                      const double *__restrict__ la1,
                                                      const double *__restrict__ lj1, int jsplit,
                                                      double *part /* [nsplit][n][7] */) {
-  __shared__ VRecD td[VTILE];
+  __shared__ VRecD td[VTD];
+  pdl_wait();
+  pdl_trigger();
   eps2 += 1.0 / 4503599627370496.0;  // the force kernel's softening (+2^-52, as ph4)
   const int k = blockIdx.x * VT + threadIdx.x;
   const bool valid = k < n;
@@ -167,30 +190,23 @@ __global__ void __launch_bounds__(VT) vjp_f64_kernel(int n, double eps2,
   const double mk = m[kk];
   const double lak[3] = {la1[3 * kk], la1[3 * kk + 1], la1[3 * kk + 2]};
   const double ljk[3] = {lj1[3 * kk], lj1[3 * kk + 1], lj1[3 * kk + 2]};
-  double tot[7] = {0, 0, 0, 0, 0, 0, 0};  // gx[3], gv[3], gm
-  for (int t0 = j0; t0 < j1; t0 += VTILE) {
-    __syncthreads();
-    for (int q = threadIdx.x; q < VTILE; q += VT) {
-      const int jj = t0 + q;
-      VRecD &r = td[q];
-      if (jj < j1) {
-        for (int c = 0; c < 3; c++) {
-          r.x[c] = x[3 * jj + c];
-          r.v[c] = v[3 * jj + c];
-          r.la[c] = la1[3 * jj + c];
-          r.lj[c] = lj1[3 * jj + c];
-        }
-        r.m = m[jj];
-      } else {
-        for (int c = 0; c < 3; c++) r.x[c] = r.v[c] = r.la[c] = r.lj[c] = 0.0;
-        r.m = -1.0;
-      }
+  double acc[7] = {0, 0, 0, 0, 0, 0, 0};  // gx[3], gv[3], gm
+  for (int t0 = j0; t0 < j1; t0 += VTD) {
+    __syncwarp();
+    const int jj = min(t0 + (int)threadIdx.x, n - 1);
+    VRecD &w = td[threadIdx.x];
+    for (int c = 0; c < 3; c++) {
+      w.x[c] = x[3 * jj + c];
+      w.v[c] = v[3 * jj + c];
+      w.la[c] = la1[3 * jj + c];
+      w.lj[c] = lj1[3 * jj + c];
     }
-    __syncthreads();
-    double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-    for (int q = 0; q < VTILE; q++) {
+    w.m = m[jj];
+    __syncwarp();
+    const int nq = min(VTD, j1 - t0);
+    for (int q = 0; q < nq; q++) {
       const VRecD &r = td[q];
-      if (r.m < 0.0 || t0 + q == k) continue;
+      if (t0 + q == k) continue;
       double R[3], V[3], lam[3], mu[3];
       for (int c = 0; c < 3; c++) {
         R[c] = r.x[c] - xk[c];
@@ -198,39 +214,40 @@ __global__ void __launch_bounds__(VT) vjp_f64_kernel(int n, double eps2,
         lam[c] = mk * r.la[c] - r.m * lak[c];
         mu[c] = mk * r.lj[c] - r.m * ljk[c];
       }
-      const double s = R[0] * R[0] + R[1] * R[1] + R[2] * R[2] + eps2;
-      const double si = 1.0 / s, s1 = sqrt(si);
-      const double s3 = s1 * si, s5 = s3 * si, s7 = s5 * si;
-      const double rl = R[0] * lam[0] + R[1] * lam[1] + R[2] * lam[2];
+      const double r2 = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
+      const double s1 = rsqrt64(r2 + eps2), si = s1 * s1;
+      const double s3 = s1 * si, s5 = s3 * si;
+      // lam.r + mu.v and the other dot products
+      const double rlvm = R[0] * lam[0] + R[1] * lam[1] + R[2] * lam[2] + V[0] * mu[0] +
+                          V[1] * mu[1] + V[2] * mu[2];
       const double rm = R[0] * mu[0] + R[1] * mu[1] + R[2] * mu[2];
-      const double vm = V[0] * mu[0] + V[1] * mu[1] + V[2] * mu[2];
       const double rv = R[0] * V[0] + R[1] * V[1] + R[2] * V[2];
-      // qs = q^-1 s^-3/2 (s^-5/2 in the softened form), c7 = 15 s^-7/2 resp.
-      // 3 (2 q^-2 s^-3/2 + 3 q^-1 s^-5/2)
-      double qs, c7;
+      // q3 = -3 q^-1 s^-3/2 (-3 s^-5/2 in the softened form); the last term of
+      // cr is 15 s^-7/2 resp. 3 (2 q^-2 s^-3/2 + 3 q^-1 s^-5/2) times rv rm
+      double q3, d;
       if (HJ) {
-        const double qi = 1.0 / (R[0] * R[0] + R[1] * R[1] + R[2] * R[2]);
-        qs = qi * s3;
-        c7 = 3.0 * (2.0 * qi * qs + 3.0 * qi * s5);
+        const double qi = rcp64(r2);
+        q3 = -3.0 * (qi * s3);
+        d = 2.0 * qi + 3.0 * si;
       } else {
-        qs = s5;
-        c7 = 15.0 * s7;
+        q3 = -3.0 * s5;
+        d = 5.0 * si;
       }
-      const double cr = -3.0 * (rl * s5 + vm * s5) + rv * rm * c7;
+      const double w5 = q3 * rm, y = q3 * rv;
+      const double cr = -3.0 * (rlvm * s5) - (y * rm) * d;
       for (int c = 0; c < 3; c++) {
-        acc[c] += lam[c] * s3 + cr * R[c] - 3.0 * qs * (rm * V[c] + rv * mu[c]);
-        acc[3 + c] += mu[c] * s3 - 3.0 * rm * qs * R[c];
+        acc[c] += lam[c] * s3 + cr * R[c] + w5 * V[c] + y * mu[c];
+        acc[3 + c] += mu[c] * s3 + w5 * R[c];
       }
-      const double ga = (r.la[0] * R[0] + r.la[1] * R[1] + r.la[2] * R[2]) * s3;
-      const double lv = r.lj[0] * V[0] + r.lj[1] * V[1] + r.lj[2] * V[2];
+      const double g = r.la[0] * R[0] + r.la[1] * R[1] + r.la[2] * R[2] + r.lj[0] * V[0] +
+                       r.lj[1] * V[1] + r.lj[2] * V[2];
       const double lr = r.lj[0] * R[0] + r.lj[1] * R[1] + r.lj[2] * R[2];
-      acc[6] -= ga + lv * s3 - 3.0 * rv * lr * qs;
+      acc[6] -= g * s3 + y * lr;
     }
-    for (int c = 0; c < 7; c++) tot[c] += acc[c];
   }
   if (valid) {
     double *p = part + ((size_t)blockIdx.y * n + k) * 7;
-    for (int c = 0; c < 7; c++) p[c] = tot[c];
+    for (int c = 0; c < 7; c++) p[c] = acc[c];
   }
 }
 
@@ -263,22 +280,19 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
-__global__ void vjp_records_kernel(int n, int n_pad, const double *__restrict__ x,
-                                   const double *__restrict__ v, const double *__restrict__ m,
-                                   const double *__restrict__ la1, const double *__restrict__ lj1,
-                                   VJPair *rec) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n_pad) return;
+__device__ __forceinline__ void store_vjp_record(int s, int n, const double x[3],
+                                                 const double v[3], double m, const double la[3],
+                                                 const double lj[3], VJPair *rec) {
   float f[VF];
   if (s < n) {
     for (int k = 0; k < 3; k++) {
-      f[k] = __double2float_rn(x[3 * s + k]);
-      f[4 + k] = __double2float_rn(x[3 * s + k] - (double)f[k]);
-      f[7 + k] = __double2float_rn(v[3 * s + k]);
-      f[10 + k] = __double2float_rn(la1[3 * s + k]);
-      f[13 + k] = __double2float_rn(lj1[3 * s + k]);
+      f[k] = __double2float_rn(x[k]);
+      f[4 + k] = __double2float_rn(x[k] - (double)f[k]);
+      f[7 + k] = __double2float_rn(v[k]);
+      f[10 + k] = __double2float_rn(la[k]);
+      f[13 + k] = __double2float_rn(lj[k]);
     }
-    f[3] = __double2float_rn(m[s]);
+    f[3] = __double2float_rn(m);
   } else {
     for (int k = 0; k < VF; k++) f[k] = 0.f;
     f[0] = f[1] = f[2] = 1.0e18f;
@@ -287,11 +301,80 @@ __global__ void vjp_records_kernel(int n, int n_pad, const double *__restrict__ 
   for (int k = 0; k < VF; k++) dst[2 * k] = f[k];
 }
 
+__global__ void vjp_records_kernel(int n, int n_pad, const double *__restrict__ x,
+                                   const double *__restrict__ v, const double *__restrict__ m,
+                                   const double *__restrict__ la1, const double *__restrict__ lj1,
+                                   VJPair *rec) {
+  pdl_wait();
+  pdl_trigger();
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= n_pad) return;
+  const int e = 3 * (s < n ? s : 0);
+  store_vjp_record(s, n, x + e, v + e, m[s < n ? s : 0], la1 + e, lj1 + e, rec);
+}
+
+// Between two force VJPs of the adjoint, a body per thread.  POST: the step
+// whose VJP (gxp, gvp, gm) is done, the predictor's pull-back; lm (if not
+// NULL) accumulates the mass cotangent.  PRE: the step before it, the
+// corrector's transpose: step-output adjoints in (lx, lv, la, lj) become the
+// corrector's input-adjoint contributions (in place), and the adjoints of the
+// force outputs go into the VJP's records (split) or la1, lj1 (FP64).
+template <bool POST, bool PRE>
+__global__ void __launch_bounds__(32) adjoint_kernel(
+    int n, int n_pad, double h, double *lx, double *lv, double *la, double *lj,
+    const double *__restrict__ gxp, const double *__restrict__ gvp, double *lm,
+    const double *__restrict__ gm, const double *__restrict__ x, const double *__restrict__ v,
+    const double *__restrict__ m, double *la1, double *lj1, VJPair *rec) {
+  pdl_wait();
+  pdl_trigger();
+  const int s = blockIdx.x * 32 + threadIdx.x;
+  if (s >= n_pad) return;
+  double ca[3] = {0, 0, 0}, cj[3] = {0, 0, 0};
+  if (s < n) {
+    const double hh = 0.5 * h, h2 = h * h / 2, h12 = h * h / 12, h6 = h * h * h / 6;
+    if (POST && lm) lm[s] += gm[s];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const int e = 3 * s + k;
+      double Lx = lx[e], Lv = lv[e], La = la[e], Lj = lj[e];
+      if (POST) {
+        const double gx = gxp[e], gv = gvp[e];
+        Lx += gx;
+        Lv += gx * h + gv;
+        La += gx * h2 + gv * h;
+        Lj += gx * h6 + gv * h2;
+      }
+      if (PRE) {
+        const double Lvt = Lv + Lx * hh;
+        ca[k] = La - Lx * h12 + Lvt * hh;
+        cj[k] = Lj - Lvt * h12;
+        if (!rec) {
+          la1[e] = ca[k];
+          lj1[e] = cj[k];
+        }
+        Lv = Lx * hh + Lvt;
+        La = Lx * h12 + Lvt * hh;
+        Lj = Lvt * h12;
+      }
+      lx[e] = Lx;
+      lv[e] = Lv;
+      la[e] = La;
+      lj[e] = Lj;
+    }
+  }
+  if (PRE && rec) {
+    const int e = 3 * (s < n ? s : 0);
+    store_vjp_record(s, n, x + e, v + e, m[s < n ? s : 0], ca, cj, rec);
+  }
+}
+
 template <bool HJ>
 __global__ void __launch_bounds__(VT2) vjp_split_kernel(int n, float eps2, const VJPair *__restrict__ rec,
                                                         int jsplit, int n_pad,
                                                         double *part /* [nsplit][n][7] */) {
   __shared__ VJPair tile[VTILE / 2];
+  pdl_wait();
+  pdl_trigger();
   f2x xh[VIPT][3], xl[VIPT][3], vk[VIPT][3], mk[VIPT], lak[VIPT][3], ljk[VIPT][3];
   int kk[VIPT];
 #pragma unroll
@@ -406,18 +489,25 @@ __global__ void __launch_bounds__(VT2) vjp_split_kernel(int n, float eps2, const
   }
 }
 
+// One quantity of one body per thread: consecutive threads read consecutive
+// doubles of every split, all splits in flight (a thread per body, walking its
+// splits 56 bytes apart, took 15 us at n = 8192; this takes 4).
 __global__ void vjp_reduce_kernel(int n, int nsplit, const double *__restrict__ part, double *gx,
                                   double *gv, double *gm) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  double t[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int s = 0; s < nsplit; s++)
-    for (int c = 0; c < 7; c++) t[c] += part[((size_t)s * n + k) * 7 + c];
-  for (int c = 0; c < 3; c++) {
-    gx[3 * k + c] = t[c];
-    gv[3 * k + c] = t[3 + c];
-  }
-  gm[k] = t[6];
+  pdl_wait();
+  pdl_trigger();
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 7 * n) return;
+  double t = 0;
+#pragma unroll 8
+  for (int s = 0; s < nsplit; s++) t += part[(size_t)s * n * 7 + e];
+  const int k = e / 7, c = e - 7 * k;
+  if (c < 3)
+    gx[3 * k + c] = t;
+  else if (c < 6)
+    gv[3 * k + c - 3] = t;
+  else
+    gm[k] = t;
 }
 
 }  // namespace
@@ -426,44 +516,43 @@ extern "C" int g6k_fixed_records(const g6_jstate *js, int n, const double *x, co
                                  const double *m, int prec, cudaStream_t st) {
   const int n_pad = (n + G6_TILE - 1) / G6_TILE * G6_TILE;
   if (n <= 0 || n_pad > js->cap) return -1;
-  records_kernel<<<(n_pad + PT - 1) / PT, PT, 0, st>>>(n, n_pad, x, v, m, prec, js->jp_split,
-                                                     js->jp_f64);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return launch_pdl(records_kernel, dim3((n_pad + 31) / 32), dim3(32), 0, st, n, n_pad, x, v, m,
+                    prec, js->jp_split, js->jp_f64) == cudaSuccess
+             ? 0
+             : -3;
 }
 
-extern "C" int g6k_fixed_predict(int n, double h, const double *x, const double *v,
-                                 const double *a, const double *j, double *xp, double *vp,
-                                 cudaStream_t st) {
-  predict_kernel<<<(3 * n + PT - 1) / PT, PT, 0, st>>>(n, h, x, v, a, j, xp, vp);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+// correct: the corrector with (a1, j1); predict: the next step's prediction
+// into xp, vp and the force records.
+extern "C" int g6k_fixed_advance(const g6_jstate *js, int n, double h, int correct, int predict,
+                                 double *x, double *v, double *a, double *j, const double *a1,
+                                 const double *j1, const double *m, double *xp, double *vp,
+                                 int prec, cudaStream_t st) {
+  const int n_pad = (n + G6_TILE - 1) / G6_TILE * G6_TILE;
+  if (n <= 0 || n_pad > js->cap || (!correct && !predict)) return -1;
+  auto kern = correct ? (predict ? advance_kernel<true, true> : advance_kernel<true, false>)
+                      : advance_kernel<false, true>;
+  return launch_pdl(kern, dim3(((predict ? n_pad : n) + 31) / 32), dim3(32), 0, st, n, n_pad, h, x,
+                    v, a, j, a1, j1, m, xp, vp, prec, js->jp_split, js->jp_f64) == cudaSuccess
+             ? 0
+             : -3;
 }
 
-extern "C" int g6k_fixed_correct(int n, double h, double *x, double *v, double *a, double *j,
-                                 const double *a1, const double *j1, cudaStream_t st) {
-  correct_kernel<<<(3 * n + PT - 1) / PT, PT, 0, st>>>(n, h, x, v, a, j, a1, j1);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
-}
-
-extern "C" int g6k_fixed_adj_pre(int n, double h, double *lx, double *lv, double *la, double *lj,
-                                 double *la1, double *lj1, cudaStream_t st) {
-  adj_pre_kernel<<<(3 * n + PT - 1) / PT, PT, 0, st>>>(n, h, lx, lv, la, lj, la1, lj1);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
-}
-
-extern "C" int g6k_fixed_adj_post(int n, double h, double *lx, double *lv, double *la,
-                                  double *lj, const double *gxp, const double *gvp, double *lm,
-                                  const double *gm, cudaStream_t st) {
-  adj_post_kernel<<<(3 * n + PT - 1) / PT, PT, 0, st>>>(n, h, lx, lv, la, lj, gxp, gvp, lm, gm);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
-}
-
-// Launch shapes.  FP64: one body per thread, j split over 1/4/8 CTA rows.
-// Split: VIPT bodies per thread, j split so that there are >= 4 CTAs per SM.
+// Launch shapes.  FP64: one body per thread, one warp per CTA.
+// Split: VIPT bodies per thread, j split so that there are about 24 CTAs per SM
+// (three at a time), so that the last ones to end leave few SMs idle: call of
+// 8192 bodies 274 us at 16 splits, 241 at 64; 16384: 950 at 10, 813 at 64;
+// 32768: 3.75 ms at 5, 3.09 at 32.
 static void vjp_shape(int n, int prec, int *nsplit, int *jsplit, int *n_pad) {
   *n_pad = (n + VTILE - 1) / VTILE * VTILE;
   if (prec == G6_PREC_FP64) {
-    *nsplit = n >= 8192 ? 8 : (n >= 1024 ? 4 : 1);
-    *jsplit = (n + *nsplit - 1) / *nsplit;
+    // about eight warps for every SM, no split below 16 j
+    const int warps = (n + VT - 1) / VT, want = 8 * g6k_sm_count();
+    int ns = (want + warps - 1) / warps;
+    if (ns > n / 16) ns = n / 16;
+    if (ns < 1) ns = 1;
+    *jsplit = (n + ns - 1) / ns;
+    *nsplit = (n + *jsplit - 1) / *jsplit;
     return;
   }
   static int sms = 0;  // SM count of the (single) device, looked up once
@@ -476,7 +565,7 @@ static void vjp_shape(int n, int prec, int *nsplit, int *jsplit, int *n_pad) {
   }
   const int gx = (n + VT2 * VIPT - 1) / (VT2 * VIPT);
   const int tiles = *n_pad / VTILE;
-  int ns = (4 * sms + gx - 1) / gx;
+  int ns = (24 * sms + gx - 1) / gx;
   if (ns > tiles) ns = tiles;
   if (ns < 1) ns = 1;
   const int tp = (tiles + ns - 1) / ns;  // tiles per split
@@ -497,6 +586,30 @@ extern "C" size_t g6k_vjp_scratch_bytes(int n) {
   return need;
 }
 
+// The VJP from records (split) or la1, lj1 (FP64) that are ready.
+static int vjp_core(int n, double eps2, int prec, int hjerk, const double *x, const double *v,
+                    const double *m, const double *la1, const double *lj1, double *gx, double *gv,
+                    double *gm, void *scratch, cudaStream_t st) {
+  int nsplit, jsplit, n_pad;
+  vjp_shape(n, prec, &nsplit, &jsplit, &n_pad);
+  const VJPair *rec = reinterpret_cast<const VJPair *>(scratch);
+  double *part = reinterpret_cast<double *>(reinterpret_cast<char *>(scratch) +
+                                            (size_t)n_pad * (sizeof(VJPair) / 2));
+  if (prec == G6_PREC_FP64) {
+    launch_pdl(hjerk ? vjp_f64_kernel<true> : vjp_f64_kernel<false>,
+               dim3((n + VT - 1) / VT, nsplit), dim3(VT), 0, st, n, eps2, x, v, m, la1, lj1,
+               jsplit, part);
+  } else {
+    const float e2 = (float)eps2 + (float)(1.0 / 4503599627370496.0);
+    launch_pdl(hjerk ? vjp_split_kernel<true> : vjp_split_kernel<false>,
+               dim3((n + VT2 * VIPT - 1) / (VT2 * VIPT), nsplit), dim3(VT2), 0, st, n, e2, rec,
+               jsplit, n_pad, part);
+  }
+  launch_pdl(vjp_reduce_kernel, dim3((7 * n + 127) / 128), dim3(128), 0, st, n, nsplit,
+             (const double *)part, gx, gv, gm);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
 // hjerk: differentiate the hermite code's jerk form instead of the softened
 // one (must match the force the forward step used).
 extern "C" int g6k_force_vjp(int n, double eps2, int prec, int hjerk, const double *x,
@@ -504,26 +617,42 @@ extern "C" int g6k_force_vjp(int n, double eps2, int prec, int hjerk, const doub
                              const double *lj1, double *gx, double *gv, double *gm, void *scratch,
                              cudaStream_t st) {
   if (n <= 0) return 0;
+  if (prec != G6_PREC_FP64) {
+    int nsplit, jsplit, n_pad;
+    vjp_shape(n, prec, &nsplit, &jsplit, &n_pad);
+    launch_pdl(vjp_records_kernel, dim3((n_pad + 31) / 32), dim3(32), 0, st, n, n_pad, x, v, m, la1,
+               lj1, reinterpret_cast<VJPair *>(scratch));
+  }
+  return vjp_core(n, eps2, prec, hjerk, x, v, m, la1, lj1, gx, gv, gm, scratch, st);
+}
+
+// The adjoints of nsteps consecutive fixed steps, last first, at the predicted
+// states xp_all, vp_all ([nsteps][n][3]): per step the force VJP with its
+// reduction, and one kernel that ends the step's adjoint and begins the next
+// one's.
+extern "C" int g6k_fixed_adjoint(int n, double h, double eps2, int nsteps, int prec, int hjerk,
+                                 const double *xp_all, const double *vp_all, const double *m,
+                                 double *lx, double *lv, double *la, double *lj, double *lm,
+                                 double *la1, double *lj1, double *gxp, double *gvp, double *gm,
+                                 void *scratch, cudaStream_t st) {
+  if (n <= 0 || nsteps <= 0) return 0;
   int nsplit, jsplit, n_pad;
   vjp_shape(n, prec, &nsplit, &jsplit, &n_pad);
-  VJPair *rec = reinterpret_cast<VJPair *>(scratch);
-  double *part = reinterpret_cast<double *>(reinterpret_cast<char *>(scratch) +
-                                            (size_t)n_pad * (sizeof(VJPair) / 2));
-  if (prec == G6_PREC_FP64) {
-    dim3 grid((n + VT - 1) / VT, nsplit);
-#define G6_VJP(H) vjp_f64_kernel<H><<<grid, VT, 0, st>>>(n, eps2, x, v, m, la1, lj1, jsplit, part)
-    if (hjerk) G6_VJP(true);
-    else G6_VJP(false);
-#undef G6_VJP
-  } else {
-    vjp_records_kernel<<<(n_pad + PT - 1) / PT, PT, 0, st>>>(n, n_pad, x, v, m, la1, lj1, rec);
-    const float e2 = (float)eps2 + (float)(1.0 / 4503599627370496.0);
-    dim3 grid((n + VT2 * VIPT - 1) / (VT2 * VIPT), nsplit);
-    if (hjerk)
-      vjp_split_kernel<true><<<grid, VT2, 0, st>>>(n, e2, rec, jsplit, n_pad, part);
-    else
-      vjp_split_kernel<false><<<grid, VT2, 0, st>>>(n, e2, rec, jsplit, n_pad, part);
+  VJPair *rec = prec == G6_PREC_FP64 ? nullptr : reinterpret_cast<VJPair *>(scratch);
+  const dim3 grid(((rec ? n_pad : n) + 31) / 32), block(32);
+  const size_t step = 3 * (size_t)n;
+  for (int s = nsteps - 1; s >= -1; s--) {
+    // before the VJP of step s: the end of step s + 1, the beginning of s
+    const double *x = s >= 0 ? xp_all + step * s : nullptr, *v = s >= 0 ? vp_all + step * s : nullptr;
+    auto kern = s == nsteps - 1 ? adjoint_kernel<false, true>
+                : s >= 0        ? adjoint_kernel<true, true>
+                                : adjoint_kernel<true, false>;
+    if (launch_pdl(kern, grid, block, 0, st, n, n_pad, h, lx, lv, la, lj, (const double *)gxp,
+                   (const double *)gvp, lm, (const double *)gm, x, v, m, la1, lj1,
+                   rec) != cudaSuccess)
+      return -3;
+    if (s >= 0 && vjp_core(n, eps2, prec, hjerk, x, v, m, la1, lj1, gxp, gvp, gm, scratch, st))
+      return -3;
   }
-  vjp_reduce_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, nsplit, part, gx, gv, gm);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return 0;
 }
