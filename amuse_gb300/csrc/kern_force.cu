@@ -591,6 +591,7 @@ struct RefHdr {
   unsigned nacc;      // REF_ACC entries queued by this call
   unsigned nmt;       // REF_MT entries queued by this call
   unsigned last_mt;   // of the last refinement
+  unsigned cmt;       // entries queued for REF_MT alone
 };
 struct RefPart {  // one j-chunk of one entry, FP64
   double a[3], p, r2;
@@ -605,6 +606,11 @@ struct RefBuf {
   unsigned ticket[RCAP];
   RefPart part[RPCAP];
   unsigned xtick[XTMAX];  // force kernel: CTAs of an i-group done (reset by the last)
+  // REF_MT alone, nearly all entries of a cluster with a mass spectrum
+  int mt_list[RCAP];
+  float mt_thr[RCAP];
+  unsigned mt_ticket[RCAP];   // per group of entries
+  float2 mt_part[RPCAP][4];   // [group][chunk][entry] sums, float-float
 };
 
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
@@ -655,6 +661,14 @@ __device__ __forceinline__ float split_eps(double eps2) {
 __device__ __forceinline__ void ref_enqueue(void *buf, int i, int mode, float thr,
                                             float thr_mt) {
   RefBuf *b = reinterpret_cast<RefBuf *>(buf);
+  if (mode == REF_MT) {
+    const unsigned e = atomicAdd(&b->h.cmt, 1u);
+    if (e < (unsigned)RCAP) {
+      b->mt_list[e] = i;
+      b->mt_thr[e] = thr_mt;
+    }
+    return;
+  }
   const unsigned e = atomicAdd(&b->h.count, 1u);
   if (mode & REF_ACC) atomicAdd(&b->h.nacc, 1u);
   if (mode & REF_MT) atomicAdd(&b->h.nmt, 1u);
@@ -1358,25 +1372,161 @@ __device__ __forceinline__ void ref_nn_take(double &r2, int &slot, double or2, i
   }
 }
 
+// The entries queued for REF_MT alone.  A warp holds EL of them in its lanes
+// (and 32 / EL j-lanes where they are few), so that a record loaded serves all
+// of them and nothing is reduced across lanes for EL = 32; a CTA's eight warps
+// share a chunk of the j, and the CTA that completes a group of entries adds
+// the chunks' sums in order.  A unit of one entry per CTA, as below, spent
+// most of its time on its own start and reduction: Salpeter cluster, N =
+// 16384, 165 entries 62 us that way and 33 this, 92 entries 42 and 33, 24
+// entries 18 and 16, 2 entries 14 and 12.
+constexpr int MT_WARPS = RNT / 32;
+__device__ __forceinline__ void refine_mt(const KParams &kp, RefBuf *b, int ne,
+                                          float2 (*s_sum)[32][4], int *s_flag) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // log2 EL: as many entries per warp as still leave two CTAs for every SM when
+  // a group's merge, RNT / (4 EL) threads per quantity, is kept to 16 chunks
+  // per thread: about 1024 ne / 4^el CTAs (24 entries at EL = 32 and 512 chunks
+  // took 41 us).
+  int el = 0;
+  while (el < 5 && (1 << el) < ne && (4 << (2 * el)) * 304LL <= 1024LL * ne) el++;
+  const int EL = 1 << el, JL = 32 >> el;
+  const int groups = (ne + EL - 1) >> el;
+  const int npair = (kp.nj + 1) >> 1;
+  const int TP = min(32, RNT >> (el + 2));  // threads per quantity in the merge
+  int nch = min((int)gridDim.x / groups, 16 * TP);
+  nch = min(nch, RPCAP / (groups << el));
+  nch = min(nch, npair / (MT_WARPS * JL * 2));
+  nch = max(nch, 1);
+  const float e32 = split_eps(kp.eps2);
+  const double eps2 = kp.eps2 + 1.0 / 4503599627370496.0;  // ph4's + 2^-52
+  const float2 eps2f = make_float2((float)eps2, (float)(eps2 - (double)(float)eps2));
+  const void *rec = kp.jrec;
+  const float4 *q4 = reinterpret_cast<const float4 *>(rec);
+  for (int u = blockIdx.x; u < groups * nch; u += gridDim.x) {
+    const int g = u / nch, c = u - g * nch;
+    const int e = (g << el) + (lane & (EL - 1));
+    const bool valid = e < ne;
+    const int i = b->mt_list[valid ? e : 0];
+    const float thr = b->mt_thr[valid ? e : 0];
+    int self;
+    float ih[3], il[3];
+    if (kp.ilist) {
+      const int slot = kp.ilist[i];
+      self = kp.iself ? kp.iself[i] : slot;
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        ih[k] = g6_split_get(rec, slot, k);
+        il[k] = g6_split_get(rec, slot, 4 + k);
+      }
+    } else {
+      self = kp.iself ? kp.iself[i] : -1;
+#pragma unroll
+      for (int k = 0; k < 3; k++) SplitP::split(kp.ipos[3 * i + k], ih[k], il[k]);
+    }
+    const int p0 = (int)((long long)npair * c / nch);
+    const int p1 = (int)((long long)npair * (c + 1) / nch);
+    float ah[3] = {0.f, 0.f, 0.f}, al[3] = {0.f, 0.f, 0.f}, ph = 0.f, pl = 0.f;
+#pragma unroll 2
+    for (int rp = p0 + warp * JL + (lane >> el); rp < p1; rp += MT_WARPS * JL) {
+      const float4 A = __ldg(q4 + 6 * rp), B = __ldg(q4 + 6 * rp + 1);
+      const float4 C = __ldg(q4 + 6 * rp + 2), D = __ldg(q4 + 6 * rp + 3);
+      const int j = 2 * rp;
+      if (mt_term(A.x, A.z, B.x, B.z, D.z, C.x, C.z, D.x, ih, il, e32, thr,
+                  j == self || j >= kp.nj, ah, al, ph, pl))
+        ff_term(rec, j, ih, il, eps2f, ah, al, ph, pl);
+      if (mt_term(A.y, A.w, B.y, B.w, D.w, C.y, C.w, D.y, ih, il, e32, thr,
+                  j + 1 == self || j + 1 >= kp.nj, ah, al, ph, pl))
+        ff_term(rec, j + 1, ih, il, eps2f, ah, al, ph, pl);
+    }
+    for (int off = 16; off >= EL; off >>= 1) {
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        ff_add(ah[k], al[k], __shfl_xor_sync(0xffffffffu, ah[k], off),
+               __shfl_xor_sync(0xffffffffu, al[k], off));
+      ff_add(ph, pl, __shfl_xor_sync(0xffffffffu, ph, off), __shfl_xor_sync(0xffffffffu, pl, off));
+    }
+    if (lane < EL) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) s_sum[warp][lane][k] = make_float2(ah[k], al[k]);
+      s_sum[warp][lane][3] = make_float2(ph, pl);
+    }
+    __syncthreads();
+    // four quantities of EL entries: the warps in order
+    float2 *part = &b->mt_part[0][0] + (((size_t)g * nch) << el) * 4;
+    if (tid < 4 * EL) {
+      float2 q = s_sum[0][tid >> 2][tid & 3];
+      for (int w = 1; w < MT_WARPS; w++) {
+        const float2 o = s_sum[w][tid >> 2][tid & 3];
+        ff_add(q.x, q.y, o.x, o.y);
+      }
+      part[((size_t)c << el) * 4 + tid] = q;
+      __threadfence();
+    }
+    __syncthreads();
+    if (tid == 0) *s_flag = atomicAdd(&b->mt_ticket[g], 1u) == (unsigned)(nch - 1);
+    __syncthreads();
+    if (*s_flag) {
+      // the group's last CTA: TP threads per quantity (a power of two, in one
+      // warp), each adding chunks t, t + TP, ... in order, then a fixed tree
+      __threadfence();
+      const int t = tid & (TP - 1), x = tid / TP;
+      float2 q = make_float2(0.f, 0.f);
+      if (x < 4 * EL) {
+#pragma unroll 4
+        for (int cc = t; cc < nch; cc += TP) {
+          const float2 o = __ldcg(part + ((size_t)cc << el) * 4 + x);
+          ff_add(q.x, q.y, o.x, o.y);
+        }
+      }
+      for (int off = TP >> 1; off > 0; off >>= 1) {
+        const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, q.x, off),
+                                     __shfl_xor_sync(0xffffffffu, q.y, off));
+        // (the lower lane first, so that both ends hold the same sum)
+        float2 lo = (tid & off) ? o : q, hi = (tid & off) ? q : o;
+        ff_add(lo.x, lo.y, hi.x, hi.y);
+        q = lo;
+      }
+      const int ee = (g << el) + (x >> 2);
+      if (t == 0 && x < 4 * EL && ee < ne) {
+        const int ii = b->mt_list[ee];
+        const double v = (double)q.x + (double)q.y;
+        if ((x & 3) < 3)
+          kp.acc[3 * ii + (x & 3)] = v;
+        else
+          kp.pot[ii] = -v;
+      }
+      if (tid == 0) b->mt_ticket[g] = 0u;
+    }
+    __syncthreads();
+  }
+}
+
 __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
   pdl_wait();
   pdl_trigger();
   RefBuf *b = reinterpret_cast<RefBuf *>(kp.refine);
-  __shared__ unsigned s_cnt;
+  __shared__ unsigned s_cnt, s_cmt;
+  __shared__ float2 s_mt[MT_WARPS][32][4];
   __shared__ double s_sum[RNT / 32][4], s_r2[RNT / 32];
   __shared__ int s_slot[RNT / 32];
   __shared__ int s_last;
   __shared__ int s_due[RNT / 32][96];  // per warp: j whose REF_MT term is due in float-float
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_cnt = *reinterpret_cast<volatile unsigned *>(&b->h.count);
+  if (tid == 0) {
+    s_cnt = *reinterpret_cast<volatile unsigned *>(&b->h.count);
+    s_cmt = *reinterpret_cast<volatile unsigned *>(&b->h.cmt);
+  }
   __syncthreads();
-  const unsigned cnt = s_cnt;
-  if (cnt == 0) {  // nothing queued (most calls): record that and leave
+  const unsigned cnt = s_cnt, cmt = s_cmt;
+  if (cnt == 0 && cmt == 0) {  // nothing queued (most calls): record that and leave
     if (blockIdx.x == 0 && tid == 0) b->h.last = b->h.last_acc = b->h.last_mt = 0u;
     return;
   }
   const int ne = cnt > (unsigned)RCAP ? 0 : (int)cnt;
-  if (cnt > (unsigned)RCAP && blockIdx.x == 0 && tid == 0) atomicMax(&b->h.overflow, cnt);
+  if (max(cnt, cmt) > (unsigned)RCAP && blockIdx.x == 0 && tid == 0)
+    atomicMax(&b->h.overflow, max(cnt, cmt));
+  if (cmt > 0 && cmt <= (unsigned)RCAP) refine_mt(kp, b, (int)cmt, s_mt, &s_last);
   int nch = 1;
   if (ne > 0) {
     // One unit per CTA while the entries are few (the CTA reduces once), two
@@ -1396,7 +1546,8 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
   const float e32 = split_eps(kp.eps2);
   const double inf = __longlong_as_double(0x7ff0000000000000ll);
   const void *rec = kp.jrec;
-  for (int u = blockIdx.x; u < units; u += gridDim.x) {
+  // (from the last CTA down: the first ones hold the units of refine_mt)
+  for (int u = gridDim.x - 1 - blockIdx.x; u < units; u += gridDim.x) {
     const int e = u / nch, c = u - e * nch;
     const int i = b->list[e];
     const int mode = b->mode[e];
@@ -1587,10 +1738,11 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
     __threadfence();
     const unsigned d = atomicAdd(&b->h.done, 1u);
     if (d == gridDim.x - 1) {
-      b->h.last = cnt;
+      b->h.last = cnt + cmt;
       b->h.last_acc = b->h.nacc;
-      b->h.last_mt = b->h.nmt;
+      b->h.last_mt = b->h.nmt + cmt;
       b->h.count = 0u;
+      b->h.cmt = 0u;
       b->h.nacc = 0u;
       b->h.nmt = 0u;
       b->h.done = 0u;
