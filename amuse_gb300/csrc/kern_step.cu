@@ -120,6 +120,11 @@ __global__ void correct_kernel(g6_jstate js, int ni, const int *__restrict__ ili
     k2 = dadd(k2, __shfl_sync(0xffffffffu, pk2, base + c));
     l2 = dadd(l2, __shfl_sync(0xffffffffu, pl2, base + c));
   }
+  // the step's two inner square roots at once: lane 0 the first, lane 1 the
+  // second (an FP64 instruction costs its time whichever lanes need it)
+  const double root = __dsqrt_rn(k == 0 ? dmul(a2, k2) : dmul(j2, l2));
+  const double root_ak = __shfl_sync(0xffffffffu, root, base);
+  const double root_jl = __shfl_sync(0xffffffffu, root, base + 1);
   if (!active) return;
   if (k < 3) {
     js.x[k * cap + s] = xp;
@@ -129,12 +134,19 @@ __global__ void correct_kernel(g6_jstate js, int ni, const int *__restrict__ ili
     return;
   }
   // lane 3: the Aarseth step with power-of-two quantisation
-  double newstep = dmul(dmul(eta, dt),
-                        __dsqrt_rn(ddiv(dadd(__dsqrt_rn(dmul(a2, k2)), j2),
-                                        dadd(__dsqrt_rn(dmul(j2, l2)), k2))));
+  double newstep =
+      dmul(dmul(eta, dt), __dsqrt_rn(ddiv(dadd(root_ak, j2), dadd(root_jl, k2))));
   const double olds = js.dt[s];
-  int expo;
-  double oldstep2 = ddiv(olds, dmul(2.0, frexp(olds, &expo)));
+  const int ohi = __double2hiint(olds);
+  double oldstep2;
+  if ((unsigned)ohi - 0x00100000u < 0x7fe00000u) {
+    // olds / (2 frexp(olds)): the power of two of a positive normal double,
+    // its mantissa cleared
+    oldstep2 = __hiloint2double(ohi & 0x7ff00000, 0);
+  } else {
+    int expo;
+    oldstep2 = ddiv(olds, dmul(2.0, frexp(olds, &expo)));
+  }
   for (int guard = 0; guard < 1100 && !multiple_of_pow2(tnext, oldstep2); guard++)
     oldstep2 = dmul(oldstep2, 0.5);  // as the division by 2, to the last bit
   if (newstep < oldstep2) {
