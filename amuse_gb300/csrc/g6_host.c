@@ -1457,7 +1457,7 @@ int g6x_run(double t_end, long long *blocks, double *particle_steps) {
      neighbour and a pass before the corrector evaluates ph4's criteria.  The
      stopping test on the corrected pair runs in the first kernel of the next
      block's scheduler (or after the loop), and its stop bits reach the host
-     in that block's mailbox copy, before that block's force is launched. */
+     in that block's mailbox, before that block's force is launched. */
   const int enc = G.enc_mode;
   const double rmin = G.enc_rmin > 0 ? G.enc_rmin : 2.0 / n; /* jdata.cc:426 */
   int *d_stop = (int *)((char *)G.d_mail + 12);
@@ -1469,23 +1469,24 @@ int g6x_run(double t_end, long long *blocks, double *particle_steps) {
   g6_enc_decision_args pend; /* the last block's stopping decision, taken by the next schedule */
   memset(&pend, 0, sizeof(pend));
   /* Per block: sched_first (min of t + dt), list_predict (the block list,
-     tnext, all j predicted to tnext), the mailbox copy and the one host
+     tnext, all j predicted to tnext, the mailbox) and the one host
      synchronisation, then the force on the block (split merge in the force
      kernel, refinement pass), [encounter check], corrector.  The two
      minima alternate by block parity: each list_predict resets the other. */
   unsigned long long *dmin2 = (unsigned long long *)G.d_sched;
   int parity = 0;
-  if (g6k_sched_reset(dmin2, G.d_ni, G.st)) return G6_ERR_CUDA;
+  unsigned *ticket = (unsigned *)(dmin2 + 2);
+  if (g6k_sched_reset(dmin2, G.d_ni, ticket, G.st)) return G6_ERR_CUDA;
   while (G.run_t < t_end && nb != max_blocks) {
     ilist_identity_n = 0;
     if (g6k_sched_first(&G.js, n, dmin2 + parity, G.d_ni, pend.enc ? &pend : NULL, G.st) ||
         g6k_list_predict(&G.js, n, G.prec, dmin2 + parity, dmin2 + (parity ^ 1), G.d_ilist,
-                         G.d_ni, G.d_tnext, G.st))
+                         G.d_ni, G.d_tnext, ticket, G.h_mail, G.st))
       return G6_ERR_CUDA;
     parity ^= 1;
     pend.enc = NULL;
-    /* one 16-byte copy into pinned memory: the only host round trip per block */
-    CK(cudaMemcpyAsync(G.h_mail, G.d_mail, 16, cudaMemcpyDeviceToHost, G.st));
+    /* list_predict writes the mailbox into pinned memory: this wait is the
+       only host round trip per block */
     const double s0 = now_ms();
     CK(cudaStreamSynchronize(G.st));
     wsync += now_ms() - s0;

@@ -131,12 +131,15 @@ __global__ void __launch_bounds__(PT) predict_kernel(g6_jstate js, int nj, int n
 // *dmin); each thread lists its slot if t + dt == tn (the block: ph4's
 // scheduler, src/amuse_ph4/src/scheduler.cc) and predicts it to tn.
 // *dmin_next, the other parity's minimum, is reset to +inf for the next
-// block.
+// block.  The last CTA to finish (ticket) writes {tn, block size, stop word}
+// to `mail`, pinned host memory, which saves the host loop a copy per block
+// (about 3 us of 65).
 template <int PREC>
 __global__ void __launch_bounds__(PT) list_predict_kernel(g6_jstate js, int nj, int nj_pad,
                                                           const unsigned long long *dmin,
                                                           unsigned long long *dmin_next,
-                                                          int *ilist, int *dni, double *dtnext) {
+                                                          int *ilist, int *dni, double *dtnext,
+                                                          unsigned *ticket, void *mail) {
   pdl_wait();
   pdl_trigger();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -145,9 +148,24 @@ __global__ void __launch_bounds__(PT) list_predict_kernel(g6_jstate js, int nj, 
     *dtnext = tn;
     *dmin_next = 0x7ff0000000000000ull;
   }
-  if (s >= nj_pad) return;
-  if (s < nj && js.t[s] + js.dt[s] == tn) ilist[atomicAdd(dni, 1)] = s;
-  predict_one<PREC>(js, s, nj, tn);
+  if (s < nj_pad) {
+    if (s < nj && js.t[s] + js.dt[s] == tn) ilist[atomicAdd(dni, 1)] = s;
+    predict_one<PREC>(js, s, nj, tn);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
+      *ticket = 0u;
+      __threadfence();
+      *reinterpret_cast<volatile double *>(mail) = tn;
+      volatile int *w = reinterpret_cast<volatile int *>(mail) + 2;
+      w[0] = *reinterpret_cast<volatile int *>(dni);
+      // the stop word beside the block size (16 bytes {tnext, ni, stop})
+      w[1] = *(reinterpret_cast<volatile int *>(dni) + 1);
+      __threadfence_system();
+    }
+  }
 }
 
 // Threads per CTA: ~36 FP64 instructions per slot at 16 cycles each per warp
@@ -182,7 +200,8 @@ extern "C" int g6k_predict(const g6_jstate *js, int nj, double ti, int prec, cud
 
 extern "C" int g6k_list_predict(const g6_jstate *js, int nj, int prec,
                                 const unsigned long long *dmin, unsigned long long *dmin_next,
-                                int *d_ilist, int *d_ni, double *d_tnext, cudaStream_t st) {
+                                int *d_ilist, int *d_ni, double *d_tnext, unsigned *ticket,
+                                void *mail, cudaStream_t st) {
   if (nj <= 0) return 0;
   const int nj_pad = (nj + G6_TILE - 1) / G6_TILE * G6_TILE;
   if (nj_pad > js->cap) return -1;
@@ -191,8 +210,8 @@ extern "C" int g6k_list_predict(const g6_jstate *js, int nj, int prec,
   const cudaError_t e =
       prec == G6_PREC_FP64
           ? launch_pdl(list_predict_kernel<G6_PREC_FP64>, dim3(grid), dim3(threads), 0, st, *js, nj,
-                       nj_pad, dmin, dmin_next, d_ilist, d_ni, d_tnext)
+                       nj_pad, dmin, dmin_next, d_ilist, d_ni, d_tnext, ticket, mail)
           : launch_pdl(list_predict_kernel<G6_PREC_SPLIT>, dim3(grid), dim3(threads), 0, st, *js, nj,
-                       nj_pad, dmin, dmin_next, d_ilist, d_ni, d_tnext);
+                       nj_pad, dmin, dmin_next, d_ilist, d_ni, d_tnext, ticket, mail);
   return e == cudaSuccess ? 0 : -3;
 }

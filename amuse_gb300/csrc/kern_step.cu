@@ -370,9 +370,10 @@ __global__ void sched_min_first(g6_jstate js, int nj, unsigned long long *dmin, 
   }
 }
 
-__global__ void sched_reset(unsigned long long *dmin, int *dni) {
+__global__ void sched_reset(unsigned long long *dmin, int *dni, unsigned *ticket) {
   dmin[0] = dmin[1] = 0x7ff0000000000000ull;
   *dni = 0;
+  *ticket = 0u;
 }
 
 __global__ void initial_step_kernel(g6_jstate js, int nj, double eta, double fac, double limit,
@@ -487,8 +488,9 @@ extern "C" int g6k_store_forces(const g6_jstate *js, int ni, const int *ilist, c
 // per block g6k_sched_first (minimum into dmin[parity]) and
 // g6k_list_predict (kern_predict.cu: the block list, tnext, the prediction,
 // and dmin[1 - parity] reset for the next block).
-extern "C" int g6k_sched_reset(unsigned long long *dmin2, int *d_ni, cudaStream_t st) {
-  sched_reset<<<1, 1, 0, st>>>(dmin2, d_ni);
+extern "C" int g6k_sched_reset(unsigned long long *dmin2, int *d_ni, unsigned *ticket,
+                               cudaStream_t st) {
+  sched_reset<<<1, 1, 0, st>>>(dmin2, d_ni, ticket);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
