@@ -433,6 +433,27 @@ __device__ __forceinline__ double sqrt64(double x) {
   const double y = rsqrt64(x), q = x * y;
   return __fma_rn(__fma_rn(-q, q, x), 0.5 * y, q);
 }
+// Quotients by one b, rounded as a / b is: div_by with rcp64's y.
+struct Div {
+  double b, y;
+  bool mid;
+  __device__ __forceinline__ explicit Div(double d) : b(d), y(rcp64(d)), mid(mid_range(d)) {}
+  __device__ __forceinline__ double operator()(double a) const { return div_by(a, b, y, mid); }
+  __device__ __forceinline__ double inv() const {  // 1 / b rounded
+    return mid ? __fma_rn(__fma_rn(-b, y, 1.0), y, y) : y;
+  }
+};
+__device__ __forceinline__ double div64(double a, double b) { return Div(b)(a); }
+// a b + c d and a . b with the order of their roundings fixed (left to the
+// compiler, it varies with the surroundings): the split mode's FP32 pair terms
+// turn a last bit of the FP64 state into 6e-8 of a term now and then, and a
+// hard binary amplifies that to 1e-6 of a position within 0.05 crossing times.
+__device__ __forceinline__ double two(double a, double b, double c, double d) {
+  return __fma_rn(a, b, __dmul_rn(c, d));
+}
+__device__ __forceinline__ double dot3(const double a[3], const double b[3]) {
+  return __fma_rn(a[2], b[2], two(a[0], b[0], a[1], b[1]));
+}
 // Stumpff functions C(z) = (1 - cos sqrt z) / z, S(z) = (sqrt z - sin sqrt z)
 // / z^(3/2) (cosh, sinh for z < 0), both from one sincos (one exp) of
 // sqrt(|z|) / 2: 1 - cos s = 2 sin^2(s/2) (no cancellation), sin s = 2
@@ -444,15 +465,13 @@ __device__ __forceinline__ void kst_cs(double z, double &C, double &S) {
     const double s = sqrt64(z);
     double sh, ch;
     sincos(0.5 * s, &sh, &ch);
-    const double i = rcp64(s * z);  // 1 / z^(3/2)
-    C = 2.0 * sh * sh * (s * i);
-    S = (s - 2.0 * sh * ch) * i;
+    C = div64(2.0 * sh * sh, z);
+    S = div64(s - 2.0 * sh * ch, s * z);
   } else if (z < -0.1) {
-    const double s = sqrt64(-z), e = exp(0.5 * s), ei = rcp64(e);
+    const double s = sqrt64(-z), e = exp(0.5 * s), ei = Div(e).inv();
     const double sh = 0.5 * (e - ei), ch = 0.5 * (e + ei);
-    const double i = rcp64(s * -z);
-    C = 2.0 * sh * sh * (s * i);
-    S = (2.0 * sh * ch - s) * i;
+    C = div64(2.0 * sh * sh, -z);
+    S = div64(2.0 * sh * ch - s, s * -z);
   } else {
     C = 1.0 / 2 +
         z * (-1.0 / 24 +
@@ -479,35 +498,42 @@ __device__ __forceinline__ void kst_cs(double z, double &C, double &S) {
 // orbit), xw + sqrt(mu) (dt - dtw) / rw (dx/dt = sqrt(mu) / r); x grows with
 // dt, so xw then also bounds the root from one side.  The C and S of the
 // step whose correction is below 1e-15 x give the f and g functions.
+// LAST: which of F's first two terms is added last (the force evaluations
+// round one way, the tree's decisions the other).
+template <bool LAST>
 __device__ __noinline__ void kep_prop(double mu, const double r0[3], const double v0[3], double dt,
                          double r[3], double v[3], double *xw = nullptr, double *dtw = nullptr,
                          double *rw = nullptr) {
-  const double r2 = r0[0] * r0[0] + r0[1] * r0[1] + r0[2] * r0[2];
-  const double irn = rsqrt64(r2), rn = sqrt64(r2);
-  const double v2 = v0[0] * v0[0] + v0[1] * v0[1] + v0[2] * v0[2];
-  const double rv = r0[0] * v0[0] + r0[1] * v0[1] + r0[2] * v0[2];
-  const double ismu = rsqrt64(mu), smu = sqrt64(mu);
-  const double alpha = 2.0 * irn - v2 * (ismu * ismu);
-  const double c1 = rv * ismu, c2 = 1.0 - alpha * rn;
+  const double rn = sqrt64(dot3(r0, r0));
+  const double v2 = dot3(v0, v0), rv = dot3(r0, v0);
+  const double smu = sqrt64(mu);
+  const Div by_rn(rn), by_smu(smu);
+  const double alpha = by_rn(2.0) - div64(v2, mu);
+  const double c1 = by_smu(rv), c2 = 1.0 - alpha * rn;
   if (dt == 0.0) {
     for (int k = 0; k < 3; k++) r[k] = r0[k], v[k] = v0[k];
     return;
   }
+  const double sd = __dmul_rn(smu, dt);
+  auto Fcs = [&](double x, double C, double S) {
+    const double a = c1 * x * x, b = c2 * x * x * x;
+    return __dsub_rn(__fma_rn(rn, x, LAST ? two(b, S, a, C) : two(a, C, b, S)), sd);
+  };
   auto Fx = [&](double x) {
     double C, S;
     kst_cs(alpha * x * x, C, S);
-    return c1 * x * x * C + c2 * x * x * x * S + rn * x - smu * dt;
+    return Fcs(x, C, S);
   };
   const bool warm = xw && *dtw > 0.0 && dt > 0.0;
   const double inf = __longlong_as_double(0x7ff0000000000000ll);
-  double x0 = alpha > 0.0 ? smu * dt * alpha : smu * dt * irn;  // sign of dt
+  double x0 = alpha > 0.0 ? smu * dt * alpha : by_rn(smu * dt);  // sign of dt
   double lo, hi;
   if (warm) {
     // The root lies above xw when dt >= dtw (F(xw) <= 0), else in (0, xw).
     // No evaluation before the first Newton step: with hi = +inf, steps from
     // below (F < 0, dF > 0) only move up, until one lands above the root and
     // bounds it.
-    x0 = *xw + smu * (dt - *dtw) * rcp64(*rw);
+    x0 = *xw + div64(smu * (dt - *dtw), *rw);
     lo = dt >= *dtw ? *xw : 0.0;
     hi = dt >= *dtw ? inf : *xw;
     if (!(x0 > lo && x0 < hi)) x0 = hi < inf ? 0.5 * (lo + hi) : lo + fabs(lo) + 1e-300;
@@ -523,14 +549,14 @@ __device__ __noinline__ void kep_prop(double mu, const double r0[3], const doubl
   for (int it = 0; it < 200; it++) {
     const double z = alpha * x * x;
     kst_cs(z, C, S);
-    const double F = c1 * x * x * C + c2 * x * x * x * S + rn * x - smu * dt;
-    const double dF = c1 * x * (1.0 - z * S) + c2 * x * x * C + rn;
+    const double F = Fcs(x, C, S);
+    const double dF = __dadd_rn(two(c2 * x * x, C, c1 * x, __fma_rn(-z, S, 1.0)), rn);
     if (F == 0.0 || fabs(F) <= 1e-15 * fabs(x * dF)) break;  // x is the root: C, S belong to it
     if (F < 0.0)
       lo = x;
     else
       hi = x;
-    const double newton = F * rcp64(dF);
+    const double newton = div64(F, dF);
     double xn = x - newton;
     if (hi < inf && (!(xn > lo && xn < hi) || fabs(2.0 * F) > fabs(step_old * dF))) {
       step_old = step;
@@ -543,12 +569,12 @@ __device__ __noinline__ void kep_prop(double mu, const double r0[3], const doubl
     if (xn == x) break;
     x = xn;
   }
-  const double f = 1.0 - x * x * C * irn, g = dt - x * x * x * S * ismu;
-  for (int k = 0; k < 3; k++) r[k] = f * r0[k] + g * v0[k];
-  const double rr2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
-  const double irr = rsqrt64(rr2), rr = sqrt64(rr2);
-  const double fd = smu * (irr * irn) * (alpha * x * x * x * S - x), gd = 1.0 - x * x * C * irr;
-  for (int k = 0; k < 3; k++) v[k] = fd * r0[k] + gd * v0[k];
+  const double f = 1.0 - by_rn(x * x * C), g = dt - by_smu(x * x * x * S);
+  for (int k = 0; k < 3; k++) r[k] = two(f, r0[k], g, v0[k]);
+  const double rr = sqrt64(dot3(r, r));
+  const double fd = div64(smu, rr * rn) * (alpha * x * x * x * S - x);
+  const double gd = 1.0 - div64(x * x * C, rr);
+  for (int k = 0; k < 3; k++) v[k] = two(fd, r0[k], gd, v0[k]);
   if (xw && dt > 0.0) {
     *xw = x;
     *dtw = dt;
@@ -561,15 +587,15 @@ __device__ __noinline__ void kep_prop(double mu, const double r0[3], const doubl
 // Barker's equation near e = 1.
 __device__ __noinline__ int kep_peri(double mu, const double r[3], const double v[3], double *dt_peri,
                         double *period) {
-  const double rn = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
-  const double v2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-  const double rv = r[0] * v[0] + r[1] * v[1] + r[2] * v[2];
+  const double rn = sqrt(dot3(r, r));
+  const double v2 = dot3(v, v);
+  const double rv = dot3(r, v);
   *period = __longlong_as_double(0x7ff0000000000000ll);
   if (rv >= 0.0) return 0;
   const double alpha = 2.0 / rn - v2 / mu;
-  const double h0 = r[1] * v[2] - r[2] * v[1], h1 = r[2] * v[0] - r[0] * v[2],
-               h2 = r[0] * v[1] - r[1] * v[0];
-  const double p = (h0 * h0 + h1 * h1 + h2 * h2) / mu;
+  const double h[3] = {two(r[1], v[2], -r[2], v[1]), two(r[2], v[0], -r[0], v[2]),
+                       two(r[0], v[1], -r[1], v[0])};
+  const double p = dot3(h, h) / mu;
   const double e = sqrt(fmax(0.0, 1.0 - p * alpha));
   if (fabs(alpha) * rn < 1e-8 || e < 1e-12) {
     const double D = rv / sqrt(mu * p);
@@ -594,10 +620,9 @@ __device__ __noinline__ int kep_peri(double mu, const double r[3], const double 
   return 1;
 }
 
-// 1 / |a - b|
-__device__ __forceinline__ double idist(const double a[3], const double4_16 &b) {
-  const double d0 = a[0] - b.x, d1 = a[1] - b.y, d2 = a[2] - b.z;
-  return rsqrt64(d0 * d0 + d1 * d1 + d2 * d2);
+__device__ __forceinline__ double dist3(const double a[3], const double4_16 &b) {
+  const double d[3] = {a[0] - b.x, a[1] - b.y, a[2] - b.z};
+  return sqrt64(dot3(d, d));
 }
 
 // The relative state of a binary at time t (frozen when fully unperturbed).
@@ -605,16 +630,17 @@ __device__ __forceinline__ void bin_rel(const BinRec &b, double t, double r[3], 
   if (b.full) {
     for (int k = 0; k < 3; k++) r[k] = b.r0[k], v[k] = b.v0[k];
   } else {
-    kep_prop(b.mi + b.mj, b.r0, b.v0, t - b.t0, r, v);
+    kep_prop<false>(b.mi + b.mj, b.r0, b.v0, t - b.t0, r, v);
   }
 }
 // The same, starting the Kepler solve from the binary's last solution and
 // keeping this one (the force evaluations: a few per step, at nearby times).
+template <bool LAST>
 __device__ __forceinline__ void bin_rel_warm(BinRec &b, double t, double r[3], double v[3]) {
   if (b.full) {
     for (int k = 0; k < 3; k++) r[k] = b.r0[k], v[k] = b.v0[k];
   } else {
-    kep_prop(b.mi + b.mj, b.r0, b.v0, t - b.t0, r, v, &b.xw, &b.dtw, &b.rw);
+    kep_prop<LAST>(b.mi + b.mj, b.r0, b.v0, t - b.t0, r, v, &b.xw, &b.dtw, &b.rw);
   }
 }
 
@@ -643,8 +669,8 @@ __device__ __noinline__ double tidal_pot(const UnpSmem &S, int n, int lane, int 
   for (int q = 0; q < 2; q++) {
     const int k = lane + 32 * q;
     if (k >= n || S.nd[k] != k || k == li || k == lj) continue;
-    phi += S.nm[k] * (-mi * idist(xi, S.d.pp[k]) - mj * idist(xj, S.d.pp[k]) +
-                      (mi + mj) * idist(xc, S.d.pp[k]));
+    phi += S.nm[k] * (div64(-mi, dist3(xi, S.d.pp[k])) - div64(mj, dist3(xj, S.d.pp[k])) +
+                      div64(mi + mj, dist3(xc, S.d.pp[k])));
   }
   return warp_sum(phi);
 }
@@ -780,12 +806,12 @@ __device__ __forceinline__ void pair_terms(const Pair2 &i, const Pair2 &j, bool 
 template <bool TREE, int NQ>
 __device__ __forceinline__ void pairs_split(UnpSmem &S, int n, int lane, double la[2][3],
                                             double lj[2][3], float tsq[2], int pq[2]) {
-  float a[NQ][3], jk[NQ][3], wb[NQ];
+  float a[NQ][3], jk[NQ][3], wb[NQ], ws[NQ];
   int jb[NQ], ni[NQ];
   bool near[2] = {false, false};
 #pragma unroll
   for (int q = 0; q < NQ; q++) {
-    wb[q] = 0.f;
+    wb[q] = ws[q] = 0.f;
     jb[q] = -1;
     ni[q] = TREE ? S.nd[min(lane + 32 * q, n - 1)] : lane + 32 * q;
   }
@@ -804,7 +830,9 @@ __device__ __forceinline__ void pairs_split(UnpSmem &S, int n, int lane, double 
         A[k] = f2_fma(f, dx[k], A[k]);
         J[k] = f2_fma(f, u[k], J[k]);
       }
+      ws[0] = fmaxf(ws[0], fminf(w0, wb[0]));
       if (w0 > wb[0]) wb[0] = w0, jb[0] = j;
+      ws[NQ - 1] = fmaxf(ws[NQ - 1], fminf(w1, wb[NQ - 1]));
       if (w1 > wb[NQ - 1]) wb[NQ - 1] = w1, jb[NQ - 1] = j;
     }
 #pragma unroll
@@ -828,7 +856,9 @@ __device__ __forceinline__ void pairs_split(UnpSmem &S, int n, int lane, double 
         a[0][k] = fmaf(f2_hi(f), f2_hi(dx[k]), fmaf(f2_lo(f), f2_lo(dx[k]), a[0][k]));
         jk[0][k] = fmaf(f2_hi(f), f2_hi(u[k]), fmaf(f2_lo(f), f2_lo(u[k]), jk[0][k]));
       }
+      ws[0] = fmaxf(ws[0], fminf(w0, wb[0]));
       if (w0 > wb[0]) wb[0] = w0, jb[0] = j;
+      ws[0] = fmaxf(ws[0], fminf(w1, wb[0]));
       if (w1 > wb[0]) wb[0] = w1, jb[0] = j + 1;
     }
     near[0] |= near[1];
@@ -836,23 +866,30 @@ __device__ __forceinline__ void pairs_split(UnpSmem &S, int n, int lane, double 
 #pragma unroll
   for (int q = 0; q < NQ; q++) {
 #pragma unroll
-    for (int k = 0; k < 3; k++) la[q][k] = (double)a[q][k], lj[q][k] = (double)jk[q][k];
+    for (int k = 0; k < 3; k++) la[q][k] = lj[q][k] = 0.0;
     const int i = lane + 32 * q;
     tsq[q] = __int_as_float(0x7f800000);
     pq[q] = 0x7fffffff;
     if (i >= n) continue;
     const Leaf me = get_leaf<TREE>(S, i);
-    if (jb[q] >= 0) {
-      const Leaf b = get_leaf<TREE>(S, jb[q]);
+    // another pair's measure as large to within the measures' errors: the
+    // quotients of all of them decide
+    const bool all = ws[q] >= wb[q] * (1.0f - 0x1p-17f);
+    for (int j = all ? 0 : jb[q]; j >= 0 && j < n; j++) {
+      if (!all && j != jb[q]) break;
+      const Leaf b = get_leaf<TREE>(S, j);
+      if (b.node == ni[q]) continue;
       const float d0 = __fadd_rn(__fsub_rn(b.h.x, me.h.x), __fsub_rn(b.l.x, me.l.x));
       const float d1 = __fadd_rn(__fsub_rn(b.h.y, me.h.y), __fsub_rn(b.l.y, me.l.y));
       const float d2 = __fadd_rn(__fsub_rn(b.h.z, me.h.z), __fsub_rn(b.l.z, me.l.z));
       const float c0 = b.c.x - me.c.x, c1 = b.c.y - me.c.y, c2 = b.c.z - me.c.z;
       const float dd = fmaf(d2, d2, fmaf(d1, d1, d0 * d0));
+      if (dd < 1e-18f) continue;
       const float v2 = fmaf(c2, c2, fmaf(c1, c1, c0 * c0));
-      tsq[q] = fminf(__fdividef(0.5f * dd * (dd * rsqrt_approx(dd)), me.v.w + b.v.w),
-                     __fdividef(dd, v2));
-      pq[q] = ni[q] < b.node ? ni[q] * MAXN + b.node : b.node * MAXN + ni[q];
+      const float ts = fminf(__fdividef(0.5f * dd * (dd * rsqrt_approx(dd)), me.v.w + b.v.w),
+                             __fdividef(dd, v2));
+      const int pid = ni[q] < b.node ? ni[q] * MAXN + b.node : b.node * MAXN + ni[q];
+      if (ts < tsq[q] || (ts == tsq[q] && pid < pq[q])) tsq[q] = ts, pq[q] = pid;
     }
     if (near[q]) {  // pairs too close for FP32: FP64
       for (int j = 0; j < n; j++) {
@@ -880,6 +917,8 @@ __device__ __forceinline__ void pairs_split(UnpSmem &S, int n, int lane, double 
         if (ts < tsq[q] || (ts == tsq[q] && pid < pq[q])) tsq[q] = ts, pq[q] = pid;
       }
     }
+#pragma unroll
+    for (int k = 0; k < 3; k++) la[q][k] += (double)a[q][k], lj[q][k] += (double)jk[q][k];
   }
 }
 
@@ -954,7 +993,7 @@ __device__ __forceinline__ double tree_forces(UnpSmem &S, int n, int lane, Comp<
   if (nb > 0) {
     if (lane < nb) {  // a lane per binary: its components' relative state at t
       double r[3], v[3];
-      bin_rel_warm(S.bin[lane], t, r, v);
+      bin_rel_warm<false>(S.bin[lane], t, r, v);
       for (int k = 0; k < 3; k++) S.kr[lane][k] = r[k], S.kr[lane][3 + k] = v[k];
     }
     __syncwarp();
@@ -969,7 +1008,8 @@ __device__ __forceinline__ double tree_forces(UnpSmem &S, int n, int lane, Comp<
         store_leaf<MODE, true>(S, s, k, B.pp[r], B.pv[r], B.pv[r]);
       } else {
         const BinRec &bb = S.bin[b];
-        const double iM = rcp64(bb.mi + bb.mj), fi = bb.mj * iM, fj = bb.mi * iM;
+        const Div by_M(bb.mi + bb.mj);
+        const double fi = by_M(bb.mj), fj = by_M(bb.mi);
         const double x = S.kr[b][k], v = S.kr[b][3 + k];
         store_leaf<MODE, true>(S, bb.li, k, B.pp[r] - fi * x, B.pv[r] - fi * v, B.pv[r]);
         store_leaf<MODE, true>(S, bb.lj, k, B.pp[r] + fj * x, B.pv[r] + fj * v, B.pv[r]);
@@ -1031,9 +1071,9 @@ __device__ __forceinline__ double tree_forces(UnpSmem &S, int n, int lane, Comp<
       B.jerk[r] = node ? S.lj[s][k] : 0.0;
     } else {
       const BinRec &bb = S.bin[b];
-      const double iM = rcp64(bb.mi + bb.mj);
-      B.acc[r] = (bb.mi * S.la[bb.li][k] + bb.mj * S.la[bb.lj][k]) * iM;
-      B.jerk[r] = (bb.mi * S.lj[bb.li][k] + bb.mj * S.lj[bb.lj][k]) * iM;
+      const Div by_M(bb.mi + bb.mj);
+      B.acc[r] = by_M(two(bb.mi, S.la[bb.li][k], bb.mj, S.la[bb.lj][k]));
+      B.jerk[r] = by_M(two(bb.mi, S.lj[bb.li][k], bb.mj, S.lj[bb.lj][k]));
     }
   }
   return dt;
@@ -1103,11 +1143,12 @@ __device__ __forceinline__ int tree_step(UnpSmem &S, int n, int lane, Comp<NS> &
     const double d2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
     const double rv = r[0] * v[0] + r[1] * v[1] + r[2] * v[2];
     if (leaves && d2 <= P.r2_crit && rv <= 0.0) {
-      const double mi = S.nm[i], mj = S.nm[j], M = mi + mj, iM = rcp64(M);
+      const double mi = S.nm[i], mj = S.nm[j], M = mi + mj;
+      const Div by_M(M);
       double cm[3], cmv[3];
       for (int k = 0; k < 3; k++) {
-        cm[k] = (mi * xi[k] + mj * xj[k]) * iM;
-        cmv[k] = (mi * vi[k] + mj * vj[k]) * iM;
+        cm[k] = by_M(two(mi, xi[k], mj, xj[k]));
+        cmv[k] = by_M(two(mi, vi[k], mj, vj[k]));
       }
       // the strongest perturber (largest m^2 / d^2 from the CM; the first
       // node on ties): each lane its two node slots, then a warp argmax
@@ -1119,8 +1160,8 @@ __device__ __forceinline__ int tree_step(UnpSmem &S, int n, int lane, Comp<NS> &
         if (k2 >= n || S.nd[k2] != k2 || k2 == i || k2 == j) continue;
         const double4_16 y = S.d.pp[k2];
         const double e0 = y.x - cm[0], e1 = y.y - cm[1], e2 = y.z - cm[2];
-        const double ee = e0 * e0 + e1 * e1 + e2 * e2;
-        const double p2 = S.nm[k2] * S.nm[k2] * rcp64(ee);
+        const double ee = fma(e2, e2, fma(e1, e1, e0 * e0));
+        const double p2 = div64(S.nm[k2] * S.nm[k2], ee);
         if (p2 > maxp) maxp = p2, nnd2 = ee, mk = S.nm[k2], kk = k2;
       }
 #pragma unroll
@@ -1134,8 +1175,8 @@ __device__ __forceinline__ int tree_step(UnpSmem &S, int n, int lane, Comp<NS> &
       }
       bool unp = true;
       if (maxp > 0.0) {
-        const double q = d2 * rcp64(nnd2);
-        unp = 4.0 * (mk * iM) * (mk * iM) * q * q * q < P.gamma2;
+        const double q = div64(d2, nnd2), mm = by_M(mk);
+        unp = 4.0 * mm * mm * q * q * q < P.gamma2;
       }
       double dtp, per;
       if (unp && kep_peri(M, r, v, &dtp, &per)) {
@@ -1170,19 +1211,21 @@ __device__ __forceinline__ int tree_step(UnpSmem &S, int n, int lane, Comp<NS> &
     const BinRec bb = S.bin[qb];
     if (bb.tpred > t) continue;
     const int i = bb.li, j = bb.lj;
-    const double M = bb.mi + bb.mj, iM = rcp64(M);
+    const double M = bb.mi + bb.mj;
+    const Div by_M(M);
+    const double gi = by_M(bb.mj), gj = by_M(bb.mi);
     double r[3], v[3], xi[3], xj[3], xc[3], vc[3];
     BinRec bw = bb;  // warm-started solve on a copy (every lane, same values)
-    bin_rel_warm(bw, t, r, v);
+    bin_rel_warm<true>(bw, t, r, v);
     get3(S.d.pp[i], xc);
     get3(S.d.pv[i], vc);
     for (int k = 0; k < 3; k++) {
-      xi[k] = xc[k] - bb.mj * iM * r[k];
-      xj[k] = xc[k] + bb.mi * iM * r[k];
+      xi[k] = xc[k] - gi * r[k];
+      xj[k] = xc[k] + gj * r[k];
     }
     const double tid = tidal_pot(S, n, lane, i, j, bb.mi, bb.mj, xi, xj, xc);
     if (!bb.full) {
-      const double mu = bb.mi * bb.mj * iM, v2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+      const double mu = by_M(bb.mi * bb.mj), v2 = dot3(v, v);
       const double fac = 1.0 - 2.0 * (tid - bb.tidal) / (mu * v2);
       if (fac > 0.0) {
         const double sf = sqrt(fac);
@@ -1242,10 +1285,10 @@ __device__ __forceinline__ int tree_step(UnpSmem &S, int n, int lane, Comp<NS> &
     // dissolve: the components become top-level nodes again
     double yi[3], yj[3], wi[3], wj[3];
     for (int k = 0; k < 3; k++) {
-      yi[k] = xc[k] - bb.mj * iM * r[k];
-      yj[k] = xc[k] + bb.mi * iM * r[k];
-      wi[k] = vc[k] - bb.mj * iM * v[k];
-      wj[k] = vc[k] + bb.mi * iM * v[k];
+      yi[k] = xc[k] - gi * r[k];
+      yj[k] = xc[k] + gj * r[k];
+      wi[k] = vc[k] - gi * v[k];
+      wj[k] = vc[k] + gj * v[k];
     }
     node_set(B, n, lane, i, yi, wi);
     node_set(B, n, lane, j, yj, wj);
@@ -1288,17 +1331,6 @@ __device__ __noinline__ void integrate(UnpSmem &S, int lane, TreeRun &run, const
   const long long max_steps = run.max_steps;
   double *pos = run.pos, *vel = run.vel;
   const double *mass = run.mass;
-  // lane & 7: one of the corrector's coefficients, a cubic in tau, a quarter
-  // included: acc = c0 oa + c1 pa + theta (c2 oj + c3 pj),
-  // jerk = (c4 oa + c5 pa) / theta + c6 oj + c7 pj (smallN.cc:487-510)
-  double q0, q1, q2, q3;
-  {
-    const int l = lane & 7;
-    q0 = l < 2 ? 0.5 : l == 2 ? 0.25 : l == 4 ? -0.75 : l == 5 ? 0.75 : -0.25;
-    q1 = l == 0 ? -0.75 : l == 1 ? 0.75 : l == 2 || l == 3 ? -0.25 : l == 6 ? -0.5 : l == 7 ? 0.5 : 0.0;
-    q2 = l < 2 ? 0.0 : l == 2 ? -0.25 : l == 3 ? 0.25 : l == 5 ? -0.75 : 0.75;
-    q3 = l == 0 || l == 2 || l == 3 ? 0.25 : l == 1 ? -0.25 : 0.0;
-  }
   Comp<NS> B;
   __syncwarp();
 #pragma unroll
@@ -1336,7 +1368,8 @@ __device__ __noinline__ void integrate(UnpSmem &S, int lane, TreeRun &run, const
     }
     // predict_loworder (hdyn.h:192-201: with the stored old force)
     {
-      const double h = dt, h3 = h * (1.0 / 3.0), h2 = h * 0.5;
+      const double h = P.on ? dt : (t + dt) - t;  // without the tree, as batch_exact_kernel's
+      const double h3 = g6_div_const(h, 3.0, 1.0 / 3.0), h2 = h * 0.5;
       FOR_COMP(r, c, n) {
         const double oj = B.ojerk[r], oa = B.oacc[r];
         B.pp[r] = fma(fma(fma(oj, h3, oa), h2, B.vel[r]), h, B.pos[r]);
@@ -1349,36 +1382,34 @@ __device__ __noinline__ void integrate(UnpSmem &S, int lane, TreeRun &run, const
     for (int it = 0; it <= nit; it++) {
       const double prev = new_dt;
       end_dt = tree_forces<MODE, NS>(S, n, lane, B, t + new_dt, eta, &bim, &bjm);
-      double iprev = 0.0;
+      const Div by_prev(prev);
       if (it < nit) {
-        iprev = rcp64(prev);
         new_dt = 0.5 * (dt + end_dt);
-        new_dt = dt + 0.5 * (end_dt - dt) * (new_dt * iprev);
+        new_dt = dt + 0.5 * (end_dt - dt) * by_prev(new_dt);
         if (new_dt >= lim) {
           new_dt = lim;
           nit = 0;
         }
       }
       if (new_dt != prev) {  // correct_acc_and_jerk(new_dt, prev)
-        const double theta = 0.5 * prev, itheta = 2.0 * iprev;
-        const double tau = (new_dt - theta) * itheta;
-        double cc = fma(fma(fma(q3, tau, q2), tau, q1), tau, q0);
-        const int l = lane & 7;
-        cc *= (l & 6) == 2 ? theta : (l & 6) == 4 ? itheta : 1.0;
-        double k[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) k[q] = __shfl_sync(0xffffffffu, cc, q);
+        const double theta = 0.5 * prev, itheta = 2.0 * by_prev.inv();
+        const double tau = 2.0 * by_prev(new_dt - theta), tau2 = tau * tau, tau3 = tau2 * tau;
         FOR_COMP(r, c, n) {
           const double pa = B.acc[r], pj = B.jerk[r], oa = B.oacc[r], oj = B.ojerk[r];
-          B.acc[r] = fma(k[3], pj, fma(k[2], oj, fma(k[1], pa, k[0] * oa)));
-          B.jerk[r] = fma(k[7], pj, fma(k[6], oj, fma(k[5], pa, k[4] * oa)));
+          B.acc[r] = 0.25 * (oa * (2 - 3 * tau + tau3) + pa * (2 + 3 * tau - tau3) +
+                             oj * theta * (1 - tau - tau2 + tau3) +
+                             pj * theta * (-1 - tau + tau2 + tau3));
+          B.jerk[r] = 0.25 * (oa * itheta * 3 * (-1 + tau2) + pa * itheta * 3 * (1 - tau2) +
+                              oj * (-1 - 2 * tau + 3 * tau2) + pj * (-1 + 2 * tau + 3 * tau2));
         }
       }
       // correct_pos_and_vel(new_dt)
-      const double hh = 0.5 * new_dt, h12 = new_dt * new_dt * (1.0 / 12.0);
+      const double nd2 = new_dt * new_dt;
       FOR_COMP(r, c, n) {
-        B.pv[r] = fma(-h12, B.jerk[r] - B.ojerk[r], fma(hh, B.acc[r] + B.oacc[r], B.vel[r]));
-        B.pp[r] = fma(-h12, B.acc[r] - B.oacc[r], fma(hh, B.pv[r] + B.vel[r], B.pos[r]));
+        B.pv[r] = B.vel[r] + new_dt * (B.acc[r] + B.oacc[r]) * 0.5 -
+                  nd2 * (B.jerk[r] - B.ojerk[r]) * (1.0 / 12.0);
+        B.pp[r] = B.pos[r] + new_dt * (B.pv[r] + B.vel[r]) * 0.5 -
+                  nd2 * (B.acc[r] - B.oacc[r]) * (1.0 / 12.0);
       }
     }
 #pragma unroll
@@ -1410,11 +1441,12 @@ __device__ __noinline__ void integrate(UnpSmem &S, int lane, TreeRun &run, const
       vel[c] = B.vel[r];
     } else if (S.nd[i] == i) {
       const BinRec &bb = S.bin[b];
-      const double iM = rcp64(bb.mi + bb.mj), x = S.kr[b][k], v = S.kr[b][3 + k];
-      pos[3 * bb.li + k] = B.pos[r] - bb.mj * iM * x;
-      vel[3 * bb.li + k] = B.vel[r] - bb.mj * iM * v;
-      pos[3 * bb.lj + k] = B.pos[r] + bb.mi * iM * x;
-      vel[3 * bb.lj + k] = B.vel[r] + bb.mi * iM * v;
+      const Div by_M(bb.mi + bb.mj);
+      const double gi = by_M(bb.mj), gj = by_M(bb.mi), x = S.kr[b][k], v = S.kr[b][3 + k];
+      pos[3 * bb.li + k] = B.pos[r] - gi * x;
+      vel[3 * bb.li + k] = B.vel[r] - gi * v;
+      pos[3 * bb.lj + k] = B.pos[r] + gj * x;
+      vel[3 * bb.lj + k] = B.vel[r] + gj * v;
     }
   }
   run.t = t;
