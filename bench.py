@@ -465,7 +465,7 @@ def run_ours(args):
                        "share_of_step": statistics.mean(rms) / (1e3 * total / args.steps),
                        "what": "refine_kernel after the force kernel: acc and pot redone in "
                                "FP64 where the FP32 sum is ill-conditioned (kappa > 48), with "
-                               "compensated FP32 sums and the large terms in FP64 where one "
+                               "compensated FP32 sums and the large terms in float-float where one "
                                "term exceeds |a|"},
             "predictor": {"ms": statistics.mean(pms), "GB_s": pred_gbs,
                           "bytes_per_j": 15 * 8 + 4 + 48,
