@@ -29,9 +29,10 @@
 //   * JL j-lanes share each i-particle (JL = 1 for large i-blocks, up to
 //     128 for tiny ones); j is also split across CTAs (grid.y) so that small
 //     active blocks still fill all 152 SMs.
-//   * Lanes of one i merge with warp shuffles (plus shared memory across
-//     warps for JL > 32); CTAs of one i merge in a second pass kernel, in
-//     fixed order, with float-float adds: deterministic.
+//   * Lanes of one i merge with warp shuffles, for JL >= 16 through a table
+//     in shared memory; CTAs of one i merge in the last CTA of the group (one
+//     or two i per group) or in a second kernel, in fixed order, with
+//     float-float adds: deterministic.
 //   * Nearest neighbour (optional, a template flag): the hot loop keeps only
 //     a running min of r2 (one FMNMX per pair) and the tile where it last
 //     improved; after the loop that tile is re-read from L2 and re-scanned
