@@ -249,3 +249,34 @@ def test_component_layout_edges(g6, mode, tol, unp):
             assert r["steps"][s] == st, n
         assert np.abs(r["pos"][a:b] - px).max() <= tol * 1e-3, n
         assert np.abs(r["vel"][a:b] - pv).max() <= tol * 1e3 * np.abs(pv).max(), n
+
+
+@pytest.mark.parametrize("unp", [False, True])
+def test_split_step_with_equal_pairs(g6, unp):
+    """Rings in circular motion: every body has two nearest pairs of the same
+    step, so the step comes from the quotients of all pairs, for one and two
+    leaves per lane.  Over 0.2 of the dynamical time (R = 1) FP32 terms move a
+    body by 1e-7 of a t^2 / 2 <= 0.1 and the end time by 1e-7 of a step; the
+    ring's own instability grows at most by e^0.8."""
+    sizes = [2, 3, 4, 31, 32, 33, 63, 64]
+    ms, xs, vs = [], [], []
+    for n in sizes:
+        a = 2 * np.pi * np.arange(n) / n
+        x = np.stack([np.cos(a), np.sin(a), 0 * a], 1)
+        pull = (1.0 / n) * (1 / (4 * np.sin(np.pi * np.arange(1, n) / n))).sum()
+        vs.append(np.sqrt(pull) * np.stack([-np.sin(a), np.cos(a), 0 * a], 1))
+        ms.append(np.full(n, 1.0 / n))
+        xs.append(x)
+    g6.batch_unperturbed(unp, dt_crit=0.0)
+    try:
+        r = g6.batch_run(np.array(sizes, np.int32), 0.2, np.concatenate(ms), np.concatenate(xs),
+                         np.concatenate(vs), mode="split", max_steps=100000)
+    finally:
+        g6.batch_unperturbed(False)
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    for s, n in enumerate(sizes):
+        px, pv, tf, st = oracle.smalln(ms[s], xs[s], vs[s], 0.14, 0.2)
+        assert r["status"][s] == 0 and r["steps"][s] == st, n
+        assert abs(r["t_final"][s] - tf) <= 1e-6
+        assert np.abs(r["pos"][off[s]:off[s + 1]] - px).max() <= 1e-6, n
+        assert np.abs(r["vel"][off[s]:off[s + 1]] - pv).max() <= 1e-6 * np.abs(pv).max(), n
