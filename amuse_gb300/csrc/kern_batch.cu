@@ -356,8 +356,8 @@ __global__ void batch_exact_kernel(const int *__restrict__ order, const int *__r
 // corrector's eight coefficients are evaluated by eight lanes at once;
 // quotients and square roots are a MUFU seed, one third-order step and one
 // corrected product, which rounds right; and comparisons of non-negative
-// values are integer compares.  4096 scatterings 20.0 -> 5.5 ms, 1024 systems
-// of 3 to 64 bodies over 0.05 crossing times 10.3 -> 6.3 ms.  A lone warp is bound by instruction latency (5.7 cycles per
+// values are integer compares.  4096 scatterings 20.4 -> 5.4 ms, 1024 systems
+// of 3 to 64 bodies over 0.05 crossing times 10.3 -> 6.1 ms.  A lone warp is bound by instruction latency (5.7 cycles per
 // instruction of 32,000 a step at n = 52), so the split mode's pair loop reads
 // a body in three or four 16-byte loads and evaluates two pairs per packed
 // f32x2 instruction.
@@ -1425,11 +1425,19 @@ __device__ __noinline__ void integrate(UnpSmem &S, int lane, TreeRun &run, const
       }
       // correct_pos_and_vel(new_dt)
       const double nd2 = new_dt * new_dt;
-      FOR_COMP(r, c, n) {
-        B.pv[r] = B.vel[r] + new_dt * (B.acc[r] + B.oacc[r]) * 0.5 -
-                  nd2 * (B.jerk[r] - B.ojerk[r]) * (1.0 / 12.0);
-        B.pp[r] = B.pos[r] + new_dt * (B.pv[r] + B.vel[r]) * 0.5 -
-                  nd2 * (B.acc[r] - B.oacc[r]) * (1.0 / 12.0);
+      if (it < nit) {  // only the next evaluation's state: two FP64 instructions fewer each
+        const double hh = 0.5 * new_dt, h12 = nd2 * (1.0 / 12.0);
+        FOR_COMP(r, c, n) {
+          B.pv[r] = fma(-h12, B.jerk[r] - B.ojerk[r], fma(hh, B.acc[r] + B.oacc[r], B.vel[r]));
+          B.pp[r] = fma(-h12, B.acc[r] - B.oacc[r], fma(hh, B.pv[r] + B.vel[r], B.pos[r]));
+        }
+      } else {
+        FOR_COMP(r, c, n) {
+          B.pv[r] = B.vel[r] + new_dt * (B.acc[r] + B.oacc[r]) * 0.5 -
+                    nd2 * (B.jerk[r] - B.ojerk[r]) * (1.0 / 12.0);
+          B.pp[r] = B.pos[r] + new_dt * (B.pv[r] + B.vel[r]) * 0.5 -
+                    nd2 * (B.acc[r] - B.oacc[r]) * (1.0 / 12.0);
+        }
       }
     }
 #pragma unroll
