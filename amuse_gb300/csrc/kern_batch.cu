@@ -357,10 +357,10 @@ __global__ void batch_exact_kernel(const int *__restrict__ order, const int *__r
 // quotients and square roots are a MUFU seed, one third-order step and one
 // corrected product, which rounds right; and comparisons of non-negative
 // values are integer compares.  4096 scatterings 20.4 -> 5.4 ms, 1024 systems
-// of 3 to 64 bodies over 0.05 crossing times 10.3 -> 6.1 ms.  A lone warp is bound by instruction latency (5.7 cycles per
-// instruction of 32,000 a step at n = 52), so the split mode's pair loop reads
-// a body in three or four 16-byte loads and evaluates two pairs per packed
-// f32x2 instruction.
+// of 3 to 64 bodies over 0.05 crossing times 10.3 -> 6.1 ms.  A lone warp is
+// bound by instruction latency (6 to 7 cycles per instruction of 32,000 a step
+// at n = 52), so the split mode's pair loop reads a body in three or four
+// 16-byte loads and evaluates two pairs per packed f32x2 instruction.
 __device__ __forceinline__ float rsqrt_approx(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
