@@ -349,12 +349,14 @@ static int check_open(void) {
 /* Apply staged j updates.  Up to UPD_DIRECT records (a block's) the scatter
    kernel reads them where they are, in pinned host memory: it needs each once,
    and a copy before it costs more than the reads (ph4's block of 8: one copy
-   and its gap, about 4 us).  More go by one copy. */
+   and its gap, about 4 us).  More go by one copy.  Calls that may allocate
+   make room for that copy whatever the number, so that a later call that may
+   not finds the buffer there. */
 #define UPD_DIRECT 1024
-static int flush_updates(void) {
+static int flush_updates(int may_alloc) {
   if (G.n_upd == 0) return 0;
   const int direct = G.n_upd <= UPD_DIRECT;
-  if (!direct && G.n_upd > G.cap_dupd) {
+  if (G.n_upd > G.cap_dupd && (may_alloc || !direct)) {
     cudaFree(G.d_upd);
     G.d_upd = NULL;
     G.cap_dupd = 0;
@@ -682,7 +684,7 @@ static int stage_force_host(int nj, int ni, const int *index, const double *xi,
     CK(cudaMemcpyAsync(G.d_in, G.h_in,
                        sizeof(double) * 6 * (size_t)ni + sizeof(int) * (size_t)ni,
                        cudaMemcpyHostToDevice, G.st));
-    rc = flush_updates();
+    rc = flush_updates(1);
     if (rc) return rc;
     rc = predict_if_needed(nj);
     if (rc) return rc;
@@ -1134,7 +1136,7 @@ int g6x_force_dev(double ti, double eps2, int nj, int ni, const double *d_xi,
   G.ti = ti;
   rc = ensure_io(1);
   if (rc) return rc;
-  rc = flush_updates();
+  rc = flush_updates(1);
   if (rc) return rc;
   rc = predict_if_needed(nj);
   if (rc) return rc;
@@ -1172,7 +1174,7 @@ int g6x_force_slots(double ti, double eps2, int nj, int ni, const int *d_ilist, 
   G.ti = ti;
   rc = ensure_io(1);
   if (rc) return rc;
-  rc = flush_updates();
+  rc = flush_updates(1);
   if (rc) return rc;
   rc = predict_if_needed(nj);
   if (rc) return rc;
@@ -1320,7 +1322,7 @@ int g6x_knn(int k, int nj, double t, int ni, const int *slots, int *ids, double 
       seterr("g6x_knn: slot %d out of [0, %d)", slots[i], nj);
       return G6_ERR_ARG;
     }
-  rc = flush_updates();
+  rc = flush_updates(1);
   if (rc) return rc;
   /* the filter reads the split records: predict them to t */
   if (g6k_predict(&G.js, nj, t, G6_PREC_SPLIT, G.st)) return G6_ERR_CUDA;
@@ -1635,7 +1637,7 @@ int g6x_force_dev_noalloc(double ti, double eps2, int nj, int ni, const double *
            "allocation", nj, G.js.cap);
     return G6_ERR_ARG;
   }
-  if (G.n_upd > G.cap_dupd) {
+  if (G.n_upd > UPD_DIRECT && G.n_upd > G.cap_dupd) { /* fewer are read in place */
     seterr("g6x_force_dev_noalloc: %d staged j updates exceed the update buffer (%d); it would "
            "need an allocation", G.n_upd, G.cap_dupd);
     return G6_ERR_ARG;
@@ -1645,7 +1647,7 @@ int g6x_force_dev_noalloc(double ti, double eps2, int nj, int ni, const double *
     return G6_ERR_STATE;
   }
   G.ti = ti;
-  rc = flush_updates(); /* copies into the existing update buffer only */
+  rc = flush_updates(0); /* reads the staging ring, or copies into the existing buffer */
   if (rc) return rc;
   rc = predict_if_needed(nj); /* the j-store already holds nj_pad slots */
   if (rc) return rc;

@@ -9,6 +9,10 @@ call's contents), in both precisions and with and without the nearest
 neighbour: the launch shape and the fixed-order merge are the same, so the
 results must be bit-identical.  This file is collected last so that a run
 stopping at the first failure has already run every other test."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -16,6 +20,7 @@ import amuse_gb300 as ag
 from amuse_gb300 import ic
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.mark.parametrize("want_nn", [True, False], ids=["nn", "no-nn"])
@@ -80,3 +85,42 @@ def test_noalloc_refuses_oversized_scratch(g6):
     with pytest.raises(ag.G6Error, match="scratch"):
         g6.force_dev_noalloc(0.0, 1e-6, n, n, dx.data_ptr(), dv.data_ptr(), None, da.data_ptr(),
                              dj.data_ptr(), dp.data_ptr(), None, sync=True)
+
+
+# A process of its own: the library keeps an update buffer once it has one.
+STAGED = """
+import numpy as np, torch
+import amuse_gb300 as ag
+from amuse_gb300 import ic
+n, first = {n}, 512
+g6 = ag.G6X(0)
+np.random.seed(33)
+m, x, v = ic.plummer(n)
+ids = np.arange(1, n + 1)
+ag.drive_load(m[:first], x[:first], v[:first], ids=ids[:first])
+ag.drive_force(first, 0.0, 1e-4, ids[:8], x[:8], v[:8])  # applies them: fewer than 1024
+ag.drive_load(2 * m, x, v, ids=ids)                        # staged when the call comes
+new = lambda *s: torch.full(s, float("nan"), dtype=torch.float64, device="cuda")
+dx, dv = (torch.tensor(q[:64], device="cuda").contiguous() for q in (x, v))
+ds = torch.arange(64, dtype=torch.int32, device="cuda")
+out = []
+for f in (g6.force_dev_noalloc, g6.force_dev):
+    o = new(64, 3), new(64, 3), new(64)
+    torch.cuda.synchronize()
+    f(0.0, 1e-4, n, 64, dx.data_ptr(), dv.data_ptr(), ds.data_ptr(), *(q.data_ptr() for q in o),
+      None, sync=True)
+    out.append([q.cpu().numpy() for q in o])
+assert all(np.array_equal(a, b) for a, b in zip(*out))
+rel = x - x[0]
+r = np.sqrt((rel[1:] ** 2).sum(1) + 1e-4)
+assert abs(out[0][2][0] + (2 * m[1:] / r).sum()) < 1e-5 * abs(out[0][2][0])
+"""
+
+
+@pytest.mark.parametrize("n", [512, 2000], ids=["read-in-place", "by-copy"])
+def test_noalloc_takes_staged_updates(lib_built, n):
+    """Updates staged before the call are taken where every earlier flush was
+    small enough to be read in place, as many as the staging ring held."""
+    r = subprocess.run([sys.executable, "-c", STAGED.format(n=n)], cwd=ROOT, text=True,
+                       stdout=subprocess.PIPE, stderr=subprocess.STDOUT, timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:]
