@@ -1807,13 +1807,15 @@ int balanced_splits(int ni, int ntiles, int jl, int ns0, int force_nsplit) {
     if (c <= 3) return (double)c * ((ntiles + ns - 1) / ns + OV) / EFF[c - 1] + merge;
     return (double)c * (tiles + OV) + merge;
   };
-  // within the fixed scratch array where the count before was
+  // within the fixed scratch array where the count before was (one split
+  // needs none)
   const size_t room = (size_t)16 << 20, rec = (size_t)ni * sizeof(SplitP::Out);
+  const bool fits = ns0 == 1 || (size_t)ns0 * rec <= room;
   int best = ns0;
   double bc = cost(ns0) * 0.99;
   const int most = ntiles < 128 ? ntiles : 128;
   for (int ns = 1; ns <= most; ns++) {
-    if (ns > ns0 && (size_t)ns0 * rec <= room && (size_t)ns * rec > room) break;
+    if (ns > ns0 && fits && (size_t)ns * rec > room) break;
     const double c = cost(ns);
     if (c < bc) {
       bc = c;

@@ -87,6 +87,29 @@ def test_noalloc_refuses_oversized_scratch(g6):
                              dj.data_ptr(), dp.data_ptr(), None, sync=True)
 
 
+@pytest.mark.parametrize("ni,nj", [(226304, 226560), (225280, 262144)])
+def test_noalloc_takes_unsplit_shapes(g6, ni, nj):
+    """So many i that one split of j fills the GPU, and whose partial records
+    would not fit the fixed array if j were split: no scratch, no refusal."""
+    torch = pytest.importorskip("torch")
+    g6.set_precision(ag.SPLIT)
+    np.random.seed(34)
+    m, x, v = ic.plummer(nj)
+    g6.load_particles(m, x, v)
+    new = lambda *s: torch.full(s, float("nan"), dtype=torch.float64, device="cuda")
+    dx, dv = (torch.tensor(q[:ni], device="cuda").contiguous() for q in (x, v))
+    ds = torch.arange(ni, dtype=torch.int32, device="cuda")
+    out = []
+    for f in (g6.force_dev_noalloc, g6.force_dev):
+        o = new(ni, 3), new(ni, 3), new(ni)
+        torch.cuda.synchronize()
+        f(0.0, 1e-4, nj, ni, dx.data_ptr(), dv.data_ptr(), ds.data_ptr(),
+          *(q.data_ptr() for q in o), None, sync=True)
+        assert g6.stats()["nsplit"] == 1
+        out.append(o)
+    assert all(torch.equal(a, b) for a, b in zip(*out)) and torch.isfinite(out[0][0]).all()
+
+
 # A process of its own: the library keeps an update buffer once it has one.
 STAGED = """
 import numpy as np, torch
