@@ -554,3 +554,21 @@ def test_lane_and_split_merges(g6, jl, ns, ni):
     assert ea.max() <= 1e-6 and ej.max() <= 1e-4
     assert np.all(np.abs(o["pot"] - ref["pot"]) <= 1e-6 * np.abs(ref["pot"]))
     assert np.array_equal(o["nn"], ref["nn"])
+
+
+def test_partial_records_bounded(g6):
+    """The scratch for the j splits' partial records (80 bytes per split and i)
+    of a large call stays at what splits of equal length take, 8 of them here."""
+    torch = pytest.importorskip("torch")
+    g6.set_precision(ag.SPLIT)
+    ni, nj = 273408, 1 << 20
+    np.random.seed(35)
+    m, x, v = ic.plummer(nj)
+    g6.load_particles(m, x, v)
+    f = dict(dtype=torch.float64, device="cuda")
+    dx, dv = (torch.tensor(q[:ni], device="cuda").contiguous() for q in (x, v))
+    out = torch.zeros(ni, 3, **f), torch.zeros(ni, 3, **f), torch.zeros(ni, **f)
+    torch.cuda.synchronize()
+    g6.force_dev(0.0, 1e-4, nj, ni, dx.data_ptr(), dv.data_ptr(), None,
+                 *(q.data_ptr() for q in out), None, sync=True)
+    assert g6.stats()["nsplit"] * ni * 80 <= 8 * ni * 80
