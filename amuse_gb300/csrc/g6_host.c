@@ -1976,9 +1976,9 @@ int g6x_batch_run(int nsys, const int *n_per_sys, const double *t_end, const dou
   return 0;
 }
 
-/* Autotuner: time every (warps per CTA, CTAs per SM) shape whose warps fit
- * the register file on a copy of the given systems (shortened to frac of
- * their end time) and keep the fastest.  out[0..2] = best wpc, cps, ms. */
+/* Autotuner: time (warps per CTA, CTAs per SM) shapes on a copy of the given
+ * systems (shortened to frac of their end time) and keep the fastest.  The
+ * launch cuts a shape to the CTAs that are resident at once.  out[0..2] = best wpc, cps, ms. */
 int g6x_batch_tune(int nsys, const int *n_per_sys, const double *t_end, const double *mass,
                    const double (*pos)[3], const double (*vel)[3], double eta, int n_iter,
                    int exact, double frac, double out[3]) {

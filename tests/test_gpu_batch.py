@@ -280,3 +280,27 @@ def test_split_step_with_equal_pairs(g6, unp):
         assert abs(r["t_final"][s] - tf) <= 1e-6
         assert np.abs(r["pos"][off[s]:off[s + 1]] - px).max() <= 1e-6, n
         assert np.abs(r["vel"][off[s]:off[s + 1]] - pv).max() <= 1e-6 * np.abs(pv).max(), n
+
+
+@pytest.mark.parametrize("mode,unp", [("split", False), ("fast", True), ("exact", False)])
+def test_shape_beyond_residency(g6, mode, unp):
+    """More CTAs per SM asked for than fit (4 x 3 and 4 x 4 warps) leave no
+    system waiting for a whole CTA to end: 400 equal systems, fewer than the
+    warps that fit at once, would take twice as long as at 4 x 2."""
+    m, x, v = ic.plummer(24, do_scale=True, rng=np.random.RandomState(13))
+    ns = np.full(400, 24, np.int32)
+    m, x, v = np.tile(m, 400), np.tile(x, (400, 1)) * 1e-3, np.tile(v, (400, 1)) / np.sqrt(1e-3)
+    t_end = 0.01 * 2 * np.sqrt(2) * 1e-3 ** 1.5
+    g6.batch_unperturbed(unp)
+    ms, pos = [], []
+    try:
+        for shape in ((4, 2), (4, 3), (4, 4)):
+            g6.batch_config(*shape)
+            r = [g6.batch_run(ns, t_end, m, x, v, mode=mode, max_steps=100000) for _ in range(4)]
+            ms.append(min(q["elapsed_ms"] for q in r[1:]))
+            pos.append(r[-1]["pos"])
+    finally:
+        g6.batch_unperturbed(False)
+        g6.batch_config(4, 2)
+    assert np.array_equal(pos[0], pos[1]) and np.array_equal(pos[0], pos[2])
+    assert max(ms) <= 1.4 * ms[0], ms
