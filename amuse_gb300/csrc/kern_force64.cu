@@ -57,6 +57,7 @@ struct K64 {
 
 constexpr unsigned long long INF_BITS = 0x7ff0000000000000ull;
 constexpr unsigned FULL = 0xffffffffu;
+constexpr int FOLD = 64;  // records per lane between folds
 
 // 1/sqrt(x), x normal: the MUFU seed y (relative error e below 2^-19, PTX
 // rsqrt.approx.ftz.f64) and one step of third order, y + y h (1/2 + 3/8 h)
@@ -133,48 +134,72 @@ __global__ void __launch_bounds__(32) force64_kernel(K64 kp, int il_log2) {
   const int j1 = min(kp.nj, j0 + kp.chunk);
   const int last = kp.nj - 1;
   Rec64 nxt = load_rec(kp.rec + min(j0 + jl, last));
+  // FOLD records at a time, then into totals: a lane's one running sum over its
+  // whole chunk (16384 i and j: 1600 terms) had three times the rounding error.
+  double ta[3] = {0.0, 0.0, 0.0}, tj[3] = {0.0, 0.0, 0.0}, tp = 0.0;
+  for (int jb = j0 + jl;;) {
+    const int je = min(j1, jb + FOLD * JL);
 #pragma unroll 2
-  for (int j = j0 + jl; j < j1; j += JL) {
-    const Rec64 r = nxt;
-    nxt = load_rec(kp.rec + min(j + JL, last));
-    const double dx = r.x - x, dy = r.y - y, dz = r.z - z;
-    double r2;
-    if (NN) {
-      // ph4's key: the unsoftened r^2 summed in component order without
-      // contraction (idata.cc:200-205,214-218), so the argmin (first slot on
-      // equal keys) is ph4's neighbour bit for bit
-      const double key = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
-                                   __dmul_rn(dz, dz));
-      const unsigned long long kb = (unsigned long long)__double_as_longlong(key);
-      if (j != self && kb < s.key) {
-        s.key = kb;
-        s.nn = j;
+    for (int j = jb; j < je; j += JL) {
+      const Rec64 r = nxt;
+      nxt = load_rec(kp.rec + min(j + JL, last));
+      const double dx = r.x - x, dy = r.y - y, dz = r.z - z;
+      double r2;
+      if (NN) {
+        // ph4's key: the unsoftened r^2 summed in component order without
+        // contraction (idata.cc:200-205,214-218), so the argmin (first slot on
+        // equal keys) is ph4's neighbour bit for bit
+        const double key = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
+                                     __dmul_rn(dz, dz));
+        const unsigned long long kb = (unsigned long long)__double_as_longlong(key);
+        if (j != self && kb < s.key) {
+          s.key = kb;
+          s.nn = j;
+        }
+        r2 = key + eps2;
+      } else {
+        r2 = __fma_rn(dz, dz, __fma_rn(dy, dy, __fma_rn(dx, dx, eps2)));
       }
-      r2 = key + eps2;
-    } else {
-      r2 = __fma_rn(dz, dz, __fma_rn(dy, dy, __fma_rn(dx, dx, eps2)));
+      double rinv = rsqrt64(r2);
+      rinv = j == self ? 0.0 : rinv;
+      const double dvx = r.vx - vx, dvy = r.vy - vy, dvz = r.vz - vz;
+      const double rv = __fma_rn(dz, dvz, __fma_rn(dy, dvy, dx * dvx));
+      const double rinv2 = rinv * rinv;
+      const double mri = r.m * rinv;
+      const double mr3i = mri * rinv2;
+      double a3;
+      if (HJ) {  // the hermite code's jerk (src/amuse_hermite/interface.cc:440-449,486)
+        const double q = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
+        a3 = j == self ? 0.0 : -3.0 * (rv * rcp64(q));
+      } else {
+        a3 = -3.0 * (rv * rinv2);
+      }
+      s.a[0] = __fma_rn(mr3i, dx, s.a[0]);
+      s.a[1] = __fma_rn(mr3i, dy, s.a[1]);
+      s.a[2] = __fma_rn(mr3i, dz, s.a[2]);
+      s.j[0] = __fma_rn(mr3i, __fma_rn(a3, dx, dvx), s.j[0]);
+      s.j[1] = __fma_rn(mr3i, __fma_rn(a3, dy, dvy), s.j[1]);
+      s.j[2] = __fma_rn(mr3i, __fma_rn(a3, dz, dvz), s.j[2]);
+      s.p += mri;
     }
-    double rinv = rsqrt64(r2);
-    rinv = j == self ? 0.0 : rinv;
-    const double dvx = r.vx - vx, dvy = r.vy - vy, dvz = r.vz - vz;
-    const double rv = __fma_rn(dz, dvz, __fma_rn(dy, dvy, dx * dvx));
-    const double rinv2 = rinv * rinv;
-    const double mri = r.m * rinv;
-    const double mr3i = mri * rinv2;
-    double a3;
-    if (HJ) {  // the hermite code's jerk (src/amuse_hermite/interface.cc:440-449,486)
-      const double q = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
-      a3 = j == self ? 0.0 : -3.0 * (rv * rcp64(q));
-    } else {
-      a3 = -3.0 * (rv * rinv2);
+    jb += FOLD * JL;
+    if (jb >= j1) break;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      ta[k] += s.a[k];
+      tj[k] += s.j[k];
+      s.a[k] = s.j[k] = 0.0;
     }
-    s.a[0] = __fma_rn(mr3i, dx, s.a[0]);
-    s.a[1] = __fma_rn(mr3i, dy, s.a[1]);
-    s.a[2] = __fma_rn(mr3i, dz, s.a[2]);
-    s.j[0] = __fma_rn(mr3i, __fma_rn(a3, dx, dvx), s.j[0]);
-    s.j[1] = __fma_rn(mr3i, __fma_rn(a3, dy, dvy), s.j[1]);
-    s.j[2] = __fma_rn(mr3i, __fma_rn(a3, dz, dvz), s.j[2]);
-    s.p += mri;
+    tp += s.p;
+    s.p = 0.0;
+  }
+  if (kp.chunk > FOLD * JL) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      s.a[k] += ta[k];
+      s.j[k] += tj[k];
+    }
+    s.p += tp;
   }
   pdl_trigger();  // j loop done: the next kernel of the chain may be scheduled
 

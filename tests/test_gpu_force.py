@@ -572,3 +572,36 @@ def test_partial_records_bounded(g6):
     g6.force_dev(0.0, 1e-4, nj, ni, dx.data_ptr(), dv.data_ptr(), None,
                  *(q.data_ptr() for q in out), None, sync=True)
     assert g6.stats()["nsplit"] * ni * 80 <= 8 * ni * 80
+
+
+@pytest.mark.skipif(np.finfo(np.longdouble).eps > 2.0 ** -80, reason="no 128-bit long double")
+def test_fp64_sums_are_folded(g6):
+    """The FP64 potential of all of 16384 bodies against 128-bit sums.  A sum of
+    m like terms in FP64, one after the other, has an rms error of about 0.4 u
+    sqrt(m / 3), u = 2^-53: 64 terms of a fold, then at most 64 folds of a chunk
+    and a few chunks, each level averaged over those above it, 0.8 u in all."""
+    torch = pytest.importorskip("torch")
+    n = 16384
+    np.random.seed(36)
+    m, x, v = ic.plummer(n)
+    m = ic.salpeter_masses(n, -2.35, 0.1, 100.0)
+    f = dict(dtype=torch.float64, device="cuda")
+    dx, dv = (torch.tensor(q, device="cuda").contiguous() for q in (x, v))
+    ds = torch.arange(n, dtype=torch.int32, device="cuda")
+    out = torch.zeros(n, 3, **f), torch.zeros(n, 3, **f), torch.zeros(n, **f)
+    g6.set_precision(ag.FP64)
+    try:
+        g6.load_particles(m, x, v)
+        torch.cuda.synchronize()
+        g6.force_dev(0.0, 1e-6, n, n, dx.data_ptr(), dv.data_ptr(), ds.data_ptr(),
+                     *(q.data_ptr() for q in out), None, sync=True)
+    finally:
+        g6.set_precision(ag.SPLIT)
+    pot, err = out[2].cpu().numpy(), []
+    X, M = x.astype(np.longdouble), m.astype(np.longdouble)
+    for i in range(0, n, n // 128):
+        r2 = ((X - X[i]) ** 2).sum(1) + (np.longdouble(1e-6) + np.longdouble(2) ** -52)
+        w = M / np.sqrt(r2)
+        w[i] = 0
+        err.append(float(-pot[i] / w.sum() - 1))
+    assert np.sqrt(np.mean(np.square(err))) <= 1.5 * 2.0 ** -53
