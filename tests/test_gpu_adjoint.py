@@ -153,3 +153,38 @@ def test_fixed_force_matches_torch(g6, precision):
             assert err.max() <= 1e-10, err.max()
         else:
             assert np.quantile(err, 0.99) <= tol_split, np.quantile(err, 0.99)
+
+
+@pytest.mark.skipif(np.finfo(np.longdouble).eps > 2.0 ** -80, reason="no 128-bit long double")
+@pytest.mark.parametrize("jerk", ["hermite", "softened"])
+def test_vjp_fp64_sums_are_folded(g6, jerk):
+    """The FP64 mass gradient of central bodies against 128-bit sums, with
+    outward cotangents, so that nearly all of a body's 16384 terms have one
+    sign.  A sum of m such terms in FP64, one after the other, has an rms error
+    of about 0.4 u sqrt(m / 3), u = 2^-53: 128 terms of four tiles, then the 16 sums
+    of a split and the eight splits, each level averaged over those above it,
+    about u in all."""
+    import amuse_gb300 as ag
+    from amuse_gb300 import ic
+    n = 16384
+    rng = np.random.RandomState(14)
+    m, x, v = ic.plummer(n, rng=rng)
+    la = x / np.linalg.norm(x, axis=1)[:, None]
+    f = dict(dtype=torch.float64, device="cuda")
+    arg = [torch.tensor(q, device="cuda") for q in (x, v, m, la, np.zeros_like(x))]
+    out = torch.zeros(n, 3, **f), torch.zeros(n, 3, **f), torch.zeros(n, **f)
+    torch.cuda.synchronize()
+    g6.set_precision(ag.FP64)
+    g6.set_fixed_jerk(ag.JERK_HERMITE if jerk == "hermite" else ag.JERK_SOFTENED)
+    try:
+        g6.force_vjp(n, 1e-4, *(q.data_ptr() for q in arg), *(q.data_ptr() for q in out))
+    finally:
+        g6.set_precision(ag.SPLIT)
+        g6.set_fixed_jerk(ag.JERK_HERMITE)
+    gm, err = out[2].cpu().numpy(), []
+    X, LA = x.astype(np.longdouble), la.astype(np.longdouble)
+    for i in np.argsort(np.linalg.norm(x, axis=1))[:96]:
+        r = X - X[i]
+        w = ((r * r).sum(1) + (np.longdouble(1e-4) + np.longdouble(2) ** -52)) ** np.longdouble(-1.5)
+        err.append(float(gm[i] / -((LA * r).sum(1) * w).sum() - 1))
+    assert np.sqrt(np.mean(np.square(err))) <= 2 * 2.0 ** -53
