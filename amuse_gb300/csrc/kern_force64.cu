@@ -57,7 +57,8 @@ struct K64 {
 
 constexpr unsigned long long INF_BITS = 0x7ff0000000000000ull;
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int FOLD = 64;  // records per lane between folds
+constexpr int LONG = 128;  // more records than this per lane are folded,
+constexpr int FOLD = 64;   // so many at a time
 
 // 1/sqrt(x), x normal: the MUFU seed y (relative error e below 2^-19, PTX
 // rsqrt.approx.ftz.f64) and one step of third order, y + y h (1/2 + 3/8 h)
@@ -100,7 +101,14 @@ __device__ __forceinline__ void nn_take(unsigned long long &k, int &n, unsigned 
   }
 }
 
-template <bool NN, bool HJ>
+// FOLDS: a lane has more than LONG records of its chunk and adds them up FOLD at a
+// time (one running sum over all of them had up to four times the rounding
+// error).  The totals take 14 registers and 8 of 28 warps off an SM, which shape64
+// allows for.  Tried for them: shared memory (an SM takes no CTA of this kernel
+// before its last one of the predictor has ended and its L1 is divided anew, and
+// the CTAs crowd on the SMs that are through: 501 i, 16384 j 576 -> 1015 us) and
+// local memory (570 us, but 675 for 605 on a call after other work).
+template <bool NN, bool HJ, bool FOLDS>
 __global__ void __launch_bounds__(32) force64_kernel(K64 kp, int il_log2) {
   pdl_wait();  // the predictor's records and the block list are complete
   const int lane = threadIdx.x;
@@ -134,11 +142,9 @@ __global__ void __launch_bounds__(32) force64_kernel(K64 kp, int il_log2) {
   const int j1 = min(kp.nj, j0 + kp.chunk);
   const int last = kp.nj - 1;
   Rec64 nxt = load_rec(kp.rec + min(j0 + jl, last));
-  // FOLD records at a time, then into totals: a lane's one running sum over its
-  // whole chunk (16384 i and j: 1600 terms) had three times the rounding error.
   double ta[3] = {0.0, 0.0, 0.0}, tj[3] = {0.0, 0.0, 0.0}, tp = 0.0;
   for (int jb = j0 + jl;;) {
-    const int je = min(j1, jb + FOLD * JL);
+    const int je = FOLDS ? min(j1, jb + FOLD * JL) : j1;
 #pragma unroll 2
     for (int j = jb; j < je; j += JL) {
       const Rec64 r = nxt;
@@ -183,7 +189,7 @@ __global__ void __launch_bounds__(32) force64_kernel(K64 kp, int il_log2) {
       s.p += mri;
     }
     jb += FOLD * JL;
-    if (jb >= j1) break;
+    if (!FOLDS || jb >= j1) break;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       ta[k] += s.a[k];
@@ -193,7 +199,7 @@ __global__ void __launch_bounds__(32) force64_kernel(K64 kp, int il_log2) {
     tp += s.p;
     s.p = 0.0;
   }
-  if (kp.chunk > FOLD * JL) {
+  if (FOLDS) {
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       s.a[k] += ta[k];
@@ -323,6 +329,13 @@ Shape64 shape64(int ni, int nj, int nn, int force_jl, int force_ns, int groups_m
       const double instr = it * PAIR + (5 - l) * LVL + FIX;
       const double per_sm = (double)((G * ns + sms - 1) / sms);
       double cost = per_sm * instr * C + 1.2 / (per_sm > 1.2 ? per_sm : 1.2) * (it * STEP + (5 - l) * 300.0);
+      if (it > LONG) {
+        // 20 warps per SM hold the totals, for 28: where that takes a second
+        // wave, the part of a warp's time by which it ends later
+        const int tail = ((int)per_sm - 1) % 20 + 1;
+        if (per_sm > 20 && per_sm <= 28) cost += (tail < 4 ? 0.5 * (5 - tail) : 0.8) * instr * C;
+        cost *= 1.004;
+      }
       if (ns > 1) cost += 2000.0 + ((ns + JL - 1) / JL) * ADD + (5 - l) * 300.0;
       if (cost < bc * 0.999) {
         bc = cost;
@@ -389,12 +402,14 @@ extern "C" int g6k_force64(const g6_force_args *a, unsigned *ticket, int groups_
     shape->threads = 32;
   }
   const dim3 grid(gx, s.nsplit), block(32);
-  if (a->hjerk)
-    launch_pdl(force64_kernel<false, true>, grid, block, 0, st, k, s.il_log2);
-  else if (a->want_nn)
-    launch_pdl(force64_kernel<true, false>, grid, block, 0, st, k, s.il_log2);
-  else
-    launch_pdl(force64_kernel<false, false>, grid, block, 0, st, k, s.il_log2);
+  const bool fold = (s.chunk + 32 / IL - 1) / (32 / IL) > LONG;
+  auto kern = a->hjerk     ? (fold ? force64_kernel<false, true, true>
+                                    : force64_kernel<false, true, false>)
+              : a->want_nn ? (fold ? force64_kernel<true, false, true>
+                                    : force64_kernel<true, false, false>)
+                           : (fold ? force64_kernel<false, false, true>
+                                    : force64_kernel<false, false, false>);
+  launch_pdl(kern, grid, block, 0, st, k, s.il_log2);
   if (a->ev_mid) cudaEventRecord(a->ev_mid, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
