@@ -1786,26 +1786,29 @@ struct ShapeKey {
 };
 ShapeKey g_shape_cache[256];
 
-// The number of splits where their lengths may differ by a tile (JL <= 4):
-// what counts is the tiles of the busiest SM.  In units of one tile's time on
-// an SM of its own, a CTA costs its tiles and OV; with up to three CTAs per SM
-// all run at once, fewer leave FP32 cycles unused (EFF); beyond that slots
-// refill as CTAs end; the partial records cost their traffic.  Another count
-// than ns0 (choose_shape's, equal lengths) is taken where it should gain 1 %.
-// Measured with the second pass: 8192 x 8192 121 -> 103 us (11 -> 32 splits:
-// 2.3 CTAs of three tiles per SM, some SMs with three, became 6.7 of one),
-// 16384 x 16384 with neighbours 449 -> 429 us, 11719 x 2^20 13.22 -> 12.97 ms
-// (11.8 CTAs per SM -> 23.0).
-int balanced_splits(int ni, int ntiles, int jl, int ns0, int force_nsplit) {
+// The number of splits where their lengths may differ by a tile (JL <= 4): what
+// counts is the tiles of the busiest SM.  In units of one tile's time there: up
+// to three CTAs per SM run at once, fewer leave a fifth of the FP32 cycles
+// unused; beyond three slots refill as CTAs end, and the longer splits cost most
+// of their tile.  OV is a CTA's start and end, and the re-scan of its best tile
+// with the nearest neighbour: counted once, and in part for each CTA that waits
+// for a slot; the partial records cost their traffic.  Another count than ns0
+// (choose_shape's, equal lengths) is taken where it should gain 1 %.  Fitted to
+// 2700 forced counts of 131 sizes: 0.9 % behind the best count on average, ns0 2.1
+// %; behind ns0 at 2 of them by 1 %.  8192 x 8192 121 -> 103 us (11 -> 32 splits),
+// 11719 x 2^20 13.22 -> 12.97 ms; 1000 x 2^18 with neighbours stays at 57 splits
+// (390 us; 408 at 76).
+int balanced_splits(int ni, int ntiles, int jl, int nn, int ns0, int force_nsplit) {
   if (force_nsplit > 0) return force_nsplit < ntiles ? force_nsplit : ntiles;
   const int sms = sm_count(), islots = (NT / jl) * IPT_SPLIT;
   const long long gx = (ni + islots - 1) / islots;
-  const double OV = 0.28 * jl, EFF[3] = {0.6, 0.9, 0.96};
+  const double OV = 0.4 + 0.9 * jl + (nn ? 1.0 + 5.5 / jl : 0.0), WAIT = nn ? 0.3 : 0.06;
   auto cost = [&](int ns) {
     const long long c = (gx * ns + sms - 1) / sms;  // CTAs of the busiest SM
-    const double tiles = (double)ntiles / ns, merge = 3e-6 * jl * ni * (double)ns;
-    if (c <= 3) return (double)c * ((ntiles + ns - 1) / ns + OV) / EFF[c - 1] + merge;
-    return (double)c * (tiles + OV) + merge;
+    const double mean = (double)ntiles / ns, most = (ntiles + ns - 1) / ns;
+    const double merge = 1e-6 * jl * ni * (double)ns;
+    if (c <= 3) return (double)c * most / (c < 3 ? 0.8 : 1.0) + OV + merge;
+    return (double)c * (mean + 0.6 * (most - mean)) + OV * (1.0 + WAIT * (double)(c - 3)) + merge;
   };
   // The partial records stay within the fixed scratch array where those of
   // the count before do (one split needs none); else within what the L2 holds,
@@ -1921,7 +1924,7 @@ void choose_shape(int ni, int nj, int nn, int force_jl, int force_nsplit, int *j
   *jl_out = bjl;
   *nsplit_out = (ntiles + tp - 1) / tp;
   *jsplit_out = tp * TJ;
-  if (bjl <= 4) *nsplit_out = balanced_splits(ni, ntiles, bjl, *nsplit_out, force_nsplit);
+  if (bjl <= 4) *nsplit_out = balanced_splits(ni, ntiles, bjl, nn, *nsplit_out, force_nsplit);
   c.ni = ni;
   c.nj = nj;
   c.nn = nn;
