@@ -198,7 +198,8 @@ int g6k_store_forces(const g6_jstate *js, int ni, const int *ilist,
    Dev. 34, theorem 3: rb is the rounded reciprocal).  3 FP64 instructions
    where the general division takes about 10 at 16 cycles each.  Outside the
    range where nothing over- or underflows (zeros among them): __ddiv_rn.
-   Checked against a / B on 3e8 mantissas (random, low and high ends).  */
+   tests/test_gpu_fp64_ops.py holds it against a / B (random mantissas and
+   both ends of their range).  */
 __device__ __forceinline__ double g6_div_const(double a, double B, double rb) {
   const unsigned e = (unsigned)__double2hiint(a) & 0x7fffffffu;
   if (e - 0x04000000u > 0x78000000u) return __ddiv_rn(a, B); /* |a| below 2^-959 or above 2^961 */

@@ -32,9 +32,12 @@
 #include <stdint.h>
 
 #include "f32x2.cuh"
+#include "fp64_approx.cuh"
 #include "g6_dev.h"
 
 namespace {
+
+using namespace fp64;
 
 constexpr int MAXN = 64;
 constexpr int WARPS_MAX = 8;
@@ -60,22 +63,6 @@ struct WarpSmem {
   double pv[MAXN][3];
   double m[MAXN];
 };
-
-// a / b correctly rounded from y, the correctly rounded 1 / b: q = a y is
-// within an ulp, its FMA residual is exact, and one correction rounds right
-// (Markstein 1990, theorem 3; checked against a / b on 4e8 operands, the ends
-// of the mantissa range among them).  3 FP64 instructions for each further
-// quotient by the same b instead of about 10.  Where a product could leave
-// the normal range (a = 0 too), the division itself.
-__device__ __forceinline__ bool mid_range(double x) {  // 2^-300 <= |x| < 2^300
-  const unsigned e = (unsigned)__double2hiint(x) & 0x7ff00000u;
-  return e - (723u << 20) < (600u << 20);
-}
-__device__ __forceinline__ double div_by(double a, double b, double y, bool bmid) {
-  if (!(bmid && mid_range(a))) return __ddiv_rn(a, b);
-  const double q = __dmul_rn(a, y);
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
 
 // Contribution of the pair (a, b), a < b in smallN's orientation, to body
 // `me` (me == a or me == b), plus the pair's Kepler time-step^2.
@@ -354,8 +341,7 @@ __global__ void batch_exact_kernel(const int *__restrict__ order, const int *__r
 // has 9 lanes at work in one pass, where a lane per body took three passes of
 // three lanes, and two more for bodies 33 .. 64 that were not there); the
 // corrector's eight coefficients are evaluated by eight lanes at once;
-// quotients and square roots are a MUFU seed, one third-order step and one
-// corrected product, which rounds right; and comparisons of non-negative
+// quotients and square roots are fp64_approx.cuh's; and comparisons of non-negative
 // values are integer compares.  4096 scatterings 20.4 -> 5.4 ms, 1024 systems
 // of 3 to 64 bodies over 0.05 crossing times 10.3 -> 6.1 ms.  A lone warp is
 // bound by instruction latency (6 to 7 cycles per instruction of 32,000 a step
@@ -405,46 +391,6 @@ struct alignas(16) UnpSmem {
   int nb;
 };
 
-__device__ __forceinline__ bool mid_positive(double x) {  // 2^-300 <= x < 2^300
-  return (unsigned)__double2hiint(x) - (723u << 20) < (600u << 20);
-}
-// 1/x: FP64 MUFU seed (relative error below 2^-19) and one third-order step,
-// x (1 + h + h^2) with h = 1 - x y; the division outside the seed's range.
-__device__ __forceinline__ double rcp64(double x) {
-  if (!mid_range(x)) return 1.0 / x;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = __fma_rn(-x, y, 1.0);
-  return __fma_rn(y, __fma_rn(h, h, h), y);
-}
-// 1/sqrt(x) the same way (y + y h (1/2 + 3/8 h), h = 1 - x y^2); for x
-// normal, in the pair loop (where the FP32 seed of before needed x in the FP32
-// range), and for any x.
-__device__ __forceinline__ double rsqrt64_normal(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = __fma_rn(-(x * y), y, 1.0);
-  return __fma_rn(h * y, __fma_rn(0.375, h, 0.5), y);
-}
-__device__ __forceinline__ double rsqrt64(double x) {
-  return mid_positive(x) ? rsqrt64_normal(x) : 1.0 / sqrt(x);
-}
-__device__ __forceinline__ double sqrt64(double x) {
-  if (!mid_positive(x)) return sqrt(x);
-  const double y = rsqrt64(x), q = x * y;
-  return __fma_rn(__fma_rn(-q, q, x), 0.5 * y, q);
-}
-// Quotients by one b, rounded as a / b is: div_by with rcp64's y.
-struct Div {
-  double b, y;
-  bool mid;
-  __device__ __forceinline__ explicit Div(double d) : b(d), y(rcp64(d)), mid(mid_range(d)) {}
-  __device__ __forceinline__ double operator()(double a) const { return div_by(a, b, y, mid); }
-  __device__ __forceinline__ double inv() const {  // 1 / b rounded
-    return mid ? __fma_rn(__fma_rn(-b, y, 1.0), y, y) : y;
-  }
-};
-__device__ __forceinline__ double div64(double a, double b) { return Div(b)(a); }
 // a b + c d and a . b with the order of their roundings fixed (left to the
 // compiler, it varies with the surroundings): the split mode's FP32 pair terms
 // turn a last bit of the FP64 state into 6e-8 of a term now and then, and a

@@ -38,6 +38,7 @@
 #include <cuda_runtime.h>
 
 #include "f32x2.cuh"
+#include "fp64_approx.cuh"
 #include "g6_dev.h"
 
 struct __align__(32) G6D4 {
@@ -141,26 +142,6 @@ struct VRecD {
   double x[3], v[3], m, la[3], lj[3];
 };
 
-// FP64 MUFU seeds and one third-order step (kern_force64.cu); the divisions
-// outside the seeds' range.
-__device__ __forceinline__ bool mid_range(double x) {
-  return (unsigned)__double2hiint(x) - (723u << 20) < (600u << 20);  // 2^-300 <= x < 2^300
-}
-__device__ __forceinline__ double rsqrt64(double x) {
-  if (!mid_range(x)) return 1.0 / sqrt(x);
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = __fma_rn(-(x * y), y, 1.0);
-  return __fma_rn(h * y, __fma_rn(0.375, h, 0.5), y);
-}
-__device__ __forceinline__ double rcp64(double x) {
-  if (!mid_range(x)) return 1.0 / x;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = __fma_rn(-x, y, 1.0);
-  return __fma_rn(y, __fma_rn(h, h, h), y);
-}
-
 // One body k per thread, one warp per CTA (an FP64 instruction takes 64 cycles
 // of the warp's scheduler: warps spread over the SMs), j in shared-memory
 // tiles of VTD, the j range split over gridDim.y CTA rows.  Of n = 128 .. 1024
@@ -220,7 +201,7 @@ __global__ void __launch_bounds__(VT) vjp_f64_kernel(int n, double eps2,
         mu[c] = mk * r.lj[c] - r.m * ljk[c];
       }
       const double r2 = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
-      const double s1 = rsqrt64(r2 + eps2), si = s1 * s1;
+      const double s1 = fp64::rsqrt64(r2 + eps2), si = s1 * s1;
       const double s3 = s1 * si, s5 = s3 * si;
       // lam.r + mu.v and the other dot products
       const double rlvm = R[0] * lam[0] + R[1] * lam[1] + R[2] * lam[2] + V[0] * mu[0] +
@@ -231,7 +212,7 @@ __global__ void __launch_bounds__(VT) vjp_f64_kernel(int n, double eps2,
       // cr is 15 s^-7/2 resp. 3 (2 q^-2 s^-3/2 + 3 q^-1 s^-5/2) times rv rm
       double q3, d;
       if (HJ) {
-        const double qi = rcp64(r2);
+        const double qi = fp64::rcp64(r2);
         q3 = -3.0 * (qi * s3);
         d = 2.0 * qi + 3.0 * si;
       } else {

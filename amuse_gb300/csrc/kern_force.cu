@@ -45,6 +45,7 @@
 #include <stdint.h>
 
 #include "f32x2.cuh"
+#include "fp64_approx.cuh"
 #include "g6_dev.h"
 
 namespace {
@@ -1243,14 +1244,6 @@ __global__ void __launch_bounds__(128) reduce_kernel(KParams kp) {
 // a time, listed per warp in shared memory and evaluated 32 at a time; lane
 // sums merge in float-float.  REF_ACC entries exchange halves of their four
 // FP64 quantities across lanes (6 additions for 20).
-//
-// 1/sqrt(x) as in kern_force64.cu: FP64 MUFU seed and one third-order step.
-__device__ __forceinline__ double refine_rsqrt(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = __fma_rn(-(x * y), y, 1.0);
-  return __fma_rn(h * y, __fma_rn(0.375, h, 0.5), y);
-}
 
 // FP64 term of j on the i at xi, added to sa and sp.
 __device__ __forceinline__ void f64_term(const void *rec, int j, const double xi[3], double eps2,
@@ -1261,7 +1254,7 @@ __device__ __forceinline__ void f64_term(const void *rec, int j, const double xi
     dx[k] = ((double)g6_split_get(rec, j, k) + (double)g6_split_get(rec, j, 4 + k)) - xi[k];
   const double m = (double)g6_split_get(rec, j, 3) + (double)g6_split_get(rec, j, 7);
   const double r2 = __fma_rn(dx[2], dx[2], __fma_rn(dx[1], dx[1], __fma_rn(dx[0], dx[0], eps2)));
-  const double rinv = refine_rsqrt(r2);
+  const double rinv = fp64::rsqrt64_normal(r2);
   const double mri = m * rinv;
   const double mr3i = mri * (rinv * rinv);
 #pragma unroll

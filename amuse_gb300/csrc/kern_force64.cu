@@ -26,6 +26,7 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "fp64_approx.cuh"
 #include "g6_dev.h"
 
 namespace {
@@ -59,28 +60,6 @@ constexpr unsigned long long INF_BITS = 0x7ff0000000000000ull;
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int LONG = 128;  // more records than this per lane are folded,
 constexpr int FOLD = 64;   // so many at a time
-
-// 1/sqrt(x), x normal: the MUFU seed y (relative error e below 2^-19, PTX
-// rsqrt.approx.ftz.f64) and one step of third order, y + y h (1/2 + 3/8 h)
-// with h = 1 - x y^2 (the binomial series of (1 - h)^(-1/2)): 5/16 e^3
-// < 2^-58 remains, below the rounding of the last FMA.
-__device__ __forceinline__ double rsqrt64(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = __fma_rn(-(x * y), y, 1.0);
-  return __fma_rn(h * y, __fma_rn(0.375, h, 0.5), y);
-}
-
-// 1/x the same way (y + y (h + h^2), h = 1 - x y, of third order).  Outside
-// the seed's range (a subnormal or infinite x or result) the plain division.
-__device__ __forceinline__ double rcp64(double x) {
-  const unsigned e = (unsigned)__double2hiint(x);
-  if (e - 0x02000000u > 0x7c000000u) return 1.0 / x;  // hi word below 2^-990 or above 2^990
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = __fma_rn(-x, y, 1.0);
-  return __fma_rn(y, __fma_rn(h, h, h), y);
-}
 
 __device__ __forceinline__ Rec64 load_rec(const Rec64 *p) {
   const double2 *q = reinterpret_cast<const double2 *>(p);
@@ -166,7 +145,7 @@ __global__ void __launch_bounds__(32) force64_kernel(K64 kp, int il_log2) {
       } else {
         r2 = __fma_rn(dz, dz, __fma_rn(dy, dy, __fma_rn(dx, dx, eps2)));
       }
-      double rinv = rsqrt64(r2);
+      double rinv = fp64::rsqrt64_normal(r2);
       rinv = j == self ? 0.0 : rinv;
       const double dvx = r.vx - vx, dvy = r.vy - vy, dvz = r.vz - vz;
       const double rv = __fma_rn(dz, dvz, __fma_rn(dy, dvy, dx * dvx));
@@ -176,7 +155,7 @@ __global__ void __launch_bounds__(32) force64_kernel(K64 kp, int il_log2) {
       double a3;
       if (HJ) {  // the hermite code's jerk (src/amuse_hermite/interface.cc:440-449,486)
         const double q = __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
-        a3 = j == self ? 0.0 : -3.0 * (rv * rcp64(q));
+        a3 = j == self ? 0.0 : -3.0 * (rv * fp64::rcp64(q));
       } else {
         a3 = -3.0 * (rv * rinv2);
       }
