@@ -304,3 +304,63 @@ def test_shape_beyond_residency(g6, mode, unp):
         g6.batch_config(4, 2)
     assert np.array_equal(pos[0], pos[1]) and np.array_equal(pos[0], pos[2])
     assert max(ms) <= 1.4 * ms[0], ms
+
+
+def _with_binaries(n, pairs, rng):
+    """A Plummer system in which the two bodies of each pair circle the first
+    one's place, 1e-3 of the nearest other body apart, e = 0.6, inbound."""
+    m, x, v = ic.plummer(n, do_scale=True, rng=rng)
+    for a, b in pairs:
+        d = np.sqrt(((x - x[a]) ** 2).sum(1))
+        d[[a, b]] = np.inf
+        sma, mt, e, ea = 1e-3 * d.min(), m[a] + m[b], 0.6, 1.5 * np.pi
+        u = rng.normal(size=3)
+        u /= np.linalg.norm(u)
+        w = np.cross(u, rng.normal(size=3))
+        w /= np.linalg.norm(w)
+        f, g = np.sqrt(1 - e * e), np.sqrt(mt / sma) / (1 - e * np.cos(ea))
+        r = sma * ((np.cos(ea) - e) * u + f * np.sin(ea) * w)
+        s = g * (-np.sin(ea) * u + f * np.cos(ea) * w)
+        c, cv = x[a].copy(), v[a].copy()
+        x[a], x[b] = c - m[b] / mt * r, c + m[a] / mt * r
+        v[a], v[b] = cv - m[b] / mt * s, cv + m[a] / mt * s
+    return m, x * 1e-3, v / np.sqrt(1e-3)
+
+
+BINARIES = {11: [(0, 10)], 21: [(0, 20)], 22: [(3, 21)], 32: [(0, 31), (5, 17)], 33: [(4, 32)],
+            43: [(31, 32), (7, 42)], 54: [(9, 50), (33, 34)], 63: [(0, 62), (31, 33)],
+            64: [(0, 63), (30, 40), (7, 8)]}
+
+
+@pytest.mark.parametrize("mode", ["fast", "split"])
+@pytest.mark.parametrize("full,t", [(True, 0.02), (False, 0.0005)], ids=["frozen", "dissolving"])
+def test_binaries_at_layout_edges(g6, mode, full, t):
+    """Hard binaries inside systems at the edges of the component slots, members
+    on both sides of the 32nd slot, against orc_smalln_unpert: frozen over whole
+    periods, or made and dissolved every period (up to 46 times here).  Inputs
+    moved by 1e-15 of themselves move the oracle's end by up to 1e-13 of the size,
+    1e-11 of the end time and 1e-9 of the velocities (fast: a hundred times that
+    allowed and more); by 1e-8, 1e-4 of a binary's separation, by 1e-6, 1e-4 and
+    1e-2 (split: FP32 terms are a thousand times more exact than that)."""
+    tx, tt, tv = (1e-9, 1e-7, 1e-6) if mode == "fast" else (1e-6, 1e-4, 1e-2)
+    made = {n: _with_binaries(n, p, np.random.RandomState(n)) for n, p in BINARIES.items()}
+    ns = np.array(list(made), np.int32)
+    m, x, v = (np.concatenate([made[n][k] for n in made]) for k in range(3))
+    t_end = t * 2 * np.sqrt(2) * 1e-3 ** 1.5
+    g6.batch_unperturbed(True, allow_full=full)
+    try:
+        r = g6.batch_run(ns, t_end, m, x, v, mode=mode, max_steps=100000)
+        nbin = g6.batch_binaries(len(ns))
+    finally:
+        g6.batch_unperturbed(False)
+    off = np.concatenate([[0], np.cumsum(ns)])
+    for s, n in enumerate(ns):
+        a, b = off[s], off[s + 1]
+        px, pv, tf, st, nb = oracle.smalln_unpert(m[a:b], x[a:b], v[a:b], 0.14, t_end,
+                                                  allow_full=full, max_steps=100000)
+        assert r["status"][s] == 0 and nbin[s] >= len(BINARIES[n]), n
+        if mode == "fast":
+            assert r["steps"][s] == st and nbin[s] == nb, n
+        assert abs(r["t_final"][s] - tf) <= tt * tf, n
+        assert np.abs(r["pos"][a:b] - px).max() <= tx * 1e-3, n
+        assert np.abs(r["vel"][a:b] - pv).max() <= tv * np.abs(pv).max(), n
