@@ -2052,7 +2052,8 @@ extern "C" int g6k_force(const g6_force_args *a, g6_shape *shape, cudaStream_t s
   kp.kappa2 = a->kappa > 0.0 ? a->kappa * a->kappa : 0.0;
   kp.stall = a->stall_test;
   kp.wait_ns = a->stall_test ? STALL_TEST_NS : WAIT_NS;
-  const size_t need = nsplit > 1 ? (size_t)nsplit * (size_t)a->ni * sizeof(SplitP::Out) : 0;
+  const size_t need =
+      nsplit > 1 ? g6k_scratch_bytes(a->ni, a->nj, a->prec, a->want_nn, jl, nsplit) : 0;
   if (need > a->scratch_bytes) return -4;
   const int islots = (NT / jl) * IPT_SPLIT;
   const int gx = (a->ni + islots - 1) / islots;
