@@ -120,6 +120,10 @@ typedef struct {
   /* i / out buffers: pinned host block + device block, capacity cap_i */
   int cap_i;
   int io_n; /* the n of the call the blocks are laid out for: each moves in one copy */
+  /* two input blocks of in_bytes: io_half the staged call's, last_half that of
+     the last force call, of last_n, kept for g6_read_neighbour_list */
+  int io_half, last_half, last_n;
+  size_t in_bytes;
   void *h_in, *d_in;   /* [ipos 3n][ivel 3n] doubles, [iself n (even)] ints, [h2 n] doubles */
   void *h_out, *d_out; /* [err 2 ints][acc 3n][jerk 3n][pot n] doubles, [nn n] ints, [nnr2 n] floats */
   int *d_err;
@@ -288,6 +292,7 @@ static int ensure_io(int ni) {
   int cap = G.cap_i ? G.cap_i : 1024;
   while (cap < ni) cap *= 2;
   size_t in_b = (size_t)cap * (7 * sizeof(double) + sizeof(int)) + sizeof(double);
+  in_b = (in_b + 255) / 256 * 256;
   size_t out_b = 16 + (size_t)cap * (7 * sizeof(double) + sizeof(int) + sizeof(float));
   if (G.h_in) cudaFreeHost(G.h_in);
   if (G.h_out) cudaFreeHost(G.h_out);
@@ -295,9 +300,10 @@ static int ensure_io(int ni) {
   cudaFree(G.d_out);
   G.h_in = G.h_out = G.d_in = G.d_out = NULL;
   G.cap_i = 0;
-  G.h_in = pin_alloc(in_b);
+  G.in_bytes = in_b;
+  G.h_in = pin_alloc(2 * in_b);
   G.h_out = pin_alloc(out_b);
-  if (!G.h_in || !G.h_out || cudaMalloc(&G.d_in, in_b) != cudaSuccess ||
+  if (!G.h_in || !G.h_out || cudaMalloc(&G.d_in, 2 * in_b) != cudaSuccess ||
       cudaMalloc(&G.d_out, out_b) != cudaSuccess) {
     seterr("cannot allocate i/o buffers for %d i-particles", cap);
     return G6_ERR_NOMEM;
@@ -313,10 +319,13 @@ static int ensure_io(int ni) {
 }
 
 /* Views into the i/o blocks for the current call's io_n particles. */
-#define IN_POS(b) ((double *)(b))
-#define IN_VEL(b) ((double *)(b) + 3 * (size_t)G.io_n)
-#define IN_SELF(b) ((int *)((double *)(b) + 6 * (size_t)G.io_n))
-#define IN_H2(b) ((double *)(b) + 6 * (size_t)G.io_n + ((size_t)G.io_n + 1) / 2)
+#define IN_AT(b, half) ((double *)((char *)(b) + (size_t)(half) * G.in_bytes))
+#define IN_SELF_OF(p, n) ((int *)((p) + 6 * (size_t)(n)))
+#define IN_H2_OF(p, n) ((p) + 6 * (size_t)(n) + ((size_t)(n) + 1) / 2)
+#define IN_POS(b) IN_AT(b, G.io_half)
+#define IN_VEL(b) (IN_POS(b) + 3 * (size_t)G.io_n)
+#define IN_SELF(b) IN_SELF_OF(IN_POS(b), G.io_n)
+#define IN_H2(b) IN_H2_OF(IN_POS(b), G.io_n)
 #define OUT_ERR(b) ((int *)(b))
 #define OUT_ACC(b) ((double *)((char *)(b) + 16))
 #define OUT_JERK(b) (OUT_ACC(b) + 3 * (size_t)G.io_n)
@@ -663,6 +672,7 @@ static int stage_force_host(int nj, int ni, const int *index, const double *xi,
     rc = ensure_io(ni);
     if (rc) return rc;
     G.io_n = ni;
+    G.io_half = 1 - G.last_half;
     memcpy(IN_POS(G.h_in), xi, sizeof(double) * 3 * (size_t)ni);
     memcpy(IN_VEL(G.h_in), vi, sizeof(double) * 3 * (size_t)ni);
     if (h2)
@@ -681,7 +691,7 @@ static int stage_force_host(int nj, int ni, const int *index, const double *xi,
     /* One copy of positions, velocities and self slots (a copy each cost
        about 3 us apiece); first, so that the kernels below follow each other
        without a copy between them. */
-    CK(cudaMemcpyAsync(G.d_in, G.h_in,
+    CK(cudaMemcpyAsync(IN_POS(G.d_in), IN_POS(G.h_in),
                        sizeof(double) * 6 * (size_t)ni + sizeof(int) * (size_t)ni,
                        cudaMemcpyHostToDevice, G.st));
     rc = flush_updates(1);
@@ -708,6 +718,8 @@ static int launch_force_host(int want_nn) {
   G.pending = 1;
   G.pending_ni = ni;
   if (ni == 0) return 0;
+  G.last_half = G.io_half;
+  G.last_n = ni;
   g6_force_args a;
   memset(&a, 0, sizeof(a));
   a.ni = ni;
@@ -841,6 +853,22 @@ static void ngb_free(void) {
   ngb_cap = ngb_ni = ngb_valid = 0;
 }
 
+/* The lists of particles [first, first + count) of an input block of n. */
+static int ngb_rows(int half, int n, int first, int count) {
+  if (count <= 0) return 0;
+  double *hp = IN_AT(G.h_in, half), *dp = IN_AT(G.d_in, half);
+  double *dh2 = IN_H2_OF(dp, n) + first;
+  CK(cudaMemcpyAsync(dh2, IN_H2_OF(hp, n) + first, sizeof(double) * (size_t)count,
+                     cudaMemcpyHostToDevice, G.st));
+  if (g6k_neighbours(&G.js, G.pending_nj, count, G.prec, dp + 3 * (size_t)first, dh2,
+                     IN_SELF_OF(dp, n) + first, d_ngb + (size_t)(G6_NGB_MAX + 1) * (size_t)first,
+                     G6_NGB_MAX, G.st)) {
+    seterr("neighbour kernel launch failed");
+    return G6_ERR_CUDA;
+  }
+  return 0;
+}
+
 int g6_read_neighbour_list_(int *cluster_id) {
   (void)cluster_id;
   int rc = check_open();
@@ -849,8 +877,7 @@ int g6_read_neighbour_list_(int *cluster_id) {
     seterr("g6_read_neighbour_list before g6calc_lasthalf");
     return G6_ERR_STATE;
   }
-  /* (a firsthalf since then may have laid the block out for fewer) */
-  const int ni = G.pending_ni < G.io_n ? G.pending_ni : G.io_n;
+  const int ni = G.pending_ni;
   if (ni <= 0) return 0;
   const size_t per = (size_t)(G6_NGB_MAX + 1);
   if (ni > ngb_cap) {
@@ -864,13 +891,11 @@ int g6_read_neighbour_list_(int *cluster_id) {
     }
     ngb_cap = ni;
   }
-  CK(cudaMemcpyAsync(IN_H2(G.d_in), IN_H2(G.h_in), sizeof(double) * (size_t)ni,
-                     cudaMemcpyHostToDevice, G.st));
-  if (g6k_neighbours(&G.js, G.pending_nj, ni, G.prec, IN_POS(G.d_in), IN_H2(G.d_in),
-                     IN_SELF(G.d_in), d_ngb, G6_NGB_MAX, G.st)) {
-    seterr("neighbour kernel launch failed");
-    return G6_ERR_CUDA;
-  }
+  /* a firsthalf since the last force call has replaced its first particles */
+  const int fresh = staged ? (staged_ni < ni ? staged_ni : ni) : 0;
+  rc = ngb_rows(G.io_half, G.io_n, 0, fresh);
+  if (rc == 0) rc = ngb_rows(G.last_half, G.last_n, fresh, ni - fresh);
+  if (rc) return rc;
   CK(cudaMemcpyAsync(h_ngb, d_ngb, sizeof(int) * per * (size_t)ni, cudaMemcpyDeviceToHost, G.st));
   CK(cudaStreamSynchronize(G.st));
   ngb_ni = ni;

@@ -14,6 +14,8 @@ Tolerances (per-particle relative errors against ph4's FP64 CPU loop):
   nn (both): the oracle's index (ph4: smallest FP64 r^2, first j on equal
   values), except where the two indices' FP64 r^2 are equal.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -269,6 +271,42 @@ def test_neighbour_lists(g6, prec):
             continue
         assert np.array_equal(got, want), q
     assert over == (1 if any_over else 0)
+
+
+@pytest.mark.parametrize("again", [7, 40, 5000])
+def test_neighbour_lists_after_a_firsthalf(g6, prec, again):
+    """g6_read_neighbour_list between the next call's two halves: the lists of
+    the last call's particles, of which the firsthalf has replaced the first
+    ones (fewer, as many, or more than the i/o block held)."""
+    np.random.seed(18)
+    n, ni = 3000, 40
+    m, x, v = ic.plummer(n)
+    ids = np.arange(1, n + 1, dtype=np.int32)
+    ag.drive_load(m, x, v, ids=ids)
+    g6.set_ti(0.0)
+    sel = np.arange(0, n, n // ni)[:ni]
+    h2 = np.linspace(0.01, 0.04, ni)
+    g6.calc(n, ids[sel], x[sel], v[sel], 1e-4, h2=h2)
+    new = (np.arange(again) * 37 + 5) % n
+    nh2 = np.full(again, 0.02)
+    args = [np.ascontiguousarray(q) for q in (ids[new], x[new], v[new], np.zeros((again, 3)), nh2)]
+    c = lambda q, t=ctypes.c_double: q.ctypes.data_as(ctypes.POINTER(t))
+    cid, cnj, cni, eps2 = ctypes.c_int(0), ctypes.c_int(n), ctypes.c_int(again), ctypes.c_double(1e-4)
+    R = ctypes.byref
+    g6.lib.g6calc_firsthalf_(R(cid), R(cnj), R(cni), c(args[0], ctypes.c_int), c(args[1]), c(args[2]),
+                             c(args[3]), c(args[3]), c(nh2), R(eps2), c(nh2))
+    g6.read_neighbour_list()
+    for q in range(ni):
+        i, r2 = (new[q], nh2[q]) if q < again else (sel[q], h2[q])
+        want = np.sort(ids[(((x - x[i]) ** 2).sum(1) <= r2) & (np.arange(n) != i)])
+        got, rc = g6.get_neighbour_list(q)
+        assert len(want) > ag.NGB_MAX or np.array_equal(got, want), q
+    acc, jerk, pot = np.zeros((again, 3)), np.zeros((again, 3)), np.zeros(again)
+    assert g6.lib.g6calc_lasthalf_(R(cid), R(cnj), R(cni), c(args[0], ctypes.c_int), c(args[1]),
+                                   c(args[2]), R(eps2), c(nh2), c(acc), c(jerk), c(pot)) == 0
+    ref = oracle.force(m, x, v, 1e-4, x[new], v[new])
+    assert (np.linalg.norm(acc - ref["acc"], axis=1)
+            <= 1e-6 * np.linalg.norm(ref["acc"], axis=1)).all()
 
 
 def test_error_codes(g6):
