@@ -1747,6 +1747,15 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
   }
 }
 
+// The wait-expiry hook in FP64, whose kernel has no wait of its own: the same
+// bounded wait on a barrier that nothing arrives on, then the error word.
+__global__ void expiry_kernel(int *err, unsigned long long wait_ns) {
+  __shared__ __align__(8) uint64_t never;
+  mbar_init(&never, 1);
+  fence_barrier_init();
+  if (!mbar_wait_bounded(&never, 0, wait_ns)) atomicOr(err, ERR_TMA_TIMEOUT);
+}
+
 int g_sms = 0;
 
 int sm_count() {
@@ -2016,6 +2025,8 @@ extern "C" int g6k_force(const g6_force_args *a, g6_shape *shape, cudaStream_t s
   if (!a->ilist && (!a->ipos || !a->ivel)) return -1;
   if (a->hjerk && (a->want_nn || (a->force_jl != 0 && a->force_jl != 1))) return -2;
   if (a->force_jl < 0 || a->force_jl > JLMAX || (a->force_jl & (a->force_jl - 1))) return -2;
+  if (a->prec == G6_PREC_FP64 && a->stall_test)
+    expiry_kernel<<<1, 1, 0, st>>>(a->err, STALL_TEST_NS);
   if (a->prec == G6_PREC_FP64)
     return g6k_force64(a, a->refine ? reinterpret_cast<RefBuf *>(a->refine)->xtick : nullptr,
                        a->refine ? XTMAX : 0, shape, st);

@@ -165,3 +165,24 @@ def test_bounded_wait_expiry(g6):
     ref = oracle.force(m, x, v, 1e-4, x[sel], v[sel])
     e = np.linalg.norm(out["acc"] - ref["acc"], axis=1) / np.linalg.norm(ref["acc"], axis=1)
     assert e.max() <= 1e-6
+
+
+def test_bounded_wait_expiry_fp64(g6):
+    """The hook's contract in FP64 precision: G6_ERR_KERNEL once, then a
+    correct call."""
+    np.random.seed(41)
+    n = 1024
+    m, x, v = ic.plummer(n)
+    sel = np.arange(0, n, 8)
+    g6.set_precision(ag.FP64)
+    try:
+        g6.load_particles(m, x, v)
+        g6.test_wait_expiry(True)
+        with pytest.raises(ag.G6Error) as ei:
+            g6.force(0.0, 1e-4, n, x[sel], v[sel], self_slot=sel)
+        assert "error word" in str(ei.value)
+        out = g6.force(0.0, 1e-4, n, x[sel], v[sel], self_slot=sel)
+    finally:
+        g6.set_precision(ag.SPLIT)
+    ref = oracle.force(m, x, v, 1e-4, x[sel], v[sel])
+    assert np.abs(out["acc"] - ref["acc"]).max() <= 1e-12 * np.abs(ref["acc"]).max()
