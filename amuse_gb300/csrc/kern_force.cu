@@ -70,7 +70,7 @@ namespace {
 #define G6_MINB 3
 #endif
 #ifndef G6_XMERGE_MAX
-#define G6_XMERGE_MAX 2  // split merge in the force kernel up to this many i per group
+#define G6_XMERGE_MAX 2  // split merge in the force kernel at most for so many i per group
 #endif
 #ifndef G6_JCHUNK
 #define G6_JCHUNK 32  // split: records per jerk fold
@@ -2075,14 +2075,14 @@ extern "C" int g6k_force(const g6_force_args *a, g6_shape *shape, cudaStream_t s
     shape->grid_y = nsplit;
     shape->threads = NT;
   }
-  // The in-kernel split merge runs in the one CTA that completes an i-group,
-  // a warp per i: it saves a launch where the group holds one or two i
-  // (JL = 128), but with more i per group that CTA's warps merge them one
-  // after another and the tail outlasts a second launch that gives every i
-  // its own warp (measured, force with merge: 722 i at JL = 4, 136 us in the
-  // kernel against 83 us with the second launch; 64 i at JL = 32, 44 us
-  // against 32 us; 1 i at JL = 128, 21 us against 24 us).
-  kp.xtick = (a->refine && nsplit > 1 && gx <= XTMAX && islots <= G6_XMERGE_MAX)
+  // The in-kernel split merge runs in the one CTA that completes an i-group of
+  // one or two i (JL = 128).  It saves a launch, but that CTA works alone at the
+  // end, and the refinement pass, released meanwhile, crowds on the SMs that are
+  // through.  It pays for many splits: 1 i, 205 splits 15.6 us against 17.9 with the
+  // second launch, 86 splits 12.1 and 12.6, 8 i, 114 splits 20.0 and 20.8; but 8 i, 86
+  // splits 17.2 and 15.6, 1 to 16 i, 2 to 16 splits 10.5 and 9.6, and 16 i, 32 splits
+  // with one entry to refine 63.8 and 31.3.  (More i per group, JL = 64 and 32: 44.9 and 33.1, 25.0 and 22.6.)
+  kp.xtick = (a->refine && nsplit >= (gx == 1 ? 64 : 96) && gx <= XTMAX && islots <= G6_XMERGE_MAX)
                  ? reinterpret_cast<RefBuf *>(a->refine)->xtick
                  : nullptr;
   kp.jrec = a->js->jp_split;

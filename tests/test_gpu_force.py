@@ -643,3 +643,30 @@ def test_fp64_sums_are_folded(g6):
         w[i] = 0
         err.append(float(-pot[i] / w.sum() - 1))
     assert np.sqrt(np.mean(np.square(err))) <= 1.5 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("splits", [1, 59, 118], ids=["none", "second-launch", "in-kernel"])
+@pytest.mark.parametrize("ni", [1, 2, 5])
+def test_split_merge_of_few_i(g6, ni, splits):
+    """One or two i per group: the splits' sums merged in the force kernel's last
+    CTA (96 splits and more) or by the second launch, twice in a row (the tickets
+    return to zero)."""
+    n = 30000
+    np.random.seed(37)
+    m, x, v = ic.plummer(n)
+    g6.set_precision(ag.SPLIT)
+    g6.load_particles(m, x, v)
+    sel = np.arange(0, n, n // ni)[:ni]
+    ref = oracle.force(m, x, v, 1e-4, x[sel], v[sel])
+    g6.set_shape(128, splits)
+    try:
+        out = [g6.force(0.0, 1e-4, n, x[sel], v[sel], self_slot=sel) for _ in range(2)]
+        assert g6.stats()["jl"] == 128 and g6.stats()["nsplit"] == splits
+    finally:
+        g6.set_shape(0, 0)
+    for o in out:
+        err = np.linalg.norm(o["acc"] - ref["acc"], axis=1) / np.linalg.norm(ref["acc"], axis=1)
+        assert err.max() <= 1e-6
+        assert (np.abs(o["pot"] / ref["pot"] - 1) <= 1e-6).all()
+        assert np.array_equal(o["nn"], ref["nn"])
+    assert np.array_equal(out[0]["acc"], out[1]["acc"])
