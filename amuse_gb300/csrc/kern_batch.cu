@@ -343,7 +343,8 @@ __global__ void batch_exact_kernel(const int *__restrict__ order, const int *__r
 // corrector's eight coefficients are evaluated by eight lanes at once;
 // quotients and square roots are fp64_approx.cuh's; and comparisons of non-negative
 // values are integer compares.  4096 scatterings 20.4 -> 5.4 ms, 1024 systems
-// of 3 to 64 bodies over 0.05 crossing times 10.3 -> 6.1 ms.  A lone warp is
+// of 3 to 64 bodies over 0.05 crossing times 10.3 -> 6.1 ms (one draw; its longest
+// system sets the time, and other draws take 5 to 31).  A lone warp is
 // bound by instruction latency (6 to 7 cycles per instruction of 32,000 a step
 // at n = 52), so the split mode's pair loop reads a body in three or four
 // 16-byte loads and evaluates two pairs per packed f32x2 instruction.

@@ -60,9 +60,6 @@ namespace {
 #ifndef G6_UNROLL_NN
 #define G6_UNROLL_NN 4  // j-loop unroll factor of the nearest-neighbour variant
 #endif
-#ifndef G6_ACHUNK
-#define G6_ACHUNK 0  // split: fold the acceleration partials with the jerk's
-#endif
 #ifndef G6_UNROLL
 #define G6_UNROLL 8
 #endif
@@ -404,11 +401,6 @@ struct SplitP {
       ff_acc(t.jh[k], t.jl[k], f2_lo(q.j[k]));
       ff_acc(t.jh[k], t.jl[k], f2_hi(q.j[k]));
       q.j[k] = 0ull;
-      if (G6_ACHUNK) {
-        ff_acc(t.ah[k], t.al[k], f2_lo(q.a[k]));
-        ff_acc(t.ah[k], t.al[k], f2_hi(q.a[k]));
-        q.a[k] = 0ull;
-      }
     }
   }
   __device__ static f2x eps(double eps2) {
@@ -1527,9 +1519,9 @@ __global__ void __launch_bounds__(RNT) refine_kernel(KParams kp) {
   if (ne > 0) {
     // One unit per CTA while the entries are few (the CTA reduces once), two
     // once they are many, for balance.  Salpeter cluster, N = 16384, 4 CTAs
-    // per SM: 165 entries 72 us at one, 62 at two, 61 at four; 59 entries 26,
-    // 28, 30; at 2 CTAs per SM and four units 78 and 39.  (With the FP64
-    // terms and reductions this pass had before: 87 and 54 us.)
+    // per SM, at one, two and four: 67 entries for kappa (and 155 in refine_mt)
+    // 109, 108 and 108 us, 12 of them 34 at each; at 2 CTAs per SM an earlier
+    // build took a quarter more.
     const int upc = ne * 4 > (int)gridDim.x ? G6_REF_UNITS : 1;
     nch = (upc * (int)gridDim.x + ne - 1) / ne;
     nch = min(nch, RCHMAX);
@@ -1768,8 +1760,6 @@ int sm_count() {
   return g_sms;
 }
 
-// Launch shape: JL from the i-block size, nsplit so that the grid covers
-// about two resident CTAs per SM, with at least 4 tiles per split.
 // Launch shape from a small cost model.  A CTA streams tiles_per tiles of
 // its j-range; per tile each thread spends ~A issue slots of fixed work
 // (wait, release, bookkeeping) plus B per j-record for its IPT i-particles
@@ -1780,8 +1770,9 @@ int sm_count() {
 // Candidates: JL from the smallest that does not waste CTA i-slots up to
 // 256 (more j-lanes = more CTAs for small blocks), and every distinct split
 // count up to 4 resident waves' worth.  Large blocks (a full wave of CTAs at
-// JL = 1) stay at JL = 1.  The last few shapes are cached (block steps
-// repeat the same ni).
+// JL = 1) stay at JL = 1; balanced_splits below has the last word on the
+// splits for JL <= 4.  The last few shapes are cached (block steps repeat the
+// same ni).
 struct ShapeKey {
   int ni, nj, nn, fjl, fns;
   int jl, nsplit, jsplit;
