@@ -1782,26 +1782,27 @@ ShapeKey g_shape_cache[256];
 // The number of splits where their lengths may differ by a tile (JL <= 4): what
 // counts is the tiles of the busiest SM.  In units of one tile's time there: up
 // to three CTAs per SM run at once, fewer leave a fifth of the FP32 cycles
-// unused; beyond three slots refill as CTAs end, and the longer splits cost most
-// of their tile.  OV is a CTA's start and end, and the re-scan of its best tile
-// with the nearest neighbour: counted once, and in part for each CTA that waits
-// for a slot; the partial records cost their traffic.  Another count than ns0
-// (choose_shape's, equal lengths) is taken where it should gain 1 %.  Fitted to
-// 2700 forced counts of 131 sizes: 0.9 % behind the best count on average, ns0 2.1
-// %; behind ns0 at 2 of them by 1 %.  8192 x 8192 121 -> 103 us (11 -> 32 splits),
-// 11719 x 2^20 13.22 -> 12.97 ms; 1000 x 2^18 with neighbours stays at 57 splits
-// (390 us; 408 at 76).
+// unused; beyond three slots refill as CTAs end, and the longer splits cost half
+// of their tile.  OV is a CTA's start and end, with the nearest neighbour the
+// re-scan of its best tile too (the dearer the farther apart the tiles lie, up to
+// 65536 j): counted once, and in part for each CTA that waits for a slot.  Another
+// count than ns0 (choose_shape's, equal lengths) is taken where it should gain half
+// a per cent.  Fitted to 3800 forced counts of 211 sizes: 0.6 % behind the best
+// count on average, ns0 2.1 %.  At 190 other sizes where the count is not ns0 it
+// gains 3.0 %; seven of them lose 2 to 7 %.  8192 x 8192 121 -> 103 us (11 -> 32
+// splits), 11719 x 2^20 13.20 -> 13.10 ms, 11850 x 11850 with neighbours 312 -> 256
+// us (8 -> 16); 1000 x 2^18 with neighbours stays at 57 (390 us; 408 at 76).
 int balanced_splits(int ni, int ntiles, int jl, int nn, int ns0, int force_nsplit) {
   if (force_nsplit > 0) return force_nsplit < ntiles ? force_nsplit : ntiles;
   const int sms = sm_count(), islots = (NT / jl) * IPT_SPLIT;
   const long long gx = (ni + islots - 1) / islots;
-  const double OV = 0.4 + 0.9 * jl + (nn ? 1.0 + 5.5 / jl : 0.0), WAIT = nn ? 0.3 : 0.06;
+  const double rescan = nn ? (1.5 + 7.0 / jl) * (ntiles < 256 ? ntiles / 256.0 : 1.0) : 0.0;
+  const double OV = 0.8 * jl + rescan, WAIT = nn ? 0.28 : 0.1;
   auto cost = [&](int ns) {
     const long long c = (gx * ns + sms - 1) / sms;  // CTAs of the busiest SM
     const double mean = (double)ntiles / ns, most = (ntiles + ns - 1) / ns;
-    const double merge = 1e-6 * jl * ni * (double)ns;
-    if (c <= 3) return (double)c * most / (c < 3 ? 0.8 : 1.0) + OV + merge;
-    return (double)c * (mean + 0.6 * (most - mean)) + OV * (1.0 + WAIT * (double)(c - 3)) + merge;
+    if (c <= 3) return (double)c * most / (c < 3 ? 0.8 : 1.0) + OV;
+    return (double)c * (mean + 0.45 * (most - mean)) + OV * (1.0 + WAIT * (double)(c - 3));
   };
   // The partial records stay within the fixed scratch array where those of
   // the count before do (one split needs none); else within what the L2 holds,
@@ -1811,7 +1812,7 @@ int balanced_splits(int ni, int ntiles, int jl, int nn, int ns0, int force_nspli
   const size_t rec = (size_t)ni * sizeof(SplitP::Out), was = ns0 > 1 ? (size_t)ns0 * rec : 0;
   const size_t limit = was <= room ? room : was > l2 ? was : l2;
   int best = ns0;
-  double bc = cost(ns0) * 0.99;
+  double bc = cost(ns0) * 0.995;
   const int most = ntiles < 128 ? ntiles : 128;
   for (int ns = 1; ns <= most; ns++) {
     if (ns > ns0 && (size_t)ns * rec > limit) break;
